@@ -86,22 +86,32 @@ extern "C" int ti_test_wait_runs_out(unsigned limit, int* gave_up, cudaStream_t 
     return 0;
 }
 
-int ti_make_tensor_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
-                               uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_cols) {
+static int make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, const void* base, uint64_t rows, uint64_t cols,
+                              uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_cols) {
     if (int rc = load_encode()) return rc;
     TI_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "tensor map: base address is not 16-byte aligned");
     TI_REQUIRE(row_stride_bytes % 16 == 0, "tensor map: row stride of %llu bytes is not a multiple of 16",
                (unsigned long long)row_stride_bytes);
-    TI_REQUIRE(box_cols * 2 == 128 && box_rows >= 1 && box_rows <= 256, "tensor map: box of %u x %u is not supported",
+    TI_REQUIRE((int)box_cols * elem_bytes == 128 && box_rows >= 1 && box_rows <= 256, "tensor map: box of %u x %u is not supported",
                box_rows, box_cols);
     cuuint64_t dims[2] = {cols, rows};
     cuuint64_t strides[1] = {row_stride_bytes};
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = g_encode(map, type, 2, const_cast<void*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     TI_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code %d (rows %llu, cols %llu, stride %llu)", (int)r,
                (unsigned long long)rows, (unsigned long long)cols, (unsigned long long)row_stride_bytes);
     return 0;
+}
+
+int ti_make_tensor_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
+                               uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_cols) {
+    return make_tensor_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, row_stride_bytes, box_rows, box_cols);
+}
+
+int ti_make_tensor_map_2d_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
+                              uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_cols) {
+    return make_tensor_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, row_stride_bytes, box_rows, box_cols);
 }

@@ -30,6 +30,9 @@ __device__ __forceinline__ void ti_report(int* status, int code) { atomicCAS(sta
 // box_rows x box_cols (box_cols * 2 bytes must be 128 for the 128-byte swizzle).
 int ti_make_tensor_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                                uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_cols);
+// The same for float32 (box_cols * 4 bytes must be 128).
+int ti_make_tensor_map_2d_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
+                              uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_cols);
 
 // ---------------------------------------------------------------------------
 // device: shared-memory addresses, mbarriers, TMA

@@ -318,7 +318,7 @@ def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, act: str = "silu", lim
     M, K = x.shape
     N = w_pairs.shape[0]
     ldx, ldw = _row_stride(x, "linear x"), _row_stride(w_pairs, "linear w")
-    if gemm.tc_eligible(x, w_pairs, K, ldx, ldw):
+    if gemm.tc_eligible(x, w_pairs, K, ldx, ldw) or gemm.f32_eligible(x, w_pairs, M, K, ldx, ldw):
         out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
         gemm.run(x, w_pairs, out, M, N, K, ldx, ldw, gated=1 + GATE_ACTS[act], gate_limit=limit)      # the kernels' codes: 1 silu, 2 gelu, 3 clamped
         return out
@@ -338,7 +338,7 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, act: str) -> torch.Tensor:
     M, K = x.shape
     N = w.shape[0]
     ldx, ldw = _row_stride(x, "linear x"), _row_stride(w, "linear w")
-    if gemm.tc_eligible(x, w, K, ldx, ldw):
+    if gemm.tc_eligible(x, w, K, ldx, ldw) or gemm.f32_eligible(x, w, M, K, ldx, ldw):
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
         gemm.run(x, w, out, M, N, K, ldx, ldw, gated=POINTWISE_ACTS[act])
         return out

@@ -30,6 +30,8 @@ SKINNY_MAX_TOKENS = 8    # up to this many: mma.sync with both operands loaded s
 SKINNY_SMALL_MAX_TOKENS = 16
 SKINNY_SMALL_MAX_K = 3072
 SKINNY_SMALL_MAX_WEIGHTS = 8_500_000
+# float32: from how many tokens on the product runs on the tensor cores (below, the few-row kernel reads the weights once)
+F32_TC_MIN_TOKENS = 17
 _tickets = {}
 _plans = {}         # (M, N, K, sms) -> (workspace floats, tickets) as ti_linear_tc_plan answers
 _sm_counts = {}
@@ -76,6 +78,13 @@ def tc_eligible(x, w, K, ldx, ldw) -> bool:
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def f32_eligible(x, w, M, K, ldx, ldw) -> bool:
+    """Whether the float32 product runs as split bfloat16 parts on the tensor cores (csrc/gemm_f32_split.cu): more tokens
+    than the few-row kernel takes, rows on 16-byte boundaries."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and M >= F32_TC_MIN_TOKENS and ldx % 4 == 0
+            and ldw % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def run(x, w, out, M, N, K, ldx, ldw, gated: int = 0, late_start: bool = False, gate_limit: float = 0.0) -> None:
     """``gated``: 1 (or True) for up * silu(gate), 2 for up * gelu(gate) in the tanh form, 3 for the clamped pair
     g' sigmoid(1.702 g') (u' + 1) with g' = min(gate, gate_limit), u' = clamp(up, -gate_limit, gate_limit), over paired
@@ -114,7 +123,20 @@ def run(x, w, out, M, N, K, ldx, ldw, gated: int = 0, late_start: bool = False, 
         _call(lib.ti_linear_tc, _ptr(x), _ptr(w), _ptr(out), M, N, K, ldx, ldw, out.stride(0), out_f32, int(gated), float(gate_limit),
               sms, _ptr(workspace), _ptr(tickets), _stream())
         return
+    if f32_eligible(x, w, M, K, ldx, ldw):
+        sms = sm_count(x.device)
+        plan = _plans.get((M, N, K, -sms))
+        if plan is None:        # (pairs of blocks, workspace floats) of this shape: asked once
+            units, ws = ctypes.c_int(), ctypes.c_longlong()
+            _call(lib.ti_linear_f32_plan, M, N, K, sms, ctypes.byref(units), ctypes.byref(ws), launches=0)
+            if len(_plans) > 4096:
+                _plans.clear()
+            plan = _plans[(M, N, K, -sms)] = (units.value, ws.value)
+        workspace = torch.empty(plan[1], dtype=torch.float32, device=x.device) if plan[1] else None
+        _call(lib.ti_linear_f32_tc, _ptr(x), _ptr(w), _ptr(out), M, N, K, ldx, ldw, out.stride(0), plan[0], _ptr(workspace), int(gated),
+              float(gate_limit), _stream(), launches=2 if plan[1] else 1)
+        return
     if gated:
-        raise RuntimeError("linear: the gated epilogue exists in the tensor-core kernel only")
+        raise RuntimeError("linear: the gated epilogue exists in the tensor-core kernels only")
     _call(lib.ti_linear_simt, _ptr(x), _ptr(w), _ptr(out), M, N, K, ldx, ldw, out.stride(0),
           _code(x, "linear"), out_f32, _stream())
