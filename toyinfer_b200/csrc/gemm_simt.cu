@@ -1,8 +1,8 @@
 // out[M, N] = x[M, K] * W[N, K]^T on the CUDA cores, 32-bit accumulation.
 //
-// Two kernels.  `gemm_tile_kernel` (128x128x16 tiles, 8x8 per thread) is the whole
-// 32-bit engine's matrix product (FFMA only, no reduced-precision tensor mode) and
-// the fallback of the bfloat16 engine for shapes its tensor-core kernel refuses.
+// Two kernels.  `gemm_tile_kernel` (128x128x16 tiles, 8x8 per thread, FFMA) is the product of
+// more than 16 tokens whose rows do not start on 16-byte boundaries: what the tensor-core kernels
+// (gemm_tcgen05.cu, and gemm_f32_split.cu for float32) cannot load.
 // `gemv_rows_kernel` serves a handful of tokens (M <= 16): each warp streams weight
 // rows once and multiplies them with all M activation rows, so decode at a small
 // batch is bound by the read of W.

@@ -2,8 +2,8 @@
 
 bfloat16 operands whose rows are 16-byte aligned go to the tcgen05 kernel (the weights play
 the 128-row operand when there are at most 64 tokens), or, for up to 8 tokens (16 for small
-matrices), to kernels that only stream the weights (CUDA cores for one token, mma.sync beyond); everything else,
-and the whole 32-bit engine, runs on the CUDA-core kernels.
+matrices), to kernels that only stream the weights (CUDA cores for one token, mma.sync beyond).  float32 operands of more than
+16 tokens go to the tcgen05 kernel that splits them into bfloat16 parts; everything else runs on the CUDA-core kernels.
 """
 from __future__ import annotations
 
@@ -30,7 +30,11 @@ SKINNY_MAX_TOKENS = 8    # up to this many: mma.sync with both operands loaded s
 SKINNY_SMALL_MAX_TOKENS = 16
 SKINNY_SMALL_MAX_K = 3072
 SKINNY_SMALL_MAX_WEIGHTS = 8_500_000
-# float32: from how many tokens on the product runs on the tensor cores (below, the few-row kernel reads the weights once)
+# float32: from how many tokens on the product runs on the tensor cores (csrc/gemm_f32_split.cu).  Below, the few-row kernel of
+# gemm_simt.cu is ahead: it starts in 2 us where a pair of blocks with its tensor memory takes 6, and at 16 tokens, us, few-row /
+# tensor cores: 384 x 96 3.2 / 6.4, 1,024 x 1,024 10.5 / 13.9, 4,096 x 1,024 19.7 / 18.8, 19,456 x 2,560 195 / 92.  At 24 tokens
+# the tensor cores are at 7.3, 14.4, 19.8 and 95 where the tiled FFMA kernel took 15, 150, 150 and 910; at 500 tokens of
+# 19,456 x 2,560 at 290 (172 TFLOP/s) where it took 2,390.
 F32_TC_MIN_TOKENS = 17
 _tickets = {}
 _plans = {}         # (M, N, K, sms) -> (workspace floats, tickets) as ti_linear_tc_plan answers
