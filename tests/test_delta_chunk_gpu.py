@@ -1,0 +1,92 @@
+"""The delta rule in chunks (csrc/delta_chunk.cu) against 64 bits and against the token-by-token scan: at edges of its chunks, with
+both kinds of decay, several sequences, strided rows, decays down to zero and states that are not zero."""
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def KR():
+    from toyinfer_b200.kernels import recurrent
+    return recurrent
+
+
+def exact(q, k, v, decay, dt, rate, beta, state, lens, head):
+    F = torch.float64
+    q, k, v, decay, beta, dt, rate = (t.to(F) for t in (q, k, v, decay, beta, dt, rate))
+    G, d = q.shape[1:]
+    H, dv = v.shape[1:]
+    unit = lambda x: x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)
+    q, k = (unit(q) * d ** -0.5).repeat_interleave(H // G, 1), unit(k).repeat_interleave(H // G, 1)
+    soft = torch.nn.functional.softplus(decay + dt, threshold=100)
+    g = torch.exp(-rate[:, None] * (soft[:, :, None].expand(-1, H, d) if head else soft.view(-1, H, d)))
+    beta = torch.sigmoid(beta)
+    out, left, t = [], [], 0
+    for b, n in enumerate(lens):
+        S = state[b].to(F).clone()
+        for _ in range(n):
+            S = g[t, :, :, None] * S
+            e = beta[t, :, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t, :, :, None] * e[:, None]
+            out.append(torch.einsum("hdv,hd->hv", S, q[t]))
+            t += 1
+        left.append(S)
+    return torch.stack(out), torch.stack(left)
+
+
+def make(dtype, head, d, dv, H, G, lens, seed, strong):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    M = sum(lens)
+    rows = r(M, 2 * G * d + H * dv + 8).to(dtype)            # as one projection leaves them: strided views
+    q, k = rows[:, :G * d].view(M, G, d), rows[:, G * d:2 * G * d].view(M, G, d)
+    v = rows[:, 2 * G * d:2 * G * d + H * dv].view(M, H, dv)
+    decay = r(M, H).to(dtype) if head else r(M, H * d)
+    dt = r(H if head else H * d) - 2.0
+    rate = torch.exp(r(H) * 0.5)
+    beta = r(M, H).to(dtype)
+    if strong:      # some tokens forget everything, some write nothing or all, some keys are next to nothing
+        decay[5::17] = 3000.0
+        beta[3::11], beta[4::13] = 60.0, -60.0
+        rows[7::19, G * d:2 * G * d] *= 1e-4
+    state = r(len(lens), H, d, dv)
+    return q, k, v, decay, dt, rate, beta, state
+
+
+def run(KR, args, lens, head):
+    q, k, v, decay, dt, rate, beta, state = args
+    n = len(lens)
+    H, d, dv = state.shape[1:]
+    store = torch.zeros(n + 1, H * d * dv + 3, device="cuda")
+    store[:n, 3:] = state.reshape(n, -1)
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32)
+    batch = SimpleNamespace(cu_new=cu, seq_slot=torch.arange(n, dtype=torch.int32, device="cuda"), n_seq=n, max_new=max(lens))
+    o = KR.delta_rule(q, k, v, decay, dt, rate, beta, store, 3, batch, head_decay=head)
+    return o.view(-1, H, dv), store[:n, 3:].view(n, H, d, dv)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head", [True, False])
+@pytest.mark.parametrize("d,dv,H,G,lens,strong", [(64, 64, 2, 2, [32], False), (128, 128, 2, 1, [33, 1, 31], False), (64, 16, 4, 2, [100, 64], True),
+                                                  (128, 48, 3, 3, [2, 65, 200], True), (128, 128, 1, 1, [700], False), (64, 256, 2, 1, [40], False)])
+def test_against_the_scan(KR, monkeypatch, dtype, head, d, dv, H, G, lens, strong):
+    args = make(dtype, head, d, dv, H, G, lens, d + dv + sum(lens), strong)
+    want = exact(*args, lens, head)
+    assert KR.delta_chunked(args[0], args[2], SimpleNamespace(max_new=max(lens), n_seq=len(lens)))
+    got = run(KR, args, lens, head)
+    monkeypatch.setattr(KR, "DELTA_CHUNKED_FROM", 1 << 30)
+    scan = run(KR, args, lens, head)
+    for g, s, w in zip(got, scan, want):
+        off = lambda x: float((x.double() - w).norm() / w.norm())
+        assert torch.isfinite(g).all()
+        # every write passes two sums of 32-bit products (over the state, then over the chunk's earlier writes) where the scan's
+        # passes one: at most twice as far off (both some 1e-7)
+        assert off(g) <= max(2.0 * off(s), 2e-7), (off(g), off(s))
+        print(f"{off(g):.2e} against the scan's {off(s):.2e}")
+        worst = (g.double() - w).abs().max() / w.abs().max()
+        assert worst <= 4e-6, worst

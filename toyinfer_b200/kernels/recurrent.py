@@ -84,6 +84,21 @@ def rglru_scan(gates: torch.Tensor, u: torch.Tensor, z: torch.Tensor, gate_bias_
     return out
 
 
+# New tokens of one sequence from which the delta rule runs in chunks of 32 (csrc/delta_chunk.cu)
+DELTA_CHUNKED_FROM = 32
+DELTA_CHUNK_SCRATCH = 1 << 30       # ... while its operands, some four floats per element of q, take no more bytes than this
+
+
+def delta_chunked(q: torch.Tensor, v: torch.Tensor, batch) -> int:
+    """Floats of scratch with which a step's delta rule runs in chunks, or 0: it goes token by token."""
+    M, G, dim = q.shape
+    H, vdim = v.shape[1], v.shape[2]
+    if batch.max_new < DELTA_CHUNKED_FROM or dim not in (64, 128) or vdim % 16:
+        return 0
+    need = (M // 32 + batch.n_seq) * H * _fn("ti_delta_chunk_floats", [I, I])(dim, vdim)
+    return need if 4 * need <= DELTA_CHUNK_SCRATCH else 0
+
+
 def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: torch.Tensor, dt_bias: torch.Tensor,
                rate: torch.Tensor, beta_logit: torch.Tensor, state: torch.Tensor, state_offset: int, batch,
                head_decay: bool = False) -> torch.Tensor:
@@ -110,6 +125,14 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
     _vec(rate, H, "delta_rule: the rates")
     base, stride = _state_part(state, state_offset, H * dim * vdim, "delta_rule")
     o = torch.zeros((M, H * vdim), dtype=torch.float32, device=q.device)
+    chunked = delta_chunked(q, v, batch)
+    if chunked:
+        scratch = torch.empty(chunked, dtype=torch.float32, device=q.device)
+        _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, P]),
+              _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(decay_logit), decay_logit.stride(0), 1 if head_decay else 0,
+              _ptr(dt_bias), _ptr(rate), _ptr(beta_logit), beta_logit.stride(0), _ptr(o), base, stride, _ptr(scratch), _ptr(batch.cu_new),
+              _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, H, G, dim, vdim, _code(q, "delta_rule"), _stream(), launches=2)
+        return o
     # unit queries and keys, decays and betas of all tokens, made by a kernel of their own before the recurrence
     scratch = torch.empty(M * (2 * G * dim + n_decay + H), dtype=torch.float32, device=q.device)
     _call(_fn("ti_delta_rule_scan", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, P]),
