@@ -120,10 +120,15 @@ delta_chunk_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
         if constexpr (HEAD) gh[tid] = tid < n ? expf(-rt * dc_softplus(to_f32(decay_logit[(size_t)(tok0 + tid) * decay_stride + h]) + dt_bias[h])) : 1.f;
     }
     __syncthreads();
-    for (int i = tid; i < CH * vdim; i += DC_THREADS) {
-        const int t = i / vdim, e = i - t * vdim;
-        a.bv[((cid * (vdim / DC_COLS) + e / DC_COLS) * CH + t) * DC_COLS + e % DC_COLS] =
-            t < n ? bs[t] * to_f32(v[(size_t)(tok0 + t) * v_stride + (size_t)h * vdim + e]) : 0.f;
+    for (int i = tid; i < CH * (vdim / 4); i += DC_THREADS) {       // four values of a row: [column group][token][16]
+        const int e = i % 4 * 4, t = i / 4 % CH, grp = i / (4 * CH);
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        if (t < n) {
+            const T* from = v + (size_t)(tok0 + t) * v_stride + (size_t)h * vdim + grp * DC_COLS + e;
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] = bs[t] * to_f32(from[j]);
+        }
+        *reinterpret_cast<float4*>(a.bv + cid * CH * vdim + 4 * i) = make_float4(x[0], x[1], x[2], x[3]);
     }
     if constexpr (HEAD) {
         if (warp == 0) {
@@ -137,7 +142,7 @@ delta_chunk_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
         __syncthreads();
         // A and P: two rows and two columns of either per thread
         const int t0 = (tid >> 4) * 2, s0 = (tid & 15) * 2;
-        float aa[2][2] = {}, pp[2][2] = {};
+        float2 aa[2][2] = {}, pp[2][2] = {};
         if (s0 <= t0 + 1) {
 #pragma unroll 4
             for (int e = 0; e < D; e += 4) {
@@ -152,8 +157,10 @@ delta_chunk_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
                 for (int i = 0; i < 2; i++)
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
-                        aa[i][j] = dot4(kt[i], kk[j], aa[i][j]);
-                        pp[i][j] = dot4(qt[i], kk[j], pp[i][j]);
+                        fma2(aa[i][j], make_float2(kt[i].x, kt[i].y), make_float2(kk[j].x, kk[j].y));
+                        fma2(aa[i][j], make_float2(kt[i].z, kt[i].w), make_float2(kk[j].z, kk[j].w));
+                        fma2(pp[i][j], make_float2(qt[i].x, qt[i].y), make_float2(kk[j].x, kk[j].y));
+                        fma2(pp[i][j], make_float2(qt[i].z, qt[i].w), make_float2(kk[j].z, kk[j].w));
                     }
             }
         }
@@ -163,8 +170,8 @@ delta_chunk_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
             for (int j = 0; j < 2; j++) {
                 const int t = t0 + i, s = s0 + j;
                 const float d = gs[t * P_PITCH + s];
-                As[t * P_PITCH + s] = s < t ? bs[t] * d * aa[i][j] : 0.f;
-                Ps[t * P_PITCH + s] = s <= t ? d * pp[i][j] : 0.f;
+                As[t * P_PITCH + s] = s < t ? bs[t] * d * (aa[i][j].x + aa[i][j].y) : 0.f;
+                Ps[t * P_PITCH + s] = s <= t ? d * (pp[i][j].x + pp[i][j].y) : 0.f;
             }
         __syncthreads();
     } else {
@@ -286,7 +293,7 @@ constexpr int R_PITCH = DC_COLS + 4, E_PITCH = DC_COLS + 8;     // (eight, or fo
 
 template <int D> constexpr int state_buf_floats() { return Ops<D>::floats + CH * DC_COLS; }
 template <int D> constexpr size_t state_smem_bytes() {
-    return (size_t)(2 * state_buf_floats<D>() + DC_COLS * (D + 4) + CH * (R_PITCH + E_PITCH)) * sizeof(float);
+    return (size_t)(2 * state_buf_floats<D>() + DC_COLS * (D + 4) + CH * (R_PITCH + E_PITCH + DC_COLS)) * sizeof(float);
 }
 
 // x[0 .. 2 N) summed over the lanes whose numbers differ in bit `bit`: the lane with it set goes on with the upper half.
@@ -310,6 +317,7 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, float* __restr
     float* St = sm + 2 * BUF;                    // [DC_COLS][PITCH]: S transposed
     float* Rs = St + DC_COLS * PITCH;            // [CH][R_PITCH]
     float* Es = Rs + CH * R_PITCH;               // [CH][E_PITCH]
+    float* Qs = Es + CH * E_PITCH;               // [CH][DC_COLS]: (G q) S
     __shared__ uint64_t ready[2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int groups = a.vdim / DC_COLS, h = blockIdx.x / groups, grp = blockIdx.x - h * groups, col0 = grp * DC_COLS, b = blockIdx.y;
@@ -376,14 +384,16 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, float* __restr
 #pragma unroll
                 for (int j = 0; j < 4; j++) all[i * 4 + j] = acc[i][j].x + acc[i][j].y;
         }
+        float half[16], quarter[8], mine[4];
+        halve<16>(all, half, 4);
+        halve<8>(half, quarter, 2);
+        halve<4>(quarter, mine, 1);
         if (warp < 4) {
-            float half[16], quarter[8], mine[4];
-            halve<16>(all, half, 4);
-            halve<8>(half, quarter, 2);
-            halve<4>(quarter, mine, 1);
             const int t = warp * 8 + kq;
             const float4 u = *reinterpret_cast<const float4*>(buf + O::floats + t * DC_COLS + ct * 4);
             *reinterpret_cast<float4*>(Rs + t * R_PITCH + ct * 4) = make_float4(u.x - mine[0], u.y - mine[1], u.z - mine[2], u.w - mine[3]);
+        } else {
+            *reinterpret_cast<float4*>(Qs + ((warp - 4) * 8 + kq) * DC_COLS + ct * 4) = make_float4(mine[0], mine[1], mine[2], mine[3]);
         }
         __syncthreads();
         {
@@ -451,26 +461,28 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, float* __restr
                 *reinterpret_cast<float4*>(St + (sc + j) * PITCH + d0) = make_float4(S[j][0], S[j][1], S[j][2], S[j][3]);
             }
         }
-        if (warp >= 4) {
-            // O = (G q) S + P E: the tokens kq, kq + 8, ... on what this lane has of the first product
+        {
+            // O = (G q) S + P E, as E = T R
+            float acc[16] = {};
 #pragma unroll
             for (int m = 0; m < 4; m++) {
                 const float4 e = *reinterpret_cast<const float4*>(Es + (kq + 8 * m) * E_PITCH + ct * 4);
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float w = buf[O::p + ((warp - 4) * 8 + i) * P_PITCH + kq + 8 * m];
-                    all[i * 4] = fmaf(w, e.x, all[i * 4]);
-                    all[i * 4 + 1] = fmaf(w, e.y, all[i * 4 + 1]);
-                    all[i * 4 + 2] = fmaf(w, e.z, all[i * 4 + 2]);
-                    all[i * 4 + 3] = fmaf(w, e.w, all[i * 4 + 3]);
+                for (int i = 0; i < 4; i++) {
+                    const float w = buf[O::p + (warp * 4 + i) * P_PITCH + kq + 8 * m];
+                    acc[i * 4] = fmaf(w, e.x, acc[i * 4]);
+                    acc[i * 4 + 1] = fmaf(w, e.y, acc[i * 4 + 1]);
+                    acc[i * 4 + 2] = fmaf(w, e.z, acc[i * 4 + 2]);
+                    acc[i * 4 + 3] = fmaf(w, e.w, acc[i * 4 + 3]);
                 }
             }
-            float half[16], quarter[8], mine[4];
-            halve<16>(all, half, 4);
-            halve<8>(half, quarter, 2);
-            halve<4>(quarter, mine, 1);
-            const int t = c * CH + (warp - 4) * 8 + kq;
-            if (t < n) *reinterpret_cast<float4*>(o + ((size_t)(first + t) * H + h) * a.vdim + col0 + ct * 4) = make_float4(mine[0], mine[1], mine[2], mine[3]);
+            float half[8], quarter[4], mine[2];
+            halve<8>(acc, half, 4);
+            halve<4>(half, quarter, 2);
+            halve<2>(quarter, mine, 1);
+            const int r = warp * 4 + (kq >> 1), e = ct * 4 + (kq & 1) * 2, t = c * CH + r;
+            const float2 q = *reinterpret_cast<const float2*>(Qs + r * DC_COLS + e);
+            if (t < n) *reinterpret_cast<float2*>(o + ((size_t)(first + t) * H + h) * a.vdim + col0 + e) = make_float2(q.x + mine[0], q.y + mine[1]);
         }
         __syncthreads();                         // this chunk's operands are used up
         if (tid == 0 && c + 2 < chunks) fetch(c + 2);
@@ -486,19 +498,24 @@ int run_chunks(const void* q, const void* k, const void* v, long long q_stride, 
                long long decay_stride, const float* dt_bias, const float* rate, const void* beta_logit, long long beta_stride, float* o,
                float* state, long long slot_stride, const DeltaChunkArgs& a, int n_seq, int max_new, cudaStream_t stream) {
     constexpr size_t prep = prep_smem_floats<D, HEAD>() * sizeof(float), smem = state_smem_bytes<D>();
+    constexpr size_t ALONE = 120 * 1024;        // shared memory of a block that shares its SM with no other
     int* status = ti_status_ptr();
     TI_REQUIRE(status != nullptr, "delta_rule: no status word");
     static bool configured = false;
     if (!configured) {
         TI_CUDA(cudaFuncSetAttribute(delta_chunk_prep_kernel<T, L, D, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep));
-        TI_CUDA(cudaFuncSetAttribute(delta_chunk_state_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        TI_CUDA(cudaFuncSetAttribute(delta_chunk_state_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem < ALONE ? ALONE : smem)));
         configured = true;
     }
     TI_CUDA(ti_launch(delta_chunk_prep_kernel<T, L, D, HEAD>, dim3((max_new + CH - 1) / CH, a.n_heads, n_seq), dim3(DC_THREADS), prep, stream,
                       (const T*)q, (const T*)k, (const T*)v, q_stride, k_stride, v_stride, (const L*)decay_logit, decay_stride, dt_bias, rate,
                       (const T*)beta_logit, beta_stride, a));
     TI_CHECK_LAUNCH("delta_rule (chunks)");
-    TI_CUDA(ti_launch(delta_chunk_state_kernel<D>, dim3(a.n_heads * (a.vdim / DC_COLS), n_seq), dim3(DC_THREADS), smem, stream, a, o, state,
+    // blocks that have an SM each must not start two on the SM that the kernel before left first: the walk is a chain, and its
+    // time is the slowest block's (64 heads' columns of 64 on two-block SMs: 245 us, spread out 165)
+    const long long blocks = (long long)a.n_heads * (a.vdim / DC_COLS) * n_seq;
+    const size_t room = blocks <= 148 && smem < ALONE ? ALONE : smem;
+    TI_CUDA(ti_launch(delta_chunk_state_kernel<D>, dim3(a.n_heads * (a.vdim / DC_COLS), n_seq), dim3(DC_THREADS), room, stream, a, o, state,
                       slot_stride, status));
     TI_CHECK_LAUNCH("delta_rule (chunk states)");
     return 0;
