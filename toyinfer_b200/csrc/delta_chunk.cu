@@ -16,7 +16,10 @@
 //
 // What bounds the second kernel: the shared memory that its multiply-adds read, 128 bytes a cycle whatever lanes share them.
 // Hence tiles of 8 x 4 results a thread with the contraction shared out over neighbouring lanes (a thread reads 1.5 bytes a
-// multiply-add where tiles of 4 x 4 and 4 x 2 read 2 and 3) and each lane left with its part of the sums after a few exchanges.
+// multiply-add where tiles of 4 x 4 and 4 x 2 read 2 and 3) and each lane left with its part of the sums after a few exchanges:
+// a chunk takes 5,500 cycles, 2,000 of them the products with S.  2,048 tokens of 16 heads of 128 x 128, us, the scan / chunks:
+// one decay per head 632 / 228, per key channel 964 / 299; heads of 64 x 64 473 / 169 and 783 / 189; a run of 32 tokens 21.8 /
+// 15.7 and 23.6 / 24.4, of 16 tokens 14.9 / 15.4 and 16.0 / 21.8 (hence the scan below 32).
 #include "tma.cuh"
 
 #include <type_traits>
@@ -363,21 +366,27 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, float* __restr
         float all[32];
         {
             float2 acc[8][4] = {};
+            float4 x[2][8], y[2][4];             // the next step's operands are on their way while this one's are multiplied
+            auto load = [&](int it) {
+                const int e = it * 32 + kq * 4;
+#pragma unroll
+                for (int j = 0; j < 4; j++) y[it & 1][j] = *reinterpret_cast<const float4*>(St + (ct * 4 + j) * PITCH + e);
+#pragma unroll
+                for (int i = 0; i < 8; i++) x[it & 1][i] = *reinterpret_cast<const float4*>(buf + (warp * 8 + i) * PITCH + e);      // (queries follow keys)
+            };
+            load(0);
 #pragma unroll
             for (int it = 0; it < D / 32; it++) {
-                const int e = it * 32 + kq * 4;
-                float4 y[4];
+                if (it + 1 < D / 32) load(it + 1);
+                asm volatile("" ::: "memory");
 #pragma unroll
-                for (int j = 0; j < 4; j++) y[j] = *reinterpret_cast<const float4*>(St + (ct * 4 + j) * PITCH + e);
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float4 x = *reinterpret_cast<const float4*>(buf + (warp * 8 + i) * PITCH + e);        // (queries follow keys)
+                for (int i = 0; i < 8; i++)
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        fma2(acc[i][j], make_float2(x.x, x.y), make_float2(y[j].x, y[j].y));
-                        fma2(acc[i][j], make_float2(x.z, x.w), make_float2(y[j].z, y[j].w));
+                        const float4 &u = x[it & 1][i], &v = y[it & 1][j];
+                        fma2(acc[i][j], make_float2(u.x, u.y), make_float2(v.x, v.y));
+                        fma2(acc[i][j], make_float2(u.z, u.w), make_float2(v.z, v.w));
                     }
-                }
             }
 #pragma unroll
             for (int i = 0; i < 8; i++)
@@ -512,7 +521,7 @@ int run_chunks(const void* q, const void* k, const void* v, long long q_stride, 
                       (const T*)beta_logit, beta_stride, a));
     TI_CHECK_LAUNCH("delta_rule (chunks)");
     // blocks that have an SM each must not start two on the SM that the kernel before left first: the walk is a chain, and its
-    // time is the slowest block's (64 heads' columns of 64 on two-block SMs: 245 us, spread out 165)
+    // time is the slowest block's (64 blocks of 64 x 16: 245 us, spread out 169)
     const long long blocks = (long long)a.n_heads * (a.vdim / DC_COLS) * n_seq;
     const size_t room = blocks <= 148 && smem < ALONE ? ALONE : smem;
     TI_CUDA(ti_launch(delta_chunk_state_kernel<D>, dim3(a.n_heads * (a.vdim / DC_COLS), n_seq), dim3(DC_THREADS), room, stream, a, o, state,

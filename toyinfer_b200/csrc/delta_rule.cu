@@ -13,7 +13,8 @@
 //
 // delta_rule_prep makes unit q and k, decays and betas of all the step's tokens at once.
 // delta_rule_scan: a sequence's new tokens are scanned in order from the state in its slot, which
-// is updated in place: whole prompts, single tokens and anything between are one kernel.  Grid
+// is updated in place: whole prompts, single tokens and anything between are one kernel (runs of 32 tokens and more of heads
+// of 64 and 128 go in chunks instead: delta_chunk.cu).  Grid
 // (heads * column groups of 8, sequences): sixteen neighbouring lanes share one column of S (a
 // sixteenth of its rows in registers each) and add up the two sums over the column by shuffles, so that
 // a single sequence still gives every SM several warps; q, k, g and v of a run of tokens are staged in
