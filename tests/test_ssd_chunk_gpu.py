@@ -1,0 +1,85 @@
+"""The Mamba-2 recurrence in chunks (csrc/ssd_chunk.cu) against 64 bits and against the token-by-token scan: at edges of its
+chunks and tiles, several sequences, strided rows, decays from none to total and states that are not zero."""
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def KR():
+    from toyinfer_b200.kernels import recurrent
+    return recurrent
+
+
+def make(H, G, N, V, lens, seed, strong=False):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    M = sum(lens)
+    rows = r(M, H * V + 2 * G * N + H + (-H % 8)).to(torch.bfloat16)       # as the projection leaves them, the step sizes beside
+    xbc, dt = rows[:, :H * V + 2 * G * N], rows[:, H * V + 2 * G * N:H * V + 2 * G * N + H]
+    if strong:
+        dt[5::17], dt[9::23] = 5000.0, -60.0        # some tokens forget everything, some write nothing and forget nothing
+    bias, rate, skip = r(H) * 0.5 - 1.0, torch.exp(r(H)), 1.0 + 0.2 * r(H)
+    return xbc, dt, bias, rate, skip, r(len(lens), H, V, N)
+
+
+def exact(args, H, G, N, V, lens):
+    xbc, dt, bias, rate, skip, state = (t.double() for t in args)
+    d = torch.nn.functional.softplus(dt + bias, threshold=100)
+    a = torch.exp(-rate * d)
+    x = xbc[:, :H * V].view(-1, H, V)
+    B, C = (xbc[:, H * V + i * G * N:H * V + (i + 1) * G * N].view(-1, G, N).repeat_interleave(H // G, 1) for i in (0, 1))
+    out, left, t = [], [], 0
+    for b, n in enumerate(lens):
+        S = state[b].clone()
+        for _ in range(n):
+            S = a[t, :, None, None] * S + (d[t, :, None] * x[t])[:, :, None] * B[t, :, None]
+            out.append(torch.einsum("hvn,hn->hv", S, C[t]) + skip[:, None] * x[t])
+            t += 1
+        left.append(S)
+    return torch.stack(out), torch.stack(left)
+
+
+def run(KR, args, H, G, N, V, lens):
+    xbc, dt, bias, rate, skip, state = args
+    n = len(lens)
+    store = torch.zeros(n + 1, H * N * V + 3, device="cuda")
+    store[:n, 3:] = state.reshape(n, -1)
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32)
+    batch = SimpleNamespace(cu_new=cu, seq_slot=torch.arange(n, dtype=torch.int32, device="cuda"), n_seq=n, max_new=max(lens))
+    y = KR.ssd_scan(xbc, dt, bias, rate, skip, H, G, N, V, store, 3, batch)
+    return y.view(-1, H, V), store[:n, 3:].view(n, H, V, N)
+
+
+@pytest.mark.parametrize("H,G,N,V,lens,strong", [(2, 1, 64, 32, [80], False), (4, 2, 128, 64, [127, 1, 129], False), (8, 8, 128, 64, [16, 128, 17], True),
+                                                 (6, 1, 64, 64, [300], True), (24, 2, 128, 32, [256, 5], False), (3, 3, 128, 64, [600], False)])
+def test_against_the_scan(KR, monkeypatch, H, G, N, V, lens, strong):
+    args = make(H, G, N, V, lens, H + N + V + sum(lens), strong)
+    want = exact(args, H, G, N, V, lens)
+    assert KR.ssd_chunked(args[0], H, N, V, SimpleNamespace(max_new=max(lens), n_seq=len(lens)))
+    got = run(KR, args, H, G, N, V, lens)
+    monkeypatch.setattr(KR, "SSD_CHUNKED_FROM", 1 << 30)
+    scan = run(KR, args, H, G, N, V, lens)
+    for g, s, w in zip(got, scan, want):
+        off = lambda x: float((x.double() - w).norm() / w.norm())
+        # the tensor cores' sums truncate: at most a step of 2^-23 for each of the 8 products of 16 that a sum over 128 has,
+        # half of it on average, where the scan rounds to nearest token by token
+        assert off(g) <= max(1.5 * off(s), 2.5e-7), (off(g), off(s))
+        print(f"{off(g):.2e} against the scan's {off(s):.2e}")
+        assert ((g.double() - w).abs().max() / w.abs().max()) <= 4e-6
+
+
+def test_rows_that_are_not_aligned_take_the_scan(KR):
+    args = list(make(2, 1, 64, 32, [90], 3))
+    wide = torch.zeros(90, args[0].shape[1] + 1, dtype=torch.bfloat16, device="cuda")
+    wide[:, 1:] = args[0]
+    args[0] = wide[:, 1:]
+    assert KR.ssd_chunked(args[0], 2, 64, 32, SimpleNamespace(max_new=90, n_seq=1)) == 0
+    want = exact(args, 2, 1, 64, 32, [90])
+    for g, w in zip(run(KR, args, 2, 1, 64, 32, [90]), want):
+        assert float((g.double() - w).norm() / w.norm()) < 1e-6

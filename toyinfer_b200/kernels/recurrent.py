@@ -190,6 +190,17 @@ def block_diag_linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 
 
 SSD_SEGMENT = 256               # tokens of a segment; a step whose longest sequence brings two or more runs them in parallel
+SSD_CHUNKED_FROM = 80           # new tokens of one sequence from which bfloat16 steps run in chunks of 128 on the tensor cores
+SSD_CHUNK_SCRATCH = 1 << 30     # ... while the chunks' states take no more bytes than this
+
+
+def ssd_chunked(xbc: torch.Tensor, n_heads: int, n_state: int, vdim: int, batch) -> int:
+    """Floats of scratch with which a step's Mamba-2 recurrence runs in chunks (csrc/ssd_chunk.cu), or 0: token by token."""
+    if (batch.max_new < SSD_CHUNKED_FROM or xbc.dtype != torch.bfloat16 or n_state not in (64, 128) or vdim not in (32, 64)
+            or xbc.stride(0) % 8 or xbc.data_ptr() % 16):
+        return 0
+    need = (xbc.shape[0] // 128 + batch.n_seq) * n_heads * (vdim * n_state + 1)
+    return need if 4 * need <= SSD_CHUNK_SCRATCH else 0
 
 
 def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, rate: torch.Tensor, skip: Optional[torch.Tensor],
@@ -210,6 +221,14 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, rat
         _vec(t, n_heads, f"ssd_scan: the {what}")
     base, stride = _state_part(state, state_offset, inner * n_state, "ssd_scan")
     y = torch.zeros((M, inner), dtype=torch.float32, device=xbc.device)         # rows that are nobody's stay zero
+    chunked = ssd_chunked(xbc, n_heads, n_state, vdim, batch)
+    if chunked:
+        scratch = torch.empty(chunked, dtype=torch.float32, device=xbc.device)
+        _call(_fn("ti_ssd_chunked", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, P, P]),
+              _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0), _ptr(dt_bias), _ptr(rate), _ptr(skip), base, stride, _ptr(y),
+              _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, int(n_heads), int(groups), int(n_state), int(vdim),
+              _ptr(scratch), _stream(), launches=3)
+        return y
     seg = int(SSD_SEGMENT)
     n_seg = (batch.max_new + seg - 1) // seg if batch.max_new >= 2 * seg else 1
     scratch = decay = None
