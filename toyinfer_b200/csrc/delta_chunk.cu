@@ -312,7 +312,7 @@ __device__ __forceinline__ void halve(const float* x, float* out, int bit) {
 
 template <int D>
 __global__ void __launch_bounds__(DC_THREADS)
-delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, float* __restrict__ state, long long slot_stride, int* status) {
+delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* __restrict__ state, long long slot_stride, int* status) {
     ti_pdl_trigger();
     using O = Ops<D>;
     constexpr int PITCH = D + 4, BUF = state_buf_floats<D>();
@@ -326,6 +326,8 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, float* __restr
     const int groups = a.vdim / DC_COLS, h = blockIdx.x / groups, grp = blockIdx.x - h * groups, col0 = grp * DC_COLS, b = blockIdx.y;
     if (tid == 0) { mbar_init(&ready[0], 1); mbar_init(&ready[1], 1); mbar_fence_init(); }
     ti_pdl_sync();
+    if (b == 0)          // rows past the last sequence's are nobody's
+        for (int m = a.cu_new[gridDim.y] + (tid >> 4); m < M; m += DC_THREADS / DC_COLS) o[((size_t)m * a.n_heads + h) * a.vdim + col0 + (tid & 15)] = 0.f;
     const int first = a.cu_new[b], n = a.cu_new[b + 1] - first;
     if (n <= 0) return;
     const int H = a.n_heads, chunks = (n + CH - 1) / CH;
@@ -505,7 +507,7 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, float* __restr
 template <typename T, typename L, int D, bool HEAD>
 int run_chunks(const void* q, const void* k, const void* v, long long q_stride, long long k_stride, long long v_stride, const void* decay_logit,
                long long decay_stride, const float* dt_bias, const float* rate, const void* beta_logit, long long beta_stride, float* o,
-               float* state, long long slot_stride, const DeltaChunkArgs& a, int n_seq, int max_new, cudaStream_t stream) {
+               float* state, long long slot_stride, const DeltaChunkArgs& a, int n_seq, int max_new, int M, cudaStream_t stream) {
     constexpr size_t prep = prep_smem_floats<D, HEAD>() * sizeof(float), smem = state_smem_bytes<D>();
     constexpr size_t ALONE = 120 * 1024;        // shared memory of a block that shares its SM with no other
     int* status = ti_status_ptr();
@@ -524,7 +526,7 @@ int run_chunks(const void* q, const void* k, const void* v, long long q_stride, 
     // time is the slowest block's (64 blocks of 64 x 16: 245 us, spread out 169)
     const long long blocks = (long long)a.n_heads * (a.vdim / DC_COLS) * n_seq;
     const size_t room = blocks <= 148 && smem < ALONE ? ALONE : smem;
-    TI_CUDA(ti_launch(delta_chunk_state_kernel<D>, dim3(a.n_heads * (a.vdim / DC_COLS), n_seq), dim3(DC_THREADS), room, stream, a, o, state,
+    TI_CUDA(ti_launch(delta_chunk_state_kernel<D>, dim3(a.n_heads * (a.vdim / DC_COLS), n_seq), dim3(DC_THREADS), room, stream, a, o, M, state,
                       slot_stride, status));
     TI_CHECK_LAUNCH("delta_rule (chunk states)");
     return 0;
@@ -557,9 +559,9 @@ extern "C" int ti_delta_rule_chunked(const void* q, const void* k, const void* v
             constexpr int D = decltype(dc)::value;
             if (head_decay)
                 return run_chunks<T, T, D, true>(q, k, v, q_stride, k_stride, v_stride, decay_logit, decay_stride, dt_bias, rate, beta_logit, beta_stride, o,
-                                                 state, slot_stride, a, n_seq, max_new, stream);
+                                                 state, slot_stride, a, n_seq, max_new, M, stream);
             return run_chunks<T, float, D, false>(q, k, v, q_stride, k_stride, v_stride, decay_logit, decay_stride, dt_bias, rate, beta_logit, beta_stride, o,
-                                                  state, slot_stride, a, n_seq, max_new, stream);
+                                                  state, slot_stride, a, n_seq, max_new, M, stream);
         };
         return dim == 64 ? go(std::integral_constant<int, 64>()) : go(std::integral_constant<int, 128>());
     });

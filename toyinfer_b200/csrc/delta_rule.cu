@@ -288,6 +288,50 @@ __global__ void head_gated_rmsnorm_kernel(const float* __restrict__ o, const T* 
     }
 }
 
+// The same where rows can be read 16 bytes at a time: vdim / 8 lanes a head (a power of two up to 32), eight values a lane, read
+// once.
+template <typename T>
+__global__ void head_gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long gate_stride,
+                                              const float* __restrict__ w, T* __restrict__ out, long long out_stride, long long rows,
+                                              int n_heads, int vdim, float eps, int gate_silu, float out_scale) {
+    ti_pdl_trigger();
+    ti_pdl_sync();
+    o = ti_dependent(o); gate = ti_dependent(gate);
+    const int lanes = vdim / 8;
+    const long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x, r = item / lanes;
+    const bool live = r < rows;
+    const long long m = live ? r / n_heads : 0;
+    const int i = (int)(item - r * lanes) * 8, at = live ? (int)(r - m * n_heads) * vdim + i : 0;
+    float x[8];
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    T g[8];
+    if (live) {
+        a = *reinterpret_cast<const float4*>(o + (size_t)r * vdim + i);
+        b = *reinterpret_cast<const float4*>(o + (size_t)r * vdim + i + 4);
+#pragma unroll
+        for (int k = 0; k < 8 * (int)sizeof(T); k += 16)
+            *reinterpret_cast<uint4*>(reinterpret_cast<char*>(g) + k) =
+                *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(gate + (size_t)m * gate_stride + at) + k);
+    }
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; e++) ss = fmaf(x[e], x[e], ss);
+    for (int k = lanes >> 1; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
+    if (!live) return;
+    const float inv = rsqrtf(ss / (float)vdim + eps) * out_scale;
+    T y[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const float gl = to_f32(g[e]);
+        const float ga = (gate_silu ? gl : 1.0f) / (1.0f + expf(-gl));
+        y[e] = from_f32<T>(x[e] * inv * (w ? w[i + e] : 1.0f) * ga);
+    }
+#pragma unroll
+    for (int k = 0; k < 8 * (int)sizeof(T); k += 16)
+        *reinterpret_cast<uint4*>(reinterpret_cast<char*>(out + (size_t)m * out_stride + at) + k) = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(y) + k);
+}
+
 template <typename F>
 int dispatch_dim(int dim, F&& f) {
     if (dim <= 32) return f(std::integral_constant<int, 32>());
@@ -367,6 +411,14 @@ extern "C" int ti_head_gated_rmsnorm(const float* o, const void* gate, long long
     const long long rows = (long long)M * n_heads;
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
+        const int V = 16 / (int)sizeof(T);
+        if (vdim >= 8 && vdim <= 256 && (vdim & (vdim - 1)) == 0 && gate_stride % V == 0 && out_stride % V == 0 &&
+            ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+            TI_CUDA(ti_launch_class<1>(head_gated_rmsnorm_vec_kernel<T>, dim3((unsigned)((rows * (vdim / 8) + 127) / 128)), dim3(128), 0, stream, o,
+                                       (const T*)gate, gate_stride, w, (T*)out, out_stride, rows, n_heads, vdim, eps, gate_silu, out_scale));
+            TI_CHECK_LAUNCH("head_gated_rmsnorm");
+            return 0;
+        }
         TI_CUDA(ti_launch_class<1>(head_gated_rmsnorm_kernel<T>, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, stream, o, (const T*)gate,
                                    gate_stride, w, (T*)out, out_stride, rows, n_heads, vdim, eps, gate_silu, out_scale));
         TI_CHECK_LAUNCH("head_gated_rmsnorm");

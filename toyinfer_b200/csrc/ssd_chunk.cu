@@ -81,13 +81,21 @@ __device__ __forceinline__ double chunk_decays(const SsdArgs& g, int tok0, int n
     return all;
 }
 
-// Rows of COLS bfloat16 (64 or 128; or 32 in rows of 64) into the swizzled boxes of mma_utils.cuh; rows past the end are zeros.
+__device__ __forceinline__ void async16(uint32_t to, const void* from, bool live) {
+    const int bytes = live ? 16 : 0;            // the rest is filled with zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// Rows of COLS bfloat16 (64 or 128; or 32 in rows of 64) into the swizzled boxes of mma_utils.cuh, on their way until
+// async_wait(); rows past the end are zeros.
 template <int COLS>
-__device__ __forceinline__ void load_rows(unsigned char* to, const bf16* from, long long ld, int n) {
+__device__ __forceinline__ void load_rows(uint32_t to, const bf16* from, long long ld, int n) {
+#pragma unroll
     for (int i = threadIdx.x; i < SC * (COLS / 8); i += SSD_THREADS) {
         const int t = i / (COLS / 8), e = (i % (COLS / 8)) * 8;
-        const uint4 v = t < n ? *reinterpret_cast<const uint4*>(from + (size_t)t * ld + e) : make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(to + swizzled_offset<SC>(t, e)) = v;
+        async16(to + swizzled_offset<SC>(t, e), from + (size_t)(t < n ? t : 0) * ld + e, t < n);
     }
 }
 
@@ -98,9 +106,7 @@ __global__ void __launch_bounds__(SSD_THREADS)
 ssd_chunk_state_kernel(SsdArgs g) {
     ti_pdl_trigger();
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char* bt = smem;                                   // B [SC][N]
-    unsigned char* xt = smem + SC * N * 2;                      // x [SC][V] (in rows of 64)
-    __shared__ float ds[SC], lh[SC], ll[SC], w[SC];
+    __shared__ float ds[SC], lh[SC], ll[SC], w[SC];             // smem: B [SC][N], x [SC][V] (in rows of 64)
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     ti_pdl_sync();
     g.xbc = ti_dependent(g.xbc); g.dt = ti_dependent(g.dt);
@@ -108,8 +114,10 @@ ssd_chunk_state_kernel(SsdArgs g) {
     if (n <= 0) return;
     const int inner = g.heads * V, grp = h / (g.heads / g.groups);
     const bf16* row0 = g.xbc + (size_t)tok0 * g.ld_xbc;
-    load_rows<N>(bt, row0 + inner + grp * N, g.ld_xbc, n);
-    load_rows<V>(xt, row0 + h * V, g.ld_xbc, n);
+    const uint32_t bs = (uint32_t)__cvta_generic_to_shared(smem), xs = bs + SC * N * 2;
+    load_rows<N>(bs, row0 + inner + grp * N, g.ld_xbc, n);
+    load_rows<V>(xs, row0 + h * V, g.ld_xbc, n);
+    async_commit();
     const size_t id = ssd_chunk_id(first, b, c) * g.heads + h;
     if (warp == 0) {
         const double all = chunk_decays(g, tok0, n, h, ds, lh, ll);
@@ -121,11 +129,11 @@ ssd_chunk_state_kernel(SsdArgs g) {
         }
         if (lane == 0) g.decay[id] = (float)exp2(all);
     }
+    async_wait();
     __syncthreads();
     constexpr int VT = V / 16, NSPLIT = 8 / VT, NT = N / NSPLIT;        // warps side by side along N; columns of N of a warp
     const int v0 = (warp % VT) * 16, n0 = (warp / VT) * NT;
     float acc[NT / 8][4] = {}, low[NT / 8][4] = {};      // (the small parts in sums of their own: an accumulator is truncated at its own size with every MMA)
-    const uint32_t xs = (uint32_t)__cvta_generic_to_shared(xt), bs = (uint32_t)__cvta_generic_to_shared(bt);
     for (int s0 = 0; s0 < SC; s0 += 16) {
         if (s0 >= n) break;
         // x transposed: matrices (v 0-7, s 0-7), (v 8-15, s 0-7), (v 0-7, s 8-15), (v 8-15, s 8-15)
@@ -199,12 +207,14 @@ __global__ void ssd_chunk_carry_kernel(SsdArgs g, int per_head) {
 // stays in registers for all of the block's heads, as does C.
 template <int N, int V>
 __global__ void __launch_bounds__(SSD_THREADS, 1)
-ssd_chunk_out_kernel(SsdArgs g, int run) {
+ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
     ti_pdl_trigger();
     extern __shared__ __align__(1024) unsigned char smem[];
-    constexpr int X_BYTES = SC * 64 * 2, PART = V * N * 2;
-    unsigned char* xt = smem;                                   // x [SC][V] (in rows of 64), where C is at first
-    unsigned char* st = smem + X_BYTES;                         // S [V][N] in three parts, where B is at first
+    constexpr int X_BYTES = SC * 64 * 2, PART = V * N * 2, RAW = 3 * PART;
+    // S [V][N] in three parts and as it is in memory; x [SC][V] (in rows of 64) of this head and the next.  C and B are where the
+    // parts of S are, and behind them, at first.
+    unsigned char* st = smem;
+    unsigned char* xt = smem + RAW + V * N * 4;
     __shared__ float ds[8][SC], lh[8][SC], ll[8][SC];
     const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     ti_pdl_sync();
@@ -214,19 +224,33 @@ ssd_chunk_out_kernel(SsdArgs g, int run) {
     const int inner = g.heads * V, per_group = g.heads / g.groups, runs = (per_group + run - 1) / run;
     const int grp = blockIdx.y / runs, h0 = grp * per_group + (blockIdx.y - grp * runs) * run, h1 = min(h0 + run, (grp + 1) * per_group);
     const bf16* row0 = g.xbc + (size_t)tok0 * g.ld_xbc;
-    if (warp < h1 - h0) chunk_decays(g, tok0, n, h0 + warp, ds[warp], lh[warp], ll[warp]);      // (runs of up to 8 heads)
-    const uint32_t xs = (uint32_t)__cvta_generic_to_shared(xt), ss = (uint32_t)__cvta_generic_to_shared(st);
+    if (b == 0 && c == 0) {      // rows past the last sequence's are nobody's
+        const int cols = (h1 - h0) * V;
+        for (int i = tid; i < (M - g.cu_new[gridDim.z]) * cols; i += SSD_THREADS)
+            g.y[(size_t)(g.cu_new[gridDim.z] + i / cols) * inner + (size_t)h0 * V + i % cols] = 0.f;
+    }
+    const uint32_t ss = (uint32_t)__cvta_generic_to_shared(st), x0 = (uint32_t)__cvta_generic_to_shared(xt);
+    auto fetch = [&](int h) {
+        load_rows<V>(x0 + ((h - h0) & 1) * X_BYTES, row0 + h * V, g.ld_xbc, n);
+        const float* from = g.scratch + (ssd_chunk_id(first, b, c) * g.heads + h) * (size_t)(V * N);
+#pragma unroll
+        for (int i = tid; i < V * N / 4; i += SSD_THREADS) async16(ss + RAW + i * 16, from + i * 4, true);
+        async_commit();
+    };
     const int tile = warp < 4 ? warp : 11 - warp;       // a scheduler's two warps see nine tiles of 16 tokens between them
     const int t0 = tile * 16, ra = lane >> 2, ca = (lane & 3) * 2;
-    load_rows<N>(smem, row0 + inner + (g.groups + grp) * N, g.ld_xbc, n);                       // C, and B behind it
-    load_rows<N>(smem + SC * N * 2, row0 + inner + grp * N, g.ld_xbc, n);
+    load_rows<N>(ss, row0 + inner + (g.groups + grp) * N, g.ld_xbc, n);                         // C, and B behind it
+    load_rows<N>(ss + SC * N * 2, row0 + inner + grp * N, g.ld_xbc, n);
+    async_commit();
+    if (warp < h1 - h0) chunk_decays(g, tok0, n, h0 + warp, ds[warp], lh[warp], ll[warp]);      // (runs of up to 8 heads)
+    async_wait();
     __syncthreads();
     uint32_t cf[N / 16][4];
 #pragma unroll
     for (int k = 0; k < N / 16; k++)
-        ldmatrix_x4(cf[k][0], cf[k][1], cf[k][2], cf[k][3], xs + swizzled_offset<SC>(t0 + (lane & 15), k * 16 + ((lane >> 4) << 3)));
+        ldmatrix_x4(cf[k][0], cf[k][1], cf[k][2], cf[k][3], ss + swizzled_offset<SC>(t0 + (lane & 15), k * 16 + ((lane >> 4) << 3)));
     float cb[SC / 8][4] = {};                   // C_t . B_s; a warp's tokens see those up to their own
-    const uint32_t bs = xs + SC * N * 2;
+    const uint32_t bs = ss + SC * N * 2;
 #pragma unroll
     for (int j = 0; j < SC / 16; j++) {
         if (j <= tile) {
@@ -239,13 +263,15 @@ ssd_chunk_out_kernel(SsdArgs g, int run) {
             }
         }
     }
+    __syncthreads();                            // C and B are used up
+    fetch(h0);
     for (int h = h0; h < h1; h++) {
-        __syncthreads();                        // the tiles before are used up
-        load_rows<V>(xt, row0 + h * V, g.ld_xbc, n);
-        const float* from = g.scratch + (ssd_chunk_id(first, b, c) * g.heads + h) * (size_t)(V * N);
+        async_wait();
+        __syncthreads();                        // this head's x and S are there; the parts of the head before are used up
+#pragma unroll
         for (int i = tid; i < V * N / 8; i += SSD_THREADS) {
             const int v = i / (N / 8), e = (i % (N / 8)) * 8;
-            const float4 p = *reinterpret_cast<const float4*>(from + (size_t)v * N + e), q = *reinterpret_cast<const float4*>(from + (size_t)v * N + e + 4);
+            const float4 p = *reinterpret_cast<const float4*>(st + RAW + i * 32), q = *reinterpret_cast<const float4*>(st + RAW + i * 32 + 16);
             uint4 hi, mid, lo;
             parts2(p.x, p.y, hi.x, mid.x, lo.x);
             parts2(p.z, p.w, hi.y, mid.y, lo.y);
@@ -257,6 +283,9 @@ ssd_chunk_out_kernel(SsdArgs g, int run) {
             *reinterpret_cast<uint4*>(to + 2 * PART) = lo;
         }
         __syncthreads();
+        if (h + 1 < h1) fetch(h + 1);           // on its way while this head's outputs are formed
+        const uint32_t xs = x0 + ((h - h0) & 1) * X_BYTES;
+        const unsigned char* xh = xt + ((h - h0) & 1) * X_BYTES;
         const int hh = h - h0;
         // A_t S C_t
         float acc[V / 8][4] = {};
@@ -317,7 +346,7 @@ ssd_chunk_out_kernel(SsdArgs g, int run) {
             for (int r = 0; r < 2; r++) {
                 const int t = ra + 8 * r, v = j * 8 + ca;
                 if (t0 + t < n) {
-                    const uint32_t x = *reinterpret_cast<const uint32_t*>(xt + swizzled_offset<SC>(t0 + t, v));
+                    const uint32_t x = *reinterpret_cast<const uint32_t*>(xh + swizzled_offset<SC>(t0 + t, v));
                     *reinterpret_cast<float2*>(yo + (size_t)t * inner + v) =
                         make_float2(fmaf(skip, __uint_as_float(x << 16), acc[j][2 * r] + low[j][2 * r]),
                                     fmaf(skip, __uint_as_float(x & 0xffff0000u), acc[j][2 * r + 1] + low[j][2 * r + 1]));
@@ -327,8 +356,8 @@ ssd_chunk_out_kernel(SsdArgs g, int run) {
 }
 
 template <int N, int V>
-int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, cudaStream_t stream) {
-    constexpr size_t state_smem = (size_t)SC * N * 2 + SC * 64 * 2, out_smem = std::max<size_t>((size_t)SC * N * 4, (size_t)SC * 64 * 2 + 3 * V * N * 2);
+int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t stream) {
+    constexpr size_t state_smem = (size_t)SC * N * 2 + SC * 64 * 2, out_smem = std::max<size_t>((size_t)SC * N * 4, (size_t)2 * SC * 64 * 2 + V * N * 10);
     static bool configured = false;
     if (!configured) {
         TI_CUDA(cudaFuncSetAttribute(ssd_chunk_state_kernel<N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)state_smem));
@@ -350,7 +379,7 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, cudaStream_t stream
         const double cost = (double)((blocks + 147) / 148) * (1.3 + r);
         if (r == 1 || cost < best) { best = cost; run = r; }
     }
-    TI_CUDA(ti_launch(ssd_chunk_out_kernel<N, V>, dim3(chunks, g.groups * ((per_group + run - 1) / run), n_seq), dim3(SSD_THREADS), out_smem, stream, g, run));
+    TI_CUDA(ti_launch(ssd_chunk_out_kernel<N, V>, dim3(chunks, g.groups * ((per_group + run - 1) / run), n_seq), dim3(SSD_THREADS), out_smem, stream, g, run, M));
     TI_CHECK_LAUNCH("ssd_scan (chunks' outputs)");
     return 0;
 }
@@ -371,6 +400,6 @@ extern "C" int ti_ssd_chunked(const void* xbc, long long ld_xbc, const void* dt_
                (reinterpret_cast<uintptr_t>(y) & 15) == 0, "ssd_scan: rows must start on 16-byte boundaries");
     SsdArgs g{(const bf16*)xbc, ld_xbc, (const bf16*)dt_raw, ld_dt, dt_bias, rate, skip, state, slot_stride, y, cu_new, seq_slot, heads, groups,
               scratch, scratch + (size_t)(M / SC + n_seq) * heads * vdim * N};
-    if (N == 64) return vdim == 32 ? run_ssd_chunks<64, 32>(g, n_seq, max_new, stream) : run_ssd_chunks<64, 64>(g, n_seq, max_new, stream);
-    return vdim == 32 ? run_ssd_chunks<128, 32>(g, n_seq, max_new, stream) : run_ssd_chunks<128, 64>(g, n_seq, max_new, stream);
+    if (N == 64) return vdim == 32 ? run_ssd_chunks<64, 32>(g, n_seq, max_new, M, stream) : run_ssd_chunks<64, 64>(g, n_seq, max_new, M, stream);
+    return vdim == 32 ? run_ssd_chunks<128, 32>(g, n_seq, max_new, M, stream) : run_ssd_chunks<128, 64>(g, n_seq, max_new, M, stream);
 }

@@ -45,11 +45,11 @@ def short_conv(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, state_o
     if act not in ACTS:
         raise KernelError(f"short_conv: unknown activation {act!r}")
     base, stride = _state_part(state, state_offset, (n - 1) * C, "short_conv")
-    out = torch.zeros((M, C), dtype=x.dtype, device=x.device)       # rows that are nobody's stay zero
-    _call(_fn("ti_short_conv", [P, L, P, P, P, I, P, L, P, L, P, P, I, I, I, I, I, P]),
+    out = torch.empty((M, C), dtype=x.dtype, device=x.device)       # (the kernel makes rows that are nobody's zero)
+    _call(_fn("ti_short_conv", [P, L, P, P, P, I, P, L, P, L, P, P, I, I, I, I, I, I, P]),
           _ptr(x), x.stride(0), _ptr(in_bias), _ptr(taps), _ptr(out_bias), ACTS[act], base, stride, _ptr(out), C,
-          _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, C, n, _code(x, "short_conv"), _stream(),
-          launches=2 if (batch.max_new > 64 and n > 1) else 1)
+          _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, C, n, _code(x, "short_conv"), _stream(),
+          launches=2 if (batch.max_new > (16 if n <= 4 else 64) and n > 1) else 1)
     return out
 
 
@@ -124,8 +124,9 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
     _vec(dt_bias, n_decay, "delta_rule: the decay bias")
     _vec(rate, H, "delta_rule: the rates")
     base, stride = _state_part(state, state_offset, H * dim * vdim, "delta_rule")
-    o = torch.zeros((M, H * vdim), dtype=torch.float32, device=q.device)
     chunked = delta_chunked(q, v, batch)
+    # rows that are nobody's are zero (the chunked form's kernels see to it themselves)
+    o = (torch.empty if chunked else torch.zeros)((M, H * vdim), dtype=torch.float32, device=q.device)
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=q.device)
         _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, P]),
@@ -220,8 +221,9 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, rat
     for t, what in ((dt_bias, "step-size bias"), (rate, "rate"), (skip, "skip weight")):
         _vec(t, n_heads, f"ssd_scan: the {what}")
     base, stride = _state_part(state, state_offset, inner * n_state, "ssd_scan")
-    y = torch.zeros((M, inner), dtype=torch.float32, device=xbc.device)         # rows that are nobody's stay zero
     chunked = ssd_chunked(xbc, n_heads, n_state, vdim, batch)
+    # rows that are nobody's are zero (the chunked form's kernels see to it themselves)
+    y = (torch.empty if chunked else torch.zeros)((M, inner), dtype=torch.float32, device=xbc.device)
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=xbc.device)
         _call(_fn("ti_ssd_chunked", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, P, P]),
