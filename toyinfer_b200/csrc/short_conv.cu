@@ -13,9 +13,8 @@
 // chunk gets its state updated by the same block; for longer ones short_conv_tail runs afterwards
 // (other blocks still read the old state while the chunk with the last tokens is at work).
 //
-// short_conv_vec: the same for up to four taps and rows that can be read 16 bytes at a time: a thread owns the channels of one
-// such read and walks 16 tokens, eight rows on their way together.  (A thread a channel waits for memory once a token:
-// 2,048 tokens of 6,144 channels 36 us, now VEC_US.)
+// short_conv_vec: the same for up to four taps and rows that can be read four channels at a time: a thread owns
+// four channels and walks 16 tokens, eight rows on their way together.
 // Rows past the last sequence's are nobody's; they are set to zero.
 #include "common.cuh"
 
@@ -83,7 +82,8 @@ short_conv_vec_kernel(const T* __restrict__ x, long long ldx, const float* __res
                       const float* __restrict__ out_bias, int act, float* __restrict__ state, long long slot_stride,
                       T* __restrict__ out, long long ldo, const int* __restrict__ cu_new, const int* __restrict__ seq_slot, int C, int M) {
     ti_pdl_trigger();
-    constexpr int V = 16 / (int)sizeof(T), AHEAD = 8;
+    constexpr int V = 4, AHEAD = 8;
+    using Run = std::conditional_t<sizeof(T) == 2, uint2, uint4>;       // four channels
     const int c = (blockIdx.y * CONV_THREADS + threadIdx.x) * V;
     if (c >= C) return;
     float w[V][N], ib[V], ob[V];
@@ -98,7 +98,7 @@ short_conv_vec_kernel(const T* __restrict__ x, long long ldx, const float* __res
     x = ti_dependent(x);
     const int b = blockIdx.z;
     if (b == 0 && blockIdx.x == 0)
-        for (int m = cu_new[gridDim.z]; m < M; m++) *reinterpret_cast<uint4*>(out + (size_t)m * ldo + c) = make_uint4(0, 0, 0, 0);
+        for (int m = cu_new[gridDim.z]; m < M; m++) *reinterpret_cast<Run*>(out + (size_t)m * ldo + c) = Run{};
     const int tok0 = cu_new[b], n = cu_new[b + 1] - tok0;
     const int t0 = blockIdx.x * VEC_CHUNK;
     if (t0 >= n) return;
@@ -111,7 +111,7 @@ short_conv_vec_kernel(const T* __restrict__ x, long long ldx, const float* __res
     for (int j = 0; j < N - 1; j++) {
         const int s = t0 - (N - 1 - j);
         if (s >= 0) {
-            const uint4 r = *reinterpret_cast<const uint4*>(xr + ((long long)j - (N - 1)) * ldx);
+            const Run r = *reinterpret_cast<const Run*>(xr + ((long long)j - (N - 1)) * ldx);
 #pragma unroll
             for (int e = 0; e < V; e++) win[j][e] = to_f32(reinterpret_cast<const T*>(&r)[e]) + ib[e];
         } else {
@@ -123,14 +123,14 @@ short_conv_vec_kernel(const T* __restrict__ x, long long ldx, const float* __res
         }
     }
     for (int u0 = 0; u0 < nt; u0 += AHEAD) {
-        uint4 r[AHEAD];
+        Run r[AHEAD];
 #pragma unroll
         for (int u = 0; u < AHEAD; u++)
-            if (u0 + u < nt) r[u] = *reinterpret_cast<const uint4*>(xr + (size_t)(u0 + u) * ldx);
+            if (u0 + u < nt) r[u] = *reinterpret_cast<const Run*>(xr + (size_t)(u0 + u) * ldx);
 #pragma unroll
         for (int u = 0; u < AHEAD; u++) {
             if (u0 + u >= nt) break;
-            uint4 y;
+            Run y;
 #pragma unroll
             for (int e = 0; e < V; e++) {
                 const float cur = to_f32(reinterpret_cast<const T*>(&r[u])[e]) + ib[e];
@@ -138,12 +138,12 @@ short_conv_vec_kernel(const T* __restrict__ x, long long ldx, const float* __res
 #pragma unroll
                 for (int j = 0; j < N - 1; j++) a = fmaf(w[e][j], win[j][e], a);
                 a = fmaf(w[e][N - 1], cur, a);
-                reinterpret_cast<T*>(&y)[e] = from_f32<T>(conv_act(a, act));
+                reinterpret_cast<T*>(&y)[e] = from_f32<T>(act == 1 ? ti_sigmoid_gate<T>(a) : a);
 #pragma unroll
                 for (int j = 0; j + 1 < N - 1; j++) win[j][e] = win[j + 1][e];
                 if constexpr (N > 1) win[N - 2][e] = cur;
             }
-            *reinterpret_cast<uint4*>(out + (size_t)(tok0 + t0 + u0 + u) * ldo + c) = y;
+            *reinterpret_cast<Run*>(out + (size_t)(tok0 + t0 + u0 + u) * ldo + c) = y;
         }
     }
     if (n <= VEC_CHUNK) {
@@ -201,9 +201,10 @@ extern "C" int ti_short_conv(const void* x, long long ldx, const float* in_bias,
     TI_REQUIRE(act == 0 || act == 1, "short_conv: unknown activation %d", act);
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
-        constexpr int V = 16 / (int)sizeof(T);
+        constexpr int V = 4;
         const bool vec = n_taps <= 4 && C % V == 0 && ldx % V == 0 && ldo % V == 0 && slot_stride % 4 == 0 &&
-                         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(state)) & 15) == 0;
+                         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & (V * sizeof(T) - 1)) == 0 &&
+                         (reinterpret_cast<uintptr_t>(state) & 15) == 0;
         const int chunk = vec ? VEC_CHUNK : CONV_CHUNK, per_block = CONV_THREADS * (vec ? V : 1);
         const int chunks = (max_new + chunk - 1) / chunk, groups = (C + per_block - 1) / per_block;
         TI_REQUIRE(groups <= 65535, "short_conv: %d channels are too many for one launch", C);

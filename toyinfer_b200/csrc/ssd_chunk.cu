@@ -99,69 +99,80 @@ __device__ __forceinline__ void load_rows(uint32_t to, const bf16* from, long lo
     }
 }
 
-// U = sum_s a_(128,s) d_s x_s B_s^T of a chunk and head: a block per (chunk, head, sequence); a warp has a run of 16 values of
-// x and its share of N.
+// U = sum_s a_(128,s) d_s x_s B_s^T of a chunk: a block per (chunk, run of heads of one group, sequence); a warp has a run of 16
+// values of x and its share of N.  The heads share B; the next one's x is on its way while one is multiplied.
+constexpr int STATE_RUN = 4;
 template <int N, int V>
-__global__ void __launch_bounds__(SSD_THREADS)
-ssd_chunk_state_kernel(SsdArgs g) {
+__global__ void __launch_bounds__(SSD_THREADS, 2)
+ssd_chunk_state_kernel(SsdArgs g, int run) {
     ti_pdl_trigger();
+    constexpr int X_BYTES = SC * 64 * 2;
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ float ds[SC], lh[SC], ll[SC], w[SC];             // smem: B [SC][N], x [SC][V] (in rows of 64)
-    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ float ds[STATE_RUN][SC], lh[STATE_RUN][SC], ll[STATE_RUN][SC], w[STATE_RUN][SC];   // smem: B [SC][N], x [SC][V] twice (in rows of 64)
+    const int c = blockIdx.x, b = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     ti_pdl_sync();
     g.xbc = ti_dependent(g.xbc); g.dt = ti_dependent(g.dt);
     const int first = g.cu_new[b], tok0 = first + c * SC, n = min(SC, g.cu_new[b + 1] - tok0);
     if (n <= 0) return;
-    const int inner = g.heads * V, grp = h / (g.heads / g.groups);
+    const int inner = g.heads * V, per_group = g.heads / g.groups, runs = (per_group + run - 1) / run;
+    const int grp = blockIdx.y / runs, h0 = grp * per_group + (blockIdx.y - grp * runs) * run, h1 = min(h0 + run, (grp + 1) * per_group);
     const bf16* row0 = g.xbc + (size_t)tok0 * g.ld_xbc;
-    const uint32_t bs = (uint32_t)__cvta_generic_to_shared(smem), xs = bs + SC * N * 2;
+    const uint32_t bs = (uint32_t)__cvta_generic_to_shared(smem), x0 = bs + SC * N * 2;
     load_rows<N>(bs, row0 + inner + grp * N, g.ld_xbc, n);
-    load_rows<V>(xs, row0 + h * V, g.ld_xbc, n);
+    load_rows<V>(x0, row0 + h0 * V, g.ld_xbc, n);
     async_commit();
-    const size_t id = ssd_chunk_id(first, b, c) * g.heads + h;
-    if (warp == 0) {
-        const double all = chunk_decays(g, tok0, n, h, ds, lh, ll);
+    const size_t id0 = ssd_chunk_id(first, b, c) * g.heads;
+    if (warp < h1 - h0) {
+        const double all = chunk_decays(g, tok0, n, h0 + warp, ds[warp], lh[warp], ll[warp]);
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int t = lane * 4 + i;
-            w[t] = ds[t] * exp2f((float)(all - (double)lh[t] - (double)ll[t]));
+            w[warp][t] = ds[warp][t] * exp2f((float)(all - (double)lh[warp][t] - (double)ll[warp][t]));
         }
-        if (lane == 0) g.decay[id] = (float)exp2(all);
+        if (lane == 0) g.decay[id0 + h0 + warp] = (float)exp2(all);
     }
-    async_wait();
-    __syncthreads();
     constexpr int VT = V / 16, NSPLIT = 8 / VT, NT = N / NSPLIT;        // warps side by side along N; columns of N of a warp
     const int v0 = (warp % VT) * 16, n0 = (warp / VT) * NT;
-    float acc[NT / 8][4] = {}, low[NT / 8][4] = {};      // (the small parts in sums of their own: an accumulator is truncated at its own size with every MMA)
-    for (int s0 = 0; s0 < SC; s0 += 16) {
-        if (s0 >= n) break;
-        // x transposed: matrices (v 0-7, s 0-7), (v 8-15, s 0-7), (v 0-7, s 8-15), (v 8-15, s 8-15)
-        uint32_t a[4], hi[4], mid[4], lo[4];
-        ldmatrix_x4_trans(a[0], a[1], a[2], a[3], xs + swizzled_offset<SC>(s0 + (lane & 7) + ((lane >> 4) << 3), v0 + (((lane >> 3) & 1) << 3)));
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int s = s0 + (i >> 1) * 8 + (lane & 3) * 2;
-            parts2(__uint_as_float(a[i] << 16) * w[s], __uint_as_float(a[i] & 0xffff0000u) * w[s + 1], hi[i], mid[i], lo[i]);
+    for (int h = h0; h < h1; h++) {
+        async_wait();
+        __syncthreads();                        // this head's x is there; the other place is no longer read
+        if (h + 1 < h1) {
+            load_rows<V>(x0 + ((h + 1 - h0) & 1) * X_BYTES, row0 + (h + 1) * V, g.ld_xbc, n);
+            async_commit();
         }
+        const uint32_t xs = x0 + ((h - h0) & 1) * X_BYTES;
+        const float* wh = w[h - h0];
+        float acc[NT / 8][4] = {}, low[NT / 8][4] = {};     // (the small parts in sums of their own: an accumulator is truncated at its own size with every MMA)
+        for (int s0 = 0; s0 < SC; s0 += 16) {
+            if (s0 >= n) break;
+            // x transposed: matrices (v 0-7, s 0-7), (v 8-15, s 0-7), (v 0-7, s 8-15), (v 8-15, s 8-15)
+            uint32_t a[4], hi[4], mid[4], lo[4];
+            ldmatrix_x4_trans(a[0], a[1], a[2], a[3], xs + swizzled_offset<SC>(s0 + (lane & 7) + ((lane >> 4) << 3), v0 + (((lane >> 3) & 1) << 3)));
 #pragma unroll
-        for (int j = 0; j < NT; j += 16) {
-            uint32_t q[4];      // B: matrices (s 0-7, n 0-7), (s 8-15, n 0-7), (s 0-7, n 8-15), (s 8-15, n 8-15), transposed on the way
-            ldmatrix_x4_trans(q[0], q[1], q[2], q[3], bs + swizzled_offset<SC>(s0 + (lane & 7) + (((lane >> 3) & 1) << 3), n0 + j + ((lane >> 4) << 3)));
+            for (int i = 0; i < 4; i++) {
+                const float2 ww = *reinterpret_cast<const float2*>(wh + s0 + (i >> 1) * 8 + (lane & 3) * 2);
+                parts2(__uint_as_float(a[i] << 16) * ww.x, __uint_as_float(a[i] & 0xffff0000u) * ww.y, hi[i], mid[i], lo[i]);
+            }
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                mma_bf16(low[j / 8 + u], lo, q[2 * u], q[2 * u + 1]);
-                mma_bf16(low[j / 8 + u], mid, q[2 * u], q[2 * u + 1]);
-                mma_bf16(acc[j / 8 + u], hi, q[2 * u], q[2 * u + 1]);
+            for (int j = 0; j < NT; j += 16) {
+                uint32_t q[4];      // B: matrices (s 0-7, n 0-7), (s 8-15, n 0-7), (s 0-7, n 8-15), (s 8-15, n 8-15), transposed on the way
+                ldmatrix_x4_trans(q[0], q[1], q[2], q[3], bs + swizzled_offset<SC>(s0 + (lane & 7) + (((lane >> 3) & 1) << 3), n0 + j + ((lane >> 4) << 3)));
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    mma_bf16(low[j / 8 + u], lo, q[2 * u], q[2 * u + 1]);
+                    mma_bf16(low[j / 8 + u], mid, q[2 * u], q[2 * u + 1]);
+                    mma_bf16(acc[j / 8 + u], hi, q[2 * u], q[2 * u + 1]);
+                }
             }
         }
-    }
-    float* to = g.scratch + id * (size_t)(V * N);
+        float* to = g.scratch + (id0 + h) * (size_t)(V * N);
 #pragma unroll
-    for (int j = 0; j < NT / 8; j++) {
-        const int v = v0 + (lane >> 2), e = n0 + j * 8 + (lane & 3) * 2;
-        *reinterpret_cast<float2*>(to + (size_t)v * N + e) = make_float2(acc[j][0] + low[j][0], acc[j][1] + low[j][1]);
-        *reinterpret_cast<float2*>(to + (size_t)(v + 8) * N + e) = make_float2(acc[j][2] + low[j][2], acc[j][3] + low[j][3]);
+        for (int j = 0; j < NT / 8; j++) {
+            const int v = v0 + (lane >> 2), e = n0 + j * 8 + (lane & 3) * 2;
+            *reinterpret_cast<float2*>(to + (size_t)v * N + e) = make_float2(acc[j][0] + low[j][0], acc[j][1] + low[j][1]);
+            *reinterpret_cast<float2*>(to + (size_t)(v + 8) * N + e) = make_float2(acc[j][2] + low[j][2], acc[j][3] + low[j][3]);
+        }
     }
 }
 
@@ -357,7 +368,7 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
 
 template <int N, int V>
 int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t stream) {
-    constexpr size_t state_smem = (size_t)SC * N * 2 + SC * 64 * 2, out_smem = std::max<size_t>((size_t)SC * N * 4, (size_t)2 * SC * 64 * 2 + V * N * 10);
+    constexpr size_t state_smem = (size_t)SC * N * 2 + 2 * SC * 64 * 2, out_smem = std::max<size_t>((size_t)SC * N * 4, (size_t)2 * SC * 64 * 2 + V * N * 10);
     static bool configured = false;
     if (!configured) {
         TI_CUDA(cudaFuncSetAttribute(ssd_chunk_state_kernel<N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)state_smem));
@@ -365,13 +376,16 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t
         configured = true;
     }
     const int chunks = (max_new + SC - 1) / SC;
-    TI_CUDA(ti_launch(ssd_chunk_state_kernel<N, V>, dim3(chunks, g.heads, n_seq), dim3(SSD_THREADS), state_smem, stream, g));
+    const int per_group = g.heads / g.groups;
+    int state_run = std::min(STATE_RUN, per_group);       // (heads share B; as long as two blocks an SM are left)
+    while (state_run > 1 && (long long)chunks * n_seq * g.groups * ((per_group + state_run - 1) / state_run) < 200) state_run /= 2;
+    TI_CUDA(ti_launch(ssd_chunk_state_kernel<N, V>, dim3(chunks, g.groups * ((per_group + state_run - 1) / state_run), n_seq), dim3(SSD_THREADS),
+                      state_smem, stream, g, state_run));
     TI_CHECK_LAUNCH("ssd_scan (chunks' parts)");
     TI_CUDA(ti_launch(ssd_chunk_carry_kernel, dim3((V * N / 4 + 255) / 256, g.heads, n_seq), dim3(256), 0, stream, g, V * N));
     TI_CHECK_LAUNCH("ssd_scan (chunks' states)");
     // heads of a block, up to the eight that fit: forming C . B costs a block about as much as a head and a third does, and
     // blocks go round by round, one on an SM
-    const int per_group = g.heads / g.groups;
     int run = 1;
     double best = 0.0;
     for (int r = 1; r <= std::min(8, per_group); r++) {
