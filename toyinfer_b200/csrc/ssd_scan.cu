@@ -15,7 +15,7 @@
 // serves both), whose partial sums of y meet by three shuffles for both columns; B, C, x
 // and the step sizes of a run of 16 tokens are staged in shared memory, the next run's fetched
 // into registers meanwhile (16 bytes a read where the rows allow it).
-// Long prompts are cut into segments that run in parallel (the recurrence is linear in the state
+// Long prompts of bfloat16 tokens go in chunks on the tensor cores (ssd_chunk.cu); others are cut into segments that run in parallel (the recurrence is linear in the state
 // and a segment's decays multiply to one number per head): a first launch finds every segment's own
 // effect on a zero state, a second walks each sequence's segments and leaves every segment's start
 // state, the third runs the recurrence of all segments at once.
