@@ -29,6 +29,8 @@
 #include "common.cuh"
 #include "attn_decode.cuh"
 
+#include <algorithm>
+
 namespace {
 
 struct LatentPages {
@@ -157,6 +159,41 @@ latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* 
     }
     __syncthreads();
     const T* ukh = uk + (size_t)h * plain * rank;
+    if (sizeof(T) == 2 && (rank & 7) == 0 && (reinterpret_cast<uintptr_t>(ukh) & 15) == 0) {
+        // eight elements of a row a read, the rows shared out over as many groups of threads as a row leaves room for; a
+        // group's sums meet in shared memory
+        const int pieces = rank >> 3, lanes = min(pieces, 128), groups = 128 / lanes, grp = t / lanes;
+        float* part = sm + plain;        // [groups][rank]
+        for (int c0 = 0; c0 < pieces; c0 += lanes) {
+            const int c = c0 + t - grp * lanes;
+            if (grp < groups && c < pieces) {
+                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                const int n = (plain - grp + groups - 1) / groups;         // rows grp, grp + groups, ...
+                for (int j0 = 0; j0 < n; j0 += 8) {
+                    uint4 w[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        w[j] = j0 + j < n ? reinterpret_cast<const uint4*>(ukh + (size_t)(grp + (j0 + j) * groups) * rank)[c] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const float qv = j0 + j < n ? qs[grp + (j0 + j) * groups] : 0.f;
+                        const bf16* wv = reinterpret_cast<const bf16*>(&w[j]);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) acc[e] = fmaf(qv, to_f32(wv[e]), acc[e]);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 8; e++) part[grp * rank + c * 8 + e] = acc[e];
+            }
+        }
+        __syncthreads();
+        for (int r = t; r < rank; r += 128) {
+            float x = 0.f;
+            for (int k = 0; k < groups; k++) x += part[k * rank + r];
+            dst[r] = x;
+        }
+        return;
+    }
     for (int r0 = 0; r0 < rank; r0 += 128 * 4) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
@@ -205,9 +242,14 @@ latent_merge_expand_kernel(const float* __restrict__ part_o, const float* __rest
     if (gate) inv *= head_gate(ti_dependent(gate), gate_stride, b, h);      // (the way out is linear)
     for (int e = t; e < rank; e += 128) {
         float acc = 0.f;
-        for (int s = 0; s < n_splits; s++) {
-            const float w = w_s[s];
-            if (w > 0.f) acc = fmaf(w, part_o[(base + s) * rank + e], acc);      // an empty split's numbers were never written
+        for (int s0 = 0; s0 < n_splits; s0 += 8) {      // eight splits' numbers on their way together
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++)          // (an empty split's numbers were never written)
+                x[j] = s0 + j < n_splits && w_s[s0 + j] > 0.f ? part_o[(base + s0 + j) * rank + e] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                if (s0 + j < n_splits) acc = fmaf(w_s[s0 + j], x[j], acc);
         }
         res[e] = acc * inv;
     }
@@ -526,16 +568,30 @@ latent_attn_kernel(const float* __restrict__ qa, const T* __restrict__ lat, floa
 // ---------------------------------------------------------------------------
 // One query per sequence, bfloat16, on the tensor cores (`mma.sync m16n8k16`, float32 accumulation).  A block takes one
 // sequence, 16 * MT heads and one share of the keys, 32 positions at a time: the rows [c | r] of a tile go to shared memory
-// as they are; S = Qa L^T (a warp per 8 keys), the softmax of a row by one thread in 32-bit, P rounded to bfloat16 as the
-// second product's operand, O += P L[:, :rank] (the latent's columns shared out over the warps, a key pair per register
-// fetched as two 16-bit loads).  Unnormalised sums, maxima and denominators go to the merging kernel when the keys are split.
+// as they are; S = Qa L^T (a warp per 8 keys), the softmax in 32-bit where the scores are (a row's maximum meets over the
+// warps in shared memory), P rounded to bfloat16 as the second product's operand, O += P L[:, :rank] (the latent's columns
+// shared out over the warps).  Unnormalised sums, maxima and denominators go to the merging kernel when the keys are split.
 // Rows of a tile outside the query's reach are zeroed: a weight of zero times whatever stood there must stay zero.
-constexpr int DK = 32, D_THREADS = 128;
+//
+// What bounds it: the read of the rows.  A tile is on its way (cp.async) while the one before it is worked off, and two blocks
+// share an SM when 16 heads or fewer share the rows, so some 70 KB are in flight per SM; a tile of 37 KB takes an SM's share of
+// the memory 1,600 cycles, its arithmetic in two blocks about as long.
+constexpr int DK = 32, D_THREADS = 128, P_LD = DK + 8;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ld_matrix4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ld_matrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+template <int MT> size_t decode_mma_smem(int W) {
+    return (size_t)(16 * MT + 2 * DK) * (W + 8) * 2 + (size_t)16 * MT * P_LD * 2 + (size_t)16 * MT * 8 * 4;
 }
 
 template <int MT, int NTW>
@@ -551,19 +607,44 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
     constexpr int ROWS = 16 * MT;
     const int W = rank + rot, LD = W + 8;
     bf16* Qs = reinterpret_cast<bf16*>(smem_raw);                  // [ROWS][LD]
-    bf16* Ls = Qs + ROWS * LD;                                     // [DK][LD]
-    bf16* Ps = Ls + DK * LD;                                       // [ROWS][DK + 8]
-    float* Ss = reinterpret_cast<float*>(Ps + ROWS * (DK + 8));    // [ROWS][DK + 1]
-    float* m_s = Ss + ROWS * (DK + 1);                             // [ROWS] running maximum
-    float* l_s = m_s + ROWS;                                       // [ROWS] running denominator
-    float* a_s = l_s + ROWS;                                       // [ROWS] this tile's rescaling
-    __shared__ const bf16* row_src[DK];
+    bf16* Ls = Qs + ROWS * LD;                                     // [2][DK][LD]
+    bf16* Ps = Ls + 2 * DK * LD;                                   // [ROWS][P_LD]
+    float* mx_s = reinterpret_cast<float*>(Ps + ROWS * P_LD);      // [4][ROWS] the warps' maxima, later their denominators
     const int split = blockIdx.x, h0 = blockIdx.y * ROWS, b = blockIdx.z;
     const int tok = cu_new[b];
     if (cu_new[b + 1] - tok <= 0) return;
     const int qi = seq_start[b], slot = seq_slot[b];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
-    // (global loads in batches, so that several are on their way at a time: a block's four warps cannot hide one each)
+    const int lo = window > 0 ? max(0, qi - window + 1) : 0;
+    const int kt_first = lo / DK, kt_last = qi / DK;
+    const int per = (kt_last - kt_first + n_splits) / n_splits;
+    const int kt_a = kt_first + split * per, kt_b = min(kt_last, kt_a + per - 1);
+    const int n_tiles8 = rank >> 3;
+    // where this thread's row of a tile lives (four threads a row); null: out of the query's reach
+    auto row_of = [&](int kt) -> const bf16* {
+        const int p = kt * DK + (tid >> 2);
+        if (kt > kt_b || p > qi || p < lo) return nullptr;
+        if (p == qi) return lat + (size_t)tok * W;
+        const int row = kv.ring_rows > 0 ? p % kv.ring_rows : p;
+        const int pidx = row / kv.page_size;
+        const int page = pidx < kv.table_width ? kv.page_table[(size_t)slot * kv.table_width + pidx] : -1;
+        return page >= 0 && page < kv.n_pages ? (const bf16*)kv.pages + ((size_t)page * kv.page_size + row % kv.page_size) * W : nullptr;
+    };
+    const uint32_t ls0 = (uint32_t)__cvta_generic_to_shared(Ls), qs0 = (uint32_t)__cvta_generic_to_shared(Qs), ps0 = (uint32_t)__cvta_generic_to_shared(Ps);
+    auto fetch = [&](int kt, const bf16* src) {
+        const uint32_t to = ls0 + (uint32_t)((((kt - kt_a) & 1) * DK + (tid >> 2)) * LD) * 2;
+        const int bytes = src ? 16 : 0;                            // the rest is filled with zeros
+        const bf16* from = src ? src : lat;
+        for (int e = (tid & 3) * 8; e < W; e += 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + e * 2), "l"(src ? from + e : from), "r"(bytes) : "memory");
+    };
+    const bf16* next = nullptr;
+    if (kt_a <= kt_b) {
+        fetch(kt_a, row_of(kt_a));
+        next = row_of(kt_a + 1);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // (global loads in batches, so that several are on their way at a time)
     {
         const int per_row = W >> 2, total = ROWS * per_row;        // pieces of four floats
         for (int i0 = 0; i0 < total; i0 += 6 * D_THREADS) {
@@ -584,11 +665,17 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
             }
         }
     }
-    if (tid < ROWS) {
-        const bool with_sink = sink && split == 0 && h0 + tid < n_heads;
-        m_s[tid] = with_sink ? sink[h0 + tid] : -INFINITY;
-        l_s[tid] = with_sink ? 1.f : 0.f;
-    }
+    // per row g and g + 8 of every 16: the running maximum (the same in all threads of the row) and this thread's share of the denominator
+    float m_run[MT][2], l_run[MT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int h = h0 + mt * 16 + g + 8 * r;
+            const bool with_sink = sink && split == 0 && h < n_heads;
+            m_run[mt][r] = with_sink ? sink[h] : -INFINITY;
+            l_run[mt][r] = with_sink && warp == 0 && t4 == 0 ? 1.f : 0.f;
+        }
     float O[MT][NTW][4];
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
@@ -596,112 +683,111 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
         for (int i = 0; i < NTW; i++)
 #pragma unroll
             for (int c = 0; c < 4; c++) O[mt][i][c] = 0.f;
-    const int lo = window > 0 ? max(0, qi - window + 1) : 0;
-    const int kt_first = lo / DK, kt_last = qi / DK;
-    const int per = (kt_last - kt_first + n_splits) / n_splits;
-    const int kt_a = kt_first + split * per, kt_b = min(kt_last, kt_a + per - 1);
-    const int n_tiles8 = rank >> 3;
     for (int kt = kt_a; kt <= kt_b; kt++) {
-        const int k0 = kt * DK;
-        __syncthreads();
-        if (tid < DK) {              // where each of the tile's rows lives
-            const int p = k0 + tid;
-            const bf16* src = nullptr;
-            if (p == qi) {
-                src = lat + (size_t)tok * W;
-            } else if (p >= lo && p < qi) {
-                const int row = kv.ring_rows > 0 ? p % kv.ring_rows : p;
-                const int pidx = row / kv.page_size;
-                const int page = pidx < kv.table_width ? kv.page_table[(size_t)slot * kv.table_width + pidx] : -1;
-                if (page >= 0 && page < kv.n_pages) src = (const bf16*)kv.pages + ((size_t)page * kv.page_size + row % kv.page_size) * W;
-            }
-            row_src[tid] = src;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                 // this tile is there (at first Qs too); the other place is no longer read
+        if (kt < kt_b) {
+            fetch(kt + 1, next);
+            next = row_of(kt + 2);       // looked up a tile ahead
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const uint32_t ls = ls0 + (uint32_t)(((kt - kt_a) & 1) * DK * LD) * 2;
+        // scores: this warp's 8 keys against all rows, in four chains of sums
+        float c[MT][4][4] = {};
         {
-            const int per_row = W >> 3, total = DK * per_row;          // 16-byte pieces
-            for (int i0 = 0; i0 < total; i0 += 6 * D_THREADS) {
-                uint4 x[6];
+            const uint32_t kaddr = ls + (uint32_t)((warp * 8 + (lane & 7)) * LD + (lane >> 3) * 8) * 2;
+            const uint32_t qaddr = qs0 + (uint32_t)((lane & 15) * LD + (lane >> 4) * 8) * 2;
+            int kk = 0;
+#pragma unroll 2
+            for (; kk + 32 <= W; kk += 32) {
+                uint32_t kb[4];          // two steps of 16
+                ld_matrix4(kb, kaddr + kk * 2);
+                const int ch = (kk >> 5) & 1;
 #pragma unroll
-                for (int u = 0; u < 6; u++) {
-                    const int idx = i0 + u * D_THREADS + tid, rr = idx / per_row, e = idx - rr * per_row;
-                    const bf16* src = idx < total ? row_src[rr] : nullptr;
-                    x[u] = src ? reinterpret_cast<const uint4*>(src)[e] : make_uint4(0u, 0u, 0u, 0u);
+                for (int mt = 0; mt < MT; mt++) {
+                    uint32_t a0[4], a1[4];
+                    ld_matrix4(a0, qaddr + (uint32_t)(mt * 16 * LD + kk) * 2);
+                    ld_matrix4(a1, qaddr + (uint32_t)(mt * 16 * LD + kk + 16) * 2);
+                    if (ch) { mma_bf16_16816(c[mt][2], a0, kb[0], kb[1]); mma_bf16_16816(c[mt][3], a1, kb[2], kb[3]); }
+                    else { mma_bf16_16816(c[mt][0], a0, kb[0], kb[1]); mma_bf16_16816(c[mt][1], a1, kb[2], kb[3]); }
                 }
+            }
+            if (kk < W) {                // sixteen left
+                const bf16* krow = Ls + (size_t)((kt - kt_a) & 1) * DK * LD + (warp * 8 + g) * LD + 2 * t4 + kk;
+                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(krow), b1 = *reinterpret_cast<const uint32_t*>(krow + 8);
 #pragma unroll
-                for (int u = 0; u < 6; u++) {
-                    const int idx = i0 + u * D_THREADS + tid, rr = idx / per_row, e = idx - rr * per_row;
-                    if (idx < total) reinterpret_cast<uint4*>(Ls + rr * LD)[e] = x[u];
+                for (int mt = 0; mt < MT; mt++) {
+                    uint32_t a[4];
+                    ld_matrix4(a, qaddr + (uint32_t)(mt * 16 * LD + kk) * 2);
+                    mma_bf16_16816(c[mt][0], a, b0, b1);
                 }
             }
         }
+        const int p0 = kt * DK + warp * 8 + 2 * t4;
+        const bool in0 = p0 >= lo && p0 <= qi, in1 = p0 + 1 >= lo && p0 + 1 <= qi;
+        float s[MT][2][2];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const bool head_ok = h0 + mt * 16 + g + 8 * r < n_heads;
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const float v = (c[mt][0][2 * r + e] + c[mt][1][2 * r + e]) + (c[mt][2][2 * r + e] + c[mt][3][2 * r + e]);
+                    s[mt][r][e] = head_ok && (e ? in1 : in0) ? v * scale : -INFINITY;
+                }
+                float mx = fmaxf(s[mt][r][0], s[mt][r][1]);
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                if (t4 == 0) mx_s[warp * ROWS + mt * 16 + g + 8 * r] = mx;
+            }
         __syncthreads();
-        // scores: this warp's 8 keys against all rows
+        float alpha[MT][2];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int row = mt * 16 + g + 8 * r;
+                const float m_new = fmaxf(fmaxf(fmaxf(mx_s[row], mx_s[ROWS + row]), fmaxf(mx_s[2 * ROWS + row], mx_s[3 * ROWS + row])), m_run[mt][r]);
+                const bool any = m_new > -INFINITY;
+                alpha[mt][r] = any ? expf(m_run[mt][r] - m_new) : 1.f;
+                const float e0 = s[mt][r][0] == -INFINITY ? 0.f : expf(s[mt][r][0] - m_new);
+                const float e1 = s[mt][r][1] == -INFINITY ? 0.f : expf(s[mt][r][1] - m_new);
+                m_run[mt][r] = m_new;
+                l_run[mt][r] = l_run[mt][r] * alpha[mt][r] + (e0 + e1);
+                const __nv_bfloat162 pk = __floats2bfloat162_rn(e0, e1);
+                *reinterpret_cast<uint32_t*>(Ps + row * P_LD + warp * 8 + 2 * t4) = *reinterpret_cast<const uint32_t*>(&pk);
+            }
+        __syncthreads();
+        // O += P L: a warp has pairs of tiles of 8 columns of the latent, warp, warp + 4, ...
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
-            const bf16* qrow = Qs + (mt * 16 + g) * LD + 2 * t4;
-            const bf16* krow = Ls + (warp * 8 + g) * LD + 2 * t4;
-            for (int kk = 0; kk < W; kk += 16) {
-                uint32_t a[4];
-                a[0] = *reinterpret_cast<const uint32_t*>(qrow + kk);
-                a[1] = *reinterpret_cast<const uint32_t*>(qrow + 8 * LD + kk);
-                a[2] = *reinterpret_cast<const uint32_t*>(qrow + kk + 8);
-                a[3] = *reinterpret_cast<const uint32_t*>(qrow + 8 * LD + kk + 8);
-                mma_bf16_16816(c, a, *reinterpret_cast<const uint32_t*>(krow + kk), *reinterpret_cast<const uint32_t*>(krow + kk + 8));
-            }
-            float* srow = Ss + (mt * 16 + g) * (DK + 1) + warp * 8 + 2 * t4;
-            srow[0] = c[0]; srow[1] = c[1];
-            srow[8 * (DK + 1)] = c[2]; srow[8 * (DK + 1) + 1] = c[3];
-        }
-        __syncthreads();
-        if (tid < ROWS) {
-            const float* srow = Ss + tid * (DK + 1);
-            const bool head_ok = h0 + tid < n_heads;
-            float mx = -INFINITY;
-            for (int j = 0; j < DK; j++) {
-                const int p = k0 + j;
-                if (head_ok && p >= lo && p <= qi) mx = fmaxf(mx, srow[j] * scale);
-            }
-            const float m_old = m_s[tid], m_new = fmaxf(m_old, mx);
-            const float alpha = m_new > -INFINITY ? expf(m_old - m_new) : 1.f;
-            float sum = 0.f;
-            for (int j = 0; j < DK; j++) {
-                const int p = k0 + j;
-                float pr = 0.f;
-                if (head_ok && p >= lo && p <= qi) pr = expf(srow[j] * scale - m_new);
-                sum += pr;
-                Ps[tid * (DK + 8) + j] = from_f32<bf16>(pr);
-            }
-            m_s[tid] = m_new;
-            l_s[tid] = l_s[tid] * alpha + sum;
-            a_s[tid] = alpha;
-        }
-        __syncthreads();
+            if (__any_sync(0xffffffffu, alpha[mt][0] != 1.f || alpha[mt][1] != 1.f)) {
 #pragma unroll
-        for (int mt = 0; mt < MT; mt++) {
-            const float al0 = a_s[mt * 16 + g], al1 = a_s[mt * 16 + g + 8];
-            uint32_t a[2][4];
+                for (int i = 0; i < NTW; i++) {
+                    O[mt][i][0] *= alpha[mt][0]; O[mt][i][1] *= alpha[mt][0]; O[mt][i][2] *= alpha[mt][1]; O[mt][i][3] *= alpha[mt][1];
+                }
+            }
+        }
+        uint32_t a[MT][2][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int ks = 0; ks < 2; ks++)
+                ld_matrix4(a[mt][ks], ps0 + (uint32_t)((mt * 16 + (lane & 15)) * P_LD + ks * 16 + (lane >> 4) * 8) * 2);
+#pragma unroll
+        for (int i = 0; i < NTW; i += 2) {
+            const int nt = 2 * warp + 4 * i;                      // this tile and the next
+            if (nt >= n_tiles8) continue;
+            const int second = nt + 1 < n_tiles8 ? 8 : 0;         // (a latent of an odd number of tiles: the last one twice)
 #pragma unroll
             for (int ks = 0; ks < 2; ks++) {
-                const bf16* prow = Ps + (mt * 16 + g) * (DK + 8) + ks * 16 + 2 * t4;
-                a[ks][0] = *reinterpret_cast<const uint32_t*>(prow);
-                a[ks][1] = *reinterpret_cast<const uint32_t*>(prow + 8 * (DK + 8));
-                a[ks][2] = *reinterpret_cast<const uint32_t*>(prow + 8);
-                a[ks][3] = *reinterpret_cast<const uint32_t*>(prow + 8 * (DK + 8) + 8);
-            }
+                uint32_t q[4];       // (keys 0-7, this tile), (keys 8-15, this), (keys 0-7, next), (keys 8-15, next), transposed on the way
+                ld_matrix4_trans(q, ls + (uint32_t)((ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + nt * 8 + (lane >> 4) * second) * 2);
 #pragma unroll
-            for (int i = 0; i < NTW; i++) {
-                const int nt = warp + 4 * i;
-                if (nt >= n_tiles8) continue;
-                O[mt][i][0] *= al0; O[mt][i][1] *= al0; O[mt][i][2] *= al1; O[mt][i][3] *= al1;
-                const unsigned short* col = reinterpret_cast<const unsigned short*>(Ls) + nt * 8 + g;
-#pragma unroll
-                for (int ks = 0; ks < 2; ks++) {
-                    const int kr = ks * 16 + 2 * t4;
-                    const uint32_t b0 = (uint32_t)col[(size_t)kr * LD] | ((uint32_t)col[(size_t)(kr + 1) * LD] << 16);
-                    const uint32_t b1 = (uint32_t)col[(size_t)(kr + 8) * LD] | ((uint32_t)col[(size_t)(kr + 9) * LD] << 16);
-                    mma_bf16_16816(O[mt][i], a[ks], b0, b1);
+                for (int mt = 0; mt < MT; mt++) {
+                    mma_bf16_16816(O[mt][i], a[mt][ks], q[0], q[1]);
+                    mma_bf16_16816(O[mt][i + 1], a[mt][ks], q[2], q[3]);
                 }
             }
         }
@@ -710,29 +796,29 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
+        for (int r = 0; r < 2; r++) {
+            float l = l_run[mt][r];
+            l += __shfl_xor_sync(0xffffffffu, l, 1);
+            l += __shfl_xor_sync(0xffffffffu, l, 2);
+            if (t4 == 0) mx_s[warp * ROWS + mt * 16 + g + 8 * r] = l;
+        }
+    __syncthreads();
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
         for (int half = 0; half < 2; half++) {
             const int r = mt * 16 + g + 8 * half, h = h0 + r;
             if (h >= n_heads) continue;
-            const float l = l_s[r];
-            if (part_o != nullptr) {
-                const size_t at = ((size_t)tok * n_heads + h) * n_splits + split;
-                if (t4 == 0 && warp == 0) { part_ml[at * 2] = m_s[r]; part_ml[at * 2 + 1] = l; }
+            const float l = (mx_s[r] + mx_s[ROWS + r]) + (mx_s[2 * ROWS + r] + mx_s[3 * ROWS + r]);
+            const size_t at = ((size_t)tok * n_heads + h) * n_splits + split;
+            if (part_o != nullptr && t4 == 0 && warp == 0) { part_ml[at * 2] = m_run[mt][half]; part_ml[at * 2 + 1] = l; }
+            float* dst = part_o != nullptr ? part_o + at * rank : ol + ((size_t)tok * n_heads + h) * rank;
+            const float f = part_o != nullptr ? 1.f : l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
-                for (int i = 0; i < NTW; i++) {
-                    const int nt = warp + 4 * i;
-                    if (nt >= n_tiles8) continue;
-                    float* dst = part_o + at * rank + nt * 8 + 2 * t4;
-                    dst[0] = O[mt][i][2 * half]; dst[1] = O[mt][i][2 * half + 1];
-                }
-            } else {
-                const float inv = l > 0.f ? 1.f / l : 0.f;
-#pragma unroll
-                for (int i = 0; i < NTW; i++) {
-                    const int nt = warp + 4 * i;
-                    if (nt >= n_tiles8) continue;
-                    float* dst = ol + ((size_t)tok * n_heads + h) * rank + nt * 8 + 2 * t4;
-                    dst[0] = O[mt][i][2 * half] * inv; dst[1] = O[mt][i][2 * half + 1] * inv;
-                }
+            for (int i = 0; i < NTW; i++) {
+                const int nt = 2 * warp + 4 * (i & ~1) + (i & 1);
+                if (nt >= n_tiles8) continue;
+                *reinterpret_cast<float2*>(dst + nt * 8 + 2 * t4) = make_float2(O[mt][i][2 * half] * f, O[mt][i][2 * half + 1] * f);
             }
         }
 }
@@ -744,8 +830,8 @@ int launch_decode_mma(const float* qa, const void* lat, float* ol, const int* cu
                       const void* uv = nullptr, void* o = nullptr, long long o_stride = 0, int vdim = 0, const void* gate = nullptr,
                       long long gate_stride = 0) {
     constexpr int ROWS = 16 * MT;
-    const int W = rank + rot, LD = W + 8;
-    const size_t smem = (size_t)(ROWS + DK) * LD * 2 + (size_t)ROWS * (DK + 8) * 2 + ((size_t)ROWS * (DK + 1) + 3 * ROWS) * 4;
+    const int W = rank + rot;
+    const size_t smem = decode_mma_smem<MT>(W);
     static size_t configured = 0;
     if (smem > 48 * 1024 && smem > configured) {
         TI_CUDA(cudaFuncSetAttribute(latent_decode_mma_kernel<MT, NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -861,7 +947,9 @@ extern "C" int ti_latent_prep_absorb(const void* d, long long d_stride, const vo
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
         size_t smem = (size_t)(W + 33) * sizeof(float) + (size_t)W * sizeof(T);
-        if ((size_t)plain * sizeof(float) > smem) smem = (size_t)plain * sizeof(float);
+        // (a head's query and its groups' sums: 128 / (rank / 8) groups of `rank` sums, 1,024 at most, or a row's own)
+        const size_t absorb = (size_t)(plain + std::max(1024, rank)) * sizeof(float);
+        if (absorb > smem) smem = absorb;
         TI_REQUIRE(smem <= 48 * 1024, "latent_prep_absorb: rows of %d elements are too long", W);
         TI_CUDA(ti_launch_class<2>(latent_prep_absorb_kernel<T>, dim3(M, n_heads + 1), dim3(128), smem, stream, (const T*)d, d_stride,
                                    (const T*)q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos, tok_seq,
