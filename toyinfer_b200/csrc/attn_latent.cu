@@ -125,8 +125,10 @@ __global__ void latent_prep_kernel(const T* __restrict__ d, long long d_stride, 
 // For steps of few tokens: the work of latent_prep and latent_absorb in one launch.  Grid (tokens, heads + 1): block
 // (m, h) with h < heads carries head h of token m into the latent space (the rotated part is rotated on the way, q itself
 // stays as it is); block (m, heads) does the token's row.
+constexpr int ABSORB_THREADS = 512;      // rows of Wuk that are on their way together: eight a thread, shared out over the block
+
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(ABSORB_THREADS)
 latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* __restrict__ q, long long q_stride,
                           int n_heads, int plain, int rank, int rot, const float* __restrict__ norm_w, float eps,
                           const float* __restrict__ cos_t, const float* __restrict__ sin_t, int max_pos,
@@ -145,11 +147,11 @@ latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* 
     const int hd = plain + rot, W = rank + rot, half = rot >> 1;
     const T* qh = q + (size_t)m * q_stride + (size_t)h * hd;
     float* qs = sm;                      // [plain]
-    for (int i = t; i < plain; i += 128) qs[i] = to_f32(qh[i]);
+    for (int i = t; i < plain; i += blockDim.x) qs[i] = to_f32(qh[i]);
     float* dst = qa + ((size_t)m * n_heads + h) * W;
     if (rot) {
         const int pos = min(max(tok_pos[m], 0), max_pos - 1);
-        for (int i = t; i < half; i += 128) {
+        for (int i = t; i < half; i += blockDim.x) {
             // (rounded to the engine's type as the rotation in place would have left it)
             const float u = to_f32(qh[plain + i]), v = to_f32(qh[plain + i + half]);
             const float c = cos_t[(size_t)pos * half + i], sn = sin_t[(size_t)pos * half + i];
@@ -162,7 +164,7 @@ latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* 
     if (sizeof(T) == 2 && (rank & 7) == 0 && (reinterpret_cast<uintptr_t>(ukh) & 15) == 0) {
         // eight elements of a row a read, the rows shared out over as many groups of threads as a row leaves room for; a
         // group's sums meet in shared memory
-        const int pieces = rank >> 3, lanes = min(pieces, 128), groups = 128 / lanes, grp = t / lanes;
+        const int pieces = rank >> 3, lanes = min(pieces, (int)blockDim.x), groups = blockDim.x / lanes, grp = t / lanes;
         float* part = sm + plain;        // [groups][rank]
         for (int c0 = 0; c0 < pieces; c0 += lanes) {
             const int c = c0 + t - grp * lanes;
@@ -187,27 +189,27 @@ latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* 
             }
         }
         __syncthreads();
-        for (int r = t; r < rank; r += 128) {
+        for (int r = t; r < rank; r += blockDim.x) {
             float x = 0.f;
             for (int k = 0; k < groups; k++) x += part[k * rank + r];
             dst[r] = x;
         }
         return;
     }
-    for (int r0 = 0; r0 < rank; r0 += 128 * 4) {
+    for (int r0 = 0; r0 < rank; r0 += blockDim.x * 4) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
         for (int dd = 0; dd < plain; dd++) {
             const float qv = qs[dd];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int r = r0 + t + 128 * j;
+                const int r = r0 + t + (int)blockDim.x * j;
                 if (r < rank) acc[j] = fmaf(qv, to_f32(ukh[(size_t)dd * rank + r]), acc[j]);
             }
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int r = r0 + t + 128 * j;
+            const int r = r0 + t + (int)blockDim.x * j;
             if (r < rank) dst[r] = acc[j];
         }
     }
@@ -217,7 +219,7 @@ latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* 
 // the splits' unnormalised sums are weighed and added into the latent result (shared memory), then
 // o[v] = sum_r uv[h, v, r] * result[r], a warp per output element, four elements at a time.
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(512)
 latent_merge_expand_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const T* __restrict__ uv,
                            T* __restrict__ o, long long o_stride, int n_heads, int vdim, int rank, int n_splits,
                            const T* __restrict__ gate, long long gate_stride) {
@@ -240,7 +242,7 @@ latent_merge_expand_kernel(const float* __restrict__ part_o, const float* __rest
     __syncthreads();
     float inv = l > 0.f ? 1.f / l : 0.f;
     if (gate) inv *= head_gate(ti_dependent(gate), gate_stride, b, h);      // (the way out is linear)
-    for (int e = t; e < rank; e += 128) {
+    for (int e = t; e < rank; e += blockDim.x) {
         float acc = 0.f;
         for (int s0 = 0; s0 < n_splits; s0 += 8) {      // eight splits' numbers on their way together
             float x[8];
@@ -254,10 +256,10 @@ latent_merge_expand_kernel(const float* __restrict__ part_o, const float* __rest
         res[e] = acc * inv;
     }
     __syncthreads();
-    const int warp = t >> 5, lane = t & 31;
+    const int warp = t >> 5, lane = t & 31, rows = (blockDim.x >> 5) * 4;
     if (sizeof(T) == 2 && (rank & 7) == 0 && (reinterpret_cast<uintptr_t>(uv) & 15) == 0) {
         // 16-byte pieces of four rows at a time: eight loads on their way per lane
-        for (int v0 = warp * 4; v0 < vdim; v0 += 16) {
+        for (int v0 = warp * 4; v0 < vdim; v0 += rows) {
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
             for (int c = lane; c < (rank >> 3); c += 32) {
                 uint4 w[4];
@@ -279,7 +281,7 @@ latent_merge_expand_kernel(const float* __restrict__ part_o, const float* __rest
         }
         return;
     }
-    for (int v0 = warp * 4; v0 < vdim; v0 += 16) {
+    for (int v0 = warp * 4; v0 < vdim; v0 += rows) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         for (int r = lane; r < rank; r += 32) {
             const float x = res[r];
@@ -843,7 +845,7 @@ int launch_decode_mma(const float* qa, const void* lat, float* ol, const int* cu
     TI_CHECK_LAUNCH("latent_attention (one token, tensor cores)");
     if (uv) {
         const size_t sm2 = (size_t)(rank + 64) * sizeof(float);
-        TI_CUDA(ti_launch_class<4>(latent_merge_expand_kernel<bf16>, dim3(n_tok, n_heads), dim3(128), sm2, stream, (const float*)part_o,
+        TI_CUDA(ti_launch_class<4>(latent_merge_expand_kernel<bf16>, dim3(n_tok, n_heads), dim3(rank > 256 ? 512 : 256), sm2, stream, (const float*)part_o,
                                    (const float*)part_ml, (const bf16*)uv, (bf16*)o, o_stride, n_heads, vdim, rank, n_splits,
                                    (const bf16*)gate, gate_stride));
         TI_CHECK_LAUNCH("latent_merge_expand");
@@ -947,11 +949,11 @@ extern "C" int ti_latent_prep_absorb(const void* d, long long d_stride, const vo
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
         size_t smem = (size_t)(W + 33) * sizeof(float) + (size_t)W * sizeof(T);
-        // (a head's query and its groups' sums: 128 / (rank / 8) groups of `rank` sums, 1,024 at most, or a row's own)
-        const size_t absorb = (size_t)(plain + std::max(1024, rank)) * sizeof(float);
+        // (a head's query and its groups' sums: ABSORB_THREADS / (rank / 8) groups of `rank` sums, or a row's own)
+        const size_t absorb = (size_t)(plain + std::max(8 * ABSORB_THREADS, rank)) * sizeof(float);
         if (absorb > smem) smem = absorb;
         TI_REQUIRE(smem <= 48 * 1024, "latent_prep_absorb: rows of %d elements are too long", W);
-        TI_CUDA(ti_launch_class<2>(latent_prep_absorb_kernel<T>, dim3(M, n_heads + 1), dim3(128), smem, stream, (const T*)d, d_stride,
+        TI_CUDA(ti_launch_class<2>(latent_prep_absorb_kernel<T>, dim3(M, n_heads + 1), dim3(ABSORB_THREADS), smem, stream, (const T*)d, d_stride,
                                    (const T*)q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos, tok_seq,
                                    seq_slot, (T*)lat, kv, (const T*)uk, qa));
         TI_CHECK_LAUNCH("latent_prep_absorb");

@@ -42,6 +42,10 @@ def mix(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, 
         _call(_fn("ti_lightning_chunked", [P, P, P, L, L, L, P, P, P, P, P, P, I, I, I, I, I, I, F, I, P]),
               _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(o), _ptr(state), _ptr(U), _ptr(decay),
               _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, n_chunks, nh, dim, vdim, a, float(k_scale), code, _stream(), launches=3)
+    elif batch.max_new == 1 and dim in (64, 128) and vdim in (64, 128) and state.data_ptr() % 16 == 0:
+        _call(_fn("ti_lightning_step", [P, P, P, L, L, L, P, P, P, P, P, I, I, I, I, I, F, I, P]),
+              _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(o), _ptr(state), _ptr(decay),
+              _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, nh, dim, vdim, a, float(k_scale), code, _stream())
     else:
         _call(_fn("ti_lightning_scan", [P, P, P, L, L, L, P, P, P, P, P, I, I, I, I, I, F, I, P]),
               _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(o), _ptr(state), _ptr(decay),

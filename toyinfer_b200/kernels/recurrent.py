@@ -125,8 +125,15 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
     _vec(rate, H, "delta_rule: the rates")
     base, stride = _state_part(state, state_offset, H * dim * vdim, "delta_rule")
     chunked = delta_chunked(q, v, batch)
-    # rows that are nobody's are zero (the chunked form's kernels see to it themselves)
-    o = (torch.empty if chunked else torch.zeros)((M, H * vdim), dtype=torch.float32, device=q.device)
+    single = batch.max_new == 1 and dim in (64, 128) and vdim in (64, 128) and base % 16 == 0 and stride % 4 == 0
+    # rows that are nobody's are zero (the chunked and the one-token form's kernels see to it themselves)
+    o = (torch.empty if chunked or single else torch.zeros)((M, H * vdim), dtype=torch.float32, device=q.device)
+    if single:
+        _call(_fn("ti_delta_step", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, I, I, I, I, I, I, I, P]),
+              _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(decay_logit), decay_logit.stride(0), 1 if head_decay else 0,
+              _ptr(dt_bias), _ptr(rate), _ptr(beta_logit), beta_logit.stride(0), _ptr(o), base, stride, _ptr(batch.cu_new),
+              _ptr(batch.seq_slot), batch.n_seq, M, H, G, dim, vdim, _code(q, "delta_rule"), _stream())
+        return o
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=q.device)
         _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, P]),
