@@ -7,7 +7,8 @@
 // What bounds it: reading and writing the state, 64 KB a head of 128 x 128.  A block takes a (sequence, head): a thread holds R
 // rows of four columns, all of its reads on their way together, the sums over the rows meet in shared memory (once for
 // lightning, twice for the delta rule), and the delta rule's unit vectors and decays are made by the block itself while the
-// state is on its way, so the step has no kernel before this one.
+// state is on its way, so the step has no kernel before this one.  32 sequences of 16 heads of 128 x 128 (67 MB of state read and
+// written) through lightning attention, us: the scan, a thread a column with its 128 rows one read each, 42; this 17.
 #include "common.cuh"
 
 #include <type_traits>
