@@ -333,12 +333,15 @@ __global__ void moe_combine_kernel(const T* __restrict__ z, T* __restrict__ out,
 __global__ void moe_pad_plan_kernel(const int* __restrict__ perm, const int* __restrict__ off, int n_experts, int P, int top,
                                     int rows, int* __restrict__ pad_src, int* __restrict__ pad_of_pair, int* __restrict__ tile_group) {
     ti_pdl_trigger();
-    extern __shared__ int poff[];        // [n_experts + 1] padded offsets
+    extern __shared__ int poff[];        // [n_experts + 1] padded offsets, then the offsets themselves
+    int* uoff = poff + n_experts + 1;
     ti_pdl_sync();
     perm = ti_dependent(perm); off = ti_dependent(off);
+    for (int e = threadIdx.x; e <= n_experts; e += blockDim.x) uoff[e] = off[e];
+    __syncthreads();
     if (threadIdx.x == 0) {
         int a = 0;
-        for (int e = 0; e < n_experts; e++) { poff[e] = a; a += (off[e + 1] - off[e] + 127) / 128 * 128; }
+        for (int e = 0; e < n_experts; e++) { poff[e] = a; a += (uoff[e + 1] - uoff[e] + 127) / 128 * 128; }
         poff[n_experts] = a;
     }
     for (int i = threadIdx.x; i < rows; i += blockDim.x) pad_src[i] = -1;
@@ -349,13 +352,16 @@ __global__ void moe_pad_plan_kernel(const int* __restrict__ perm, const int* __r
             if (t * 128 >= poff[e] && t * 128 < poff[e + 1]) { g = e; break; }
         tile_group[t] = g;
     }
-    for (int e = 0; e < n_experts; e++) {
-        const int lo = off[e], cnt = off[e + 1] - lo;
-        for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-            const int p = perm[lo + i], at = poff[e] + i;
-            pad_src[at] = p / top;
-            pad_of_pair[p] = at;
+    // (all pairs in one sweep: an expert after another each waited for memory, 16 experts 9 us)
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+        int lo = 0, hi = n_experts;          // the expert whose run holds place i
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (uoff[mid] <= i) lo = mid; else hi = mid;
         }
+        const int p = perm[i], at = poff[lo] + i - uoff[lo];
+        pad_src[at] = p / top;
+        pad_of_pair[p] = at;
     }
 }
 
@@ -531,8 +537,9 @@ extern "C" int ti_moe_pad_plan(const int* perm, const int* off, int n_experts, i
                                int* pad_of_pair, int* tile_group, cudaStream_t stream) {
     if (P == 0) return 0;
     TI_REQUIRE(P > 0 && n_experts > 0 && top > 0 && rows % 128 == 0 && rows >= P + 0, "moe_pad_plan: bad sizes");
-    const size_t smem = (size_t)(n_experts + 1) * sizeof(int);
-    TI_REQUIRE(smem <= 48 * 1024, "moe_pad_plan: %d experts are too many", n_experts);
+    const size_t smem = (size_t)2 * (n_experts + 1) * sizeof(int);
+    TI_REQUIRE(smem <= 96 * 1024, "moe_pad_plan: %d experts are too many", n_experts);
+    if (smem > 48 * 1024) TI_CUDA(cudaFuncSetAttribute(moe_pad_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     TI_CUDA(ti_launch_class<1>(moe_pad_plan_kernel, dim3(1), dim3(1024), smem, stream, perm, off, n_experts, P, top, rows, pad_src,
                                pad_of_pair, tile_group));
     TI_CHECK_LAUNCH("moe_pad_plan");
