@@ -103,7 +103,8 @@ __device__ __forceinline__ int place_among(int* cnt, int e) {
 
 // Routers of up to E experts without runs of experts, E a compile-time bound: a token's logits are read once, into registers,
 // and a pair's place among its expert's is known when it is counted, so that the pairs need no second count.  (One block, as
-// above: 777 tokens, 16 experts, two per token 19 us with the logits read again for every choice, 7 so.)
+// above: 777 tokens, 16 experts, two per token
+// 19 us with the logits read again for every choice, 11 so.)
 // SOFT: weights by softmax (moe_route_softmax), else by sigmoid (moe_route_topk: pair_w the score, pair_w2 its square).
 template <int E, bool SOFT>
 __global__ void __launch_bounds__(RT_THREADS)
