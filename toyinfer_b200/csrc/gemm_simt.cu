@@ -103,6 +103,7 @@ gemm_tile_kernel(const T* __restrict__ X, const T* __restrict__ W, OT* __restric
 // ---------------------------------------------------------------------------
 constexpr int GV_ROWS = 8;       // activation rows per pass
 constexpr int GV_THREADS = 256;
+constexpr int GV_AHEAD = 4;
 
 template <typename T, typename OT, int V>
 __global__ void __launch_bounds__(GV_THREADS)
@@ -122,23 +123,23 @@ gemv_rows_kernel(const T* __restrict__ X, const T* __restrict__ W, OT* __restric
 #pragma unroll
         for (int r = 0; r < GV_ROWS; r++) acc[r] = 0.f;
         const T* wrow = W + (size_t)n * ldw;
-        for (int k = lane * V; k < K; k += 32 * V) {
-            float w[V];
-            if constexpr (V == 1) {
-                w[0] = to_f32(wrow[k]);
-            } else {
-                const Pack pw = *reinterpret_cast<const Pack*>(wrow + k);
+        // GV_AHEAD pieces of the weight row on their way together (one at a time, a warp waited for memory once per 512 bytes)
+        for (int k0 = lane * V; k0 < K; k0 += 32 * V * GV_AHEAD) {
+            Pack pw[GV_AHEAD];
 #pragma unroll
-                for (int j = 0; j < V; j++) w[j] = to_f32(pw.v[j]);
-            }
+            for (int u = 0; u < GV_AHEAD; u++)
+                if (k0 + u * 32 * V < K) pw[u] = *reinterpret_cast<const Pack*>(wrow + k0 + u * 32 * V);
 #pragma unroll
-            for (int r = 0; r < GV_ROWS; r++) {
-                if (r < rows) {
-                    const T* xr = X + (size_t)(mb + r) * ldx + k;
-                    if constexpr (V == 1) {
-                        acc[r] = fmaf(w[0], to_f32(xr[0]), acc[r]);
-                    } else {
-                        const Pack px = *reinterpret_cast<const Pack*>(xr);
+            for (int u = 0; u < GV_AHEAD; u++) {
+                const int k = k0 + u * 32 * V;
+                if (k >= K) break;
+                float w[V];
+#pragma unroll
+                for (int j = 0; j < V; j++) w[j] = to_f32(pw[u].v[j]);
+#pragma unroll
+                for (int r = 0; r < GV_ROWS; r++) {
+                    if (r < rows) {
+                        const Pack px = *reinterpret_cast<const Pack*>(X + (size_t)(mb + r) * ldx + k);
 #pragma unroll
                         for (int j = 0; j < V; j++) acc[r] = fmaf(w[j], to_f32(px.v[j]), acc[r]);
                     }

@@ -584,6 +584,37 @@ __device__ void sort_descending(unsigned long long* w, int n2) {
     }
 }
 
+// The bin of 256 (from the highest down) in which the rem-th word lies: s[0] the bin, s[1] how many of it are taken, s[2] 1 when
+// there are fewer words than asked for, 2 when the bin is taken whole.  By the block's first warp, eight bins a lane (one thread
+// going through them took up to 256 reads of shared memory one after another).
+__device__ __forceinline__ void pick_bin(const int* hist, int rem, int* s) {
+    const int lane = threadIdx.x;
+    if (lane >= 32) return;
+    int n[8], own = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) { n[i] = hist[255 - 8 * lane - i]; own += n[i]; }
+    int upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
+    }
+    const unsigned reached = __ballot_sync(0xffffffffu, upto >= rem);
+    const int who = reached ? __ffs(reached) - 1 : 31;       // none: the lowest bin
+    if (lane != who) return;
+    int above = upto - own, at = 7, in = n[7];
+    bool found = false;
+#pragma unroll
+    for (int i = 0; i < 7; i++)
+        if (!found) {
+            if (above + n[i] >= rem) { found = true; at = i; in = n[i]; }
+            else above += n[i];
+        }
+    s[0] = 255 - 8 * lane - at;
+    s[1] = rem - above;
+    s[2] = above + in < rem ? 1 : in == rem - above ? 2 : 0;
+}
+
 // The k largest of the block's words (EPT per thread in registers, 0 = none, all others distinct):
 // the word of rank k by radix selection, a byte at a time from the top (counts only, so the answer
 // does not depend on the order in which threads run), then every word at or above it goes to
@@ -602,15 +633,7 @@ __device__ void select_largest(const unsigned long long (&w)[EPT], int k, unsign
         for (int e = 0; e < EPT; e++)
             if (w[e] != 0ull && (w[e] & mask) == prefix) atomicAdd(&hist[(int)((w[e] >> (8 * pass)) & 255ull)], 1);
         __syncthreads();
-        if (t == 0) {
-            int above = 0, bin = 255;
-            for (; bin > 0; bin--) {
-                if (above + hist[bin] >= rem) break;
-                above += hist[bin];
-            }
-            s[0] = bin; s[1] = rem - above;
-            s[2] = (above + hist[bin] < rem) ? 1 : (hist[bin] == rem - above ? 2 : 0);      // 1: fewer words than asked for; 2: the bin is taken whole
-        }
+        pick_bin(hist, rem, s);
         __syncthreads();
         prefix |= (unsigned long long)s[0] << (8 * pass);
         rem = s[1];
@@ -647,15 +670,7 @@ __device__ void select_largest_of(const unsigned long long* w, int n, int k, uns
             if (v != 0ull && (v & mask) == prefix) atomicAdd(&hist[(int)((v >> (8 * pass)) & 255ull)], 1);
         }
         __syncthreads();
-        if (t == 0) {
-            int above = 0, bin = 255;
-            for (; bin > 0; bin--) {
-                if (above + hist[bin] >= rem) break;
-                above += hist[bin];
-            }
-            s[0] = bin; s[1] = rem - above;
-            s[2] = (above + hist[bin] < rem) ? 1 : (hist[bin] == rem - above ? 2 : 0);
-        }
+        pick_bin(hist, rem, s);
         __syncthreads();
         prefix |= (unsigned long long)s[0] << (8 * pass);
         rem = s[1];
@@ -680,6 +695,8 @@ __device__ void select_largest_of(const unsigned long long* w, int n, int k, uns
 }
 
 constexpr int K1B = 256;      // threads of the chunk kernel: 16 entries each
+constexpr int FEW_K = 64;     // so many entries of a chunk are found by ranks
+static_assert(FEW_K * CHUNK / K1B <= MAXK && K1B <= 256, "the entries that reach the bound fit the list, the maxima the histogram's room");
 
 // the block's sum of v in a fixed order (threads in order within a warp's tree, warps in order)
 __device__ float block_sum_ordered(float v, float* sm /* 33 entries */) {
@@ -700,7 +717,7 @@ __device__ float block_sum_ordered(float v, float* sm /* 33 entries */) {
 // chunk's maximum m and sum of exp(x - m) (as softmax_chunk_kernel leaves them).
 __global__ void __launch_bounds__(K1B) topk_chunk_kernel(SampleArgs a, int k, int chunks, unsigned long long* cand, float* stats) {
     ti_pdl_trigger();
-    __shared__ int hist[256];
+    __shared__ __align__(16) int hist[256];
     __shared__ int sh[3];
     __shared__ float red[33];
     __shared__ unsigned long long kept[MAXK];
@@ -736,8 +753,54 @@ __global__ void __launch_bounds__(K1B) topk_chunk_kernel(SampleArgs a, int k, in
             stats[((size_t)row * chunks + c) * 2 + 1] = sum;
         }
     }
-    select_largest<CHUNK / K1B>(w, k, kept, hist, sh);
     unsigned long long* out = cand + ((size_t)row * chunks + c) * k;
+    if (k <= FEW_K) {
+        // Few entries: the k-th largest of the threads' own maxima is a bound that at least k entries reach, and few more do.
+        // Ranks by counting, among the maxima and then among the entries that reach the bound; no histogram (whose first byte is
+        // the same for most logits, so that its counts queue for a few words of shared memory).
+        unsigned own = 0;
+#pragma unroll
+        for (int e = 0; e < CHUNK / K1B; e++) own = max(own, (unsigned)(w[e] >> 32));
+        unsigned* key = reinterpret_cast<unsigned*>(hist);
+        int n_keys = K1B;
+        if (k <= 24) {                   // the maxima of four threads each: a quarter of the counting, a few entries more
+            own = max(own, __shfl_xor_sync(0xffffffffu, own, 1));
+            own = max(own, __shfl_xor_sync(0xffffffffu, own, 2));
+            n_keys = K1B / 4;
+            if ((t & 3) == 0) key[t >> 2] = own;
+        } else key[t] = own;
+        if (t == 0) { sh[0] = 0; sh[1] = -1; }
+        __syncthreads();
+        int above = 0;
+        for (int i = 0; i < n_keys; i += 4) {
+            const uint4 o = *reinterpret_cast<const uint4*>(key + i);
+            above += (o.x > own) + (o.y > own) + (o.z > own) + (o.w > own);
+        }
+        const unsigned least = __reduce_min_sync(0xffffffffu, above < k ? own : 0xFFFFFFFFu);
+        if ((t & 31) == 0) atomicMin(reinterpret_cast<unsigned*>(&sh[1]), least);
+        __syncthreads();
+        const unsigned bound = (unsigned)sh[1];
+#pragma unroll
+        for (int e = 0; e < CHUNK / K1B; e++)
+            if (w[e] != 0ull && (unsigned)(w[e] >> 32) >= bound) {
+                const int p = atomicAdd(&sh[0], 1);
+                if (p < MAXK) kept[p] = w[e];
+            }
+        __syncthreads();
+        const int m = sh[0];
+        if (m <= FEW_K * CHUNK / K1B) {          // (more: ties beyond count, left to the histograms)
+            for (int i = t; i < m; i += K1B) {
+                const unsigned long long mine = kept[i];
+                int r = 0;
+                for (int j = 0; j < m; j++) r += kept[j] > mine;
+                if (r < k) out[r] = mine;
+            }
+            for (int i = m + t; i < k; i += K1B) out[i] = 0ull;
+            return;
+        }
+        __syncthreads();
+    }
+    select_largest<CHUNK / K1B>(w, k, kept, hist, sh);
     for (int i = t; i < k; i += K1B) out[i] = kept[i];
 }
 

@@ -36,6 +36,8 @@ SKINNY_SMALL_MAX_WEIGHTS = 8_500_000
 # the tensor cores are at 7.3, 14.4, 19.8 and 95 where the tiled FFMA kernel took 15, 150, 150 and 910; at 500 tokens of
 # 19,456 x 2,560 at 290 (172 TFLOP/s) where it took 2,390.
 F32_TC_MIN_TOKENS = 17
+F32_FEW_ROWS = 8                # tokens that the few-row kernel takes in one pass over the weights; two passes over a matrix
+F32_TC_WEIGHTS = 8_000_000      # of so many weights take longer than the tensor cores' one
 _tickets = {}
 _plans = {}         # (M, N, K, sms) -> (workspace floats, tickets) as ti_linear_tc_plan answers
 _sm_counts = {}
@@ -85,7 +87,8 @@ def tc_eligible(x, w, K, ldx, ldw) -> bool:
 def f32_eligible(x, w, M, K, ldx, ldw) -> bool:
     """Whether the float32 product runs as split bfloat16 parts on the tensor cores (csrc/gemm_f32_split.cu): more tokens
     than the few-row kernel takes, rows on 16-byte boundaries."""
-    return (x.dtype == torch.float32 and w.dtype == torch.float32 and M >= F32_TC_MIN_TOKENS and ldx % 4 == 0
+    enough = M >= F32_TC_MIN_TOKENS or M > F32_FEW_ROWS and w.shape[0] * K >= F32_TC_WEIGHTS and F32_TC_MIN_TOKENS <= 17
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and enough and ldx % 4 == 0
             and ldw % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
