@@ -757,7 +757,8 @@ __global__ void __launch_bounds__(K1B) topk_chunk_kernel(SampleArgs a, int k, in
     if (k <= FEW_K) {
         // Few entries: the k-th largest of the threads' own maxima is a bound that at least k entries reach, and few more do.
         // Ranks by counting, among the maxima and then among the entries that reach the bound; no histogram (whose first byte is
-        // the same for most logits, so that its counts queue for a few words of shared memory).
+        // the same for most logits, so that its counts queue for a few words of shared memory).  64 rows of 151,936 logits, top_k
+        // 20: the kernel 73 us by histograms, 43 so; the merge 26 and 10 with pick_bin.
         unsigned own = 0;
 #pragma unroll
         for (int e = 0; e < CHUNK / K1B; e++) own = max(own, (unsigned)(w[e] >> 32));
