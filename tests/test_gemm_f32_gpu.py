@@ -18,7 +18,7 @@ def K():
 def cuda_cores(K, monkeypatch, fn):
     from toyinfer_b200.kernels import gemm
     with monkeypatch.context() as m:
-        m.setattr(gemm, "F32_TC_MIN_TOKENS", 1 << 30)
+        m.setattr(gemm, "f32_on_tensor_cores", False)
         return fn()
 
 
@@ -31,7 +31,7 @@ def operands(M, N, Kd, positive, pad=0):
 
 # tokens at the edges of tiles of 64, 128 and 256; weight rows and contractions at theirs (256 rows, 32 steps), down to one chunk
 @pytest.mark.parametrize("M,N,Kd", [(17, 8, 8), (63, 255, 33), (64, 256, 32), (65, 257, 64), (128, 512, 100), (129, 40, 2560), (256, 300, 31),
-                                    (257, 1030, 96), (700, 2600, 1000), (40, 2560, 9728), (500, 520, 4)])
+                                    (257, 1030, 96), (700, 2600, 1000), (40, 2560, 9728), (9, 4096, 2048), (500, 520, 4)])
 @pytest.mark.parametrize("positive", [False, True])
 def test_product(K, monkeypatch, M, N, Kd, positive):
     pad = -Kd % 4                          # rows start on 16-byte boundaries whatever the contraction's length

@@ -35,9 +35,11 @@ SKINNY_SMALL_MAX_WEIGHTS = 8_500_000
 # tensor cores: 384 x 96 3.2 / 6.4, 1,024 x 1,024 10.5 / 13.9, 4,096 x 1,024 19.7 / 18.8, 19,456 x 2,560 195 / 92.  At 24 tokens
 # the tensor cores are at 7.3, 14.4, 19.8 and 95 where the tiled FFMA kernel took 15, 150, 150 and 910; at 500 tokens of
 # 19,456 x 2,560 at 290 (172 TFLOP/s) where it took 2,390.
+# ... so it starts at 17 tokens, and at 9 for a matrix of many weights, which the few-row kernel reads twice from there on.
 F32_TC_MIN_TOKENS = 17
-F32_FEW_ROWS = 8                # tokens that the few-row kernel takes in one pass over the weights; two passes over a matrix
-F32_TC_WEIGHTS = 8_000_000      # of so many weights take longer than the tensor cores' one
+F32_TC_MIN_TOKENS_LARGE = 9
+F32_TC_LARGE = 8_000_000
+f32_on_tensor_cores = True      # tests clear this to run the CUDA-core kernels at any size
 _tickets = {}
 _plans = {}         # (M, N, K, sms) -> (workspace floats, tickets) as ti_linear_tc_plan answers
 _sm_counts = {}
@@ -87,8 +89,8 @@ def tc_eligible(x, w, K, ldx, ldw) -> bool:
 def f32_eligible(x, w, M, K, ldx, ldw) -> bool:
     """Whether the float32 product runs as split bfloat16 parts on the tensor cores (csrc/gemm_f32_split.cu): more tokens
     than the few-row kernel takes, rows on 16-byte boundaries."""
-    enough = M >= F32_TC_MIN_TOKENS or M > F32_FEW_ROWS and w.shape[0] * K >= F32_TC_WEIGHTS and F32_TC_MIN_TOKENS <= 17
-    return (x.dtype == torch.float32 and w.dtype == torch.float32 and enough and ldx % 4 == 0
+    least = F32_TC_MIN_TOKENS_LARGE if w.shape[0] * K >= F32_TC_LARGE else F32_TC_MIN_TOKENS
+    return (f32_on_tensor_cores and x.dtype == torch.float32 and w.dtype == torch.float32 and M >= least and ldx % 4 == 0
             and ldw % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
