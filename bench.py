@@ -923,7 +923,7 @@ def run_kernel(name: str, reps: int, eager: bool = False):
             opts = name.split(":")[1].split(",") if ":" in name else []
             T = int(opts[0]) if opts else PREFILL_TOKENS
             if len(opts) > 1:
-                KR.SSD_SEGMENT = int(opts[1])
+                KR.SSD_SEGMENT, KR.SSD_CHUNKED_FROM = int(opts[1]), 1 << 30      # the scan in segments, not in chunks
             heads, vd, N, groups = 64, 64, 128, 8
             inner = heads * vd
             xbc, dt = rnd(T, inner + 2 * groups * N), rnd(T, heads)

@@ -386,6 +386,31 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const T* __res
     }
 }
 
+// The same where rows can be read 16 bytes at a time: a thread holds eight values of its row, read once, gate and weight with them.
+template <typename T>
+__global__ void gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ g, long long g_stride,
+                                         const float* __restrict__ w, T* __restrict__ out, int N, float eps) {
+    ti_pdl_trigger();
+    __shared__ float red[33];
+    const int i = threadIdx.x * 8;
+    const float4 wa = *reinterpret_cast<const float4*>(w + i), wb = *reinterpret_cast<const float4*>(w + i + 4);
+    ti_pdl_sync();
+    o = ti_dependent(o); g = ti_dependent(g);
+    const size_t m = blockIdx.x;
+    struct alignas(16) Run { T v[8]; };
+    const Run gr = *reinterpret_cast<const Run*>(g + m * g_stride + i);
+    const float4 a = *reinterpret_cast<const float4*>(o + m * N + i), b = *reinterpret_cast<const float4*>(o + m * N + i + 4);
+    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, wv[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; e++) ss = fmaf(x[e], x[e], ss);
+    const float inv = rsqrtf(block_sum(ss, red) / (float)N + eps);
+    Run y;
+#pragma unroll
+    for (int e = 0; e < 8; e++) y.v[e] = from_f32<T>(x[e] * inv * wv[e] * ti_sigmoid_gate<T, false>(to_f32(gr.v[e])));
+    *reinterpret_cast<Run*>(out + m * N + i) = y;
+}
+
 template <typename F>
 int dispatch_dim(int dim, F&& f) {
     if (dim <= 32) return f(std::integral_constant<int, 32>());
@@ -467,6 +492,13 @@ extern "C" int ti_gated_rmsnorm(const float* o, const void* g, long long g_strid
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
         const int threads = N <= 256 ? 64 : N <= 1024 ? 128 : 256;
+        const int V = 16 / (int)sizeof(T);
+        if (N % 256 == 0 && N <= 8192 && g_stride % V == 0 &&
+            ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+            TI_CUDA(ti_launch_class<1>(gated_rmsnorm_vec_kernel<T>, dim3(M), dim3(N / 8), 0, stream, o, (const T*)g, g_stride, w, (T*)out, N, eps));
+            TI_CHECK_LAUNCH("gated_rmsnorm");
+            return 0;
+        }
         TI_CUDA(ti_launch_class<1>(gated_rmsnorm_kernel<T>, dim3(M), dim3(threads), 0, stream, o, (const T*)g, g_stride, w, (T*)out, N, eps));
         TI_CHECK_LAUNCH("gated_rmsnorm");
         return 0;
