@@ -314,31 +314,25 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                 tc_commit_pair(&acc_full[buf]);
             }
         } else if (warp_u == 17 && elect_one()) {
-            // TMA producer of this block: its 128 weight rows and BN / 2 tokens of every chunk.  The weights are constant:
-            // the first chunks' are asked for before the kernel before this one has finished.
-            const int pre = (int)min((long long)RAWS, chunks);
+            // TMA producer of this block: its 128 weight rows and BN / 2 tokens of every chunk.  The weights too are asked for after the
+            // wait: a float32 matrix may be the work of the kernel before this one.
+            ti_pdl_sync();
+            SplitWalk walk(total, nk, unit, g.units);
+            SplitPiece p;
+            int it = 0;
             bool ok = true;
-            for (int pass = 0; pass < 2 && ok; pass++) {
-                SplitWalk walk(total, nk, unit, g.units);
-                SplitPiece p;
-                int it = 0;
-                while (ok && walk.next(p)) {
-                    const int tn = p.tile / tiles_m, tm = p.tile - tn * tiles_m;
-                    for (int kc = p.c0; kc < p.c1; kc++, it++) {
-                        const int rs = it % RAWS;
-                        unsigned char* to = raw + (size_t)rs * RAW;
-                        if (pass == 0 && it >= pre) { ok = false; break; }
-                        if (pass == 1 && it >= pre && !mbar_wait(&raw_empty[rs], (uint32_t)(((it / RAWS) & 1) ^ 1))) {
-                            ti_report(status, TI_STATUS_PIPE_WAIT); ok = false; break;
-                        }
-                        if (pass == 0 || it >= pre) {
-                            mbar_expect_tx(&raw_full[rs], RAW);
-                            tma_load_2d(to, &w_map, kc * CHUNK, tn * 2 * WROWS + rank * WROWS, &raw_full[rs]);
-                        }
-                        if (pass == 1) tma_load_2d(to + WROWS * 128, &x_map, kc * CHUNK, tm * BN + rank * (BN / 2), &raw_full[rs]);
+            while (ok && walk.next(p)) {
+                const int tn = p.tile / tiles_m, tm = p.tile - tn * tiles_m;
+                for (int kc = p.c0; kc < p.c1; kc++, it++) {
+                    const int rs = it % RAWS;
+                    unsigned char* to = raw + (size_t)rs * RAW;
+                    if (it >= RAWS && !mbar_wait(&raw_empty[rs], (uint32_t)(((it / RAWS) & 1) ^ 1))) {
+                        ti_report(status, TI_STATUS_PIPE_WAIT); ok = false; break;
                     }
+                    mbar_expect_tx(&raw_full[rs], RAW);
+                    tma_load_2d(to, &w_map, kc * CHUNK, tn * 2 * WROWS + rank * WROWS, &raw_full[rs]);
+                    tma_load_2d(to + WROWS * 128, &x_map, kc * CHUNK, tm * BN + rank * (BN / 2), &raw_full[rs]);
                 }
-                if (pass == 0) { ok = true; ti_pdl_sync(); }
             }
         }
     }
