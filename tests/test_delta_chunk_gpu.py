@@ -85,8 +85,29 @@ def test_against_the_scan(KR, monkeypatch, dtype, head, d, dv, H, G, lens, stron
         off = lambda x: float((x.double() - w).norm() / w.norm())
         assert torch.isfinite(g).all()
         # every write passes two sums of 32-bit products (over the state, then over the chunk's earlier writes) where the scan's
-        # passes one: at most twice as far off (both some 1e-7)
-        assert off(g) <= max(2.0 * off(s), 2e-7), (off(g), off(s))
+        # passes one; these sequences' few elements spread the ratio by a third, test_no_further_off below has more of them
+        assert off(g) <= max(1.35 * off(s), 1.4e-7), (off(g), off(s))
         print(f"{off(g):.2e} against the scan's {off(s):.2e}")
         worst = (g.double() - w).abs().max() / w.abs().max()
         assert worst <= 4e-6, worst
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head", [True, False])
+@pytest.mark.parametrize("d,H,G,lens", [(64, 4, 2, [700]), (128, 2, 2, [700]), (64, 4, 4, [300, 100])])
+def test_no_further_off_than_the_scan(KR, monkeypatch, dtype, head, d, H, G, lens):
+    """q, k and v as they come from their convolution's silu."""
+    off = []
+    for seed in range(8):
+        q, k, v, *rest = make(dtype, head, d, d, H, G, lens, seed, False)
+        args = [torch.nn.functional.silu(t.float()).to(dtype) for t in (q, k, v)] + rest
+        want = exact(*args, lens, head)
+        both = []
+        for least in (KR.DELTA_CHUNKED_FROM, 1 << 30):
+            with monkeypatch.context() as m:
+                m.setattr(KR, "DELTA_CHUNKED_FROM", least)
+                both += [float((g.double() - w).norm() / w.norm()) for g, w in zip(run(KR, args, lens, head), want)]
+        off.append(both)
+    o, S, o_scan, S_scan = torch.tensor(off).mean(0).tolist()
+    print(f"o {o:.2e} against the scan's {o_scan:.2e}, state {S:.2e} against {S_scan:.2e}")
+    assert o <= 1.03 * o_scan and S <= 1.03 * S_scan         # (three hundredths: the spread of eight draws' mean)
