@@ -82,7 +82,28 @@ def test_short_conv(dtype, taps, C, lens):
         out.append((KR.short_conv(strided(x, dtype, extra), w, st, offset, batch, in_bias=ib, out_bias=ob, act="silu"), st[:, offset:offset + (taps - 1) * C]))
     (a, sa), (b, sb) = out
     assert torch.equal(sa, sb) and not a[sum(lens):].any() and not b[sum(lens):].any()
-    if dtype == torch.float32:
-        assert torch.equal(a, b)
-    else:
-        torch.testing.assert_close(a.float(), b.float(), rtol=2.0 ** -7, atol=1e-6)      # one bfloat16 step: another exponential
+    assert torch.equal(a, b)
+
+
+FAR = [-88.5, -88.0, -87.5, -87.0, -40.0, 0.0, 40.0, 88.0]        # exp(-z) up to the end of float32's range
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("extra", [8, 3])
+def test_gates_far_out(dtype, extra):
+    """Whatever form a row takes: the exact quotient, also where exp(-z) is close to the largest float32."""
+    from toyinfer_b200.kernels import lightning as KS, recurrent as KR
+    M, V = 3, 256
+    z = torch.tensor(FAR, device="cuda").repeat(M, V // len(FAR))
+    gate, o, w = strided(z, dtype, extra), rnd(M, V).abs() + 0.1, torch.ones(V, device="cuda")
+    zz = gate.double()
+    silu, sigmoid = zz * torch.sigmoid(zz), torch.sigmoid(zz)
+    rms = lambda x: x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5)
+    near = lambda got, want: torch.testing.assert_close(got.double(), want, rtol=2e-6 if dtype == torch.float32 else 2.0 ** -8, atol=3e-38)
+    near(KR.head_gated_rmsnorm(o, gate, w, 1, 1e-5, gate_act="silu"), rms(o.double()) * silu)
+    near(KR.head_gated_rmsnorm(o, gate, w, 1, 1e-5), rms(o.double()) * sigmoid)
+    near(KR.gate_group_rmsnorm(o, gate, w, 1, 1e-5), rms(o.double() * silu))
+    near(KS.gated_rmsnorm(o, gate, w, 1e-5), rms(o.double()) * sigmoid)
+    cu = torch.tensor([0, M], dtype=torch.int32, device="cuda")
+    batch = SimpleNamespace(cu_new=cu, seq_slot=torch.zeros(1, dtype=torch.int32, device="cuda"), n_seq=1, max_new=M)
+    near(KR.short_conv(gate, torch.ones(V, 1, device="cuda"), torch.zeros(1, 4, device="cuda"), 0, batch, act="silu"), silu)

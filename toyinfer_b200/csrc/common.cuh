@@ -165,13 +165,6 @@ __device__ __forceinline__ float ti_gate_act(float z, int kind) {
     return z / (1.0f + expf(-z));
 }
 
-// z sigmoid(z) (silu) or, with Z false, sigmoid(z), for a result of type T: exact in 32 bits for float32; for one that is rounded
-// to bfloat16 by the fast exponential and quotient, a few units of 2^-23 off (a third of the instructions).
-template <typename T, bool Z = true> __device__ __forceinline__ float ti_sigmoid_gate(float z) {
-    if constexpr (sizeof(T) == 2) return __fdividef(Z ? z : 1.0f, 1.0f + __expf(-z));
-    return (Z ? z : 1.0f) / (1.0f + expf(-z));
-}
-
 // What a gated product stores for its (gate, up) pair.  kind 1 and 2: up * act(gate) as above; kind 3: a clamped gate
 // under a sharpened sigmoid, times the clamped up value plus one: g' = min(gate, limit), u' = clamp(up, -limit, limit),
 // g' sigmoid(1.702 g') (u' + 1).

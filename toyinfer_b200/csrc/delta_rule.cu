@@ -324,7 +324,7 @@ __global__ void head_gated_rmsnorm_vec_kernel(const float* __restrict__ o, const
 #pragma unroll
     for (int e = 0; e < 8; e++) {
         const float gl = to_f32(g[e]);
-        const float ga = gate_silu ? ti_sigmoid_gate<T>(gl) : ti_sigmoid_gate<T, false>(gl);
+        const float ga = (gate_silu ? gl : 1.0f) / (1.0f + expf(-gl));
         y[e] = from_f32<T>(x[e] * inv * (w ? w[i + e] : 1.0f) * ga);
     }
 #pragma unroll

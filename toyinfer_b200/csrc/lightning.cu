@@ -409,7 +409,7 @@ __global__ void gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* _
     const float inv = rsqrtf(block_sum(ss, red) / (float)N + eps);
     Run y;
 #pragma unroll
-    for (int e = 0; e < 8; e++) y.v[e] = from_f32<T>(x[e] * inv * wv[e] * ti_sigmoid_gate<T, false>(to_f32(gr.v[e])));
+    for (int e = 0; e < 8; e++) y.v[e] = from_f32<T>(x[e] * inv * wv[e] * (1.0f / (1.0f + expf(-to_f32(gr.v[e])))));
     *reinterpret_cast<Run*>(out + m * N + i) = y;
 }
 

@@ -139,7 +139,7 @@ short_conv_vec_kernel(const T* __restrict__ x, long long ldx, const float* __res
 #pragma unroll
                 for (int j = 0; j < N - 1; j++) a = fmaf(w[e][j], win[j][e], a);
                 a = fmaf(w[e][N - 1], cur, a);
-                reinterpret_cast<T*>(&y)[e] = from_f32<T>(act == 1 ? ti_sigmoid_gate<T>(a) : a);
+                reinterpret_cast<T*>(&y)[e] = from_f32<T>(conv_act(a, act));
 #pragma unroll
                 for (int j = 0; j + 1 < N - 1; j++) win[j][e] = win[j + 1][e];
                 if constexpr (N > 1) win[N - 2][e] = cur;

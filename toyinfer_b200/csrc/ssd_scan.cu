@@ -322,7 +322,8 @@ __global__ void gate_group_rmsnorm_vec_kernel(const float* __restrict__ y, const
             *reinterpret_cast<uint4*>(reinterpret_cast<char*>(zv) + k) = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(z + (size_t)m * ldz + at) + k);
 #pragma unroll
         for (int e = 0; e < 8; e++) {
-            u[e] = yv[e] * ti_sigmoid_gate<T>(to_f32(zv[e]));
+            const float zi = to_f32(zv[e]);
+            u[e] = yv[e] * (zi / (1.0f + expf(-zi)));
             ss = fmaf(u[e], u[e], ss);
         }
     }
