@@ -81,3 +81,40 @@ def test_rows_off_the_boundary_take_the_other_kernel(K):
     odd = base[1:].view(96, 65)[:, :64]
     odd.copy_(w)
     torch.testing.assert_close(K.linear(x, odd), x @ w.T, rtol=1e-5, atol=4e-6)
+
+
+def microseconds(fn):
+    fn()
+    times = []
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(4):
+            fn()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b) * 250)
+    return min(times)
+
+
+@pytest.mark.parametrize("spoil", ["all nan", "a row nan", "a weight row nan", "all infinite", "a row's end infinite"])
+def test_results_that_are_not_finite_cost_little(K, monkeypatch, spoil):
+    """Activations that have become NaN or infinite: the results of the CUDA cores, at some times the product's usual cost."""
+    x, w = operands(256, 1024, 1024, False)
+    usual = microseconds(lambda: K.linear(x, w))
+    if spoil == "all nan":
+        x[:] = float("nan")
+    elif spoil == "a row nan":
+        x[100] = float("nan")
+    elif spoil == "a weight row nan":
+        w[70] = float("nan")
+    elif spoil == "all infinite":
+        x[:] = float("inf")
+    else:
+        x[255, 1023] = float("-inf")
+    got, want = K.linear(x, w), cuda_cores(K, monkeypatch, lambda: K.linear(x, w))
+    K.check_status()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[want.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    torch.testing.assert_close(got[fine], want[fine], rtol=1e-5, atol=4e-6)
+    assert microseconds(lambda: K.linear(x, w)) < 25 * usual + 100     # (a thread a result: 180 times for NaN throughout)

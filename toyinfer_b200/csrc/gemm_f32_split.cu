@@ -91,16 +91,56 @@ __device__ __forceinline__ void split8(const F8& f, uint4& hi, uint4& mid, uint4
     lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// A result that is not finite: the sum as the CUDA-core kernel forms it (gemm_simt.cu: partial sums of 128).
-__device__ __noinline__ float plain_dot(const SplitArgs& g, int m, int n) {
-    const float* a = g.x + (size_t)m * g.ldx;
-    const float* b = g.w + (size_t)n * g.ldw;
-    float total = 0.f, s = 0.f;
-    for (int k = 0; k < g.K; k++) {
-        s = fmaf(a[k], b[k], s);
-        if (k % 128 == 127) { total += s; s = 0.f; }
+// Whether a row holds a NaN; and a product of two rows by FFMA, which ends as soon as a sum has become one.  By a whole warp.
+__device__ __forceinline__ bool row_has_nan(const float* a, int K) {
+    for (int k0 = 0; k0 < K; k0 += 128) {
+        bool any = false;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = k0 + u * 32 + (threadIdx.x & 31);
+            any |= k < K && isnan(a[k < K ? k : 0]);
+        }
+        if (__any_sync(0xffffffffu, any)) return true;
     }
-    return s + total;
+    return false;
+}
+__device__ __forceinline__ float plain_dot(const float* a, const float* b, int K) {
+    float s = 0.f;
+    for (int k0 = 0; k0 < K; k0 += 128) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = k0 + u * 32 + (threadIdx.x & 31);
+            if (k < K) s = fmaf(a[k], b[k], s);
+        }
+        if (__any_sync(0xffffffffu, isnan(s))) return __int_as_float(0x7fffffff);
+    }
+    return warp_sum(s);
+}
+
+// Results of a warp (lane: weight row n; bit e of `bad`: token m0 + e) that are not finite.  Where an operand's row holds a NaN,
+// so is the result, and the row is looked at once for all of them; the others (infinities, and values that only their
+// bfloat16 parts make infinite) are formed again, a warp a result.  (A thread per result, every step of the contraction one
+// after another, took 4.4 ms where a product of 256 x 1,024 x 1,024 of NaN takes 25 us otherwise.)  Called by whole warps.
+__device__ __noinline__ void redo16(const SplitArgs& g, int m0, int n, unsigned bad, float* v) {
+    const int lane = threadIdx.x & 31;
+    const float nan = __int_as_float(0x7fffffff);
+    for (int e = 0; e < 16; e++) {
+        const unsigned who = __ballot_sync(0xffffffffu, bad >> e & 1u);
+        if (__popc(who) < 2 || !row_has_nan(g.x + (size_t)(m0 + e) * g.ldx, g.K)) continue;
+        if (bad >> e & 1u) v[e] = nan;
+        bad &= ~(1u << e);
+    }
+    for (int l = 0; l < 32; l++) {
+        unsigned left = __shfl_sync(0xffffffffu, bad, l);
+        if (left == 0) continue;
+        const float* w = g.w + (size_t)(n - lane + l) * g.ldw;
+        const bool all = __popc(left) >= 2 && row_has_nan(w, g.K);
+        for (; left != 0; left &= left - 1) {
+            const int e = __ffs(left) - 1;
+            const float s = all ? nan : plain_dot(g.x + (size_t)(m0 + e) * g.ldx, w, g.K);
+            if (lane == l) v[e] = s;
+        }
+    }
 }
 
 // Sixteen results of a thread: tokens m0 .. m0 + 15 of weight row n (lanes are consecutive n); all lanes of a warp call it
@@ -111,13 +151,19 @@ __device__ __noinline__ void store16(const SplitArgs& g, int m0, int n, float4 a
     float probe = 0.f;                  // not a number as soon as one of them is not finite
 #pragma unroll
     for (int e = 0; e < 16; e++) probe = fmaf(v[e], 0.f, probe);
-    if (probe != 0.f && n < g.N) {
-#pragma unroll
-        for (int e = 0; e < 16; e++)
-            if (m0 + e < g.M && !isfinite(v[e])) v[e] = plain_dot(g, m0 + e, n);
-    }
-    __syncwarp();
     const int live = min(16, g.M - m0);
+    if (__any_sync(0xffffffffu, probe != 0.f)) {
+        float again[16];
+        unsigned bad = 0;
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+            again[e] = v[e];
+            if (e < live && n < g.N && !isfinite(v[e])) bad |= 1u << e;
+        }
+        redo16(g, m0, n, bad, again);
+#pragma unroll
+        for (int e = 0; e < 16; e++) v[e] = again[e];
+    }
     if (g.gated >= 1 && g.gated <= 3) {
         float* o = g.out + (size_t)m0 * g.ldo + (n >> 1);
         const bool mine = n < g.N && (n & 1) == 0;
