@@ -118,3 +118,7 @@ def test_results_that_are_not_finite_cost_little(K, monkeypatch, spoil):
     fine = want.isfinite()
     torch.testing.assert_close(got[fine], want[fine], rtol=1e-5, atol=4e-6)
     assert microseconds(lambda: K.linear(x, w)) < 25 * usual + 100     # (a thread a result: 180 times for NaN throughout)
+
+
+def test_no_weight_rows(K):
+    assert K.linear(torch.ones(40, 64, device="cuda"), torch.ones(0, 64, device="cuda")).shape == (40, 0)

@@ -90,7 +90,7 @@ def f32_eligible(x, w, M, K, ldx, ldw) -> bool:
     """Whether the float32 product runs as split bfloat16 parts on the tensor cores (csrc/gemm_f32_split.cu): more tokens
     than the few-row kernel takes, rows on 16-byte boundaries."""
     least = F32_TC_MIN_TOKENS_LARGE if w.shape[0] * K >= F32_TC_LARGE else F32_TC_MIN_TOKENS
-    return (f32_on_tensor_cores and x.dtype == torch.float32 and w.dtype == torch.float32 and M >= least and ldx % 4 == 0
+    return (f32_on_tensor_cores and x.dtype == torch.float32 and w.dtype == torch.float32 and M >= least and w.shape[0] > 0 and ldx % 4 == 0
             and ldw % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
