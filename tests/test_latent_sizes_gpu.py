@@ -1,0 +1,73 @@
+"""Single tokens over a cached latent (csrc/attn_latent.cu, kernels/latent.py) at the edges of what they take, against 64 bits: rows so
+wide that one tile of keys fits beside the queries."""
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+PAGE = 64
+
+
+def layer(dtype, n_heads, plain, rot, rank, vdim, held, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    n, W = len(held), rank + rot
+    need = [-(-(h + 1) // PAGE) for h in held]
+    table = torch.full((n, max(need)), -1, dtype=torch.int32)
+    at = 0
+    for b, k in enumerate(need):
+        table[b, :k] = torch.arange(at, at + k)
+        at += k
+    pages = r(at, 1, PAGE, W).to(dtype)
+    mem = SimpleNamespace(k_pages=pages, page_table=table.cuda(), page_size=PAGE, ring_rows=0, n_kv_heads=1, head_dim=W)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    batch = SimpleNamespace(mode="extend", n_seq=n, n_tok=n, max_new=1, max_pos_after=max(held) + 1, plan_len=max(held) + 1, tok_pos=i32(held),
+                            tok_seq=i32(list(range(n))), seq_slot=i32(list(range(n))), seq_start=i32(held), seq_len=i32([h + 1 for h in held]),
+                            cu_new=i32(list(range(n + 1))))
+    angle = torch.arange(max(held) + 1, device="cuda")[:, None] * 0.01 * torch.arange(1, rot // 2 + 1, device="cuda")[None]
+    tables = (angle.cos().float().contiguous(), angle.sin().float().contiguous(), rot)
+    d, q = r(n, W).to(dtype), (r(n, n_heads, plain + rot) * 0.3).to(dtype)
+    uk, uv = ((r(n_heads * k, rank) * rank ** -0.5).to(dtype) for k in (plain, vdim))
+    return d, q, 1.0 + 0.1 * r(rank), tables, uk, uv, batch, mem
+
+
+def exact(d, q, norm_w, tables, uk, uv, batch, mem, rank, scale):
+    F = torch.float64
+    n, H, hd = q.shape
+    cos, sin, rot = tables
+    plain = hd - rot
+    pos = batch.tok_pos.long()
+    rounded = lambda x: x.to(d.dtype).to(F)                       # what the cache holds and the tensor cores multiply
+
+    def turn(x):
+        u, v = x[..., :rot // 2], x[..., rot // 2:]
+        c, s = (t[pos].to(F).view(n, *([1] * (x.dim() - 2)), rot // 2) for t in (cos, sin))
+        return torch.cat([u * c - v * s, v * c + u * s], -1)
+
+    c = d[:, :rank].to(F)
+    row = rounded(torch.cat([c / torch.sqrt((c * c).mean(-1, keepdim=True) + 1e-6) * norm_w.to(F), turn(d[:, rank:].to(F))], -1))
+    uk, uv = uk.to(F).view(H, plain, rank), uv.to(F).view(H, -1, rank)
+    qa = torch.cat([torch.einsum("nhp,hpr->nhr", q[..., :plain].to(F), uk), rounded(turn(q[..., plain:].to(F)))], -1)
+    out = []
+    for b in range(n):
+        held = int(pos[b])
+        keys = torch.cat([mem.k_pages[mem.page_table[b].clamp(min=0).long()].reshape(-1, row.shape[1])[:held].to(F), row[b:b + 1]])
+        p = torch.softmax(qa[b] @ keys.T * scale, -1)
+        out.append(torch.einsum("hr,hvr->hv", p @ keys[:, :rank], uv).reshape(-1))
+    return torch.stack(out)
+
+
+# rows of 1,200 elements over 20 heads and of 1,456 over 8: one tile; of 1,168: the widest of two
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,plain,rot,rank", [(20, 64, 688, 512), (8, 64, 944, 512), (20, 64, 656, 512), (16, 32, 32, 128)])
+def test_single_tokens(H, plain, rot, rank):
+    from toyinfer_b200.kernels import latent as KL, check_status
+    scale = (plain + rot) ** -0.5
+    d, q, norm_w, tables, uk, uv, batch, mem = layer(torch.bfloat16, H, plain, rot, rank, 48, [0, 31, 32, 200, 1000])
+    want = exact(d, q, norm_w, tables, uk, uv, batch, mem, rank, scale)
+    got = KL.attention_single(d, q, rank, rot, norm_w, 1e-6, tables, uk, uv, 48, scale, 0, None, batch, mem)
+    check_status()
+    # queries in the latent space and softmax weights are rounded to bfloat16 (2^-9 each), the result too
+    assert float((got.double() - want).norm() / want.norm()) < 1e-2

@@ -595,8 +595,8 @@ __device__ __forceinline__ void ld_matrix4_trans(uint32_t (&r)[4], uint32_t addr
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-template <int MT> size_t decode_mma_smem(int W) {
-    return (size_t)(16 * MT + 2 * DK) * (W + 8) * 2 + (size_t)16 * MT * P_LD * 2 + (size_t)16 * MT * 8 * 4;
+template <int MT> size_t decode_mma_smem(int W, int tiles) {
+    return (size_t)(16 * MT + tiles * DK) * (W + 8) * 2 + (size_t)16 * MT * P_LD * 2 + (size_t)16 * MT * 8 * 4;
 }
 
 template <int MT, int NTW>
@@ -604,16 +604,17 @@ __global__ void __launch_bounds__(D_THREADS)
 latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ lat, float* __restrict__ ol,
                          const int* __restrict__ cu_new, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
                          int n_heads, int rank, int rot, float scale, int window, const float* __restrict__ sink,
-                         LatentPages kv, int n_splits, float* __restrict__ part_o, float* __restrict__ part_ml) {
+                         LatentPages kv, int n_splits, float* __restrict__ part_o, float* __restrict__ part_ml, int tiles) {
     ti_pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ti_pdl_sync();
     qa = ti_dependent(qa); lat = ti_dependent(lat);
     constexpr int ROWS = 16 * MT;
+    const int ahead = tiles - 1;                                   // (1, or 0: rows so wide that only one tile of them fits)
     const int W = rank + rot, LD = W + 8;
     bf16* Qs = reinterpret_cast<bf16*>(smem_raw);                  // [ROWS][LD]
-    bf16* Ls = Qs + ROWS * LD;                                     // [2][DK][LD]
-    bf16* Ps = Ls + 2 * DK * LD;                                   // [ROWS][P_LD]
+    bf16* Ls = Qs + ROWS * LD;                                     // [tiles][DK][LD]
+    bf16* Ps = Ls + tiles * DK * LD;                                 // [ROWS][P_LD]
     float* mx_s = reinterpret_cast<float*>(Ps + ROWS * P_LD);      // [4][ROWS] the warps' maxima, later their denominators
     const int split = blockIdx.x, h0 = blockIdx.y * ROWS, b = blockIdx.z;
     const int tok = cu_new[b];
@@ -637,7 +638,7 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
     };
     const uint32_t ls0 = (uint32_t)__cvta_generic_to_shared(Ls), qs0 = (uint32_t)__cvta_generic_to_shared(Qs), ps0 = (uint32_t)__cvta_generic_to_shared(Ps);
     auto fetch = [&](int kt, const bf16* src) {
-        const uint32_t to = ls0 + (uint32_t)((((kt - kt_a) & 1) * DK + (tid >> 2)) * LD) * 2;
+        const uint32_t to = ls0 + (uint32_t)((((kt - kt_a) & ahead) * DK + (tid >> 2)) * LD) * 2;
         const int bytes = src ? 16 : 0;                            // the rest is filled with zeros
         const bf16* from = src ? src : lat;
         for (int e = (tid & 3) * 8; e < W; e += 32)
@@ -691,12 +692,12 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
     for (int kt = kt_a; kt <= kt_b; kt++) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                 // this tile is there (at first Qs too); the other place is no longer read
-        if (kt < kt_b) {
+        if (ahead && kt < kt_b) {
             fetch(kt + 1, next);
             next = row_of(kt + 2);       // looked up a tile ahead
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const uint32_t ls = ls0 + (uint32_t)(((kt - kt_a) & 1) * DK * LD) * 2;
+        const uint32_t ls = ls0 + (uint32_t)(((kt - kt_a) & ahead) * DK * LD) * 2;
         // scores: this warp's 8 keys against all rows, in four chains of sums
         float c[MT][4][4] = {};
         {
@@ -718,7 +719,7 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
                 }
             }
             if (kk < W) {                // sixteen left
-                const bf16* krow = Ls + (size_t)((kt - kt_a) & 1) * DK * LD + (warp * 8 + g) * LD + 2 * t4 + kk;
+                const bf16* krow = Ls + (size_t)((kt - kt_a) & ahead) * DK * LD + (warp * 8 + g) * LD + 2 * t4 + kk;
                 const uint32_t b0 = *reinterpret_cast<const uint32_t*>(krow), b1 = *reinterpret_cast<const uint32_t*>(krow + 8);
 #pragma unroll
                 for (int mt = 0; mt < MT; mt++) {
@@ -796,6 +797,12 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
                 }
             }
         }
+        if (!ahead && kt < kt_b) {
+            __syncthreads();             // the one tile is no longer read
+            fetch(kt + 1, next);
+            next = row_of(kt + 2);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
     }
     __syncthreads();
 #pragma unroll
@@ -836,7 +843,8 @@ int launch_decode_mma(const float* qa, const void* lat, float* ol, const int* cu
                       long long gate_stride = 0) {
     constexpr int ROWS = 16 * MT;
     const int W = rank + rot;
-    const size_t smem = decode_mma_smem<MT>(W);
+    const int tiles = decode_mma_smem<MT>(W, 2) <= 227 * 1024 ? 2 : 1;
+    const size_t smem = decode_mma_smem<MT>(W, tiles);
     static size_t configured = 0;
     if (smem > 48 * 1024 && smem > configured) {
         TI_CUDA(cudaFuncSetAttribute(latent_decode_mma_kernel<MT, NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -844,7 +852,7 @@ int launch_decode_mma(const float* qa, const void* lat, float* ol, const int* cu
     }
     dim3 grid(n_splits, (n_heads + ROWS - 1) / ROWS, n_seq);
     TI_CUDA(ti_launch_class<3>(latent_decode_mma_kernel<MT, NTW>, grid, dim3(D_THREADS), smem, stream, qa, (const bf16*)lat, ol, cu_new,
-                               seq_start, seq_slot, n_heads, rank, rot, scale, window, sink, kv, n_splits, part_o, part_ml));
+                               seq_start, seq_slot, n_heads, rank, rot, scale, window, sink, kv, n_splits, part_o, part_ml, tiles));
     TI_CHECK_LAUNCH("latent_attention (one token, tensor cores)");
     if (uv) {
         const size_t sm2 = (size_t)(rank + 64) * sizeof(float);
