@@ -1,5 +1,5 @@
 """Single tokens over a cached latent (csrc/attn_latent.cu, kernels/latent.py) at the edges of what they take, against 64 bits: rows so
-wide that one tile of keys fits beside the queries."""
+wide that one tile of keys fits beside the queries, and long heads."""
 from __future__ import annotations
 
 from types import SimpleNamespace
@@ -59,9 +59,9 @@ def exact(d, q, norm_w, tables, uk, uv, batch, mem, rank, scale):
     return torch.stack(out)
 
 
-# rows of 1,200 elements over 20 heads and of 1,456 over 8: one tile; of 1,168: the widest of two
+# rows of 1,200 elements over 20 heads and of 1,456 over 8: one tile; of 1,168: the widest of two; a head of 9,000 unrotated elements
 @pytest.mark.gpu
-@pytest.mark.parametrize("H,plain,rot,rank", [(20, 64, 688, 512), (8, 64, 944, 512), (20, 64, 656, 512), (16, 32, 32, 128)])
+@pytest.mark.parametrize("H,plain,rot,rank", [(20, 64, 688, 512), (8, 64, 944, 512), (20, 64, 656, 512), (16, 32, 32, 128), (1, 9000, 32, 64)])
 def test_single_tokens(H, plain, rot, rank):
     from toyinfer_b200.kernels import latent as KL, check_status
     scale = (plain + rot) ** -0.5

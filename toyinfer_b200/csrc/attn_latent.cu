@@ -959,11 +959,11 @@ extern "C" int ti_latent_prep_absorb(const void* d, long long d_stride, const vo
     const int W = rank + rot;
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
-        size_t smem = (size_t)(W + 33) * sizeof(float) + (size_t)W * sizeof(T);
+        const size_t row = (size_t)(W + 33) * sizeof(float) + (size_t)W * sizeof(T);
+        TI_REQUIRE(row <= 48 * 1024 && (size_t)plain * sizeof(float) <= 48 * 1024, "latent_prep_absorb: rows of %d elements are too long", W);
         // (a head's query and its groups' sums: ABSORB_THREADS / (rank / 8) groups of `rank` sums, or a row's own)
-        const size_t absorb = (size_t)(plain + std::max(8 * ABSORB_THREADS, rank)) * sizeof(float);
-        if (absorb > smem) smem = absorb;
-        TI_REQUIRE(smem <= 48 * 1024, "latent_prep_absorb: rows of %d elements are too long", W);
+        const size_t smem = std::max(row, (size_t)(plain + std::max(8 * ABSORB_THREADS, rank)) * sizeof(float));
+        if (smem > 48 * 1024) TI_CUDA(cudaFuncSetAttribute(latent_prep_absorb_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         TI_CUDA(ti_launch_class<2>(latent_prep_absorb_kernel<T>, dim3(M, n_heads + 1), dim3(ABSORB_THREADS), smem, stream, (const T*)d, d_stride,
                                    (const T*)q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos, tok_seq,
                                    seq_slot, (T*)lat, kv, (const T*)uk, qa));
