@@ -1,5 +1,5 @@
 """Single tokens over a cached latent (csrc/attn_latent.cu, kernels/latent.py) at the edges of what they take, against 64 bits: rows so
-wide that one tile of keys fits beside the queries, and long heads."""
+wide that one tile of keys fits beside the queries, long heads, float32 at its own number of splits.  And that number's rule."""
 from __future__ import annotations
 
 from types import SimpleNamespace
@@ -8,6 +8,20 @@ import pytest
 import torch
 
 PAGE = 64
+
+
+def test_float32_rows_take_a_second_round_only_where_tiles_are_left():
+    from toyinfer_b200.kernels.latent import decode_splits as splits
+    assert splits(4, 8, 8, 2000, 148) == 64                       # tensor cores: all blocks run at once
+    assert splits(4, 8, 8, 2000, 148, 576) == 37                  # one block an SM; a second round would leave a tile each
+    assert splits(16, 8, 8, 2000, 148, 576) == 16 and splits(16, 8, 8, 2000, 148, 288) == 18
+    assert splits(64, 16, 16, 2000, 148, 576) == 4
+    for n in (1, 3, 16, 64, 500):
+        for heads, hb in ((8, 8), (16, 16), (32, 32), (40, 32)):
+            for span in (1, 31, 200, 4000, 100000):
+                for row in (64, 424, 425, 576, 890):
+                    one = max(1, min(148 // (n * -(-heads // hb)), span // 32 + 2, 64))
+                    assert one <= splits(n, heads, hb, span, 148, row) <= splits(n, heads, hb, span, 148)
 
 
 def layer(dtype, n_heads, plain, rot, rank, vdim, held, seed=0):
@@ -71,3 +85,16 @@ def test_single_tokens(H, plain, rot, rank):
     check_status()
     # queries in the latent space and softmax weights are rounded to bfloat16 (2^-9 each), the result too
     assert float((got.double() - want).norm() / want.norm()) < 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,H,rank,rot", [(4, 8, 512, 64), (16, 8, 256, 32), (20, 16, 512, 64), (1, 3, 64, 16)])
+def test_float32_single_tokens(n, H, rank, rot):
+    from toyinfer_b200.kernels import latent as KL
+    scale = (64 + rot) ** -0.5
+    held = [(i * 613) % 1900 for i in range(n)]
+    d, q, norm_w, tables, uk, uv, batch, mem = layer(torch.float32, H, 64, rot, rank, 64, held)
+    want = exact(d, q, norm_w, tables, uk, uv, batch, mem, rank, scale)
+    lat = KL.prep(d, q, rank, rot, norm_w, 1e-6, tables, batch, mem)
+    got = KL.attention(q, lat, uk, uv, 64, rank, rot, scale, 0, None, batch, mem)
+    assert float((got.double() - want).norm() / want.norm()) < 2e-6      # sums of some 600 products and of 2,000 positions in 32 bits

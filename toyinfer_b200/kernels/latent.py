@@ -79,20 +79,35 @@ def heads_per_block(n_heads: int, one_token_each: bool) -> int:
     return hb
 
 
-def decode_splits(n_seq: int, n_heads: int, hb: int, span: int, sms: int) -> int:
-    """Blocks that share a sequence's keys when every sequence brings one query: as many as run at once in all, two per SM
-    where 16 heads or fewer share a block (its rows leave room for two), else one; a tile of 32 keys each at least, 64 at
-    most (every split costs the merging kernel a row of partial sums)."""
+def decode_splits(n_seq: int, n_heads: int, hb: int, span: int, sms: int, simt_row: int = 0) -> int:
+    """Blocks that share a sequence's keys when every sequence brings one query; a tile of 32 keys each at least, 64 at most
+    (every split costs the merging kernel a row of partial sums).  The tensor-core kernel: as many as run at once in all, two per
+    SM where 16 heads or fewer share a block (its rows leave room for two), else one.  The CUDA-core kernel (``simt_row``
+    elements a row) keeps 64 rows as float32: two blocks an SM up to 424 elements, beyond them one, and then a second round, whose
+    unequal ends even out, only where a block has four tiles left at least.  float32 layers of single tokens, us, one per SM / two
+    / by this rule, sequences x heads, positions, rows: 4 x 8, 500 to 2,000, 576 224 / 240 / 224; 16 x 8, the same 602 / 538 / 513;
+    16 x 16, 1,000 to 4,000, 576 1,573 / 1,407 / 1,406; 6 x 8, 400 to 1,500, 544 215 / 245 / 215; 16 x 8, 500 to 2,000, 288 325 / 229
+    / 229."""
     tiles = span // 32 + 2
     groups = (n_heads + hb - 1) // hb
-    return max(1, min((2 if hb <= 16 else 1) * sms // max(1, n_seq * groups), tiles, 64))
+    one = min(sms // max(1, n_seq * groups), tiles, 64)
+    two = min(2 * sms // max(1, n_seq * groups), tiles, 64) if hb <= 16 else one
+    if simt_row > 424:
+        two = max(one, min(two, tiles // 4))
+    return max(1, two)
 
 
-def plan(n_seq: int, n_heads: int, window: int, plan_len: int, device) -> int:
+def tensor_core_single(dtype, rank: int, rot: int, *tensors) -> bool:
+    """Whether a step of single tokens runs on the tensor cores (csrc/attn_latent.cu): bfloat16, sizes and rows that it takes."""
+    return (dtype == torch.bfloat16 and (rank + rot) % 16 == 0 and rank % 8 == 0 and rank <= 512
+            and all(t.dtype == torch.bfloat16 and t.data_ptr() % 16 == 0 for t in tensors))
+
+
+def plan(n_seq: int, n_heads: int, window: int, plan_len: int, device, simt_row: int = 0) -> int:
     """The splits of a step of single tokens planned for ``plan_len`` positions (what of its launches depends on the length)."""
     from .gemm import sm_count
     span = plan_len if window <= 0 else min(plan_len, window)
-    return decode_splits(n_seq, n_heads, heads_per_block(n_heads, True), span, sm_count(device))
+    return decode_splits(n_seq, n_heads, heads_per_block(n_heads, True), span, sm_count(device), simt_row)
 
 
 def _gate(gate: Optional[torch.Tensor], M: int, n_heads: int, dtype, what: str):
@@ -143,8 +158,7 @@ def prompt_eligible(q: torch.Tensor, lat: torch.Tensor, rank: int, rot: int, vdi
 
 def single_eligible(q: torch.Tensor, rank: int, rot: int, batch, mem) -> bool:
     """Whether attention_single takes this step: every sequence one token, bfloat16, sizes the tensor-core kernel takes."""
-    return (batch.mode == "extend" and q.dtype == torch.bfloat16 and (rank + rot) % 16 == 0 and rank % 8 == 0 and rank <= 512
-            and mem.k_pages.dtype == torch.bfloat16 and mem.k_pages.data_ptr() % 16 == 0)
+    return batch.mode == "extend" and tensor_core_single(q.dtype, rank, rot, mem.k_pages)
 
 
 def attention_single(d: torch.Tensor, q: torch.Tensor, rank: int, rot: int, norm_w: torch.Tensor, eps: float, tables,
@@ -206,7 +220,7 @@ def attention(q: torch.Tensor, lat: torch.Tensor, uk: torch.Tensor, uv: torch.Te
     hb = heads_per_block(nh, batch.mode == "extend")
     splits, part_o, part_ml = 1, None, None
     if batch.mode == "extend":
-        splits = plan(batch.n_seq, nh, window, batch.plan_len, q.device)
+        splits = plan(batch.n_seq, nh, window, batch.plan_len, q.device, 0 if tensor_core_single(q.dtype, rank, rot, lat, mem.k_pages) else W)
         if splits > 1:
             part_o = torch.empty((M, nh, splits, rank), dtype=torch.float32, device=q.device)
             part_ml = torch.empty((M, nh, splits, 2), dtype=torch.float32, device=q.device)

@@ -132,7 +132,8 @@ class LatentAttention(Mixer):
         return KVRequest(1, self.rank + self.rot, self.window, values=False)
 
     def launch_plan(self, n_seq: int, plan_len: int, dtype, device, n_live=None):
-        return ("latent", KL.plan(n_seq, self.n_heads, self.window, plan_len, device))    # the split of a sequence's keys over blocks
+        row = 0 if KL.tensor_core_single(dtype, self.rank, self.rot) else self.rank + self.rot
+        return ("latent", KL.plan(n_seq, self.n_heads, self.window, plan_len, device, row))    # the split of a sequence's keys over blocks
 
     def forward(self, x, batch, mem, shared) -> torch.Tensor:
         if mem is None or not hasattr(mem, "k_pages"):
