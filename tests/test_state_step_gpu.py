@@ -80,3 +80,24 @@ def test_delta(dtype, d, dv, H, G, n, head):
     close(out[0][0][:n], out[1][0][:n], o)
     close(out[0][1][at, 4:].view(S.shape), out[1][1][at, 4:].view(S.shape), S)
     assert not out[0][0][n:].any() and torch.equal(out[0][1][:, :4], state[:, :4])
+
+
+@pytest.mark.parametrize("longest", [0, 1, 100])
+def test_a_step_of_no_sequences(longest):
+    """Rows that are nobody's are zero though no kernel runs."""
+    from toyinfer_b200.kernels import recurrent as KR
+    batch = SimpleNamespace(cu_new=torch.zeros(1, dtype=torch.int32, device="cuda"), seq_slot=torch.zeros(0, dtype=torch.int32, device="cuda"),
+                            n_seq=0, n_tok=0, max_new=longest)
+    r = rnd(1)
+    state = torch.zeros(2, 2 * 64 * 64, device="cuda")
+
+    def call(fn, shape, dtype):
+        poison = torch.full(shape, float("nan"), dtype=dtype, device="cuda")       # what the result's memory holds before
+        del poison
+        y = fn()
+        assert y.shape == shape and not y.any()
+
+    call(lambda: KR.short_conv(r(5, 128).to(torch.bfloat16), r(128, 4), state, 0, batch), (5, 128), torch.bfloat16)
+    call(lambda: KR.delta_rule(r(5, 2, 64), r(5, 2, 64), r(5, 2, 64), r(5, 2), r(2), r(2), r(5, 2), state, 0, batch, head_decay=True), (5, 128), torch.float32)
+    call(lambda: KR.ssd_scan(r(5, 128 + 128).to(torch.bfloat16), r(5, 2).to(torch.bfloat16), r(2), r(2), None, 2, 1, 64, 64, state, 0, batch), (5, 128),
+         torch.float32)

@@ -45,7 +45,8 @@ def short_conv(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, state_o
     if act not in ACTS:
         raise KernelError(f"short_conv: unknown activation {act!r}")
     base, stride = _state_part(state, state_offset, (n - 1) * C, "short_conv")
-    out = torch.empty((M, C), dtype=x.dtype, device=x.device)       # (the kernel makes rows that are nobody's zero)
+    # rows that are nobody's are zero: the kernel sees to it where a sequence brings tokens
+    out = (torch.empty if batch.n_seq and batch.max_new else torch.zeros)((M, C), dtype=x.dtype, device=x.device)
     _call(_fn("ti_short_conv", [P, L, P, P, P, I, P, L, P, L, P, P, I, I, I, I, I, I, P]),
           _ptr(x), x.stride(0), _ptr(in_bias), _ptr(taps), _ptr(out_bias), ACTS[act], base, stride, _ptr(out), C,
           _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, C, n, _code(x, "short_conv"), _stream(),
@@ -93,7 +94,7 @@ def delta_chunked(q: torch.Tensor, v: torch.Tensor, batch) -> int:
     """Floats of scratch with which a step's delta rule runs in chunks, or 0: it goes token by token."""
     M, G, dim = q.shape
     H, vdim = v.shape[1], v.shape[2]
-    if batch.max_new < DELTA_CHUNKED_FROM or dim not in (64, 128) or vdim % 16:
+    if batch.n_seq == 0 or batch.max_new < DELTA_CHUNKED_FROM or dim not in (64, 128) or vdim % 16:
         return 0
     need = (M // 32 + batch.n_seq) * H * _fn("ti_delta_chunk_floats", [I, I])(dim, vdim)
     return need if 4 * need <= DELTA_CHUNK_SCRATCH else 0
@@ -125,7 +126,7 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
     _vec(rate, H, "delta_rule: the rates")
     base, stride = _state_part(state, state_offset, H * dim * vdim, "delta_rule")
     chunked = delta_chunked(q, v, batch)
-    single = batch.max_new == 1 and dim in (64, 128) and vdim in (64, 128) and base % 16 == 0 and stride % 4 == 0
+    single = batch.n_seq > 0 and batch.max_new == 1 and dim in (64, 128) and vdim in (64, 128) and base % 16 == 0 and stride % 4 == 0
     # rows that are nobody's are zero (the chunked and the one-token form's kernels see to it themselves)
     o = (torch.empty if chunked or single else torch.zeros)((M, H * vdim), dtype=torch.float32, device=q.device)
     if single:
@@ -204,7 +205,7 @@ SSD_CHUNK_SCRATCH = 1 << 30     # ... while the chunks' states take no more byte
 
 def ssd_chunked(xbc: torch.Tensor, n_heads: int, n_state: int, vdim: int, batch) -> int:
     """Floats of scratch with which a step's Mamba-2 recurrence runs in chunks (csrc/ssd_chunk.cu), or 0: token by token."""
-    if (batch.max_new < SSD_CHUNKED_FROM or xbc.dtype != torch.bfloat16 or n_state not in (64, 128) or vdim not in (32, 64)
+    if (batch.n_seq == 0 or batch.max_new < SSD_CHUNKED_FROM or xbc.dtype != torch.bfloat16 or n_state not in (64, 128) or vdim not in (32, 64)
             or xbc.stride(0) % 8 or xbc.data_ptr() % 16):
         return 0
     need = (xbc.shape[0] // 128 + batch.n_seq) * n_heads * (vdim * n_state + 1)
