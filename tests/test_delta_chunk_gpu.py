@@ -111,3 +111,21 @@ def test_no_further_off_than_the_scan(KR, monkeypatch, dtype, head, d, H, G, len
     o, S, o_scan, S_scan = torch.tensor(off).mean(0).tolist()
     print(f"o {o:.2e} against the scan's {o_scan:.2e}, state {S:.2e} against {S_scan:.2e}")
     assert o <= 1.03 * o_scan and S <= 1.03 * S_scan         # (three hundredths: the spread of eight draws' mean)
+
+
+@pytest.mark.parametrize("head", [True, False])
+@pytest.mark.parametrize("lens", [[0, 40, 0, 70], [50, 0]])
+def test_empty_sequences_and_rows_that_are_nobodys(KR, head, lens):
+    args = make(torch.float32, head, 64, 64, 2, 2, lens, 5, False)
+    q, k, v, decay, dt, rate, beta, state = args
+    wide = lambda t: torch.cat([t, torch.ones(3, *t.shape[1:], device="cuda")])
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32)
+    batch = SimpleNamespace(cu_new=cu, seq_slot=torch.arange(len(lens), dtype=torch.int32, device="cuda"), n_seq=len(lens), max_new=max(lens))
+    store = state.reshape(len(lens), -1).clone()
+    poison = torch.full((sum(lens) + 3, 128), float("nan"), device="cuda")       # what the result's memory holds before
+    del poison
+    o = KR.delta_rule(wide(q), wide(k), wide(v), wide(decay), dt, rate, wide(beta), store, 0, batch, head_decay=head)
+    want, left = exact(*args, lens, head)
+    assert not o[sum(lens):].any()
+    assert float((o[:sum(lens)].view(want.shape).double() - want).norm() / want.norm()) < 1e-6
+    assert float((store.view(left.shape).double() - left).norm() / left.norm()) < 1e-6

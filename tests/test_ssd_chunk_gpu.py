@@ -106,3 +106,22 @@ def test_no_further_off_than_the_scan(KR, monkeypatch, H, G, N, V, lens, kind):
     # each, so that outputs of one sign lose 8.6e-8 at most.  Else no further off than the scan (a tenth for six draws' spread).
     slack = 0.0 if kind == "silu" else 4e-8
     assert y <= 1.1 * y_scan + slack and S <= 1.1 * S_scan
+
+
+@pytest.mark.parametrize("lens", [[0, 90, 0, 130], [100, 0]])
+def test_empty_sequences_and_rows_that_are_nobodys(KR, lens):
+    args = make(4, 2, 64, 32, lens, 7)
+    xbc, dt, bias, rate, skip, state = args
+    M, H, N, V = sum(lens) + 3, 4, 64, 32
+    wide = lambda t: torch.cat([t, torch.ones(3, t.shape[1], dtype=t.dtype, device="cuda")])
+    xbc, dt = wide(xbc), wide(dt)
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32)
+    batch = SimpleNamespace(cu_new=cu, seq_slot=torch.arange(len(lens), dtype=torch.int32, device="cuda"), n_seq=len(lens), max_new=max(lens))
+    store = state.reshape(len(lens), -1).clone()
+    poison = torch.full((M, H * V), float("nan"), device="cuda")         # what the result's memory holds before
+    del poison
+    y = KR.ssd_scan(xbc, dt, bias, rate, skip, H, 2, N, V, store, 0, batch)
+    want, left = exact(args, 4, 2, 64, 32, lens)
+    assert not y[sum(lens):].any()
+    assert float((y[:sum(lens)].view(-1, H, V).double() - want).norm() / want.norm()) < 1e-6
+    assert float((store.view(left.shape).double() - left).norm() / left.norm()) < 1e-6

@@ -245,15 +245,15 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
     ti_pdl_sync();
     g.xbc = ti_dependent(g.xbc); g.dt = ti_dependent(g.dt); g.scratch = ti_dependent(g.scratch);
     const int first = g.cu_new[b], tok0 = first + c * SC, n = min(SC, g.cu_new[b + 1] - tok0);
-    if (n <= 0) return;
     const int inner = g.heads * V, per_group = g.heads / g.groups, runs = (per_group + run - 1) / run;
     const int grp = blockIdx.y / runs, h0 = grp * per_group + (blockIdx.y - grp * runs) * run, h1 = min(h0 + run, (grp + 1) * per_group);
-    const bf16* row0 = g.xbc + (size_t)tok0 * g.ld_xbc;
-    if (b == 0 && c == 0) {      // rows past the last sequence's are nobody's
+    if (b == 0 && c == 0) {      // rows past the last sequence's are nobody's (whether or not the first one brings tokens)
         const int cols = (h1 - h0) * V;
         for (int i = tid; i < (M - g.cu_new[gridDim.z]) * cols; i += SSD_THREADS)
             g.y[(size_t)(g.cu_new[gridDim.z] + i / cols) * inner + (size_t)h0 * V + i % cols] = 0.f;
     }
+    if (n <= 0) return;
+    const bf16* row0 = g.xbc + (size_t)tok0 * g.ld_xbc;
     const uint32_t ss = (uint32_t)__cvta_generic_to_shared(st), x0 = (uint32_t)__cvta_generic_to_shared(xt);
     auto fetch = [&](int h) {
         load_rows<V>(x0 + ((h - h0) & 1) * X_BYTES, row0 + h * V, g.ld_xbc, n);
