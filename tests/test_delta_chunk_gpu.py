@@ -114,6 +114,20 @@ def test_no_further_off_than_the_scan(KR, monkeypatch, dtype, head, d, H, G, len
 
 
 @pytest.mark.parametrize("head", [True, False])
+@pytest.mark.parametrize("what", ["q", "k", "v", "decay", "beta"])
+def test_a_token_that_is_not_finite_spoils_none_before_it(KR, head, what):
+    lens, bad = [70, 40], 45                       # the token in the first sequence's second chunk
+    args = make(torch.float32, head, 64, 64, 2, 2, lens, 5, False)
+    clean, left = (t.clone() for t in run(KR, args, lens, head))
+    args[["q", "k", "v", "decay", None, None, "beta"].index(what)][bad] = float("nan")
+    got, state = run(KR, args, lens, head)
+    keep = torch.ones(sum(lens), dtype=torch.bool, device="cuda")
+    keep[bad:lens[0]] = False
+    assert torch.equal(got[keep], clean[keep]) and torch.equal(state[1], left[1])
+    assert got[bad].isnan().all() and (what == "q" or (got[bad:lens[0]].isnan().all() and state[0].isnan().all()))
+
+
+@pytest.mark.parametrize("head", [True, False])
 @pytest.mark.parametrize("lens", [[0, 40, 0, 70], [50, 0]])
 def test_empty_sequences_and_rows_that_are_nobodys(KR, head, lens):
     args = make(torch.float32, head, 64, 64, 2, 2, lens, 5, False)

@@ -432,6 +432,7 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
                 const float4 r = *reinterpret_cast<const float4*>(Rs + (kq + 8 * m) * R_PITCH + ct * 4);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
+                    if (kq + 8 * m > warp * 4 + i) continue;       // (a later token's is not looked at: zero times a NaN is one)
                     const float w = buf[O::t + (warp * 4 + i) * P_PITCH + kq + 8 * m];
                     acc[i * 4] = fmaf(w, r.x, acc[i * 4]);
                     acc[i * 4 + 1] = fmaf(w, r.y, acc[i * 4 + 1]);
@@ -497,6 +498,7 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
                 const float4 e = *reinterpret_cast<const float4*>(Es + (kq + 8 * m) * E_PITCH + ct * 4);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
+                    if (kq + 8 * m > warp * 4 + i) continue;
                     const float w = buf[O::p + (warp * 4 + i) * P_PITCH + kq + 8 * m];
                     acc[i * 4] = fmaf(w, e.x, acc[i * 4]);
                     acc[i * 4 + 1] = fmaf(w, e.y, acc[i * 4 + 1]);
