@@ -125,3 +125,30 @@ def test_empty_sequences_and_rows_that_are_nobodys(KR, lens):
     assert not y[sum(lens):].any()
     assert float((y[:sum(lens)].view(-1, H, V).double() - want).norm() / want.norm()) < 1e-6
     assert float((store.view(left.shape).double() - left).norm() / left.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("V", [32, 64])
+@pytest.mark.parametrize("what", ["x nan", "x inf", "B", "C", "dt"])
+def test_a_token_that_is_not_finite_spoils_none_before_it(KR, V, what):
+    H, G, N, lens, bad = 4, 2, 64, [300, 90], 200                # the token in the first sequence's second chunk, amid a tile
+    args = make(H, G, N, V, lens, 3)
+    clean, left = (t.clone() for t in run(KR, args, H, G, N, V, lens))
+    xbc, dt = args[:2]
+    at = {"x nan": slice(V, V + 5), "x inf": slice(V, V + 5), "B": slice(H * V, H * V + N), "C": slice(H * V + G * N, H * V + G * N + N)}
+    if what == "dt":
+        dt[bad] = float("nan")
+    else:
+        xbc[bad, at[what]] = float("inf" if what == "x inf" else "nan")
+    y, state = run(KR, args, H, G, N, V, lens)
+    keep = torch.ones(sum(lens), dtype=torch.bool, device="cuda")
+    keep[bad:lens[0]] = False
+    assert torch.equal(y[keep], clean[keep]) and torch.equal(state[1], left[1])
+    if what[0] == "x":                                           # five channels of the second head, from the token on
+        assert not y[bad:lens[0], 1, :5].isfinite().any() and not state[0, 1, :5].isfinite().any()
+        y[:, 1, :5], clean[:, 1, :5], state[0, 1, :5], left[0, 1, :5] = 0, 0, 0, 0
+        assert torch.equal(y, clean) and torch.equal(state, left)
+    elif what == "C":
+        keep[bad + 1:lens[0]] = True
+        assert torch.equal(y[keep], clean[keep]) and y[bad, :2].isnan().all() and torch.equal(state, left)
+    else:
+        assert y[bad:lens[0], :2].isnan().all() and state[0, :2].isnan().all()

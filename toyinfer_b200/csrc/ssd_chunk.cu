@@ -102,6 +102,12 @@ __device__ __forceinline__ void mma_add(float (&acc)[4], const uint32_t (&a)[4],
     for (int e = 0; e < 4; e++) acc[e] += t[e];
 }
 
+// Two bfloat16 values without those that are not finite, and whether there was one.
+__device__ __forceinline__ bool spoilt(uint32_t x) { return (x & 0x7f80u) == 0x7f80u || (x & 0x7f800000u) == 0x7f800000u; }
+__device__ __forceinline__ uint32_t without(uint32_t x) {
+    return ((x & 0x7f80u) == 0x7f80u ? 0u : x & 0xffffu) | ((x & 0x7f800000u) == 0x7f800000u ? 0u : x & 0xffff0000u);
+}
+
 // Rows of COLS bfloat16 (64 or 128; or 32 in rows of 64) into the swizzled boxes of mma_utils.cuh, on their way until
 // async_wait(); rows past the end are zeros.
 template <int COLS>
@@ -336,6 +342,7 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
         for (int j = 0; j < V / 8; j++) { acc[j][0] *= ea; acc[j][1] *= ea; acc[j][2] *= eb; acc[j][3] *= eb; }
         // the chunk's own tokens: weights from C . B (their small parts in sums of their own, as above)
         float low[V / 8][4] = {};
+        bool bad = false;               // whether x of this warp's own 16 tokens holds values that are not finite
 #pragma unroll
         for (int j = 0; j < SC / 16; j++) {
             if (j <= tile) {
@@ -358,6 +365,12 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
                 for (int v = 0; v < V / 16; v++) {
                     uint32_t q[4];
                     ldmatrix_x4_trans(q[0], q[1], q[2], q[3], xs + swizzled_offset<SC>(j * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), v * 16 + ((lane >> 4) << 3)));
+                    if (j == tile && __any_sync(0xffffffffu, spoilt(q[0]) || spoilt(q[1]) || spoilt(q[2]) || spoilt(q[3]))) {
+                        // (a weight of zero would carry them to the tokens before them)
+                        bad = true;
+#pragma unroll
+                        for (int u = 0; u < 4; u++) q[u] = without(q[u]);
+                    }
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         mma_bf16(low[2 * v + u], lo, q[2 * u], q[2 * u + 1]);
@@ -366,6 +379,18 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
                     }
                 }
             }
+        }
+        if (bad) {                      // they spoil their own token and those after it
+#pragma unroll
+            for (int j = 0; j < V / 8; j++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    int at = 16;        // the first of them in this column
+                    for (int s = 15; s >= 0; s--)
+                        if (spoilt(*reinterpret_cast<const unsigned short*>(xh + swizzled_offset<SC>(t0 + s, j * 8 + ca + e)))) at = s;
+                    if (ra >= at) acc[j][e] = __int_as_float(0x7fffffff);
+                    if (ra + 8 >= at) acc[j][2 + e] = __int_as_float(0x7fffffff);
+                }
         }
         const float skip = g.skip ? g.skip[h] : 0.f;
         float* yo = g.y + (size_t)(tok0 + t0) * inner + (size_t)h * V;
