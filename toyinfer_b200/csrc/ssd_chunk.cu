@@ -102,11 +102,8 @@ __device__ __forceinline__ void mma_add(float (&acc)[4], const uint32_t (&a)[4],
     for (int e = 0; e < 4; e++) acc[e] += t[e];
 }
 
-// Two bfloat16 values without those that are not finite, and whether there was one.
-__device__ __forceinline__ bool spoilt(uint32_t x) { return (x & 0x7f80u) == 0x7f80u || (x & 0x7f800000u) == 0x7f800000u; }
-__device__ __forceinline__ uint32_t without(uint32_t x) {
-    return ((x & 0x7f80u) == 0x7f80u ? 0u : x & 0xffffu) | ((x & 0x7f800000u) == 0x7f800000u ? 0u : x & 0xffff0000u);
-}
+// Bit 15 (31) of the result: the lower (upper) of two bfloat16 values is not finite.
+__device__ __forceinline__ uint32_t not_finite2(uint32_t x) { return (x & 0x7f807f80u) + 0x00800080u; }
 
 // Rows of COLS bfloat16 (64 or 128; or 32 in rows of 64) into the swizzled boxes of mma_utils.cuh, on their way until
 // async_wait(); rows past the end are zeros.
@@ -148,7 +145,9 @@ ssd_chunk_state_kernel(SsdArgs g, int run) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int t = lane * 4 + i;
-            w[warp][t] = ds[warp][t] * (float)exp2(all - (double)lh[warp][t] - (double)ll[warp][t]);
+            const double x = all - (double)lh[warp][t] - (double)ll[warp][t];
+            const float r = (float)x;           // (what the exponent loses here is put back: 2^x = 2^r (1 + ln 2 (x - r)))
+            w[warp][t] = ds[warp][t] * (exp2f(r) * fmaf(0.6931472f, (float)(x - (double)r), 1.f));
         }
         if (lane == 0) g.decay[id0 + h0 + warp] = (float)exp2(all);
     }
@@ -247,6 +246,7 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
     unsigned char* st = smem;
     unsigned char* xt = smem + RAW + V * N * 4;
     __shared__ float ds[8][SC], lh[8][SC], ll[8][SC];
+    __shared__ int spoilt_from[V];
     const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     ti_pdl_sync();
     g.xbc = ti_dependent(g.xbc); g.dt = ti_dependent(g.dt); g.scratch = ti_dependent(g.scratch);
@@ -313,10 +313,29 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
             *reinterpret_cast<uint4*>(to + PART) = mid;
             *reinterpret_cast<uint4*>(to + 2 * PART) = lo;
         }
-        __syncthreads();
+        // Values of x that are not finite: a weight of zero would carry them to tokens before them.  They become zeros, and
+        // every output of their channel from their token on becomes a NaN.
+        unsigned char* xh = xt + ((h - h0) & 1) * X_BYTES;
+        uint32_t any = 0;
+#pragma unroll
+        for (int i = tid; i < SC * (V / 8); i += SSD_THREADS) {
+            const uint4 x = *reinterpret_cast<const uint4*>(xh + swizzled_offset<SC>(i / (V / 8), (i % (V / 8)) * 8));
+            any |= not_finite2(x.x) | not_finite2(x.y) | not_finite2(x.z) | not_finite2(x.w);
+        }
+        const bool bad = __syncthreads_or((any & 0x80008000u) != 0);
+        if (bad) {
+            if (tid < V) {
+                int at = SC;
+                for (int t = SC - 1; t >= 0; t--) {
+                    unsigned short* x = reinterpret_cast<unsigned short*>(xh + swizzled_offset<SC>(t, tid));
+                    if ((*x & 0x7f80u) == 0x7f80u) { at = t; *x = 0; }
+                }
+                spoilt_from[tid] = at;
+            }
+            __syncthreads();
+        }
         if (h + 1 < h1) fetch(h + 1);           // on its way while this head's outputs are formed
         const uint32_t xs = x0 + ((h - h0) & 1) * X_BYTES;
-        const unsigned char* xh = xt + ((h - h0) & 1) * X_BYTES;
         const int hh = h - h0;
         // A_t S C_t
         float acc[V / 8][4] = {};
@@ -342,7 +361,6 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
         for (int j = 0; j < V / 8; j++) { acc[j][0] *= ea; acc[j][1] *= ea; acc[j][2] *= eb; acc[j][3] *= eb; }
         // the chunk's own tokens: weights from C . B (their small parts in sums of their own, as above)
         float low[V / 8][4] = {};
-        bool bad = false;               // whether x of this warp's own 16 tokens holds values that are not finite
 #pragma unroll
         for (int j = 0; j < SC / 16; j++) {
             if (j <= tile) {
@@ -365,12 +383,6 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
                 for (int v = 0; v < V / 16; v++) {
                     uint32_t q[4];
                     ldmatrix_x4_trans(q[0], q[1], q[2], q[3], xs + swizzled_offset<SC>(j * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), v * 16 + ((lane >> 4) << 3)));
-                    if (j == tile && __any_sync(0xffffffffu, spoilt(q[0]) || spoilt(q[1]) || spoilt(q[2]) || spoilt(q[3]))) {
-                        // (a weight of zero would carry them to the tokens before them)
-                        bad = true;
-#pragma unroll
-                        for (int u = 0; u < 4; u++) q[u] = without(q[u]);
-                    }
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         mma_bf16(low[2 * v + u], lo, q[2 * u], q[2 * u + 1]);
@@ -380,18 +392,12 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
                 }
             }
         }
-        if (bad) {                      // they spoil their own token and those after it
+        if (bad)
 #pragma unroll
             for (int j = 0; j < V / 8; j++)
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    int at = 16;        // the first of them in this column
-                    for (int s = 15; s >= 0; s--)
-                        if (spoilt(*reinterpret_cast<const unsigned short*>(xh + swizzled_offset<SC>(t0 + s, j * 8 + ca + e)))) at = s;
-                    if (ra >= at) acc[j][e] = __int_as_float(0x7fffffff);
-                    if (ra + 8 >= at) acc[j][2 + e] = __int_as_float(0x7fffffff);
-                }
-        }
+                for (int e = 0; e < 4; e++)
+                    if (t0 + ra + (e >> 1) * 8 >= spoilt_from[j * 8 + ca + (e & 1)]) acc[j][e] = __int_as_float(0x7fffffff);
         const float skip = g.skip ? g.skip[h] : 0.f;
         float* yo = g.y + (size_t)(tok0 + t0) * inner + (size_t)h * V;
 #pragma unroll
