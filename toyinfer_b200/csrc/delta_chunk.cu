@@ -66,6 +66,7 @@ struct DeltaChunkArgs {
     float* bv;                  // [chunks, heads, vdim / 16][CH][16] beta v
     const int* cu_new; const int* seq_slot;
     int n_heads, qk_heads, vdim;
+    int least;                  // sequences of fewer new tokens are left to the scan
 };
 
 // A sequence's chunk c has the number tok0 / 32 + b + c: no two chunks of a step share one.
@@ -98,7 +99,7 @@ delta_chunk_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
     ti_pdl_sync();
     q = ti_dependent(q); k = ti_dependent(k); v = ti_dependent(v); decay_logit = ti_dependent(decay_logit); beta_logit = ti_dependent(beta_logit);
     const int tok0 = a.cu_new[b] + c * CH, n = min(CH, a.cu_new[b + 1] - tok0);
-    if (n <= 0) return;
+    if (n <= 0 || a.cu_new[b + 1] - a.cu_new[b] < a.least) return;
     const int hq = h / (a.n_heads / a.qk_heads), vdim = a.vdim;
     const float rt = rate[h];
     const size_t cid = chunk_id(a.cu_new[b], b, c) * a.n_heads + h;
@@ -346,7 +347,7 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
     if (b == 0)          // rows past the last sequence's are nobody's
         for (int m = a.cu_new[gridDim.y] + (tid >> 4); m < M; m += DC_THREADS / DC_COLS) o[((size_t)m * a.n_heads + h) * a.vdim + col0 + (tid & 15)] = 0.f;
     const int first = a.cu_new[b], n = a.cu_new[b + 1] - first;
-    if (n <= 0) return;
+    if (n <= 0 || n < a.least) return;
     const int H = a.n_heads, chunks = (n + CH - 1) / CH;
     const size_t id0 = chunk_id(first, b, 0);
     auto fetch = [&](int c) {                    // by one thread
@@ -557,12 +558,14 @@ int run_chunks(const void* q, const void* k, const void* v, long long q_stride, 
 extern "C" int ti_delta_chunk_floats(int dim, int vdim) { return (dim == 64 ? Ops<64>::floats : Ops<128>::floats) + CH * vdim; }
 
 // As ti_delta_rule_scan (delta_rule.cu), for dim 64 or 128 and vdim a multiple of 16.  max_new: at least the most new tokens of
-// a sequence.  scratch: float32, 16-byte aligned, (M / 32 + n_seq) * heads * ti_delta_chunk_floats(dim, vdim) values.
+// a sequence.  Sequences of fewer than `least` new tokens are passed over (ti_delta_rule_scan takes those up to its `most`).
+// scratch: float32, 16-byte aligned, (M / 32 + n_seq) * heads * ti_delta_chunk_floats(dim, vdim) values.
 extern "C" int ti_delta_rule_chunked(const void* q, const void* k, const void* v, long long q_stride, long long k_stride,
                                      long long v_stride, const void* decay_logit, long long decay_stride, int head_decay,
                                      const float* dt_bias, const float* rate, const void* beta_logit, long long beta_stride, float* o,
                                      float* state, long long slot_stride, float* scratch, const int* cu_new, const int* seq_slot, int n_seq,
-                                     int max_new, int M, int n_heads, int qk_heads, int dim, int vdim, int dtype, cudaStream_t stream) {
+                                     int max_new, int M, int n_heads, int qk_heads, int dim, int vdim, int least, int dtype,
+                                     cudaStream_t stream) {
     if (n_seq == 0 || M == 0) return 0;
     TI_REQUIRE(n_seq > 0 && n_seq <= 65535 && M > 0 && max_new > 0 && n_heads > 0 && n_heads <= 65535 && qk_heads > 0 && n_heads % qk_heads == 0 && scratch,
                "delta_rule: bad sizes");
@@ -571,7 +574,7 @@ extern "C" int ti_delta_rule_chunked(const void* q, const void* k, const void* v
     DeltaChunkArgs a;
     a.ops = scratch;
     a.bv = scratch + (size_t)(M / CH + n_seq) * n_heads * (dim == 64 ? Ops<64>::floats : Ops<128>::floats);
-    a.cu_new = cu_new; a.seq_slot = seq_slot; a.n_heads = n_heads; a.qk_heads = qk_heads; a.vdim = vdim;
+    a.cu_new = cu_new; a.seq_slot = seq_slot; a.n_heads = n_heads; a.qk_heads = qk_heads; a.vdim = vdim; a.least = least;
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
         auto go = [&](auto dc) -> int {

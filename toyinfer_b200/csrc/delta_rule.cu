@@ -45,7 +45,8 @@ __global__ void delta_rule_prep_kernel(const T* __restrict__ q, const T* __restr
                                        const L* __restrict__ decay_logit, long long decay_stride, const float* __restrict__ dt_bias,
                                        const float* __restrict__ rate, const T* __restrict__ beta_logit, long long beta_stride,
                                        float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ gg, float* __restrict__ beta,
-                                       long long rows, int n_heads, int qk_heads, int dim) {
+                                       long long rows, int n_heads, int qk_heads, int dim, const int* __restrict__ cu_new, int n_seq,
+                                       int most) {
     ti_pdl_trigger();
     ti_pdl_sync();
     q = ti_dependent(q); k = ti_dependent(k); decay_logit = ti_dependent(decay_logit); beta_logit = ti_dependent(beta_logit);
@@ -54,6 +55,14 @@ __global__ void delta_rule_prep_kernel(const T* __restrict__ q, const T* __restr
     const int lane = threadIdx.x & 31, units = qk_heads + n_heads;
     const long long m = w / units;
     const int unit = (int)(w - m * units);
+    if (most > 0) {              // only tokens of the sequences that are scanned
+        int lo = 0, hi = n_seq;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (cu_new[mid] <= m) lo = mid; else hi = mid;
+        }
+        if (cu_new[lo + 1] - cu_new[lo] > most) return;
+    }
     if (unit < qk_heads) {
         const T* qr = q + (size_t)m * q_stride + (size_t)unit * dim;
         const T* kr = k + (size_t)m * k_stride + (size_t)unit * dim;
@@ -105,7 +114,7 @@ delta_rule_scan_kernel(const float* __restrict__ qn, const float* __restrict__ k
                        const float* __restrict__ beta, const T* __restrict__ v, long long v_stride,
                        float* __restrict__ o, float* __restrict__ state, long long slot_stride,
                        const int* __restrict__ cu_new, const int* __restrict__ seq_slot,
-                       int n_heads, int qk_heads, int dim, int vdim, int groups) {
+                       int n_heads, int qk_heads, int dim, int vdim, int groups, int most) {
     ti_pdl_trigger();
     constexpr int NV = MAXD / DR_LPC >= 4 ? 4 : MAXD / DR_LPC, J = MAXD / (DR_LPC * NV), ROW = MAXD;
     constexpr int PIECES = (HEAD ? 2 : 3) * DR_TOK * ROW / 4;            // 16-byte pieces of a run's q, k, g
@@ -122,7 +131,7 @@ delta_rule_scan_kernel(const float* __restrict__ qn, const float* __restrict__ k
     const int h = blockIdx.x / groups, g = blockIdx.x - h * groups;
     const int b = blockIdx.y;
     const int tok0 = cu_new[b], n = cu_new[b + 1] - tok0;
-    if (n <= 0) return;
+    if (n <= 0 || (most > 0 && n > most)) return;
     const int hq = h / (n_heads / qk_heads);
     const int r = threadIdx.x & (DR_LPC - 1), cl = threadIdx.x / DR_LPC;
     const int col = g * DR_COLS + cl;
@@ -348,7 +357,7 @@ template <typename T, typename L, bool HEAD>
 int delta_rule_run(const void* q, const void* k, const void* v, long long q_stride, long long k_stride, long long v_stride,
                    const void* decay_logit, long long decay_stride, const float* dt_bias, const float* rate, const void* beta_logit,
                    long long beta_stride, float* o, float* state, long long slot_stride, float* scratch, const int* cu_new,
-                   const int* seq_slot, int n_seq, int M, int n_heads, int qk_heads, int dim, int vdim, cudaStream_t stream) {
+                   const int* seq_slot, int n_seq, int M, int n_heads, int qk_heads, int dim, int vdim, int most, cudaStream_t stream) {
     const int groups = (vdim + DR_COLS - 1) / DR_COLS;
     float* qn = scratch;
     float* kn = qn + (size_t)M * qk_heads * dim;
@@ -357,7 +366,7 @@ int delta_rule_run(const void* q, const void* k, const void* v, long long q_stri
     const long long rows = (long long)M * (qk_heads + n_heads);
     TI_CUDA(ti_launch(delta_rule_prep_kernel<T, L, HEAD>, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, stream, (const T*)q, (const T*)k,
                       q_stride, k_stride, (const L*)decay_logit, decay_stride, dt_bias, rate, (const T*)beta_logit, beta_stride, qn, kn, gg,
-                      beta, rows, n_heads, qk_heads, dim));
+                      beta, rows, n_heads, qk_heads, dim, cu_new, n_seq, most));
     TI_CHECK_LAUNCH("delta_rule_prep");
     return dispatch_dim(dim, [&](auto md) -> int {
         constexpr int MAXD = decltype(md)::value;
@@ -367,7 +376,7 @@ int delta_rule_run(const void* q, const void* k, const void* v, long long q_stri
             TI_CUDA(cudaFuncSetAttribute(delta_rule_scan_kernel<T, MAXD, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         TI_CUDA(ti_launch(delta_rule_scan_kernel<T, MAXD, HEAD>, dim3(n_heads * groups, n_seq), dim3(DR_THREADS), smem, stream,
                           (const float*)qn, (const float*)kn, (const float*)gg, (const float*)beta, (const T*)v, v_stride, o, state,
-                          slot_stride, cu_new, seq_slot, n_heads, qk_heads, dim, vdim, groups));
+                          slot_stride, cu_new, seq_slot, n_heads, qk_heads, dim, vdim, groups, most));
         TI_CHECK_LAUNCH("delta_rule_scan");
         return 0;
     });
@@ -379,12 +388,13 @@ int delta_rule_run(const void* q, const void* k, const void* v, long long q_stri
 // decay_logit float32 [M, heads * dim], dt_bias float32 [heads * dim]; head_decay 1: decay_logit [M, heads] of the engine's
 // type, dt_bias float32 [heads] (row stride decay_stride in both); rate: float32 [heads]; beta_logit: [M, heads] (row stride
 // given); o: float32 [M, heads * vdim]; state: float32, slot s at state + s * slot_stride holds [heads, dim, vdim];
+// most > 0: sequences of more new tokens are passed over (ti_delta_rule_chunked, delta_chunk.cu, takes them).
 // scratch: float32, M * (2 * qk_heads * dim + heads * (head_decay ? 1 : dim) + heads) values, 16-byte aligned.
 extern "C" int ti_delta_rule_scan(const void* q, const void* k, const void* v, long long q_stride, long long k_stride,
                                   long long v_stride, const void* decay_logit, long long decay_stride, int head_decay,
                                   const float* dt_bias, const float* rate, const void* beta_logit, long long beta_stride, float* o,
                                   float* state, long long slot_stride, float* scratch, const int* cu_new, const int* seq_slot, int n_seq,
-                                  int M, int n_heads, int qk_heads, int dim, int vdim, int dtype, cudaStream_t stream) {
+                                  int M, int n_heads, int qk_heads, int dim, int vdim, int most, int dtype, cudaStream_t stream) {
     if (n_seq == 0 || M == 0) return 0;
     TI_REQUIRE(n_seq > 0 && n_seq <= 65535 && M > 0 && n_heads > 0 && qk_heads > 0 && n_heads % qk_heads == 0 && dim > 0 && vdim > 0 && scratch,
                "delta_rule_scan: bad sizes");
@@ -394,10 +404,10 @@ extern "C" int ti_delta_rule_scan(const void* q, const void* k, const void* v, l
         if (head_decay)
             return delta_rule_run<T, T, true>(q, k, v, q_stride, k_stride, v_stride, decay_logit, decay_stride, dt_bias, rate, beta_logit,
                                               beta_stride, o, state, slot_stride, scratch, cu_new, seq_slot, n_seq, M, n_heads, qk_heads, dim,
-                                              vdim, stream);
+                                              vdim, most, stream);
         return delta_rule_run<T, float, false>(q, k, v, q_stride, k_stride, v_stride, decay_logit, decay_stride, dt_bias, rate, beta_logit,
                                                beta_stride, o, state, slot_stride, scratch, cu_new, seq_slot, n_seq, M, n_heads, qk_heads,
-                                               dim, vdim, stream);
+                                               dim, vdim, most, stream);
     });
 }
 

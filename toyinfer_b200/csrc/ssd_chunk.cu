@@ -34,7 +34,7 @@ struct SsdArgs {
     float* state; long long slot_stride;
     float* y;
     const int* cu_new; const int* seq_slot;
-    int heads, groups;
+    int heads, groups, least;   // sequences of fewer than `least` new tokens are left to the scan
     float* scratch;             // [chunks, heads, vdim, N]: what a chunk adds, then the state before it
     float* decay;               // [chunks, heads]
 };
@@ -130,7 +130,7 @@ ssd_chunk_state_kernel(SsdArgs g, int run) {
     ti_pdl_sync();
     g.xbc = ti_dependent(g.xbc); g.dt = ti_dependent(g.dt);
     const int first = g.cu_new[b], tok0 = first + c * SC, n = min(SC, g.cu_new[b + 1] - tok0);
-    if (n <= 0) return;
+    if (n <= 0 || g.cu_new[b + 1] - first < g.least) return;
     const int inner = g.heads * V, per_group = g.heads / g.groups, runs = (per_group + run - 1) / run;
     const int grp = blockIdx.y / runs, h0 = grp * per_group + (blockIdx.y - grp * runs) * run, h1 = min(h0 + run, (grp + 1) * per_group);
     const bf16* row0 = g.xbc + (size_t)tok0 * g.ld_xbc;
@@ -202,7 +202,7 @@ __global__ void ssd_chunk_carry_kernel(SsdArgs g, int per_head) {
     g.scratch = ti_dependent(g.scratch); g.decay = ti_dependent(g.decay);
     const int b = blockIdx.z, h = blockIdx.y, first = g.cu_new[b], n = g.cu_new[b + 1] - first;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (n <= 0 || i >= per_head) return;
+    if (n <= 0 || n < g.least || i >= per_head) return;
     const int chunks = (n + SC - 1) / SC;
     float* slot = g.state + (size_t)g.seq_slot[b] * g.slot_stride + (size_t)h * per_head + i;
     const size_t id = ssd_chunk_id(first, b, 0) * g.heads + h;
@@ -258,7 +258,7 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
         for (int i = tid; i < (M - g.cu_new[gridDim.z]) * cols; i += SSD_THREADS)
             g.y[(size_t)(g.cu_new[gridDim.z] + i / cols) * inner + (size_t)h0 * V + i % cols] = 0.f;
     }
-    if (n <= 0) return;
+    if (n <= 0 || g.cu_new[b + 1] - first < g.least) return;
     const bf16* row0 = g.xbc + (size_t)tok0 * g.ld_xbc;
     const uint32_t ss = (uint32_t)__cvta_generic_to_shared(st), x0 = (uint32_t)__cvta_generic_to_shared(xt);
     auto fetch = [&](int h) {
@@ -426,8 +426,10 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t
     }
     const int chunks = (max_new + SC - 1) / SC;
     const int per_group = g.heads / g.groups;
+    // chunks that there can be: sequences that bring fewer tokens than the longest leave blocks of the grid without work
+    const long long live = std::min((long long)chunks * n_seq, (long long)M / SC + std::min(n_seq, g.least > 0 ? M / g.least : n_seq)) * g.groups;
     int state_run = std::min(STATE_RUN, per_group);       // (heads share B; as long as two blocks an SM are left)
-    while (state_run > 1 && (long long)chunks * n_seq * g.groups * ((per_group + state_run - 1) / state_run) < 200) state_run /= 2;
+    while (state_run > 1 && live * ((per_group + state_run - 1) / state_run) < 200) state_run /= 2;
     TI_CUDA(ti_launch(ssd_chunk_state_kernel<N, V>, dim3(chunks, g.groups * ((per_group + state_run - 1) / state_run), n_seq), dim3(SSD_THREADS),
                       state_smem, stream, g, state_run));
     TI_CHECK_LAUNCH("ssd_scan (chunks' parts)");
@@ -438,7 +440,7 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t
     int run = 1;
     double best = 0.0;
     for (int r = 1; r <= std::min(8, per_group); r++) {
-        const long long blocks = (long long)chunks * n_seq * g.groups * ((per_group + r - 1) / r);
+        const long long blocks = live * ((per_group + r - 1) / r);
         const double cost = (double)((blocks + 147) / 148) * (1.3 + r);
         if (r == 1 || cost < best) { best = cost; run = r; }
     }
@@ -450,10 +452,11 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t
 }  // namespace
 
 // As ti_ssd_scan (ssd_scan.cu), for bfloat16 tokens, N 64 or 128 and vdim 32 or 64; rows of xbc on 16-byte boundaries.  max_new:
-// at least the most new tokens of a sequence.  scratch: float32, 16-byte aligned, (M / 128 + n_seq) * heads * (vdim * N + 1) values.
+// at least the most new tokens of a sequence.  Sequences of fewer than `least` are passed over (ti_ssd_scan takes those up to its
+// `most`).  scratch: float32, 16-byte aligned, (M / 128 + n_seq) * heads * (vdim * N + 1) values.
 extern "C" int ti_ssd_chunked(const void* xbc, long long ld_xbc, const void* dt_raw, long long ld_dt, const float* dt_bias,
                               const float* rate, const float* skip, float* state, long long slot_stride, float* y, const int* cu_new,
-                              const int* seq_slot, int n_seq, int max_new, int M, int heads, int groups, int N, int vdim, float* scratch,
+                              const int* seq_slot, int n_seq, int max_new, int M, int heads, int groups, int N, int vdim, int least, float* scratch,
                               cudaStream_t stream) {
     if (n_seq == 0 || M == 0) return 0;
     TI_REQUIRE(n_seq > 0 && n_seq <= 65535 && M > 0 && max_new > 0 && heads > 0 && heads <= 65535 && groups > 0 && heads % groups == 0 && scratch,
@@ -461,7 +464,7 @@ extern "C" int ti_ssd_chunked(const void* xbc, long long ld_xbc, const void* dt_
     TI_REQUIRE((N == 64 || N == 128) && (vdim == 32 || vdim == 64), "ssd_scan: states of %d x %d are not taken in chunks", vdim, N);
     TI_REQUIRE(ld_xbc % 8 == 0 && (reinterpret_cast<uintptr_t>(xbc) & 15) == 0 && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 &&
                (reinterpret_cast<uintptr_t>(y) & 15) == 0, "ssd_scan: rows must start on 16-byte boundaries");
-    SsdArgs g{(const bf16*)xbc, ld_xbc, (const bf16*)dt_raw, ld_dt, dt_bias, rate, skip, state, slot_stride, y, cu_new, seq_slot, heads, groups,
+    SsdArgs g{(const bf16*)xbc, ld_xbc, (const bf16*)dt_raw, ld_dt, dt_bias, rate, skip, state, slot_stride, y, cu_new, seq_slot, heads, groups, least,
               scratch, scratch + (size_t)(M / SC + n_seq) * heads * vdim * N};
     if (N == 64) return vdim == 32 ? run_ssd_chunks<64, 32>(g, n_seq, max_new, M, stream) : run_ssd_chunks<64, 64>(g, n_seq, max_new, M, stream);
     return vdim == 32 ? run_ssd_chunks<128, 32>(g, n_seq, max_new, M, stream) : run_ssd_chunks<128, 64>(g, n_seq, max_new, M, stream);

@@ -59,7 +59,7 @@ ssd_scan_kernel(const T* __restrict__ xbc, long long ld_xbc, const T* __restrict
                 const float* __restrict__ dt_bias, const float* __restrict__ rate, const float* __restrict__ skip,
                 float* __restrict__ state, long long slot_stride, float* __restrict__ y, const int* __restrict__ cu_new,
                 const int* __restrict__ seq_slot, int heads, int groups, int N, int vdim, int seg, int n_seg,
-                float* __restrict__ scratch, float* __restrict__ seg_decay, int vec) {
+                float* __restrict__ scratch, float* __restrict__ seg_decay, int vec, int most) {
     ti_pdl_trigger();
     constexpr int NP = LPC * R;                  // N rounded up to what the lanes hold
     constexpr int CH = R >= 4 ? 4 : 2;           // floats of one read or write of shared memory
@@ -86,7 +86,7 @@ ssd_scan_kernel(const T* __restrict__ xbc, long long ld_xbc, const T* __restrict
     xbc = ti_dependent(xbc); dt_raw = ti_dependent(dt_raw);
     const int tok0 = cu_new[b], n = cu_new[b + 1] - tok0;
     const int t_begin = p * seg, t_end = min(n, t_begin + seg);
-    if (n <= 0 || t_begin >= t_end) return;
+    if (n <= 0 || t_begin >= t_end || (most > 0 && n > most)) return;
     const bool last = t_end == n;
     if (!OUT && last) return;
     const size_t per_slot = (size_t)inner * N, at = ((size_t)h * vdim + v) * N;
@@ -354,15 +354,17 @@ __global__ void gate_group_rmsnorm_vec_kernel(const float* __restrict__ y, const
 // that run in parallel: each segment's own effect on a zero state, a walk over a sequence's segments that gives each
 // its start state, then the recurrence itself per segment.  scratch: float32 [n_seq * n_seg, heads * vdim * N];
 // seg_decay: float32 [n_seq * n_seg, heads].  Three launches instead of one.
+// most > 0 (with one segment only): sequences of more new tokens are passed over (ti_ssd_chunked, ssd_chunk.cu, takes them).
 extern "C" int ti_ssd_scan(const void* xbc, long long ld_xbc, const void* dt_raw, long long ld_dt, const float* dt_bias,
                            const float* rate, const float* skip, float* state, long long slot_stride, float* y, const int* cu_new,
                            const int* seq_slot, int n_seq, int heads, int groups, int N, int vdim, int seg, int n_seg,
-                           float* scratch, float* seg_decay, int dtype, cudaStream_t stream) {
+                           float* scratch, float* seg_decay, int most, int dtype, cudaStream_t stream) {
     if (n_seq == 0) return 0;
     TI_REQUIRE(n_seq > 0 && heads > 0 && heads <= 65535 && groups > 0 && heads % groups == 0 && N > 0 && vdim > 0, "ssd_scan: bad sizes");
     TI_REQUIRE(N <= LPC * 32, "ssd_scan: a state of %d values per column is not supported (up to %d)", N, LPC * 32);
     TI_REQUIRE(n_seg >= 1 && (long long)n_seq * n_seg <= 65535 && (n_seg == 1 || (seg > 0 && scratch && seg_decay)),
                "ssd_scan: %d sequences in %d segments", n_seq, n_seg);
+    TI_REQUIRE(most <= 0 || n_seg == 1, "ssd_scan: sequences in segments are all taken");
     if (n_seg == 1) { seg = 1 << 30; scratch = nullptr; }
     const int rows = (N + LPC - 1) / LPC;
     const int inner = heads * vdim;
@@ -377,7 +379,7 @@ extern "C" int ti_ssd_scan(const void* xbc, long long ld_xbc, const void* dt_raw
             if (n_seg > 1) {
                 TI_CUDA(ti_launch(ssd_scan_kernel<T, R, false>, grid, dim3(SCAN_THREADS), smem, stream, (const T*)xbc, ld_xbc, (const T*)dt_raw,
                                   ld_dt, dt_bias, rate, skip, state, slot_stride, y, cu_new, seq_slot, heads, groups, N, vdim, seg, n_seg,
-                                  scratch, seg_decay, vec));
+                                  scratch, seg_decay, vec, 0));
                 TI_CHECK_LAUNCH("ssd_scan (segments)");
                 const long long per_slot = (long long)inner * N;
                 TI_CUDA(ti_launch(ssd_segment_carry_kernel, dim3((unsigned)std::min<long long>((per_slot + 255) / 256, 1024), n_seq), dim3(256), 0,
@@ -387,7 +389,7 @@ extern "C" int ti_ssd_scan(const void* xbc, long long ld_xbc, const void* dt_raw
             }
             TI_CUDA(ti_launch(ssd_scan_kernel<T, R, true>, grid, dim3(SCAN_THREADS), smem, stream, (const T*)xbc, ld_xbc, (const T*)dt_raw, ld_dt,
                               dt_bias, rate, skip, state, slot_stride, y, cu_new, seq_slot, heads, groups, N, vdim, seg, n_seg, scratch,
-                              seg_decay, vec));
+                              seg_decay, vec, most));
             TI_CHECK_LAUNCH("ssd_scan");
             return 0;
         };

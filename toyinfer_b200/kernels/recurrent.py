@@ -11,6 +11,7 @@ from typing import Optional
 import torch
 
 from . import KernelError, _call, _code, _need_cuda, _ptr, _stream
+from .gemm import sm_count
 from .wide import _fn
 
 P, I, L, F = c_void_p, c_int, c_longlong, c_float
@@ -85,16 +86,42 @@ def rglru_scan(gates: torch.Tensor, u: torch.Tensor, z: torch.Tensor, gate_bias_
     return out
 
 
+def in_chunks(batch, least: int, blocks: int, places: int) -> Optional[int]:
+    """Which sequences of a step go in chunks: those of at least the returned number of new tokens (0: all of them; the others go
+    token by token in a launch of their own), or None: none does.
+
+    A sequence of fewer than ``least`` tokens costs the chunked form ``blocks`` blocks all the same, which take turns in
+    ``places``; token by token a long sequence is a chain, beside which short ones cost little.  Delta rule, 16 heads of 128, us,
+    token by token / all in chunks / shared out: 40 tokens and 2 single ones 25 / 29 / 36, 64 and 2 34 / 29 / 35, 64 and 8 35 /
+    57 / 51, 160 and 8 72 / 65 / 59, 160 and 32 98 / 160 / 114, 512 and 32 214 / 204 / 145, 2,048 and 32 841 / 366 / 346.
+
+    Every answer is right whatever the lengths (a captured step is replayed with others); where they are not known, all
+    sequences but one count as short."""
+    if batch.n_seq == 0 or batch.max_new < least:
+        return None
+    new = getattr(batch, "host_new", None)
+    short = sum(n < least for n in new) if new is not None and len(new) == batch.n_seq else batch.n_seq - 1
+    turns = short * blocks / places
+    if short == 0 or (turns <= 4 and batch.max_new >= 14 + 25 * turns):
+        return 0
+    return least if batch.max_new >= 64 + 14 * min(turns, 25) else None
+
+
 # New tokens of one sequence from which the delta rule runs in chunks of 32 (csrc/delta_chunk.cu)
 DELTA_CHUNKED_FROM = 32
 DELTA_CHUNK_SCRATCH = 1 << 30       # ... while its operands, some four floats per element of q, take no more bytes than this
+
+
+def delta_from(H: int, dim: int, vdim: int, batch, device) -> Optional[int]:
+    # (a block of the walk has an SM to itself for keys of 128, half of one for keys of 64)
+    return in_chunks(batch, DELTA_CHUNKED_FROM, H * vdim // 16, (1 if dim == 128 else 2) * sm_count(device))
 
 
 def delta_chunked(q: torch.Tensor, v: torch.Tensor, batch) -> int:
     """Floats of scratch with which a step's delta rule runs in chunks, or 0: it goes token by token."""
     M, G, dim = q.shape
     H, vdim = v.shape[1], v.shape[2]
-    if batch.n_seq == 0 or batch.max_new < DELTA_CHUNKED_FROM or dim not in (64, 128) or vdim % 16:
+    if dim not in (64, 128) or vdim % 16 or delta_from(H, dim, vdim, batch, q.device) is None:
         return 0
     need = (M // 32 + batch.n_seq) * H * _fn("ti_delta_chunk_floats", [I, I])(dim, vdim)
     return need if 4 * need <= DELTA_CHUNK_SCRATCH else 0
@@ -137,17 +164,19 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
         return o
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=q.device)
-        _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, P]),
+        least = delta_from(H, dim, vdim, batch, q.device)
+        _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, P]),
               _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(decay_logit), decay_logit.stride(0), 1 if head_decay else 0,
               _ptr(dt_bias), _ptr(rate), _ptr(beta_logit), beta_logit.stride(0), _ptr(o), base, stride, _ptr(scratch), _ptr(batch.cu_new),
-              _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, H, G, dim, vdim, _code(q, "delta_rule"), _stream(), launches=2)
-        return o
+              _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, H, G, dim, vdim, least, _code(q, "delta_rule"), _stream(), launches=2)
+        if least == 0:
+            return o
     # unit queries and keys, decays and betas of all tokens, made by a kernel of their own before the recurrence
     scratch = torch.empty(M * (2 * G * dim + n_decay + H), dtype=torch.float32, device=q.device)
-    _call(_fn("ti_delta_rule_scan", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, P]),
+    _call(_fn("ti_delta_rule_scan", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, P]),
           _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(decay_logit), decay_logit.stride(0), 1 if head_decay else 0,
           _ptr(dt_bias), _ptr(rate), _ptr(beta_logit), beta_logit.stride(0), _ptr(o), base, stride, _ptr(scratch), _ptr(batch.cu_new),
-          _ptr(batch.seq_slot), batch.n_seq, M, H, G, dim, vdim, _code(q, "delta_rule"), _stream(), launches=2)
+          _ptr(batch.seq_slot), batch.n_seq, M, H, G, dim, vdim, least - 1 if chunked else 0, _code(q, "delta_rule"), _stream(), launches=2)
     return o
 
 
@@ -203,9 +232,13 @@ SSD_CHUNKED_FROM = 80           # new tokens of one sequence from which bfloat16
 SSD_CHUNK_SCRATCH = 1 << 30     # ... while the chunks' states take no more bytes than this
 
 
+def ssd_from(n_heads: int, batch, device) -> Optional[int]:
+    return in_chunks(batch, SSD_CHUNKED_FROM, n_heads, 2 * sm_count(device) // 5)
+
+
 def ssd_chunked(xbc: torch.Tensor, n_heads: int, n_state: int, vdim: int, batch) -> int:
     """Floats of scratch with which a step's Mamba-2 recurrence runs in chunks (csrc/ssd_chunk.cu), or 0: token by token."""
-    if (batch.n_seq == 0 or batch.max_new < SSD_CHUNKED_FROM or xbc.dtype != torch.bfloat16 or n_state not in (64, 128) or vdim not in (32, 64)
+    if (ssd_from(n_heads, batch, xbc.device) is None or xbc.dtype != torch.bfloat16 or n_state not in (64, 128) or vdim not in (32, 64)
             or xbc.stride(0) % 8 or xbc.data_ptr() % 16):
         return 0
     need = (xbc.shape[0] // 128 + batch.n_seq) * n_heads * (vdim * n_state + 1)
@@ -234,21 +267,23 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, rat
     y = (torch.empty if chunked else torch.zeros)((M, inner), dtype=torch.float32, device=xbc.device)
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=xbc.device)
-        _call(_fn("ti_ssd_chunked", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, P, P]),
+        least = ssd_from(n_heads, batch, xbc.device)
+        _call(_fn("ti_ssd_chunked", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, I, P, P]),
               _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0), _ptr(dt_bias), _ptr(rate), _ptr(skip), base, stride, _ptr(y),
               _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, int(n_heads), int(groups), int(n_state), int(vdim),
-              _ptr(scratch), _stream(), launches=3)
-        return y
+              least, _ptr(scratch), _stream(), launches=3)
+        if least == 0:
+            return y
     seg = int(SSD_SEGMENT)
-    n_seg = (batch.max_new + seg - 1) // seg if batch.max_new >= 2 * seg else 1
+    n_seg = (batch.max_new + seg - 1) // seg if batch.max_new >= 2 * seg and not chunked else 1
     scratch = decay = None
     if n_seg > 1:
         scratch = torch.empty((batch.n_seq * n_seg, inner * n_state), dtype=torch.float32, device=xbc.device)
         decay = torch.empty((batch.n_seq * n_seg, n_heads), dtype=torch.float32, device=xbc.device)
-    _call(_fn("ti_ssd_scan", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, P, P, I, P]),
+    _call(_fn("ti_ssd_scan", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, P, P, I, I, P]),
           _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0), _ptr(dt_bias), _ptr(rate), _ptr(skip), base, stride, _ptr(y),
           _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, int(n_heads), int(groups), int(n_state), int(vdim), seg, n_seg,
-          _ptr(scratch), _ptr(decay), _code(xbc, "ssd_scan"), _stream(), launches=3 if n_seg > 1 else 1)
+          _ptr(scratch), _ptr(decay), least - 1 if chunked else 0, _code(xbc, "ssd_scan"), _stream(), launches=3 if n_seg > 1 else 1)
     return y
 
 
