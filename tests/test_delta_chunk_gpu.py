@@ -77,6 +77,7 @@ def run(KR, args, lens, head):
 def test_against_the_scan(KR, monkeypatch, dtype, head, d, dv, H, G, lens, strong):
     args = make(dtype, head, d, dv, H, G, lens, d + dv + sum(lens), strong)
     want = exact(*args, lens, head)
+    monkeypatch.setattr(KR, "DELTA_CHANNEL_FROM", (32, 32))
     assert KR.delta_chunked(args[0], args[2], SimpleNamespace(max_new=max(lens), n_seq=len(lens)))
     got = run(KR, args, lens, head)
     monkeypatch.setattr(KR, "DELTA_CHUNKED_FROM", 1 << 30)
@@ -129,7 +130,8 @@ def test_a_token_that_is_not_finite_spoils_none_before_it(KR, head, what):
 
 @pytest.mark.parametrize("head", [True, False])
 @pytest.mark.parametrize("lens", [[0, 40, 0, 70], [50, 0]])
-def test_empty_sequences_and_rows_that_are_nobodys(KR, head, lens):
+def test_empty_sequences_and_rows_that_are_nobodys(KR, monkeypatch, head, lens):
+    monkeypatch.setattr(KR, "DELTA_CHANNEL_FROM", (32, 32))
     args = make(torch.float32, head, 64, 64, 2, 2, lens, 5, False)
     q, k, v, decay, dt, rate, beta, state = args
     wide = lambda t: torch.cat([t, torch.ones(3, *t.shape[1:], device="cuda")])
@@ -143,3 +145,11 @@ def test_empty_sequences_and_rows_that_are_nobodys(KR, head, lens):
     assert not o[sum(lens):].any()
     assert float((o[:sum(lens)].view(want.shape).double() - want).norm() / want.norm()) < 1e-6
     assert float((store.view(left.shape).double() - left).norm() / left.norm()) < 1e-6
+
+
+def test_who_goes_in_chunks(KR):
+    step = lambda *lens: SimpleNamespace(n_seq=len(lens), max_new=max(lens), host_new=list(lens))
+    q, v = torch.empty(64, 2, 64, device="cuda"), torch.empty(64, 2, 64, device="cuda")
+    took = lambda batch, head: KR.delta_chunked(q, v, batch, head) > 0
+    assert took(step(32), True) and not took(step(31), True) and took(step(40, 33), True)
+    assert not took(step(47), False) and took(step(48), False) and not took(step(63, 63), False) and took(step(64, 64), False)

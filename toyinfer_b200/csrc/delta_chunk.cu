@@ -18,8 +18,8 @@
 // Hence tiles of 8 x 4 results a thread with the contraction shared out over neighbouring lanes (a thread reads 1.5 bytes a
 // multiply-add where tiles of 4 x 4 and 4 x 2 read 2 and 3) and each lane left with its part of the sums after a few exchanges:
 // a chunk takes 5,500 cycles, 2,000 of them the products with S.  2,048 tokens of 16 heads of 128 x 128, us, the scan / chunks:
-// one decay per head 632 / 228, per key channel 964 / 299; heads of 64 x 64 473 / 169 and 783 / 189; a run of 32 tokens 21.8 /
-// 15.7 and 23.6 / 24.4, of 16 tokens 14.9 / 15.4 and 16.0 / 21.8 (hence the scan below 32).
+// one decay per head 632 / 228, per key channel 964 / 299; heads of 64 x 64 473 / 169 and 783 / 189; a run of 32 tokens 21 /
+// 15 and 24 / 23, of 16 tokens 14 / 15 and 15 / 21 (where the line lies: kernels/recurrent.py).
 #include "tma.cuh"
 
 #include <type_traits>

@@ -107,21 +107,26 @@ def in_chunks(batch, least: int, blocks: int, places: int) -> Optional[int]:
     return least if batch.max_new >= 64 + 14 * min(turns, 25) else None
 
 
-# New tokens of one sequence from which the delta rule runs in chunks of 32 (csrc/delta_chunk.cu)
+# New tokens of one sequence from which the delta rule runs in chunks of 32 (csrc/delta_chunk.cu).  With a decay per key channel, of
+# one sequence and of several: making a chunk's operands takes longer.  us, token by token / chunks, heads of 128 and of 64: one
+# decay per head, 32 tokens 21 / 15 and 19 / 12, 4 x 40 44 / 43 and 23 / 23, 32 x 33 253 / 254 and 84 / 82; per channel, 32 tokens 24 /
+# 23 and 19 / 19, 40 28 / 30 and 22 / 22, 48 31 / 30 and 24 / 22, 4 x 48 53 / 52 and 25 / 32, 4 x 64 67 / 52 and 32 / 32.
 DELTA_CHUNKED_FROM = 32
+DELTA_CHANNEL_FROM = (48, 64)
 DELTA_CHUNK_SCRATCH = 1 << 30       # ... while its operands, some four floats per element of q, take no more bytes than this
 
 
-def delta_from(H: int, dim: int, vdim: int, batch, device) -> Optional[int]:
+def delta_from(H: int, dim: int, vdim: int, batch, device, head_decay: bool) -> Optional[int]:
+    least = DELTA_CHUNKED_FROM if head_decay else max(DELTA_CHUNKED_FROM, DELTA_CHANNEL_FROM[batch.n_seq > 1])
     # (a block of the walk has an SM to itself for keys of 128, half of one for keys of 64)
-    return in_chunks(batch, DELTA_CHUNKED_FROM, H * vdim // 16, (1 if dim == 128 else 2) * sm_count(device))
+    return in_chunks(batch, least, H * vdim // 16, (1 if dim == 128 else 2) * sm_count(device))
 
 
-def delta_chunked(q: torch.Tensor, v: torch.Tensor, batch) -> int:
+def delta_chunked(q: torch.Tensor, v: torch.Tensor, batch, head_decay: bool = True) -> int:
     """Floats of scratch with which a step's delta rule runs in chunks, or 0: it goes token by token."""
     M, G, dim = q.shape
     H, vdim = v.shape[1], v.shape[2]
-    if dim not in (64, 128) or vdim % 16 or delta_from(H, dim, vdim, batch, q.device) is None:
+    if dim not in (64, 128) or vdim % 16 or delta_from(H, dim, vdim, batch, q.device, head_decay) is None:
         return 0
     need = (M // 32 + batch.n_seq) * H * _fn("ti_delta_chunk_floats", [I, I])(dim, vdim)
     return need if 4 * need <= DELTA_CHUNK_SCRATCH else 0
@@ -152,7 +157,7 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
     _vec(dt_bias, n_decay, "delta_rule: the decay bias")
     _vec(rate, H, "delta_rule: the rates")
     base, stride = _state_part(state, state_offset, H * dim * vdim, "delta_rule")
-    chunked = delta_chunked(q, v, batch)
+    chunked = delta_chunked(q, v, batch, head_decay)
     single = batch.n_seq > 0 and batch.max_new == 1 and dim in (64, 128) and vdim in (64, 128) and base % 16 == 0 and stride % 4 == 0
     # rows that are nobody's are zero (the chunked and the one-token form's kernels see to it themselves)
     o = (torch.empty if chunked or single else torch.zeros)((M, H * vdim), dtype=torch.float32, device=q.device)
@@ -164,7 +169,7 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
         return o
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=q.device)
-        least = delta_from(H, dim, vdim, batch, q.device)
+        least = delta_from(H, dim, vdim, batch, q.device, head_decay)
         _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, P]),
               _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(decay_logit), decay_logit.stride(0), 1 if head_decay else 0,
               _ptr(dt_bias), _ptr(rate), _ptr(beta_logit), beta_logit.stride(0), _ptr(o), base, stride, _ptr(scratch), _ptr(batch.cu_new),
