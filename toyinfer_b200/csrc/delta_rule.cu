@@ -313,14 +313,11 @@ __global__ void head_gated_rmsnorm_vec_kernel(const float* __restrict__ o, const
     const int i = (int)(item - r * lanes) * 8, at = live ? (int)(r - m * n_heads) * vdim + i : 0;
     float x[8];
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-    T g[8];
+    struct alignas(16) Run { T v[8]; } g;
     if (live) {
         a = *reinterpret_cast<const float4*>(o + (size_t)r * vdim + i);
         b = *reinterpret_cast<const float4*>(o + (size_t)r * vdim + i + 4);
-#pragma unroll
-        for (int k = 0; k < 8 * (int)sizeof(T); k += 16)
-            *reinterpret_cast<uint4*>(reinterpret_cast<char*>(g) + k) =
-                *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(gate + (size_t)m * gate_stride + at) + k);
+        g = *reinterpret_cast<const Run*>(gate + (size_t)m * gate_stride + at);
     }
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
     float ss = 0.f;
@@ -329,16 +326,14 @@ __global__ void head_gated_rmsnorm_vec_kernel(const float* __restrict__ o, const
     for (int k = lanes >> 1; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
     if (!live) return;
     const float inv = rsqrtf(ss / (float)vdim + eps) * out_scale;
-    T y[8];
+    Run y;
 #pragma unroll
     for (int e = 0; e < 8; e++) {
-        const float gl = to_f32(g[e]);
+        const float gl = to_f32(g.v[e]);
         const float ga = (gate_silu ? gl : 1.0f) / (1.0f + expf(-gl));
-        y[e] = from_f32<T>(x[e] * inv * (w ? w[i + e] : 1.0f) * ga);
+        y.v[e] = from_f32<T>(x[e] * inv * (w ? w[i + e] : 1.0f) * ga);
     }
-#pragma unroll
-    for (int k = 0; k < 8 * (int)sizeof(T); k += 16)
-        *reinterpret_cast<uint4*>(reinterpret_cast<char*>(out + (size_t)m * out_stride + at) + k) = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(y) + k);
+    *reinterpret_cast<Run*>(out + (size_t)m * out_stride + at) = y;
 }
 
 template <typename F>

@@ -312,17 +312,15 @@ __global__ void gate_group_rmsnorm_vec_kernel(const float* __restrict__ y, const
     const bool live = part < parts;
     const long long m = live ? part / groups : 0;
     const int at = live ? (int)(part - m * groups) * gs + i : 0;
+    struct alignas(16) Run { T v[8]; };
     float u[8], ss = 0.f;
     if (live) {
         const float4 a = *reinterpret_cast<const float4*>(y + (size_t)m * inner + at), b = *reinterpret_cast<const float4*>(y + (size_t)m * inner + at + 4);
         const float yv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        T zv[8];
-#pragma unroll
-        for (int k = 0; k < 8 * (int)sizeof(T); k += 16)
-            *reinterpret_cast<uint4*>(reinterpret_cast<char*>(zv) + k) = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(z + (size_t)m * ldz + at) + k);
+        const Run zr = *reinterpret_cast<const Run*>(z + (size_t)m * ldz + at);
 #pragma unroll
         for (int e = 0; e < 8; e++) {
-            const float zi = to_f32(zv[e]);
+            const float zi = to_f32(zr.v[e]);
             u[e] = yv[e] * (zi / (1.0f + expf(-zi)));
             ss = fmaf(u[e], u[e], ss);
         }
@@ -337,12 +335,10 @@ __global__ void gate_group_rmsnorm_vec_kernel(const float* __restrict__ y, const
     const float inv = rsqrtf(all / (float)gs + eps);
     const float4 a = *reinterpret_cast<const float4*>(w + at), b = *reinterpret_cast<const float4*>(w + at + 4);
     const float wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    T r[8];
+    Run r;
 #pragma unroll
-    for (int e = 0; e < 8; e++) r[e] = from_f32<T>(u[e] * inv * wv[e]);
-#pragma unroll
-    for (int k = 0; k < 8 * (int)sizeof(T); k += 16)
-        *reinterpret_cast<uint4*>(reinterpret_cast<char*>(out + (size_t)m * inner + at) + k) = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(r) + k);
+    for (int e = 0; e < 8; e++) r.v[e] = from_f32<T>(u[e] * inv * wv[e]);
+    *reinterpret_cast<Run*>(out + (size_t)m * inner + at) = r;
 }
 
 }  // namespace
