@@ -380,7 +380,12 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
     __syncthreads();
     for (int c = 0; c < chunks; c++) {
         if (!mbar_wait(&ready[c & 1], (uint32_t)((c >> 1) & 1))) { ti_report(status, TI_STATUS_TMA_WAIT); ok = false; }
-        if (!__syncthreads_and(ok)) return;      // this chunk's operands and S are there
+        if (!__syncthreads_and(ok)) {            // (given up: not before the copies under way have arrived, or their waits have run out too)
+            if (tid == 0)
+                for (int k = c; k < min(c + 2, chunks); k++) mbar_wait(&ready[k & 1], (uint32_t)((k >> 1) & 1));
+            __syncthreads();
+            return;
+        }                                        // this chunk's operands and S are there
         const float* buf = sm + (c & 1) * BUF;
         // the products with S: 64 rows (32 keys, then 32 queries) x 16 columns; a warp has 8 rows, a lane 4 columns and an eighth of D
         float all[32];
