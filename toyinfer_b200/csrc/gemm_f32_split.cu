@@ -339,7 +339,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
         const long long chunks = unit_begin(total, g.units, unit + 1) - unit_begin(total, g.units, unit);
         if (warp_u == 16 && rank == 0 && elect_one()) {
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-            for (int it = 0; it < chunks; it++) {
+            int it = 0;
+            for (; it < chunks; it++) {
                 const int s = it % STAGES, buf = it & 1;
                 if (!mbar_wait_cluster(&acc_empty[buf], (uint32_t)(((it >> 1) & 1) ^ 1))) { ti_report(status, TI_STATUS_PIPE_WAIT); break; }
                 if (!mbar_wait_cluster(&full[s], (uint32_t)((it / STAGES) & 1))) { ti_report(status, TI_STATUS_PIPE_WAIT); break; }
@@ -359,6 +360,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                 tc_commit_pair(&empty[s]);
                 tc_commit_pair(&acc_full[buf]);
             }
+            if (it < chunks && it > 0) mbar_wait(&acc_full[(it - 1) & 1], (uint32_t)(((it - 1) >> 1) & 1));      // (given up: the products under way end first)
         } else if (warp_u == 17 && elect_one()) {
             // TMA producer of this block: its 128 weight rows and BN / 2 tokens of every chunk.  The weights too are asked for after the
             // wait: a float32 matrix may be the work of the kernel before this one.
@@ -380,6 +382,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                     tma_load_2d(to + WROWS * 128, &x_map, kc * CHUNK, tm * BN + rank * (BN / 2), &raw_full[rs]);
                 }
             }
+            // not before every copy has arrived, also where the warps that wait for them have given up
+            for (int k = max(0, it - RAWS); k < it; k++) mbar_wait(&raw_full[k % RAWS], (uint32_t)((k / RAWS) & 1));
         }
     }
     // neither block leaves, or gives back its tensor memory, while the other may still read its shared memory or arrive on its barriers
