@@ -430,6 +430,13 @@ gemm_f32_join_kernel(const SplitArgs g, int tiles_m, int nk, long long total) {
                     make_float4(sum[c + 8], sum[c + 9], sum[c + 10], sum[c + 11]), make_float4(sum[c + 12], sum[c + 13], sum[c + 14], sum[c + 15]));
 }
 
+// Whether a run of chunks ends inside a tile, so that pieces are left to be added.
+bool split_cuts(long long total, int units, int nk) {
+    for (int u = 1; u < units; u++)
+        if (unit_begin(total, units, u) % nk != 0) return true;
+    return false;
+}
+
 template <int BN>
 int launch_split(const SplitArgs& g, cudaStream_t stream) {
     constexpr size_t smem = (size_t)PARTS * split_stage_bytes<BN>() + (size_t)raw_stages<BN>() * raw_stage_bytes<BN>() + 1024;
@@ -465,9 +472,7 @@ int launch_split(const SplitArgs& g, cudaStream_t stream) {
     TI_CHECK_LAUNCH("linear (float32, tcgen05)");
     const int tiles_m = (g.M + BN - 1) / BN, tiles_n = (g.N + 2 * WROWS - 1) / (2 * WROWS), nk = (g.K + CHUNK - 1) / CHUNK;
     const long long total = (long long)tiles_m * tiles_n * nk;
-    bool cut = false;
-    for (int u = 1; u < g.units && !cut; u++) cut = unit_begin(total, g.units, u) % nk != 0;
-    if (cut) {
+    if (split_cuts(total, g.units, nk)) {
         TI_CUDA(ti_launch_class<5>(gemm_f32_join_kernel<BN>, dim3(g.units - 1, 2, BN / 32), dim3(WROWS), 0, stream, g, tiles_m, nk, total));
         TI_CHECK_LAUNCH("linear (float32, pieces)");
     }
@@ -485,11 +490,14 @@ int split_units(int M, int N, int K, int sms) {
 
 }  // namespace
 
-// Pairs of blocks and floats of workspace of a product.
-extern "C" int ti_linear_f32_plan(int M, int N, int K, int sms, int* units, long long* workspace) {
+// Pairs of blocks, floats of workspace and launches of a product.
+extern "C" int ti_linear_f32_plan(int M, int N, int K, int sms, int* units, long long* workspace, int* launches) {
     TI_REQUIRE(M > 0 && N > 0 && K > 0 && sms >= 2, "linear: bad sizes M=%d N=%d K=%d", M, N, K);
     *units = split_units(M, N, K, sms);
-    *workspace = *units > 1 ? (long long)*units * 4 * split_bn(M) * WROWS : 0;
+    const int bn = split_bn(M), nk = (K + CHUNK - 1) / CHUNK;
+    const bool cut = split_cuts((long long)((M + bn - 1) / bn) * ((N + 2 * WROWS - 1) / (2 * WROWS)) * nk, *units, nk);
+    *launches = cut ? 2 : 1;
+    *workspace = cut ? (long long)*units * 4 * split_bn(M) * WROWS : 0;
     return 0;
 }
 
@@ -501,7 +509,8 @@ extern "C" int ti_linear_f32_tc(const void* x, const void* w, void* out, int M, 
     TI_REQUIRE(M > 0 && N > 0 && K > 0, "linear: bad sizes M=%d N=%d K=%d", M, N, K);
     TI_REQUIRE(ldx % 4 == 0 && ldw % 4 == 0 && ldx >= K && ldw >= K && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0,
                "linear (float32): rows must start on 16-byte boundaries");
-    TI_REQUIRE(units >= 1 && units <= 32767 && (units == 1 || workspace != nullptr), "linear (float32): %d units without room", units);
+    TI_REQUIRE(units >= 1 && units <= 32767 && (workspace != nullptr || !split_cuts((long long)((M + split_bn(M) - 1) / split_bn(M)) *
+               ((N + 2 * WROWS - 1) / (2 * WROWS)) * ((K + CHUNK - 1) / CHUNK), units, (K + CHUNK - 1) / CHUNK)), "linear (float32): %d units without room", units);
     TI_REQUIRE(gated >= 0 && gated <= 5 && (gated < 1 || gated > 3 || N % 2 == 0), "linear (float32): unknown activation %d", gated);
     SplitArgs g{(const float*)x, (const float*)w, (float*)out, M, N, K, ldx, ldw, ldo, units, workspace, gated, gate_limit};
     switch (split_bn(M)) {

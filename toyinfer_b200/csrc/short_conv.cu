@@ -192,10 +192,11 @@ int dispatch_taps(int n, F&& f) {
 
 // x: [M, C] of the engine's type with row stride ldx; in_bias, out_bias: float32 [C] or null; taps: float32 [C, n];
 // state: float32, sequence slot s at state + s * slot_stride holds [n - 1, C]; out: [M, C] with row stride ldo (rows past the last
-// sequence's become zero).
+// sequence's become zero).  launched: the number of kernels.
 extern "C" int ti_short_conv(const void* x, long long ldx, const float* in_bias, const float* taps, const float* out_bias,
                              int act, float* state, long long slot_stride, void* out, long long ldo, const int* cu_new,
-                             const int* seq_slot, int n_seq, int max_new, int M, int C, int n_taps, int dtype, cudaStream_t stream) {
+                             const int* seq_slot, int n_seq, int max_new, int M, int C, int n_taps, int* launched, int dtype, cudaStream_t stream) {
+    *launched = 0;
     if (n_seq == 0 || max_new == 0) return 0;
     TI_REQUIRE(n_seq > 0 && n_seq <= 65535 && max_new > 0 && C > 0, "short_conv: bad sizes");
     TI_REQUIRE(n_taps >= 1 && n_taps <= MAX_TAPS, "short_conv: %d taps are not supported (1 to %d)", n_taps, MAX_TAPS);
@@ -220,10 +221,12 @@ extern "C" int ti_short_conv(const void* x, long long ldx, const float* in_bias,
                 TI_CUDA(ti_launch(short_conv_kernel<T, N>, dim3(chunks, groups, n_seq), dim3(CONV_THREADS), 0, stream, (const T*)x, ldx,
                                   in_bias, taps, out_bias, act, state, slot_stride, (T*)out, ldo, cu_new, seq_slot, C, M));
             TI_CHECK_LAUNCH("short_conv");
+            *launched = 1;
             if (chunks > 1 && N > 1) {
                 TI_CUDA(ti_launch(short_conv_tail_kernel<T, N>, dim3((C + CONV_THREADS - 1) / CONV_THREADS, n_seq), dim3(CONV_THREADS), 0, stream,
                                   (const T*)x, ldx, in_bias, state, slot_stride, cu_new, seq_slot, C, chunk));
                 TI_CHECK_LAUNCH("short_conv_tail");
+                *launched = 2;
             }
             return 0;
         });

@@ -53,12 +53,13 @@ def _need_cuda(*tensors, what: str) -> None:
             raise KernelError(f"{what}: tensors must be on a CUDA device (got {t.device}); there is no CPU path")
 
 
-def _call(fn, *args, launches: int = 1) -> None:
+def _call(fn, *args, launches=1) -> None:
+    """``launches``: how many kernels the call launches, or a ctypes integer that the call sets to that."""
     global launch_count
     rc = fn(*args)
     if rc != 0:
         raise KernelError(library().ti_last_error().decode("utf-8", "replace"))
-    launch_count += launches
+    launch_count += getattr(launches, "value", launches)
 
 
 def _i32(t: torch.Tensor, what: str) -> torch.Tensor:

@@ -97,8 +97,9 @@ def f32_eligible(x, w, M, K, ldx, ldw) -> bool:
 def run(x, w, out, M, N, K, ldx, ldw, gated: int = 0, late_start: bool = False, gate_limit: float = 0.0) -> None:
     """``gated``: 1 (or True) for up * silu(gate), 2 for up * gelu(gate) in the tanh form, 3 for the clamped pair
     g' sigmoid(1.702 g') (u' + 1) with g' = min(gate, gate_limit), u' = clamp(up, -gate_limit, gate_limit), over paired
-    weight rows; 4 and 5: no pairs, every value through the squared ReLU or gelu; only for shapes the tensor-core kernel takes (see tc_eligible).  ``late_start``: the
-    few-token kernels start only when the kernel before them has finished (csrc/gemm_skinny.cu)."""
+    weight rows; 4 and 5: no pairs, every value through the squared ReLU or gelu; only for shapes that a tensor-core kernel takes
+    (tc_eligible, f32_eligible).  ``late_start``: the few-token kernels start only when the kernel before them has finished
+    (csrc/gemm_skinny.cu)."""
     lib = library()
     out_f32 = 1 if (out.dtype == torch.float32 and x.dtype != torch.float32) else 0
     if tc_eligible(x, w, K, ldx, ldw) and M <= GEMV_MAX_TOKENS:
@@ -135,15 +136,15 @@ def run(x, w, out, M, N, K, ldx, ldw, gated: int = 0, late_start: bool = False, 
     if f32_eligible(x, w, M, K, ldx, ldw):
         sms = sm_count(x.device)
         plan = _plans.get((M, N, K, -sms))
-        if plan is None:        # (pairs of blocks, workspace floats) of this shape: asked once
-            units, ws = ctypes.c_int(), ctypes.c_longlong()
-            _call(lib.ti_linear_f32_plan, M, N, K, sms, ctypes.byref(units), ctypes.byref(ws), launches=0)
+        if plan is None:        # (pairs of blocks, workspace floats, launches) of this shape: asked once
+            units, ws, n = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
+            _call(lib.ti_linear_f32_plan, M, N, K, sms, ctypes.byref(units), ctypes.byref(ws), ctypes.byref(n), launches=0)
             if len(_plans) > 4096:
                 _plans.clear()
-            plan = _plans[(M, N, K, -sms)] = (units.value, ws.value)
+            plan = _plans[(M, N, K, -sms)] = (units.value, ws.value, n.value)
         workspace = torch.empty(plan[1], dtype=torch.float32, device=x.device) if plan[1] else None
         _call(lib.ti_linear_f32_tc, _ptr(x), _ptr(w), _ptr(out), M, N, K, ldx, ldw, out.stride(0), plan[0], _ptr(workspace), int(gated),
-              float(gate_limit), _stream(), launches=2 if plan[1] else 1)
+              float(gate_limit), _stream(), launches=plan[2])
         return
     if gated:
         raise RuntimeError("linear: the gated epilogue exists in the tensor-core kernels only")

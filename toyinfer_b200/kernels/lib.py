@@ -39,7 +39,7 @@ def _declare(lib) -> None:
         "ti_attn_chunk_mma": [P, P, P, P, L, L, L, L, P, P, P, I, I, I, I, I, I, F, I, P, P, P, I, I, I, I, P],
         "ti_attn_chunk_tc": [P, P, P, P, L, L, L, L, P, P, P, I, I, I, I, I, I, F, I, P, P, P, I, I, I, I, P],
         "ti_linear_tc": [P, P, P, I, I, I, L, L, L, I, I, F, I, P, P, P],
-        "ti_linear_f32_plan": [I, I, I, I, P, P],
+        "ti_linear_f32_plan": [I, I, I, I, P, P, P],
         "ti_linear_f32_tc": [P, P, P, I, I, I, L, L, L, I, P, I, F, P],
         "ti_linear_gemv": [P, P, P, I, I, I, L, L, L, I, I, F, I, I, P],
         "ti_linear_skinny": [P, P, P, I, I, I, L, L, L, I, I, F, I, I, P],

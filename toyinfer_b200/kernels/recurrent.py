@@ -5,7 +5,7 @@ Every state lives in one float32 tensor per schedule entry, [slots, n]: a kernel
 slot 0 and the distance between slots."""
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import byref, c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
 import torch
@@ -48,10 +48,11 @@ def short_conv(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, state_o
     base, stride = _state_part(state, state_offset, (n - 1) * C, "short_conv")
     # rows that are nobody's are zero: the kernel sees to it where a sequence brings tokens
     out = (torch.empty if batch.n_seq and batch.max_new else torch.zeros)((M, C), dtype=x.dtype, device=x.device)
-    _call(_fn("ti_short_conv", [P, L, P, P, P, I, P, L, P, L, P, P, I, I, I, I, I, I, P]),
+    launched = c_int()
+    _call(_fn("ti_short_conv", [P, L, P, P, P, I, P, L, P, L, P, P, I, I, I, I, I, P, I, P]),
           _ptr(x), x.stride(0), _ptr(in_bias), _ptr(taps), _ptr(out_bias), ACTS[act], base, stride, _ptr(out), C,
-          _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, C, n, _code(x, "short_conv"), _stream(),
-          launches=2 if (batch.max_new > (16 if n <= 4 else 64) and n > 1) else 1)
+          _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, C, n, byref(launched), _code(x, "short_conv"), _stream(),
+          launches=launched)
     return out
 
 
