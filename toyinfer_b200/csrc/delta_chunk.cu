@@ -532,7 +532,7 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
 template <typename T, typename L, int D, bool HEAD>
 int run_chunks(const void* q, const void* k, const void* v, long long q_stride, long long k_stride, long long v_stride, const void* decay_logit,
                long long decay_stride, const float* dt_bias, const float* rate, const void* beta_logit, long long beta_stride, float* o,
-               float* state, long long slot_stride, const DeltaChunkArgs& a, int n_seq, int max_new, int M, cudaStream_t stream) {
+               float* state, long long slot_stride, const DeltaChunkArgs& a, int n_seq, int max_new, int M, int sms, cudaStream_t stream) {
     constexpr size_t prep = prep_smem_floats<D, HEAD>() * sizeof(float), smem = state_smem_bytes<D>();
     constexpr size_t ALONE = 120 * 1024;        // shared memory of a block that shares its SM with no other
     int* status = ti_status_ptr();
@@ -550,7 +550,7 @@ int run_chunks(const void* q, const void* k, const void* v, long long q_stride, 
     // blocks that have an SM each must not start two on the SM that the kernel before left first: the walk is a chain, and its
     // time is the slowest block's (64 blocks of 64 x 16: 245 us, spread out 169)
     const long long blocks = (long long)a.n_heads * (a.vdim / DC_COLS) * n_seq;
-    const size_t room = blocks <= 148 && smem < ALONE ? ALONE : smem;
+    const size_t room = blocks <= sms && smem < ALONE ? ALONE : smem;
     TI_CUDA(ti_launch(delta_chunk_state_kernel<D>, dim3(a.n_heads * (a.vdim / DC_COLS), n_seq), dim3(DC_THREADS), room, stream, a, o, M, state,
                       slot_stride, status));
     TI_CHECK_LAUNCH("delta_rule (chunk states)");
@@ -564,12 +564,12 @@ extern "C" int ti_delta_chunk_floats(int dim, int vdim) { return (dim == 64 ? Op
 
 // As ti_delta_rule_scan (delta_rule.cu), for dim 64 or 128 and vdim a multiple of 16.  max_new: at least the most new tokens of
 // a sequence.  Sequences of fewer than `least` new tokens are passed over (ti_delta_rule_scan takes those up to its `most`).
-// scratch: float32, 16-byte aligned, (M / 32 + n_seq) * heads * ti_delta_chunk_floats(dim, vdim) values.
+// sms: the device's SMs.  scratch: float32, 16-byte aligned, (M / 32 + n_seq) * heads * ti_delta_chunk_floats(dim, vdim) values.
 extern "C" int ti_delta_rule_chunked(const void* q, const void* k, const void* v, long long q_stride, long long k_stride,
                                      long long v_stride, const void* decay_logit, long long decay_stride, int head_decay,
                                      const float* dt_bias, const float* rate, const void* beta_logit, long long beta_stride, float* o,
                                      float* state, long long slot_stride, float* scratch, const int* cu_new, const int* seq_slot, int n_seq,
-                                     int max_new, int M, int n_heads, int qk_heads, int dim, int vdim, int least, int dtype,
+                                     int max_new, int M, int n_heads, int qk_heads, int dim, int vdim, int least, int sms, int dtype,
                                      cudaStream_t stream) {
     if (n_seq == 0 || M == 0) return 0;
     TI_REQUIRE(n_seq > 0 && n_seq <= 65535 && M > 0 && max_new > 0 && n_heads > 0 && n_heads <= 65535 && qk_heads > 0 && n_heads % qk_heads == 0 && scratch,
@@ -586,9 +586,9 @@ extern "C" int ti_delta_rule_chunked(const void* q, const void* k, const void* v
             constexpr int D = decltype(dc)::value;
             if (head_decay)
                 return run_chunks<T, T, D, true>(q, k, v, q_stride, k_stride, v_stride, decay_logit, decay_stride, dt_bias, rate, beta_logit, beta_stride, o,
-                                                 state, slot_stride, a, n_seq, max_new, M, stream);
+                                                 state, slot_stride, a, n_seq, max_new, M, sms, stream);
             return run_chunks<T, float, D, false>(q, k, v, q_stride, k_stride, v_stride, decay_logit, decay_stride, dt_bias, rate, beta_logit, beta_stride, o,
-                                                  state, slot_stride, a, n_seq, max_new, M, stream);
+                                                  state, slot_stride, a, n_seq, max_new, M, sms, stream);
         };
         return dim == 64 ? go(std::integral_constant<int, 64>()) : go(std::integral_constant<int, 128>());
     });

@@ -416,7 +416,7 @@ ssd_chunk_out_kernel(SsdArgs g, int run, int M) {
 }
 
 template <int N, int V>
-int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t stream) {
+int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, int sms, cudaStream_t stream) {
     constexpr size_t state_smem = (size_t)SC * N * 2 + 2 * SC * 64 * 2, out_smem = std::max<size_t>((size_t)SC * N * 4, (size_t)2 * SC * 64 * 2 + V * N * 10);
     static bool configured = false;
     if (!configured) {
@@ -428,8 +428,8 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t
     const int per_group = g.heads / g.groups;
     // chunks that there can be: sequences that bring fewer tokens than the longest leave blocks of the grid without work
     const long long live = std::min((long long)chunks * n_seq, (long long)M / SC + std::min(n_seq, g.least > 0 ? M / g.least : n_seq)) * g.groups;
-    int state_run = std::min(STATE_RUN, per_group);       // (heads share B; as long as two blocks an SM are left)
-    while (state_run > 1 && live * ((per_group + state_run - 1) / state_run) < 200) state_run /= 2;
+    int state_run = std::min(STATE_RUN, per_group);       // (heads share B, as long as most SMs have two blocks left)
+    while (state_run > 1 && live * ((per_group + state_run - 1) / state_run) < 4 * sms / 3) state_run /= 2;
     TI_CUDA(ti_launch(ssd_chunk_state_kernel<N, V>, dim3(chunks, g.groups * ((per_group + state_run - 1) / state_run), n_seq), dim3(SSD_THREADS),
                       state_smem, stream, g, state_run));
     TI_CHECK_LAUNCH("ssd_scan (chunks' parts)");
@@ -441,7 +441,7 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t
     double best = 0.0;
     for (int r = 1; r <= std::min(8, per_group); r++) {
         const long long blocks = live * ((per_group + r - 1) / r);
-        const double cost = (double)((blocks + 147) / 148) * (1.3 + r);
+        const double cost = (double)((blocks + sms - 1) / sms) * (1.3 + r);
         if (r == 1 || cost < best) { best = cost; run = r; }
     }
     TI_CUDA(ti_launch(ssd_chunk_out_kernel<N, V>, dim3(chunks, g.groups * ((per_group + run - 1) / run), n_seq), dim3(SSD_THREADS), out_smem, stream, g, run, M));
@@ -453,10 +453,10 @@ int run_ssd_chunks(const SsdArgs& g, int n_seq, int max_new, int M, cudaStream_t
 
 // As ti_ssd_scan (ssd_scan.cu), for bfloat16 tokens, N 64 or 128 and vdim 32 or 64; rows of xbc on 16-byte boundaries.  max_new:
 // at least the most new tokens of a sequence.  Sequences of fewer than `least` are passed over (ti_ssd_scan takes those up to its
-// `most`).  scratch: float32, 16-byte aligned, (M / 128 + n_seq) * heads * (vdim * N + 1) values.
+// `most`).  sms: the device's SMs.  scratch: float32, 16-byte aligned, (M / 128 + n_seq) * heads * (vdim * N + 1) values.
 extern "C" int ti_ssd_chunked(const void* xbc, long long ld_xbc, const void* dt_raw, long long ld_dt, const float* dt_bias,
                               const float* rate, const float* skip, float* state, long long slot_stride, float* y, const int* cu_new,
-                              const int* seq_slot, int n_seq, int max_new, int M, int heads, int groups, int N, int vdim, int least, float* scratch,
+                              const int* seq_slot, int n_seq, int max_new, int M, int heads, int groups, int N, int vdim, int least, int sms, float* scratch,
                               cudaStream_t stream) {
     if (n_seq == 0 || M == 0) return 0;
     TI_REQUIRE(n_seq > 0 && n_seq <= 65535 && M > 0 && max_new > 0 && heads > 0 && heads <= 65535 && groups > 0 && heads % groups == 0 && scratch,
@@ -466,6 +466,6 @@ extern "C" int ti_ssd_chunked(const void* xbc, long long ld_xbc, const void* dt_
                (reinterpret_cast<uintptr_t>(y) & 15) == 0, "ssd_scan: rows must start on 16-byte boundaries");
     SsdArgs g{(const bf16*)xbc, ld_xbc, (const bf16*)dt_raw, ld_dt, dt_bias, rate, skip, state, slot_stride, y, cu_new, seq_slot, heads, groups, least,
               scratch, scratch + (size_t)(M / SC + n_seq) * heads * vdim * N};
-    if (N == 64) return vdim == 32 ? run_ssd_chunks<64, 32>(g, n_seq, max_new, M, stream) : run_ssd_chunks<64, 64>(g, n_seq, max_new, M, stream);
-    return vdim == 32 ? run_ssd_chunks<128, 32>(g, n_seq, max_new, M, stream) : run_ssd_chunks<128, 64>(g, n_seq, max_new, M, stream);
+    if (N == 64) return vdim == 32 ? run_ssd_chunks<64, 32>(g, n_seq, max_new, M, sms, stream) : run_ssd_chunks<64, 64>(g, n_seq, max_new, M, sms, stream);
+    return vdim == 32 ? run_ssd_chunks<128, 32>(g, n_seq, max_new, M, sms, stream) : run_ssd_chunks<128, 64>(g, n_seq, max_new, M, sms, stream);
 }

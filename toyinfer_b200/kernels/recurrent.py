@@ -124,7 +124,7 @@ def delta_from(H: int, dim: int, vdim: int, batch, device, head_decay: bool) -> 
 
 
 def delta_chunked(q: torch.Tensor, v: torch.Tensor, batch, head_decay: bool = True) -> int:
-    """Floats of scratch with which a step's delta rule runs in chunks, or 0: it goes token by token."""
+    """Floats of scratch with which a step's delta rule runs in chunks (all of it or its long sequences), or 0: it goes token by token."""
     M, G, dim = q.shape
     H, vdim = v.shape[1], v.shape[2]
     if dim not in (64, 128) or vdim % 16 or delta_from(H, dim, vdim, batch, q.device, head_decay) is None:
@@ -171,10 +171,11 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logit: t
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=q.device)
         least = delta_from(H, dim, vdim, batch, q.device, head_decay)
-        _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, P]),
+        _call(_fn("ti_delta_rule_chunked", [P, P, P, L, L, L, P, L, I, P, P, P, L, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, I, P]),
               _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(decay_logit), decay_logit.stride(0), 1 if head_decay else 0,
               _ptr(dt_bias), _ptr(rate), _ptr(beta_logit), beta_logit.stride(0), _ptr(o), base, stride, _ptr(scratch), _ptr(batch.cu_new),
-              _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, H, G, dim, vdim, least, _code(q, "delta_rule"), _stream(), launches=2)
+              _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, H, G, dim, vdim, least, sm_count(q.device), _code(q, "delta_rule"),
+              _stream(), launches=2)
         if least == 0:
             return o
     # unit queries and keys, decays and betas of all tokens, made by a kernel of their own before the recurrence
@@ -239,11 +240,15 @@ SSD_CHUNK_SCRATCH = 1 << 30     # ... while the chunks' states take no more byte
 
 
 def ssd_from(n_heads: int, batch, device) -> Optional[int]:
+    # (of the states of 64 heads that a short sequence's chunk reads and writes, some two thirds of an SM's worth take turns; us, 64
+    # heads of 64 x 128, token by token / all in chunks / shared out: 100 tokens and 2 single ones 41 / 35 / 38, 160 and 4 63 / 46 /
+    # 47, 160 and 8 64 / 80 / 53, 256 and 32 106 / 218 / 97, 512 and 32 241 / 227 / 118, 2,048 and 32 512 / 330 / 163)
     return in_chunks(batch, SSD_CHUNKED_FROM, n_heads, 2 * sm_count(device) // 5)
 
 
 def ssd_chunked(xbc: torch.Tensor, n_heads: int, n_state: int, vdim: int, batch) -> int:
-    """Floats of scratch with which a step's Mamba-2 recurrence runs in chunks (csrc/ssd_chunk.cu), or 0: token by token."""
+    """Floats of scratch with which a step's Mamba-2 recurrence runs in chunks (csrc/ssd_chunk.cu; all of it or its long
+    sequences), or 0: token by token."""
     if (ssd_from(n_heads, batch, xbc.device) is None or xbc.dtype != torch.bfloat16 or n_state not in (64, 128) or vdim not in (32, 64)
             or xbc.stride(0) % 8 or xbc.data_ptr() % 16):
         return 0
@@ -256,8 +261,10 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, rat
     """The Mamba-2 recurrence over every sequence's new tokens (csrc/ssd_scan.cu).  xbc [M, heads * vdim + 2 * groups *
     n_state]: x, B and C after their convolution and silu; dt_raw [M, heads] the raw step sizes (rows may be strided);
     dt_bias, rate (= exp(A_log)) and skip float32 [heads].  Returns float32 y [M, heads * vdim]; the state
-    [heads, vdim, n_state] per slot is left as it is after the step's tokens.  Sequences that bring more than
-    ``2 * SSD_SEGMENT`` tokens run as segments in parallel (three launches)."""
+    [heads, vdim, n_state] per slot is left as it is after the step's tokens.  bfloat16 sequences of SSD_CHUNKED_FROM tokens and
+    more go in chunks on the tensor cores (csrc/ssd_chunk.cu: three launches; in_chunks says which of a step's sequences do);
+    else sequences that bring ``2 * SSD_SEGMENT`` tokens and more run as segments in parallel (three launches), and others token
+    by token."""
     _need_cuda(xbc, dt_raw, dt_bias, rate, skip, state, what="ssd_scan")
     M = xbc.shape[0]
     inner = n_heads * vdim
@@ -274,10 +281,10 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, rat
     if chunked:
         scratch = torch.empty(chunked, dtype=torch.float32, device=xbc.device)
         least = ssd_from(n_heads, batch, xbc.device)
-        _call(_fn("ti_ssd_chunked", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, I, P, P]),
+        _call(_fn("ti_ssd_chunked", [P, L, P, L, P, P, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, P, P]),
               _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0), _ptr(dt_bias), _ptr(rate), _ptr(skip), base, stride, _ptr(y),
               _ptr(batch.cu_new), _ptr(batch.seq_slot), batch.n_seq, batch.max_new, M, int(n_heads), int(groups), int(n_state), int(vdim),
-              least, _ptr(scratch), _stream(), launches=3)
+              least, sm_count(xbc.device), _ptr(scratch), _stream(), launches=3)
         if least == 0:
             return y
     seg = int(SSD_SEGMENT)
