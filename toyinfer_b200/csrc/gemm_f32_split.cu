@@ -10,6 +10,10 @@
 // contraction: a chunk of 32 is multiplied into one of two accumulators (the five small products first, then hi * hi, whose two
 // MMAs are the only ones that truncate at the size of the result), and the epilogue warps add it to sums in registers,
 // rounded to nearest, while the next chunk goes into the other.
+// What the two large MMAs of a chunk cut off is left: results come out 4 to 5e-8 too small.  Error against 64 bits (2-norm) at
+// contractions of 64 / 2,560 / 9,728, this and FFMA tiles: operands of mixed signs 0.6, 1.1, 1.4e-7 and 1.4, 2.2, 2.6e-7; of one sign,
+// where every cut errs the same way, 0.6, 0.8, 1.0e-7 and 1.2, 0.7, 1.2e-7.  The few-row kernel, whose 9 to 16 tokens of a large
+// matrix come here, is at 1.0 to 3.2e-7 on mixed signs (this 0.9 to 1.5e-7) and at 0.3 to 0.5e-7 on one sign (0.7 to 1.1e-7).
 //
 // What bounds it: six bfloat16 MMAs per product (a sixth of the bfloat16 rate); beside them, per chunk of a tile of 256 x 256
 // on a pair of SMs (1,536 cycles of MMA), a block's issue slots are about a quarter splitting its 256 rows of operands and a
@@ -143,27 +147,9 @@ __device__ __noinline__ void redo16(const SplitArgs& g, int m0, int n, unsigned 
     }
 }
 
-// Sixteen results of a thread: tokens m0 .. m0 + 15 of weight row n (lanes are consecutive n); all lanes of a warp call it
-// together.  One copy of the code for all columns of a tile: written out for each of 128 columns it was fetched from L2
-// instruction by instruction, 40 us a tile.
-__device__ __noinline__ void store16(const SplitArgs& g, int m0, int n, float4 a, float4 b, float4 c, float4 d) {
-    float v[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
-    float probe = 0.f;                  // not a number as soon as one of them is not finite
-#pragma unroll
-    for (int e = 0; e < 16; e++) probe = fmaf(v[e], 0.f, probe);
+// Stores sixteen results of a thread: tokens m0 .. m0 + 15 of weight row n (lanes are consecutive n).
+__device__ __forceinline__ void put16(const SplitArgs& g, int m0, int n, float (&v)[16]) {
     const int live = min(16, g.M - m0);
-    if (__any_sync(0xffffffffu, probe != 0.f)) {
-        float again[16];
-        unsigned bad = 0;
-#pragma unroll
-        for (int e = 0; e < 16; e++) {
-            again[e] = v[e];
-            if (e < live && n < g.N && !isfinite(v[e])) bad |= 1u << e;
-        }
-        redo16(g, m0, n, bad, again);
-#pragma unroll
-        for (int e = 0; e < 16; e++) v[e] = again[e];
-    }
     if (g.gated >= 1 && g.gated <= 3) {
         float* o = g.out + (size_t)m0 * g.ldo + (n >> 1);
         const bool mine = n < g.N && (n & 1) == 0;
@@ -183,6 +169,28 @@ __device__ __noinline__ void store16(const SplitArgs& g, int m0, int n, float4 a
 #pragma unroll
     for (int e = 0; e < 16; e++)
         if (e < live) o[(size_t)e * g.ldo] = v[e];
+}
+
+// The same where one of a warp's results is not finite.
+__device__ __noinline__ void store16_again(const SplitArgs& g, int m0, int n, float4 a, float4 b, float4 c, float4 d) {
+    float v[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+    unsigned bad = 0;
+#pragma unroll
+    for (int e = 0; e < 16; e++)
+        if (m0 + e < g.M && n < g.N && !isfinite(v[e])) bad |= 1u << e;
+    redo16(g, m0, n, bad, v);
+    put16(g, m0, n, v);
+}
+
+// All lanes of a warp call it together.  One copy of the code for all columns of a tile: written out for each of 128 columns it was
+// fetched from L2 instruction by instruction, 40 us a tile.
+__device__ __noinline__ void store16(const SplitArgs& g, int m0, int n, float4 a, float4 b, float4 c, float4 d) {
+    float v[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+    float probe = 0.f;                  // not a number as soon as one of them is not finite
+#pragma unroll
+    for (int e = 0; e < 16; e++) probe = fmaf(v[e], 0.f, probe);
+    if (__any_sync(0xffffffffu, probe != 0.f)) store16_again(g, m0, n, a, b, c, d);
+    else put16(g, m0, n, v);
 }
 
 __host__ __device__ __forceinline__ long long unit_begin(long long total, int units, int u) { return total * u / units; }
@@ -420,8 +428,12 @@ gemm_f32_join_kernel(const SplitArgs g, int tiles_m, int nk, long long total) {
         const long long b = unit_begin(total, g.units, v);
         const int place = (b >= t0 ? 0 : 1);                                // the unit's run begins inside this tile, or before it
         const float* ws = ti_dependent(g.workspace) + (((size_t)v * 2 + place) * 2 + rank) * (size_t)(BN * WROWS) + (size_t)j0 * WROWS + threadIdx.x;
+        float x[32];                    // (a piece's numbers all on their way together)
 #pragma unroll
-        for (int j = 0; j < 32; j++) sum[j] += __ldcg(ws + (size_t)j * WROWS);
+        for (int j = 0; j < 32; j++) x[j] = __ldcg(ws + (size_t)j * WROWS);
+        asm volatile("" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 32; j++) sum[j] += x[j];
     }
 #pragma unroll
     for (int c = 0; c < 32; c += 16)
