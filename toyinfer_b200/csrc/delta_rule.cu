@@ -298,7 +298,7 @@ __global__ void head_gated_rmsnorm_kernel(const float* __restrict__ o, const T* 
 }
 
 // The same where rows can be read 16 bytes at a time: vdim / 8 lanes a head (a power of two up to 32), eight values a lane, read
-// once.
+// once.  Rows of 16 heads of 128, us: 32 tokens 2.5 -> 1.9, 2,048 12.8 -> 7.7.
 template <typename T>
 __global__ void head_gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long gate_stride,
                                               const float* __restrict__ w, T* __restrict__ out, long long out_stride, long long rows,

@@ -387,8 +387,8 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const T* __res
 }
 
 // The same where rows can be read 16 bytes at a time: a thread holds eight values of its row, read
-// once, gate and weight with them.  Bound by latency: a row of 4,096 was a chain of 16 dependent reads a thread, twice over; 32
-// tokens of a decode step's layer 50 -> 44 us a pass.
+// once, gate and weight with them.  Bound by latency: a row of 4,096 was a chain of 16 dependent reads a thread, twice over: 32
+// tokens 10.3 -> 2.2 us, rows of 2,048 5.6 -> 1.9, 2,048 such rows 12.4 -> 6.7.
 template <typename T>
 __global__ void gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ g, long long g_stride,
                                          const float* __restrict__ w, T* __restrict__ out, int N, float eps) {

@@ -14,8 +14,9 @@
 // (other blocks still read the old state while the chunk with the last tokens is at work).
 //
 // short_conv_vec: the same for up to four taps and rows that can be read four channels at a time: a thread owns
-// four channels and walks 16 tokens, eight rows on their way together.  2,048 tokens of 6,144 channels: 36 us a thread a channel
-// (a wait for memory per token), 21 so; eight channels a thread took 40 (162 registers: three blocks an SM).
+// four channels and walks 16 tokens, eight rows on their way together.  2,048 tokens of 6,144 channels: 39 us a thread a channel
+// (a wait for memory per token), 27 so (float32 47 and 32); 64 tokens 17 and 8.  Eight channels a thread: 162 registers, three
+// blocks an SM, twice the time.
 // Rows past the last sequence's are nobody's; they are set to zero.
 #include "common.cuh"
 
