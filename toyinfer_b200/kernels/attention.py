@@ -25,7 +25,7 @@ def check_supported(n_heads: int, n_kv_heads: int, head_dim: int, dtype) -> None
     if not tensor_cores:
         if group * head_dim > 32 * 128:
             raise KernelError(f"attention_decode: {group} query heads per kv head of size {head_dim} exceed this kernel's "
-                              f"{32 * 128} outputs per block")
+                              f"{32 * 128} outputs per kv head")
         smem = (group * head_dim + 64 * (head_dim + 1) + 64 * head_dim + group * 64 + 3 * group) * 4
         if smem > 227 * 1024:
             raise KernelError(f"attention_decode: {group} query heads per kv head of size {head_dim} need {smem} bytes "
@@ -52,7 +52,7 @@ def prefill(q, k, v, out, scale, window, batch) -> None:
           _code(q, "attention_prefill"), _stream())
 
 
-MAX_CLUSTER = 16     # splits that the tensor-core decode kernel merges itself, as one thread-block cluster
+MAX_CLUSTER = 16     # splits that the decode kernels merge themselves, as one thread-block cluster
 
 
 def chunk(q, k, v, mem, out, scale, window, batch) -> None:
@@ -177,7 +177,7 @@ def decode(q, mem, out, scale, window, batch) -> None:
           _ptr(pt), pt.shape[1], mem.page_size, mem.ring_rows, mem.k_pages.shape[0],
           _ptr(batch.seq_slot), _ptr(batch.seq_len), B, nh, nkv, hd, scale, window, splits,
           _ptr(out), out.stride(0), _ptr(part_o), _ptr(part_ml), _code(q, "attention_decode"), *extra, _stream(),
-          launches=2 if (splits > 1 and mode != 2) else 1)
+          launches=2 if splits > (1 if tensor_cores else MAX_CLUSTER) and mode != 2 else 1)
 
 
 def decode_fused_eligible(q, k, v, q_w, k_w, tables, mem) -> bool:
