@@ -79,3 +79,56 @@ def test_padded_plan(counts):
         at += 128 * pad
     assert torch.equal(src.cpu(), want_src) and torch.equal(tile.cpu(), want_tile)
     assert torch.equal(src[place.long()], torch.arange(n, dtype=torch.int32, device="cuda"))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,E,top,H", [(1, 1, 1, 8), (3, 8, 8, 264), (40, 9, 2, 1024), (777, 16, 2, 2048), (4099, 17, 1, 136), (600, 32, 16, 1032)])
+@pytest.mark.parametrize("kind", ["plain", "biased", "corrected"])
+def test_router_with_its_product(dtype, M, E, top, H, kind):
+    from toyinfer_b200.kernels import moe as KM
+    g = torch.Generator(device="cuda").manual_seed(M + E + H)
+    x = torch.randn(M, H + 8, generator=g, device="cuda").to(dtype)[:, :H]
+    w = (torch.randn(E, H, generator=g, device="cuda") / H ** 0.5).to(dtype)
+    extra = 0.1 * torch.randn(E, generator=g, device="cuda")
+    bias, corr = (extra if kind == "biased" else None), (extra if kind == "corrected" else None)
+    z = x.double() @ w.double().T + (bias.double() if bias is not None else 0)
+    s = torch.softmax(z, dim=1)
+    c = s + corr if corr is not None else z
+    ff = 64
+    assert KM.route_rows_eligible(x, w, 0, top)
+    perm, off, weight, plan = KM.route_rows(x, w, corr, top, 1.5, bias, ff)
+    chosen = choose(c, top)
+    want = 1.5 * s.gather(1, chosen) / s.gather(1, chosen).sum(1, keepdim=True)
+    # sums of H products and an exponential in 32 bits; tokens whose choices lie within 1e-5 may fall either way
+    order = torch.sort(c, dim=1, descending=True).values
+    sure = (order[:, :-1] - order[:, 1:])[:, :top].amin(1) > 1e-5 if E > 1 else torch.ones(M, dtype=torch.bool, device="cuda")
+    torch.testing.assert_close(weight.view(M, top).double()[sure], want[sure], rtol=1e-5, atol=0)
+    assert (plan is not None) == (dtype == torch.bfloat16 and M * top >= KM.TC_MIN_GROUP * E)
+    if plan is None:
+        runs = perm.long(), off.long()
+    else:
+        pad_src, place, tile = plan
+        assert torch.equal(pad_src[place.long()].long(), torch.arange(M * top, device="cuda") // top)
+        assert int((pad_src >= 0).sum()) == M * top
+        e_of = tile[place.long() // 128].long()
+        runs = e_of.sort(stable=True).indices, torch.cat([torch.zeros(1, dtype=torch.long, device="cuda"), torch.bincount(e_of, minlength=E).cumsum(0)])
+    perm, off = runs
+    assert torch.equal(perm.sort().values, torch.arange(M * top, device="cuda"))
+    for e in range(E):
+        mine = torch.zeros(M * top, dtype=torch.bool, device="cuda")
+        mine[perm[int(off[e]):int(off[e + 1])]] = True
+        wrong = mine != (chosen.reshape(-1) == e)
+        assert not (wrong.view(M, top) & sure[:, None]).any()
+
+
+def test_router_with_its_product_not_a_number():
+    """The lowest open expert is kept against every other where its score is not a number; elsewhere such a score never wins."""
+    from toyinfer_b200.kernels import moe as KM
+    x, w = torch.eye(8, device="cuda")[:3].contiguous(), torch.zeros(4, 8, device="cuda")
+    nan = float("nan")
+    w[:, 0] = torch.tensor([nan, 3.0, 2.0, 1.0])          # x = unit vectors: a row's logits are w's columns; 0 * nan reaches the others
+    perm, off, _, _ = KM.route_rows(x[:1].contiguous(), w, None, 2, 1.0, None, 64)
+    assert sorted(perm.tolist()) == [0, 1] and off.tolist() == [0, 1, 2, 2, 2]
+    w[:, 0] = torch.tensor([0.0, nan, -0.0, -1.0])
+    perm, off, _, _ = KM.route_rows(x[:1].contiguous(), w, None, 2, 1.0, None, 64)
+    assert off.tolist() == [0, 1, 2, 2, 2] or off.tolist() == [0, 1, 1, 2, 2]

@@ -7,14 +7,14 @@
 // The order inside a group is whatever the atomics gave; no result depends on it, since every
 // pair's rows are computed for themselves.
 //
-// `moe_grouped` is the product kernel, used twice:
+// `moe_grouped` is the product, used twice:
 //   first product   rows of x gathered by pair (token perm[i] / top), expert e's gate and up
 //                   matrices, then the expert's activation, into y[i] (places, grouped)
 //   second product  rows y[i], expert e's down matrix, result scattered to z[perm[i]] (pairs in
 //                   the tokens' order), scaled by the pair's weight
-// Tiles of 32 places x 64 weight rows; a tile lies inside one expert's group (groups are
-// walked tile by tile: the grid has an upper bound of tiles, ceil(P / 32) + experts).
-// Arithmetic on the CUDA cores in 32-bit; operands of the engine's type.
+// A tile of places lies inside one expert's group (groups are walked tile by tile: the grid has an upper bound of tiles,
+// ceil(P / tile) + experts).  32-bit operands, and bfloat16 groups of few places, run from registers (moe_rows.cuh); bfloat16
+// groups of some tens of places as shared-memory tiles on mma.sync (below), of many on tcgen05 (gemm_tcgen05_grouped.cu).
 //
 // `moe_combine`: out[m] = sum_j z[m * top + j], summed in the order of j.
 //
@@ -22,6 +22,7 @@
 // y = g' * sigmoid(alpha * g') * (u' + shift).  (limit = infinity, alpha = 1, shift = 0: silu(g) * u.)
 // `relu2` (the dense feed-forward's activation, x -> max(x, 0)^2) is here as well.
 #include "common.cuh"
+#include "moe_rows.cuh"
 
 namespace {
 
@@ -62,119 +63,18 @@ __global__ void moe_route_table_kernel(const int* __restrict__ ids, const int* _
     }
 }
 
-constexpr int GM = 32, GN = 64, GK = 32, G_THREADS = 256;
-
-enum { ACT_NONE = 0, ACT_CLAMPED_SWISH = 1 };
-
-// A: rows of `a` ([*, K], row stride lda); row of place i is a[(GATHER ? perm[i] / top : i)].
-// W: [n_experts, N, K] (and W2 of the same shape when PAIR: the up matrix beside the gate matrix).
-// out: PAIR -> y[i, n] = act(gate, up);  else z[(SCATTER ? perm[i] : i), n] = product * scale.
-template <typename T, bool PAIR>
-__global__ void __launch_bounds__(G_THREADS)
-moe_grouped_kernel(const T* __restrict__ a, long long lda, const T* __restrict__ W, const T* __restrict__ W2,
-                   T* __restrict__ out, long long ldo, const int* __restrict__ perm, const int* __restrict__ off,
-                   int n_experts, int N, int K, int top, int gather, int scatter, float scale, float limit, float alpha, float shift,
-                   long long w_estride) {
-    ti_pdl_trigger();
-    __shared__ float As[GK][GM + 1];
-    __shared__ float Ws[GK][GN + 1];
-    __shared__ float W2s[PAIR ? GK : 1][GN + 1];
-    __shared__ int rows[GM];
-    __shared__ int where[3];             // expert, first place, places in the tile
-    ti_pdl_sync();
-    a = ti_dependent(a); perm = ti_dependent(perm); off = ti_dependent(off);
-    if (threadIdx.x == 0) {
-        // tile blockIdx.x of the walk over the groups
-        int t = blockIdx.x, e = 0, found = -1, first = 0, cnt = 0;
-        for (; e < n_experts; e++) {
-            const int lo = off[e], hi = off[e + 1];
-            const int tiles = (hi - lo + GM - 1) / GM;
-            if (t < tiles) { found = e; first = lo + t * GM; cnt = min(GM, hi - first); break; }
-            t -= tiles;
-        }
-        where[0] = found; where[1] = first; where[2] = cnt;
-    }
-    __syncthreads();
-    const int e = where[0], first = where[1], cnt = where[2];
-    if (e < 0) return;
-    const int n0 = blockIdx.y * GN;
-    if (threadIdx.x < GM) {
-        const int i = first + threadIdx.x;
-        int r = -1;
-        if (threadIdx.x < cnt) r = gather ? perm[i] / top : i;
-        rows[threadIdx.x] = r;
-    }
-    __syncthreads();
-    const T* We = W + (size_t)e * w_estride;
-    const T* W2e = PAIR ? W2 + (size_t)e * w_estride : nullptr;
-    // thread (ty, tx): places ty, ty + 8, ty + 16, ty + 24; weight rows tx, tx + 32
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    float acc[4][2], acc2[4][2];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++) { acc[i][j] = 0.f; acc2[i][j] = 0.f; }
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        for (int idx = threadIdx.x; idx < GM * GK; idx += G_THREADS) {
-            const int r = idx / GK, kk = idx - r * GK;
-            const int src = rows[r];
-            As[kk][r] = (src >= 0 && k0 + kk < K) ? to_f32(a[(size_t)src * lda + k0 + kk]) : 0.f;
-        }
-        for (int idx = threadIdx.x; idx < GN * GK; idx += G_THREADS) {
-            const int r = idx / GK, kk = idx - r * GK;
-            const bool ok = n0 + r < N && k0 + kk < K;
-            Ws[kk][r] = ok ? to_f32(We[(size_t)(n0 + r) * K + k0 + kk]) : 0.f;
-            if constexpr (PAIR) W2s[kk][r] = ok ? to_f32(W2e[(size_t)(n0 + r) * K + k0 + kk]) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int kk = 0; kk < GK; kk++) {
-            float av[4], wv[2], w2v[2];
-#pragma unroll
-            for (int i = 0; i < 4; i++) av[i] = As[kk][ty + 8 * i];
-#pragma unroll
-            for (int j = 0; j < 2; j++) { wv[j] = Ws[kk][tx + 32 * j]; w2v[j] = PAIR ? W2s[kk][tx + 32 * j] : 0.f; }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-                    if constexpr (PAIR) acc2[i][j] = fmaf(av[i], w2v[j], acc2[i][j]);
-                }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = ty + 8 * i;
-        if (r >= cnt) continue;
-        const int place = first + r;
-        const size_t orow = scatter ? (size_t)perm[place] : (size_t)place;
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int n = n0 + tx + 32 * j;
-            if (n >= N) continue;
-            float y;
-            if constexpr (PAIR) {
-                // the two products are rounded to the engine's type first, as a kernel after the product would find them
-                const float g = fminf(to_f32(from_f32<T>(acc[i][j])), limit);
-                const float u = fminf(fmaxf(to_f32(from_f32<T>(acc2[i][j])), -limit), limit);
-                y = g * (1.0f / (1.0f + expf(-alpha * g))) * (u + shift);
-            } else {
-                y = acc[i][j] * scale;
-            }
-            out[orow * ldo + n] = from_f32<T>(y);
-        }
-    }
-}
-
-// The same product for bfloat16 on the tensor cores: `mma.sync m16n8k16` with float32 accumulation.  Tiles of 32 places x
+// The product for bfloat16 groups of some tens of places: `mma.sync m16n8k16` with float32 accumulation.  Tiles of 32 places x
 // 128 weight rows, contraction in steps of 64; 8 warps as 2 (places) x 4 (weight rows), a warp 16 x 32.  The tiles of the
 // next step are fetched into registers while this step's are multiplied.  Rows in shared memory are padded by 16 bytes, so
 // that the eight rows a fragment load touches fall into different banks.  Needs K, lda and the matrices' rows in multiples of
 // 8 elements (16-byte loads).  With MI = 2 a tile has 64 places (a warp 32 x 32): every weight fragment then feeds two
 // multiplications, which is what the shared memory's bandwidth allows the tensor cores; groups of few places take MI = 1.
 constexpr int TN = 128, TK = 64, T_THREADS = 256, T_LD = TK + 8;
+// Places an expert on average: beyond the first a block of the 32-bit product takes 32 of them (30 places, 1,024 x 600, 86 us a step
+// against 102; at 5 they would leave three of four warps idle); up to the second bfloat16 runs from registers (20 places 97 us against
+// 118; at 31 the tiles below, which read a weight once for 32 places, take 84).
+constexpr int ROWS_SMALL_PLACES = 12;
+constexpr int SKINNY_MAX_PLACES = 24;
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -197,15 +97,10 @@ moe_grouped_mma_kernel(const bf16* __restrict__ a, long long lda, const bf16* __
     __shared__ int where[3];
     ti_pdl_sync();
     a = ti_dependent(a); perm = ti_dependent(perm); off = ti_dependent(off);
-    if (threadIdx.x == 0) {
-        int t = blockIdx.x, e = 0, found = -1, first = 0, cnt = 0;
-        for (; e < n_experts; e++) {
-            const int lo = off[e], hi = off[e + 1];
-            const int tiles = (hi - lo + TM - 1) / TM;
-            if (t < tiles) { found = e; first = lo + t * TM; cnt = min(TM, hi - first); break; }
-            t -= tiles;
-        }
-        where[0] = found; where[1] = first; where[2] = cnt;
+    if (threadIdx.x < 32) {
+        int found = -1, at = 0, n = 0;
+        if (!timoe::find_tile<TM>(off, n_experts, blockIdx.x, found, at, n)) found = -1;
+        if (threadIdx.x == 0) { where[0] = found; where[1] = at; where[2] = n; }
     }
     __syncthreads();
     const int e = where[0], first = where[1], cnt = where[2];
@@ -492,6 +387,12 @@ extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const
     TI_REQUIRE(!pair || W2, "moe_grouped: the paired form needs a second matrix");
     const bool tensor_cores = dtype == TI_BF16 && K % 8 == 0 && lda % 8 == 0 && ((uintptr_t)a & 15) == 0 && ((uintptr_t)W & 15) == 0 &&
                               (!W2 || ((uintptr_t)W2 & 15) == 0);
+    timoe::RowsArgs r{a, lda, W, pair ? W2 : nullptr, out, ldo, perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride};
+    if (tensor_cores && P <= SKINNY_MAX_PLACES * n_experts) {
+        if (P <= 2 * n_experts) return timoe::launch_skinny<1>(r, P, stream);
+        if (P <= 8 * n_experts) return timoe::launch_skinny<2>(r, P, stream);
+        return timoe::launch_skinny<4>(r, P, stream);
+    }
     if (tensor_cores) {
         const bool big = P >= 48 * n_experts;         // groups of 48 places and more on average: tiles of 64
         const int tm = big ? 64 : 32;
@@ -506,19 +407,13 @@ extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const
         TI_CHECK_LAUNCH("moe_grouped");
         return 0;
     }
-    const int tiles = (P + GM - 1) / GM + n_experts;
-    const int nblk = (N + GN - 1) / GN;
-    TI_REQUIRE(nblk <= 65535, "moe_grouped: %d weight rows are too many for one launch", N);
     return ti_dispatch_dtype(dtype, [&](auto t) -> int {
         using T = decltype(t);
-        if (pair)
-            TI_CUDA(ti_launch(moe_grouped_kernel<T, true>, dim3(tiles, nblk), dim3(G_THREADS), 0, stream, (const T*)a, lda,
-                              (const T*)W, (const T*)W2, (T*)out, ldo, perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride));
-        else
-            TI_CUDA(ti_launch(moe_grouped_kernel<T, false>, dim3(tiles, nblk), dim3(G_THREADS), 0, stream, (const T*)a, lda,
-                              (const T*)W, (const T*)W2, (T*)out, ldo, perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride));
-        TI_CHECK_LAUNCH("moe_grouped");
-        return 0;
+        constexpr int V = 16 / sizeof(T);
+        const bool vec = K % V == 0 && lda % V == 0 && w_estride % V == 0 && (((uintptr_t)a | (uintptr_t)W | (uintptr_t)r.W2) & 15) == 0;
+        if constexpr (sizeof(T) == 4)
+            if (vec) return P > ROWS_SMALL_PLACES * n_experts ? timoe::launch_rows<T, V, 4>(r, P, stream) : timoe::launch_rows<T, V, 1>(r, P, stream);
+        return timoe::launch_rows<T, 1, 1>(r, P, stream);
     });
 }
 

@@ -189,6 +189,157 @@ int route_few(const float* z, long long ldz, const float* logit_bias, const floa
     return go(std::integral_constant<int, 32>());
 }
 
+// A softmax router of up to 32 experts with its product: a block takes TOK tokens.  Its eight warps take every eighth expert's row
+// each, lanes along the row (16 bytes, AHEAD pieces of every row on their way together), and then, a warp a token and a lane an
+// expert, choose as moe_route_few_kernel does.  The choices go to moe_place_kernel, which counts and places the pairs.
+// (The product alone, a tcgen05 tile of which 16 of 128 rows were used, took 12 us at 40 to 777 tokens, and the one-block router after
+// it 7 us at one token and 9 at 777: what bounds both is a chain of dependent steps, not work.)
+constexpr int RK_THREADS = 256;
+
+// Smaller than every number's key: not a number.  Equal numbers (zeros of both signs too) have equal keys.
+__device__ __forceinline__ unsigned order_key(float c) {
+    if (c != c) return 0u;
+    const unsigned b = __float_as_uint(c + 0.0f);
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+
+template <typename T, int EPW, int TOK>
+__global__ void __launch_bounds__(RK_THREADS, TOK == 1 ? 2 : 3)
+moe_router_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ w, int K, const float* __restrict__ logit_bias,
+                  const float* __restrict__ correction, int n_experts, int top, float scale, int M, int* __restrict__ pair_expert,
+                  float* __restrict__ pair_w) {
+    ti_pdl_trigger();
+    constexpr int V = 16 / sizeof(T), AHEAD = TOK == 1 ? 4 : 1;
+    struct alignas(16) Pack { T v[V]; };
+    __shared__ float logits[TOK][32];
+    ti_pdl_sync();
+    x = ti_dependent(x); w = ti_dependent(w);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m0 = blockIdx.x * TOK;
+    float acc[EPW][TOK];
+#pragma unroll
+    for (int i = 0; i < EPW; i++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) acc[i][t] = 0.f;
+    for (int k0 = lane * V; k0 < K; k0 += 32 * V * AHEAD) {
+        Pack px[AHEAD][TOK], pw[AHEAD][EPW];
+#pragma unroll
+        for (int u = 0; u < AHEAD; u++) {
+            const int k = k0 + u * 32 * V;
+            if (k >= K) break;
+#pragma unroll
+            for (int t = 0; t < TOK; t++) px[u][t] = *reinterpret_cast<const Pack*>(x + (size_t)min(m0 + t, M - 1) * ldx + k);
+#pragma unroll
+            for (int i = 0; i < EPW; i++)
+                if (warp + 8 * i < n_experts) pw[u][i] = *reinterpret_cast<const Pack*>(w + (size_t)(warp + 8 * i) * K + k);
+        }
+#pragma unroll
+        for (int u = 0; u < AHEAD; u++) {
+            if (k0 + u * 32 * V >= K) break;
+#pragma unroll
+            for (int i = 0; i < EPW; i++)
+                if (warp + 8 * i < n_experts) {
+#pragma unroll
+                    for (int t = 0; t < TOK; t++)
+#pragma unroll
+                        for (int j = 0; j < V; j++) acc[i][t] = fmaf(to_f32(px[u][t].v[j]), to_f32(pw[u][i].v[j]), acc[i][t]);
+                }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < EPW; i++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) {
+            const float s = warp_sum(acc[i][t]);
+            if (lane == 0 && warp + 8 * i < n_experts) logits[t][warp + 8 * i] = s;
+        }
+    __syncthreads();
+    const int m = m0 + warp;
+    if (warp >= TOK || m >= M) return;
+    const bool has = lane < n_experts;
+    const float l = has ? logits[warp][lane] + (logit_bias ? logit_bias[lane] : 0.f) : -INFINITY;
+    const float zmax = warp_max(l);
+    const float ex = has ? expf(l - zmax) : 0.f;
+    const float inv = 1.0f / warp_sum(ex);
+    const float s = ex * inv, c = correction ? (has ? s + correction[lane] : 0.f) : l;
+    const unsigned key = order_key(c);
+    bool open = has;
+    float mine = 0.f, total = 0.f;
+    int rank = -1;
+    for (int j = 0; j < top; j++) {
+        // the lowest open index where that one is not a number (it is kept against every other), else the largest, lowest index first
+        const int lowest = __ffs(__ballot_sync(0xffffffffu, open)) - 1;
+        const unsigned most = __reduce_max_sync(0xffffffffu, open ? key : 0u);
+        const int largest = __ffs(__ballot_sync(0xffffffffu, open && key == most)) - 1;
+        const int best = __shfl_sync(0xffffffffu, key, lowest) == 0u ? lowest : largest;
+        total += __shfl_sync(0xffffffffu, s, best);
+        if (lane == best) { open = false; rank = j; mine = s; }
+    }
+    if (rank >= 0) {
+        pair_expert[(size_t)m * top + rank] = lane;
+        pair_w[(size_t)m * top + rank] = mine * (scale / (total + 1e-20f));
+    }
+}
+
+// Counts the pairs of every expert (up to 32) and writes them out grouped by expert.  One block.  Without pad_src: perm and off.
+// With it: the plan of moe_pad_plan (moe_grouped.cu) instead, every expert's places padded to whole tiles of 128.
+__global__ void __launch_bounds__(RT_THREADS)
+moe_place_kernel(int* __restrict__ pair_expert, int n_experts, int top, int P, int* __restrict__ perm, int* __restrict__ off,
+                 int rows, int* __restrict__ pad_src, int* __restrict__ pad_of_pair, int* __restrict__ tile_group) {
+    ti_pdl_trigger();
+    __shared__ int cnt[32], offs[33];
+    if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+    ti_pdl_sync();
+    pair_expert = ti_dependent(pair_expert);
+    __syncthreads();
+    if (pad_src) for (int i = threadIdx.x; i < rows; i += RT_THREADS) pad_src[i] = -1;
+    constexpr int KEEP = 4;                    // pairs whose place a thread keeps in registers; further ones go back to pair_expert
+    int e_of[KEEP], at_of[KEEP];
+#pragma unroll
+    for (int i = 0; i < KEEP; i++) {
+        const int p = i * RT_THREADS + threadIdx.x;
+        e_of[i] = p < P ? pair_expert[p] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < KEEP; i++)
+        if (i * RT_THREADS < P) at_of[i] = place_among(cnt, e_of[i]);
+    for (int p0 = KEEP * RT_THREADS; p0 < P; p0 += RT_THREADS) {
+        const int p = p0 + threadIdx.x, e = p < P ? pair_expert[p] : -1, at = place_among(cnt, e);
+        if (p < P) pair_expert[p] = e + at * 32;                 // (P * 32 is below 2^31, see the entry)
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int n = (int)threadIdx.x < n_experts ? cnt[threadIdx.x] : 0;
+        int upto = pad_src ? (n + 127) / 128 * 128 : n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int below = __shfl_up_sync(0xffffffffu, upto, o);
+            if ((int)threadIdx.x >= o) upto += below;
+        }
+        offs[threadIdx.x + 1] = upto;
+        if (threadIdx.x == 0) offs[0] = 0;
+    }
+    __syncthreads();
+    auto put = [&](int p, int e, int at) {
+        const int i = offs[e] + at;
+        if (pad_src) { pad_src[i] = p / top; pad_of_pair[p] = i; }
+        else perm[i] = p;
+    };
+#pragma unroll
+    for (int i = 0; i < KEEP; i++)
+        if (e_of[i] >= 0) put(i * RT_THREADS + threadIdx.x, e_of[i], at_of[i]);
+    for (int p = KEEP * RT_THREADS + threadIdx.x; p < P; p += RT_THREADS) put(p, pair_expert[p] & 31, pair_expert[p] >> 5);
+    if (!pad_src) {
+        if ((int)threadIdx.x <= n_experts) off[threadIdx.x] = offs[threadIdx.x];
+        return;
+    }
+    for (int t = threadIdx.x; t < rows / 128; t += RT_THREADS) {
+        int g = -1;
+        for (int e = 0; e < n_experts; e++)
+            if (t * 128 >= offs[e] && t * 128 < offs[e + 1]) g = e;
+        tile_group[t] = g;
+    }
+}
+
 constexpr int MAX_GROUPS = 64;
 
 __global__ void moe_route_softmax_kernel(const float* __restrict__ z, long long ldz, const float* __restrict__ logit_bias,
@@ -364,6 +515,40 @@ extern "C" int ti_moe_route_softmax(const float* z, long long ldz, const float* 
     TI_CUDA(ti_launch_class<1>(moe_route_softmax_kernel, dim3(1), dim3(RT_THREADS), smem, stream, z, ldz, logit_bias, correction, n_experts,
                                top, n_groups, keep, scale, M, perm, off, pair_expert, pair_w));
     TI_CHECK_LAUNCH("moe_route_softmax");
+    return 0;
+}
+
+// The softmax router with its product, for up to 32 experts without runs: x [M, K] (row stride ldx), w [n_experts, K] dense, both of
+// one type, rows on 16-byte boundaries.  pair_expert: int32 scratch [M * top]; pair_w: float32 [M * top].  With pad_src null: perm
+// and off as ti_moe_route_softmax gives them; else pad_src [rows], pad_of_pair and tile_group as ti_moe_pad_plan does.
+extern "C" int ti_moe_route_rows(const void* x, long long ldx, const void* w, int K, const float* logit_bias, const float* correction,
+                                 int n_experts, int top, float scale, int M, int* pair_expert, float* pair_w, int* perm, int* off,
+                                 int rows, int* pad_src, int* pad_of_pair, int* tile_group, int dtype, cudaStream_t stream) {
+    if (M == 0) return 0;
+    TI_REQUIRE(M > 0 && K > 0 && n_experts > 0 && n_experts <= 32 && top >= 1 && top <= n_experts && top <= MAX_TOP && (long long)M * top * 32 < (1LL << 31),
+               "moe_route_rows: bad sizes (%d experts, %d per token; at most 32 and %d)", n_experts, top, MAX_TOP);
+    TI_REQUIRE(pad_src ? rows % 128 == 0 && rows >= M * top && pad_of_pair && tile_group : perm && off, "moe_route_rows: incomplete plan");
+    const int code = ti_dispatch_dtype(dtype, [&](auto t) -> int {
+        using T = decltype(t);
+        constexpr int V = 16 / sizeof(T);
+        TI_REQUIRE(K % V == 0 && ldx % V == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0, "moe_route_rows: rows are not 16-byte aligned");
+        auto go = [&](auto tok) -> int {
+            constexpr int TOK = decltype(tok)::value;
+            auto kernel = n_experts <= 8 ? moe_router_kernel<T, 1, TOK> : n_experts <= 16 ? moe_router_kernel<T, 2, TOK> : moe_router_kernel<T, 4, TOK>;
+            TI_CUDA(ti_launch_class<1>(kernel, dim3((M + TOK - 1) / TOK), dim3(RK_THREADS), 0, stream, (const T*)x, ldx, (const T*)w, K, logit_bias,
+                                       correction, n_experts, top, scale, M, pair_expert, pair_w));
+            return 0;
+        };
+        // a token a block while all blocks fit the device at once
+        const int rc = M <= 296 ? go(std::integral_constant<int, 1>()) : go(std::integral_constant<int, 4>());
+        if (rc) return rc;
+        TI_CHECK_LAUNCH("moe_route_rows");
+        return 0;
+    });
+    if (code) return code;
+    TI_CUDA(ti_launch_class<1>(moe_place_kernel, dim3(1), dim3(RT_THREADS), 0, stream, pair_expert, n_experts, top, M * top, perm, off, rows, pad_src,
+                               pad_of_pair, tile_group));
+    TI_CHECK_LAUNCH("moe_route_rows (places)");
     return 0;
 }
 

@@ -49,16 +49,31 @@ def route_by_table(ids: torch.Tensor, table: torch.Tensor, n_experts: int):
 TC_MIN_GROUP = 64          # places per expert on average from which the tcgen05 grouped product runs (groups are padded to 128)
 
 
+def padded_eligible(x: torch.Tensor, n_experts: int, ff: int, top: int) -> bool:
+    """Whether ``expert_pairs`` pads the experts' groups and runs on tcgen05."""
+    M, H = x.shape
+    return (x.dtype == torch.bfloat16 and H % 8 == 0 and ff % 8 == 0 and M * top >= TC_MIN_GROUP * n_experts and x.stride(0) % 8 == 0
+            and x.data_ptr() % 16 == 0)
+
+
+def _plan_tensors(pairs: int, n_experts: int, dev):
+    """(pad_src, pad_of_pair, tile_group) of a step's padded groups, not yet written."""
+    rows = (pairs + 127 * n_experts + 127) // 128 * 128
+    return (torch.empty(rows, dtype=torch.int32, device=dev), torch.empty(pairs, dtype=torch.int32, device=dev),
+            torch.empty(rows // 128, dtype=torch.int32, device=dev))
+
+
 def expert_pairs(x: torch.Tensor, perm: torch.Tensor, off: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, top: int,
-                 limit: float, alpha: float, shift: float = 1.0, weight: float = 1.0):
+                 limit: float, alpha: float, shift: float = 1.0, weight: float = 1.0, plan=None):
     """Every (token, choice) pair's expert output, not yet summed: x[M, H]; w_gate_up [experts, 2 * ff, H] (an expert's gate
     rows, then its up rows); w_down [experts, H, ff]; the expert's activation is g' sigmoid(alpha g') (u' + shift) with
     g' = min(g, limit), u' = clamp(u, -limit, limit) (limit = inf, alpha = 1, shift = 0: silu(g) u).  Returns
     (z, place_of_pair): pair p's row, times ``weight``, is z[place_of_pair[p]], or z[p] when place_of_pair is None.
 
     bfloat16 steps with many tokens per expert pad every expert's tokens to tiles of 128 rows and run both products on
-    tcgen05 (csrc/gemm_tcgen05_grouped.cu; ``weight`` is then left to the caller's sum); everything else runs the grouped
-    tiles of csrc/moe_grouped.cu."""
+    tcgen05 (csrc/gemm_tcgen05_grouped.cu; ``weight`` is then left to the caller's sum; ``plan``: the padded places where
+    the router gave them already, ``perm`` and ``off`` are None then); everything else runs the grouped products of
+    csrc/moe_grouped.cu."""
     _need_cuda(x, perm, off, w_gate_up, w_down, what="moe")
     M, H = x.shape
     E, ff2, H2 = w_gate_up.shape
@@ -70,15 +85,14 @@ def expert_pairs(x: torch.Tensor, perm: torch.Tensor, off: torch.Tensor, w_gate_
             raise KernelError("moe: the experts' matrices must be dense and of the tokens' dtype")
     Pn = M * top
     code = _code(x, "moe")
-    if (x.dtype == torch.bfloat16 and H % 8 == 0 and ff % 8 == 0 and Pn >= TC_MIN_GROUP * E and x.stride(0) % 8 == 0
-            and x.data_ptr() % 16 == 0):
-        rows = (Pn + 127 * E + 127) // 128 * 128
+    if padded_eligible(x, E, ff, top):
         dev = x.device
-        pad_src = torch.empty(rows, dtype=torch.int32, device=dev)
-        pad_of_pair = torch.empty(Pn, dtype=torch.int32, device=dev)
-        tile_group = torch.empty(rows // 128, dtype=torch.int32, device=dev)
-        _call(_fn("ti_moe_pad_plan", [P, P, I, I, I, I, P, P, P, P]), _ptr(perm), _ptr(off), E, Pn, top, rows, _ptr(pad_src),
-              _ptr(pad_of_pair), _ptr(tile_group), _stream())
+        if plan is None:
+            pad_src, pad_of_pair, tile_group = plan = _plan_tensors(Pn, E, dev)
+            _call(_fn("ti_moe_pad_plan", [P, P, I, I, I, I, P, P, P, P]), _ptr(perm), _ptr(off), E, Pn, top, pad_src.numel(), _ptr(pad_src),
+                  _ptr(pad_of_pair), _ptr(tile_group), _stream())
+        pad_src, pad_of_pair, tile_group = plan
+        rows = pad_src.numel()
         xs = torch.empty((rows, H), dtype=x.dtype, device=dev)
         _call(_fn("ti_moe_gather_rows", [P, L, P, P, I, I, I, P]), _ptr(x), x.stride(0), _ptr(pad_src), _ptr(xs), rows, H, code, _stream())
         grouped = _fn("ti_linear_grouped_tc", [P, P, P, P, I, I, I, I, L, P])
@@ -154,6 +168,40 @@ def route_softmax(z: torch.Tensor, correction, n_experts: int, top: int, n_group
     _call(_fn("ti_moe_route_softmax", [P, L, P, P, I, I, I, I, F, I, P, P, P, P, P]), _ptr(z), z.stride(0), _ptr(logit_bias), _ptr(correction),
           int(n_experts), int(top), int(n_groups), int(keep), float(scale), M, _ptr(perm), _ptr(off), _ptr(scratch), _ptr(weight), _stream())
     return perm, off, weight
+
+
+def route_rows_eligible(x: torch.Tensor, w: torch.Tensor, n_groups: int, top: int) -> bool:
+    """Whether ``route_rows`` takes this router: up to 32 experts, no runs, rows on 16-byte boundaries."""
+    E, H = w.shape
+    v = 16 // x.element_size()
+    return (E <= 32 and n_groups <= 1 and top <= 16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] == H and x.dtype == w.dtype
+            and w.is_contiguous() and H % v == 0 and x.stride(0) % v == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and x.shape[0] * top * 32 < 2 ** 31)
+
+
+def route_rows(x: torch.Tensor, w: torch.Tensor, correction, top: int, scale: float, logit_bias, ff: int):
+    """``route_softmax`` (without runs) of the logits x w^T, the product included: x [M, H], w [experts, H] ->
+    (perm, off, weight, plan): for experts of width ``ff`` that ``expert_pairs`` runs on padded groups (``padded_eligible``) the
+    padded places as ``plan``, perm and off None; else perm and off, plan None (csrc/moe_router.cu)."""
+    _need_cuda(x, w, correction, logit_bias, what="moe_route_rows")
+    E, H = w.shape
+    for t in (correction, logit_bias):
+        if t is not None and (t.dtype != torch.float32 or tuple(t.shape) != (E,) or not t.is_contiguous()):
+            raise KernelError("moe_route_rows: the correction and the logits' bias must be dense float32 [experts]")
+    M = x.shape[0]
+    dev = x.device
+    scratch = torch.empty(M * top, dtype=torch.int32, device=dev)
+    weight = torch.empty(M * top, dtype=torch.float32, device=dev)
+    perm = off = None
+    plan = _plan_tensors(M * top, E, dev) if padded_eligible(x, E, ff, top) else None
+    if plan is None:
+        perm = torch.empty(M * top, dtype=torch.int32, device=dev)
+        off = torch.empty(E + 1, dtype=torch.int32, device=dev)
+    pad_src, pad_of_pair, tile_group = plan or (None, None, None)
+    _call(_fn("ti_moe_route_rows", [P, L, P, I, P, P, I, I, F, I, P, P, P, P, I, P, P, P, I, P]), _ptr(x), x.stride(0), _ptr(w), H, _ptr(logit_bias),
+          _ptr(correction), E, int(top), float(scale), M, _ptr(scratch), _ptr(weight), _ptr(perm), _ptr(off), pad_src.numel() if plan else 0,
+          _ptr(pad_src), _ptr(pad_of_pair), _ptr(tile_group), _code(x, "moe_route_rows"), _stream(), launches=2)
+    return perm, off, weight, plan
 
 
 def route_topk(z: torch.Tensor, n_experts: int, top: int):

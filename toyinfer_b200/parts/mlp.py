@@ -324,9 +324,13 @@ class SoftmaxMoE(FeedForward):
     def forward(self, x, batch) -> torch.Tensor:
         from ..kernels import moe as KM
         M = x.shape[0]
-        z = K.linear(x, self.w_router, out_dtype=torch.float32)
-        perm, off, weight = KM.route_softmax(z, self.correction, self.n_experts, self.top, self.n_groups, self.keep, self.scale, self.b_router)
-        y, place, _ = KM.expert_pairs(x, perm, off, self.w_gate_up, self.w_down, self.top, float("inf"), 1.0, 0.0)
+        plan = None
+        if KM.route_rows_eligible(x, self.w_router, self.n_groups, self.top):
+            perm, off, weight, plan = KM.route_rows(x, self.w_router, self.correction, self.top, self.scale, self.b_router, self.inter)
+        else:
+            z = K.linear(x, self.w_router, out_dtype=torch.float32)
+            perm, off, weight = KM.route_softmax(z, self.correction, self.n_experts, self.top, self.n_groups, self.keep, self.scale, self.b_router)
+        y, place, _ = KM.expert_pairs(x, perm, off, self.w_gate_up, self.w_down, self.top, float("inf"), 1.0, 0.0, plan=plan)
         shared = K.linear(K.linear_swiglu(x, self.ws_gate_up, "silu"), self.ws_down) if self.shared else None
         return KM.combine_gated(y, place, weight, shared, None, M, self.top)
 
