@@ -90,7 +90,7 @@ __global__ void attn_decode_combine_kernel(const float* __restrict__ part_o, con
         const int d = threadIdx.x + e * blockDim.x;
         if (d < hd) {
             float o = l > 0.f ? acc[e] / l : 0.f;
-            if (gate) o /= 1.f + expf(-to_f32(gate[(size_t)b * gate_stride + (size_t)h * hd + d]));
+            if (gate) o = ti_over(o, 1.f + expf(-to_f32(gate[(size_t)b * gate_stride + (size_t)h * hd + d])));
             out[(size_t)b * o_stride + (size_t)h * hd + d] = from_f32<T>(o);
         }
     }

@@ -533,7 +533,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
             if (d == 0) { fin_ml[r * 2] = m; fin_ml[r * 2 + 1] = l; }
         } else if (a.n_splits == 1) {
             float res = (sig ? acc : (l > 0.f ? acc / l : 0.f)) * (WIN ? a.out_scale : 1.f);
-            if ((WIN || EXTRA) && a.gate) res /= 1.f + expf(-to_f32(ti_dependent((const bf16*)a.gate)[(size_t)b * a.gate_stride + (size_t)h * HD + d]));
+            if ((WIN || EXTRA) && a.gate) res = ti_over(res, 1.f + expf(-to_f32(ti_dependent((const bf16*)a.gate)[(size_t)b * a.gate_stride + (size_t)h * HD + d])));
             if (WIN && a.out_f32) ((float*)a.out)[(size_t)b * a.o_stride + (size_t)h * HD + d] = res;
             else ((bf16*)a.out)[(size_t)b * a.o_stride + (size_t)h * HD + d] = __float2bfloat16_rn(res);
         } else {
@@ -563,7 +563,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                 }
             }
             float res = l > 0.f ? acc / l : 0.f;
-            if (EXTRA && a.gate) res /= 1.f + expf(-to_f32(ti_dependent((const bf16*)a.gate)[(size_t)b * a.gate_stride + (size_t)(h0 + r) * HD + d]));
+            if (EXTRA && a.gate) res = ti_over(res, 1.f + expf(-to_f32(ti_dependent((const bf16*)a.gate)[(size_t)b * a.gate_stride + (size_t)(h0 + r) * HD + d])));
             ((bf16*)a.out)[(size_t)b * a.o_stride + (size_t)(h0 + r) * HD + d] = __float2bfloat16_rn(res);
         }
         cluster_sync_all();     // nobody leaves while its shared memory may still be read

@@ -42,7 +42,7 @@ struct LatentPages {
 // sigmoid of a head's gate logit: logits [M, heads], row stride in elements
 template <typename T>
 __device__ __forceinline__ float head_gate(const T* gate, long long stride, size_t token, int head) {
-    return 1.0f / (1.0f + expf(-to_f32(gate[token * stride + head])));
+    return ti_over(1.0f, 1.0f + expf(-to_f32(gate[token * stride + head])));
 }
 
 template <typename T>

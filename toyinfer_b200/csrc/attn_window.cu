@@ -55,7 +55,7 @@ struct Pages {
     const int* page_table; int table_width; int page_size; int n_pages;
 };
 
-__device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
+__device__ __forceinline__ float sigmoidf(float x) { return ti_over(1.0f, 1.0f + expf(-x)); }
 
 // A logit per element of a token's results (engine type, row stride in elements), or none.
 struct Gate {

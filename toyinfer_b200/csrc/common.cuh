@@ -155,6 +155,18 @@ static inline cudaError_t ti_launch_after(void (*kernel)(KArgs...), dim3 grid, d
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// z / d for d >= 1 (infinity and NaN included): what sigmoids and silu divide by.  The compiler's division branches to a slow path,
+// which keeps the values that a thread works on from running side by side: the gated epilogue of a tile of 128 x 128 took 7.6 us,
+// the plain one 1.5.  Here the approximate reciprocal's quotient gets the remainder's correction in one fused multiply-add each
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), without a branch; where the
+// remainder is not finite (d or the quotient infinite) the quotient stands as it is.
+__device__ __forceinline__ float ti_over(float z, float d) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = z * r, rest = fmaf(-q, d, z);
+    return fabsf(rest) < INFINITY ? fmaf(rest, r, q) : q;
+}
+
 // The activation of a gated product's gate.  kind 1: silu, z / (1 + exp(-z)); kind 2: the tanh form of gelu,
 // 0.5 z (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))).
 __device__ __forceinline__ float ti_gate_act(float z, int kind) {
@@ -162,7 +174,7 @@ __device__ __forceinline__ float ti_gate_act(float z, int kind) {
         const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
         return 0.5f * z * (1.0f + tanhf(u));
     }
-    return z / (1.0f + expf(-z));
+    return ti_over(z, 1.0f + expf(-z));
 }
 
 // What a gated product stores for its (gate, up) pair.  kind 1 and 2: up * act(gate) as above; kind 3: a clamped gate
@@ -171,7 +183,7 @@ __device__ __forceinline__ float ti_gate_act(float z, int kind) {
 __device__ __forceinline__ float ti_gate_pair(float gate, float up, int kind, float limit) {
     if (kind == 3) {
         const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-        return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
+        return ti_over(g, 1.0f + expf(-1.702f * g)) * (u + 1.0f);
     }
     return up * ti_gate_act(gate, kind);
 }

@@ -132,7 +132,7 @@ delta_chunk_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
         }
     }
     if (tid < CH) {
-        bs[tid] = tid < n ? 1.0f / (1.0f + expf(-to_f32(beta_logit[(size_t)(tok0 + tid) * beta_stride + h]))) : 0.f;
+        bs[tid] = tid < n ? ti_over(1.0f, 1.0f + expf(-to_f32(beta_logit[(size_t)(tok0 + tid) * beta_stride + h]))) : 0.f;
         if constexpr (HEAD) gh[tid] = tid < n ? expf(-rt * dc_softplus(to_f32(decay_logit[(size_t)(tok0 + tid) * decay_stride + h]) + dt_bias[h])) : 1.f;
     }
     __syncthreads();

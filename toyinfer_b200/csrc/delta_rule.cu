@@ -86,7 +86,7 @@ __global__ void delta_rule_prep_kernel(const T* __restrict__ q, const T* __restr
             float* go = gg + ((size_t)m * n_heads + h) * dim;
             for (int i = lane; i < dim; i += 32) go[i] = expf(-rt * softplus_f(to_f32(l[i]) + dt_bias[(size_t)h * dim + i]));
         }
-        if (lane == 0) beta[(size_t)m * n_heads + h] = 1.0f / (1.0f + expf(-to_f32(beta_logit[(size_t)m * beta_stride + h])));
+        if (lane == 0) beta[(size_t)m * n_heads + h] = ti_over(1.0f, 1.0f + expf(-to_f32(beta_logit[(size_t)m * beta_stride + h])));
     }
 }
 
@@ -292,7 +292,7 @@ __global__ void head_gated_rmsnorm_kernel(const float* __restrict__ o, const T* 
     const float inv = rsqrtf(ss / (float)vdim + eps) * out_scale;
     for (int i = lane; i < vdim; i += 32) {
         const float gl = to_f32(gate[(size_t)m * gate_stride + (size_t)h * vdim + i]);
-        const float ga = (gate_silu ? gl : 1.0f) / (1.0f + expf(-gl));
+        const float ga = ti_over(gate_silu ? gl : 1.0f, 1.0f + expf(-gl));
         out[(size_t)m * out_stride + (size_t)h * vdim + i] = from_f32<T>(orow[i] * inv * (w ? w[i] : 1.0f) * ga);
     }
 }
@@ -330,7 +330,7 @@ __global__ void head_gated_rmsnorm_vec_kernel(const float* __restrict__ o, const
 #pragma unroll
     for (int e = 0; e < 8; e++) {
         const float gl = to_f32(g.v[e]);
-        const float ga = (gate_silu ? gl : 1.0f) / (1.0f + expf(-gl));
+        const float ga = ti_over(gate_silu ? gl : 1.0f, 1.0f + expf(-gl));
         y.v[e] = from_f32<T>(x[e] * inv * (w ? w[i + e] : 1.0f) * ga);
     }
     *reinterpret_cast<Run*>(out + (size_t)m * out_stride + at) = y;

@@ -262,7 +262,7 @@ __global__ void swiglu_pairs_kernel(const T* __restrict__ gu, T* __restrict__ ou
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const float g = to_f32(gu[2 * idx]), u = to_f32(gu[2 * idx + 1]);
-        out[idx] = from_f32<T>(u * (g / (1.0f + expf(-g))));
+        out[idx] = from_f32<T>(u * (ti_over(g, 1.0f + expf(-g))));
     }
 }
 
@@ -280,7 +280,7 @@ __global__ void swiglu_kernel(const T* __restrict__ gu, T* __restrict__ out, int
         load_vec<T, V>(gu + m * 2 * I + i, g);
         load_vec<T, V>(gu + m * 2 * I + I + i, u);
 #pragma unroll
-        for (int j = 0; j < V; j++) g[j] = u[j] * (g[j] / (1.0f + expf(-g[j])));
+        for (int j = 0; j < V; j++) g[j] = u[j] * (ti_over(g[j], 1.0f + expf(-g[j])));
         store_vec<T, V>(out + m * I + i, g);
     }
 }

@@ -28,7 +28,7 @@
 
 namespace {
 
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu_f(float z) { return ti_over(z, 1.0f + expf(-z)); }
 
 // what q, k and v pass as they enter the recurrence
 struct Entry { int act; float k_scale; };
@@ -381,7 +381,7 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const T* __res
     ss = block_sum(ss, red);
     const float inv = rsqrtf(ss / (float)N + eps);
     for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        const float gate = 1.0f / (1.0f + expf(-to_f32(g[m * g_stride + i])));
+        const float gate = ti_over(1.0f, 1.0f + expf(-to_f32(g[m * g_stride + i])));
         out[m * N + i] = from_f32<T>(orow[i] * inv * w[i] * gate);
     }
 }
@@ -409,7 +409,7 @@ __global__ void gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* _
     const float inv = rsqrtf(block_sum(ss, red) / (float)N + eps);
     Run y;
 #pragma unroll
-    for (int e = 0; e < 8; e++) y.v[e] = from_f32<T>(x[e] * inv * wv[e] * (1.0f / (1.0f + expf(-to_f32(gr.v[e])))));
+    for (int e = 0; e < 8; e++) y.v[e] = from_f32<T>(x[e] * inv * wv[e] * (ti_over(1.0f, 1.0f + expf(-to_f32(gr.v[e])))));
     *reinterpret_cast<Run*>(out + m * N + i) = y;
 }
 

@@ -200,7 +200,7 @@ moe_grouped_mma_kernel(const bf16* __restrict__ a, long long lda, const bf16* __
                 if constexpr (PAIR) {
                     const float gt = fminf(to_f32(from_f32<bf16>(acc[m][j][2 * half + c])), limit);
                     const float u = fminf(fmaxf(to_f32(from_f32<bf16>(acc2[m][j][2 * half + c])), -limit), limit);
-                    y = gt * (1.0f / (1.0f + expf(-alpha * gt))) * (u + shift);
+                    y = gt * (ti_over(1.0f, 1.0f + expf(-alpha * gt))) * (u + shift);
                 } else {
                     y = acc[m][j][2 * half + c] * scale;
                 }
@@ -293,7 +293,7 @@ __global__ void moe_act_pair_vec_kernel(const bf16* __restrict__ gu, bf16* __res
         for (int e = 0; e < 8; e++) {
             const float g = fminf(to_f32(gp[e]), limit);
             const float u = fminf(fmaxf(to_f32(up[e]), -limit), limit);
-            op[e] = from_f32<bf16>(g * (1.0f / (1.0f + expf(-alpha * g))) * (u + shift));
+            op[e] = from_f32<bf16>(g * (ti_over(1.0f, 1.0f + expf(-alpha * g))) * (u + shift));
         }
         reinterpret_cast<uint4*>(y)[idx] = o4;
     }
@@ -329,7 +329,7 @@ __global__ void moe_act_pair_kernel(const T* __restrict__ gu, T* __restrict__ y,
         const int f = (int)(idx - i * ff);
         const float g = fminf(to_f32(gu[i * 2 * ff + f]), limit);
         const float u = fminf(fmaxf(to_f32(gu[i * 2 * ff + ff + f]), -limit), limit);
-        y[idx] = from_f32<T>(g * (1.0f / (1.0f + expf(-alpha * g))) * (u + shift));
+        y[idx] = from_f32<T>(g * (ti_over(1.0f, 1.0f + expf(-alpha * g))) * (u + shift));
     }
 }
 

@@ -52,7 +52,7 @@ __global__ void moe_route_topk_kernel(const float* __restrict__ z, long long ldz
             }
             chosen[j] = best;
             const int p = m * top + j;
-            const float s = 1.0f / (1.0f + expf(-bz));
+            const float s = ti_over(1.0f, 1.0f + expf(-bz));
             pair_expert[p] = best;
             pair_score[p] = s;
             pair_score2[p] = s * s;
@@ -147,7 +147,7 @@ moe_route_few_kernel(const float* __restrict__ z, long long ldz, const float* __
                 if (e < n_experts && !(taken >> e & 1u) && (best < 0 || c[e] > bc)) { best = e; bc = c[e]; bl = l[e]; }     // a row of NaN keeps the lowest free index
             taken |= 1u << best;
             chosen[j] = best;
-            s_of[j] = SOFT ? expf(bl - zmax) * inv : 1.0f / (1.0f + expf(-bl));
+            s_of[j] = SOFT ? expf(bl - zmax) * inv : ti_over(1.0f, 1.0f + expf(-bl));
             total += s_of[j];
         }
         const float norm = SOFT ? scale / (total + 1e-20f) : 1.f;
@@ -420,7 +420,7 @@ __global__ void moe_combine_gated_kernel(const T* __restrict__ z, const int* __r
     z = ti_dependent(z); place_of_pair = ti_dependent(place_of_pair); pair_w = ti_dependent(pair_w);
     shared_out = ti_dependent(shared_out); gate_logit = ti_dependent(gate_logit);
     const size_t m = blockIdx.x;
-    const float g = (shared_out && gate_logit) ? 1.0f / (1.0f + expf(-gate_logit[m * gate_stride])) : 1.f;
+    const float g = (shared_out && gate_logit) ? ti_over(1.0f, 1.0f + expf(-gate_logit[m * gate_stride])) : 1.f;
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
         float s = 0.f;
         for (int j = 0; j < top; j++) {
@@ -443,7 +443,7 @@ __global__ void moe_combine_gated_vec_kernel(const T* __restrict__ z, const int*
     z = ti_dependent(z); place_of_pair = ti_dependent(place_of_pair); pair_w = ti_dependent(pair_w);
     shared_out = ti_dependent(shared_out); gate_logit = ti_dependent(gate_logit);
     const size_t m = blockIdx.x;
-    const float g = (shared_out && gate_logit) ? 1.0f / (1.0f + expf(-gate_logit[m * gate_stride])) : 1.f;
+    const float g = (shared_out && gate_logit) ? ti_over(1.0f, 1.0f + expf(-gate_logit[m * gate_stride])) : 1.f;
     struct alignas(16) Run { T v[8]; };
     for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
         float s[8] = {};

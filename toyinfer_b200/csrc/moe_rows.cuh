@@ -64,7 +64,7 @@ template <typename T>
 __device__ __forceinline__ float pair_act(const RowsArgs& a, float gate, float up) {
     const float g = fminf(to_f32(from_f32<T>(gate)), a.limit);
     const float u = fminf(fmaxf(to_f32(from_f32<T>(up)), -a.limit), a.limit);
-    return g * (1.0f / (1.0f + expf(-a.alpha * g))) * (u + a.shift);
+    return g * (ti_over(1.0f, 1.0f + expf(-a.alpha * g))) * (u + a.shift);
 }
 
 // 32-bit arithmetic on the CUDA cores.  A warp takes four weight rows (two of each matrix of a pair) and eight places; its lanes

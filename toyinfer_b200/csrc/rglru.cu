@@ -15,7 +15,7 @@ namespace {
 
 constexpr int LRU_THREADS = 128, LRU_AHEAD = 4;
 
-__device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float sigmoid_f(float z) { return ti_over(1.0f, 1.0f + expf(-z)); }
 __device__ __forceinline__ float gelu_tanh_f(float z) {
     return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }

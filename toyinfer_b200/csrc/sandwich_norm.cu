@@ -203,7 +203,7 @@ __device__ __forceinline__ float gate_act(float g, int act) {
         const float u = 0.7978845608028654f * (g + 0.044715f * g * g * g);
         return 0.5f * g * (1.0f + tanhf(u));
     }
-    return g / (1.0f + expf(-g));       // silu
+    return ti_over(g, 1.0f + expf(-g));       // silu
 }
 
 template <typename T>
@@ -220,7 +220,7 @@ __global__ void gated_act_kernel(const T* __restrict__ gu, long long ld, T* __re
         const float u = to_f32(pairs ? row[2 * i + 1] : row[I + i]);
         if (act == 2) {      // a clamped gate with a sharpened sigmoid, times the clamped up value plus one
             const float gc = fminf(g, limit), uc = fminf(fmaxf(u, -limit), limit);
-            out[idx] = from_f32<T>(gc / (1.0f + expf(-1.702f * gc)) * (uc + 1.0f));
+            out[idx] = from_f32<T>(ti_over(gc, 1.0f + expf(-1.702f * gc)) * (uc + 1.0f));
         } else {
             out[idx] = from_f32<T>(gate_act(g, act) * u);
         }

@@ -27,7 +27,7 @@ namespace {
 constexpr int VEC_CHUNK = 16;       // tokens of a block of short_conv_vec
 constexpr int CONV_CHUNK = 64, CONV_THREADS = 128, MAX_TAPS = 8;
 
-__device__ __forceinline__ float conv_act(float z, int act) { return act == 1 ? z / (1.0f + expf(-z)) : z; }
+__device__ __forceinline__ float conv_act(float z, int act) { return act == 1 ? ti_over(z, 1.0f + expf(-z)) : z; }
 
 template <typename T, int N>
 __global__ void __launch_bounds__(CONV_THREADS)

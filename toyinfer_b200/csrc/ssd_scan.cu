@@ -286,13 +286,13 @@ __global__ void gate_group_rmsnorm_kernel(const float* __restrict__ y, const T* 
     float ss = 0.f;
     for (int i = threadIdx.x; i < gs; i += blockDim.x) {
         const float zi = to_f32(zr[i]);
-        const float u = yr[i] * (zi / (1.0f + expf(-zi)));
+        const float u = yr[i] * (ti_over(zi, 1.0f + expf(-zi)));
         ss = fmaf(u, u, ss);
     }
     const float inv = rsqrtf(block_sum(ss, red) / (float)gs + eps);
     for (int i = threadIdx.x; i < gs; i += blockDim.x) {
         const float zi = to_f32(zr[i]);
-        const float u = yr[i] * (zi / (1.0f + expf(-zi)));
+        const float u = yr[i] * (ti_over(zi, 1.0f + expf(-zi)));
         out[(size_t)m * inner + base + i] = from_f32<T>(u * inv * w[base + i]);
     }
 }
@@ -322,7 +322,7 @@ __global__ void gate_group_rmsnorm_vec_kernel(const float* __restrict__ y, const
 #pragma unroll
         for (int e = 0; e < 8; e++) {
             const float zi = to_f32(zr.v[e]);
-            u[e] = yv[e] * (zi / (1.0f + expf(-zi)));
+            u[e] = yv[e] * (ti_over(zi, 1.0f + expf(-zi)));
             ss = fmaf(u[e], u[e], ss);
         }
     }

@@ -62,12 +62,12 @@ state_step_kernel(StepArgs a) {
         lam = ((const float*)a.decay)[h];
         for (int i = tid; i < D; i += ST_THREADS) {
             const float x = to_f32(kr[i]), y = to_f32(qr[i]);
-            ks[i] = (a.act ? x / (1.0f + expf(-x)) : x) * a.k_scale;
-            qs[i] = a.act ? y / (1.0f + expf(-y)) : y;
+            ks[i] = (a.act ? ti_over(x, 1.0f + expf(-x)) : x) * a.k_scale;
+            qs[i] = a.act ? ti_over(y, 1.0f + expf(-y)) : y;
         }
         for (int i = tid; i < V; i += ST_THREADS) {
             const float x = to_f32(v[(size_t)tok * a.v_stride + (size_t)h * V + i]);
-            es[i] = a.act ? x / (1.0f + expf(-x)) : x;
+            es[i] = a.act ? ti_over(x, 1.0f + expf(-x)) : x;
         }
     } else {
         if (warp < 2) {         // unit key, unit query times dim^-1/2
@@ -93,7 +93,7 @@ state_step_kernel(StepArgs a) {
                 gs[i] = expf(-rt * st_softplus(l + dt));
             }
         } else if (warp == 6) {
-            if (lane == 0) s_beta = 1.0f / (1.0f + expf(-to_f32(((const T*)a.beta)[(size_t)tok * a.beta_stride + h])));
+            if (lane == 0) s_beta = ti_over(1.0f, 1.0f + expf(-to_f32(((const T*)a.beta)[(size_t)tok * a.beta_stride + h])));
         }
     }
     __syncthreads();
