@@ -13,8 +13,8 @@
 //
 // delta_chunk_prep_kernel makes T, P and the decayed queries and keys of all chunks at once: a block per (chunk, value head).
 // delta_chunk_state_kernel walks a sequence's chunks: a block per (head, 16 columns of S), S kept in registers and, for the two
-// products with it, transposed in shared memory; the next chunk's operands come as one bulk copy meanwhile (the first kernel
-// leaves them in the layout that this one reads).
+// products with it, transposed in shared memory; the next chunk's operands come by bulk copies into the parts of one buffer that
+// are used up (the first kernel leaves them in the layout that this one reads).
 //
 // What bounds the second kernel: the shared memory that its multiply-adds read, 128 bytes a cycle whatever lanes share them.
 // Hence tiles of 8 x 4 results a thread with the contraction shared out over neighbouring lanes (a thread reads 1.5 bytes a
@@ -316,7 +316,7 @@ constexpr int R_PITCH = DC_COLS + 4, E_PITCH = DC_COLS + 8;     // (eight, or fo
 
 template <int D> constexpr int state_buf_floats() { return Ops<D>::floats + CH * DC_COLS; }
 template <int D> constexpr size_t state_smem_bytes() {
-    return (size_t)(2 * state_buf_floats<D>() + DC_COLS * (D + 4) + CH * (R_PITCH + E_PITCH + DC_COLS)) * sizeof(float);
+    return (size_t)(state_buf_floats<D>() + DC_COLS * (D + 4) + CH * (R_PITCH + E_PITCH + DC_COLS)) * sizeof(float);
 }
 
 // x[0 .. 2 N) summed over the lanes whose numbers differ in bit `bit`: the lane with it set goes on with the upper half.
@@ -331,13 +331,13 @@ __device__ __forceinline__ void halve(const float* x, float* out, int bit) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(DC_THREADS)
+__global__ void __launch_bounds__(DC_THREADS, 2)
 delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* __restrict__ state, long long slot_stride, int* status) {
     ti_pdl_trigger();
     using O = Ops<D>;
     constexpr int PITCH = D + 4, BUF = state_buf_floats<D>();
     extern __shared__ __align__(16) float sm[];
-    float* St = sm + 2 * BUF;                    // [DC_COLS][PITCH]: S transposed
+    float* St = sm + BUF;                        // [DC_COLS][PITCH]: S transposed
     float* Rs = St + DC_COLS * PITCH;            // [CH][R_PITCH]
     float* Es = Rs + CH * R_PITCH;               // [CH][E_PITCH]
     float* Qs = Es + CH * E_PITCH;               // [CH][DC_COLS]: (G q) S
@@ -352,17 +352,23 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
     if (n <= 0 || n < a.least) return;
     const int H = a.n_heads, chunks = (n + CH - 1) / CH;
     const size_t id0 = chunk_id(first, b, 0);
-    auto fetch = [&](int c) {                    // by one thread
-        float* buf = sm + (c & 1) * BUF;
-        const size_t cid = (id0 + c) * H + h;
-        mbar_expect_tx(&ready[c & 1], BUF * 4);
+    // One buffer, in two parts that come when what they replace is used up: the keys, queries and values of the next chunk once the
+    // products with S are made, the rest of a chunk's operands while they are.
+    auto copy = [&](uint64_t* bar, float* to, const float* from, int floats) {
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(smem_u32(buf)), "l"(a.ops + cid * O::floats), "r"(O::floats * 4), "r"(smem_u32(&ready[c & 1])) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(smem_u32(buf + O::floats)), "l"(a.bv + (cid * groups + grp) * (CH * DC_COLS)), "r"(CH * DC_COLS * 4),
-                       "r"(smem_u32(&ready[c & 1])) : "memory");
+                     ::"r"(smem_u32(to)), "l"(from), "r"(floats * 4), "r"(smem_u32(bar)) : "memory");
     };
-    if (tid == 0) { fetch(0); if (chunks > 1) fetch(1); }
+    auto fetch_rows = [&](int c) {               // by one thread
+        const size_t cid = (id0 + c) * H + h;
+        mbar_expect_tx(&ready[0], (O::d + CH * DC_COLS) * 4);
+        copy(&ready[0], sm, a.ops + cid * O::floats, O::d);
+        copy(&ready[0], sm + O::floats, a.bv + (cid * groups + grp) * (CH * DC_COLS), CH * DC_COLS);
+    };
+    auto fetch_rest = [&](int c) {
+        mbar_expect_tx(&ready[1], (O::floats - O::d) * 4);
+        copy(&ready[1], sm + O::d, a.ops + ((id0 + c) * H + h) * O::floats + O::d, O::floats - O::d);
+    };
+    if (tid == 0) fetch_rows(0);
     // k^T E: tiles of 8 rows and 4 columns of S, a tile's tokens shared out over SG lanes; of its sums this thread keeps four
     // rows (d0 ..) and NC columns (sc ..), its piece of S
     constexpr int SG = D == 128 ? 4 : 8, NC = D == 128 ? 2 : 1;
@@ -380,15 +386,15 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
     const int kq = lane & 7, ct = lane >> 3;
     bool ok = true;
     __syncthreads();
+    const float* buf = sm;
     for (int c = 0; c < chunks; c++) {
-        if (!mbar_wait(&ready[c & 1], (uint32_t)((c >> 1) & 1))) { ti_report(status, TI_STATUS_TMA_WAIT); ok = false; }
-        if (!__syncthreads_and(ok)) {            // (given up: not before the copies under way have arrived, or their waits have run out too)
-            if (tid == 0)
-                for (int k = c; k < min(c + 2, chunks); k++) mbar_wait(&ready[k & 1], (uint32_t)((k >> 1) & 1));
+        if (!mbar_wait(&ready[0], (uint32_t)(c & 1))) { ti_report(status, TI_STATUS_TMA_WAIT); ok = false; }
+        if (!__syncthreads_and(ok)) {            // (given up: not before the copy under way has arrived, or its wait has run out too)
+            if (tid == 0) mbar_wait(&ready[0], (uint32_t)(c & 1));
             __syncthreads();
             return;
-        }                                        // this chunk's operands and S are there
-        const float* buf = sm + (c & 1) * BUF;
+        }                                        // this chunk's rows and S are there, the last one's operands are used up
+        if (tid == 0) fetch_rest(c);
         // the products with S: 64 rows (32 keys, then 32 queries) x 16 columns; a warp has 8 rows, a lane 4 columns and an eighth of D
         float all[32];
         {
@@ -431,7 +437,13 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
         } else {
             *reinterpret_cast<float4*>(Qs + ((warp - 4) * 8 + kq) * DC_COLS + ct * 4) = make_float4(mine[0], mine[1], mine[2], mine[3]);
         }
-        __syncthreads();
+        if (!mbar_wait(&ready[1], (uint32_t)(c & 1))) { ti_report(status, TI_STATUS_TMA_WAIT); ok = false; }
+        if (!__syncthreads_and(ok)) {
+            if (tid == 0) mbar_wait(&ready[1], (uint32_t)(c & 1));
+            __syncthreads();
+            return;
+        }                                        // R, (G q) S and the chunk's other operands are there, its rows are used up
+        if (tid == 0 && c + 1 < chunks) fetch_rows(c + 1);
         {
             // E = T R: a warp has 4 rows, a lane 4 columns and the tokens kq, kq + 8, ...
             float acc[16] = {};
@@ -522,8 +534,6 @@ delta_chunk_state_kernel(DeltaChunkArgs a, float* __restrict__ o, int M, float* 
             const float2 q = *reinterpret_cast<const float2*>(Qs + r * DC_COLS + e);
             if (t < n) *reinterpret_cast<float2*>(o + ((size_t)(first + t) * H + h) * a.vdim + col0 + e) = make_float2(q.x + mine[0], q.y + mine[1]);
         }
-        __syncthreads();                         // this chunk's operands are used up
-        if (tid == 0 && c + 2 < chunks) fetch(c + 2);
     }
 #pragma unroll
     for (int j = 0; j < NC; j++)
@@ -549,10 +559,12 @@ int run_chunks(const void* q, const void* k, const void* v, long long q_stride, 
                       (const T*)q, (const T*)k, (const T*)v, q_stride, k_stride, v_stride, (const L*)decay_logit, decay_stride, dt_bias, rate,
                       (const T*)beta_logit, beta_stride, a));
     TI_CHECK_LAUNCH("delta_rule (chunks)");
-    // blocks that have an SM each must not start two on the SM that the kernel before left first: the walk is a chain, and its
-    // time is the slowest block's (64 blocks of 64 x 16: 245 us, spread out 169)
+    // Blocks that have an SM each must not start two on the SM that the kernel before left first: the walk is a chain, and its
+    // time is the slowest block's (64 blocks of 64 x 16: 245 us, spread out 169).  Two blocks of heads of 128 on an SM get 1.35 times one
+    // block's work done, so that pays from the third round on: 384 blocks (500, 383 and 200 tokens) 86 us alone, 65 in pairs, but 256
+    // (1,348 and 700) 176 and 183, where pairs of two long sequences' blocks end last.
     const long long blocks = (long long)a.n_heads * (a.vdim / DC_COLS) * n_seq;
-    const size_t room = blocks <= sms && smem < ALONE ? ALONE : smem;
+    const size_t room = blocks <= (D == 128 ? 2 : 1) * (long long)sms && smem < ALONE ? ALONE : smem;
     TI_CUDA(ti_launch(delta_chunk_state_kernel<D>, dim3(a.n_heads * (a.vdim / DC_COLS), n_seq), dim3(DC_THREADS), room, stream, a, o, M, state,
                       slot_stride, status));
     TI_CHECK_LAUNCH("delta_rule (chunk states)");
