@@ -110,8 +110,15 @@ class _KVGroup:
         self.dirty.pop(slot, None)
 
     def flush(self) -> None:
-        for slot, (lo, hi) in self.dirty.items():
-            self.table[slot, lo:hi].copy_(torch.from_numpy(self.table_host[slot, lo:hi]))
+        if not self.dirty:
+            return
+        first, last = min(self.dirty), max(self.dirty)
+        if len(self.dirty) > 1 and (last + 1 - first) * self.pages_per_seq <= 8192:
+            # one copy of the rows from the first to the last (those between them are the same on both sides, or nobody's)
+            self.table[first:last + 1].copy_(torch.from_numpy(self.table_host[first:last + 1]))
+        else:
+            for slot, (lo, hi) in self.dirty.items():
+                self.table[slot, lo:hi].copy_(torch.from_numpy(self.table_host[slot, lo:hi]))
         self.dirty.clear()
 
     def view(self, entry: int) -> KVView:

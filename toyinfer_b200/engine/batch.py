@@ -39,31 +39,65 @@ class BatchBuffers:
         self.total = off
         device = torch.device(device)
         pin = device.type == "cuda"
-        self.host = torch.zeros(self.total, dtype=torch.int32, pin_memory=pin)
-        self.host_np = self.host.numpy()
+        # two host buffers in turn, so that a step can be written while the upload of the one before still waits for its place
+        # in the stream
+        self._hosts = [_HostBuffer(self.total, self.offsets, pin) for _ in range(2 if pin else 1)]
+        self._at = 0
         self.dev = torch.zeros(self.total, dtype=torch.int32, device=device)
-        self._copied = torch.cuda.Event() if pin else None
-        self._pending = False
+        self._dev_views = {}
+
+    @property
+    def host(self) -> torch.Tensor:
+        """The host buffer that is being written, or was last."""
+        return self._hosts[self._at].data
+
+    @property
+    def host_np(self) -> np.ndarray:
+        return self._hosts[self._at].np
 
     def host_view(self, name: str) -> np.ndarray:
-        off, n = self.offsets[name]
-        return self.host_np[off:off + n]
+        return self._hosts[self._at].fields[name]
 
     def dev_view(self, name: str) -> torch.Tensor:
         off, n = self.offsets[name]
         return self.dev[off:off + n]
 
-    def begin_fill(self) -> None:
-        """The host buffer may be rewritten only after its last upload has left it."""
-        if self._pending:
-            self._copied.synchronize()
-            self._pending = False
+    def dev_views(self, n_tok: int, n_seq: int):
+        """The step's device views (fields of ``StepBatch``) for so many token rows and sequences; kept, as their making takes
+        longer than the rest of a single-token step's preparation."""
+        views = self._dev_views.get((n_tok, n_seq))
+        if views is None:
+            if len(self._dev_views) >= 64:
+                self._dev_views.clear()
+            sizes = {"token_ids": n_tok, "tok_pos": n_tok, "tok_seq": n_tok, "cu_new": n_seq + 1}
+            views = self._dev_views[(n_tok, n_seq)] = {name: self.dev_view(name)[:sizes.get(name, n_seq)] for name in self.FIELDS}
+        return views
+
+    def begin_fill(self) -> "_HostBuffer":
+        """The host buffer to write: it may be rewritten only after its last upload has left it."""
+        self._at = (self._at + 1) % len(self._hosts)
+        h = self._hosts[self._at]
+        if h.pending:
+            h.copied.synchronize()
+            h.pending = False
+        return h
 
     def upload(self) -> None:
-        self.dev.copy_(self.host, non_blocking=True)
-        if self._copied is not None:
-            self._copied.record()
-            self._pending = True
+        h = self._hosts[self._at]
+        self.dev.copy_(h.data, non_blocking=True)
+        if h.copied is not None:
+            h.copied.record()
+            h.pending = True
+
+
+class _HostBuffer:
+    def __init__(self, total: int, offsets, pin: bool):
+        self.data = torch.zeros(total, dtype=torch.int32, pin_memory=pin)
+        self.np = self.data.numpy()
+        self.fields = {name: self.np[off:off + n] for name, (off, n) in offsets.items()}
+        self.copied = torch.cuda.Event() if pin else None
+        self.pending = False
+        self.holds = None       # (sequences, padded, scratch slot) of the step of single tokens that the buffer holds, if it holds one
 
 
 @dataclass
@@ -116,10 +150,33 @@ def fill_batch(buf: BatchBuffers, mode: str, slots: Sequence[int], starts: Seque
     spare = n_tok > n_used
     if n_seq + spare > buf.n_seq or n_tok > buf.n_tok or n_used > n_tok:
         raise ValueError(f"step of {n_seq + spare} sequences / {max(n_tok, n_used)} tokens exceeds buffers for {buf.n_seq} / {buf.n_tok}")
-    buf.begin_fill()
-    ids, pos, seq = buf.host_view("token_ids"), buf.host_view("tok_pos"), buf.host_view("tok_seq")
-    sl, st, nw, ln, cu = (buf.host_view("seq_slot"), buf.host_view("seq_start"), buf.host_view("seq_new"),
-                          buf.host_view("seq_len"), buf.host_view("cu_new"))
+    h = buf.begin_fill()
+    f = h.fields
+    layout = (n_real, n_seq, scratch_slot) if mode == "extend" and new.count(1) == n_real and not spare else None
+    if layout is not None and h.holds == layout:
+        # single tokens of as many sequences as before: what does not follow from that alone
+        f["token_ids"][:n_real] = [t[0] for t in tokens]
+        f["tok_pos"][:n_real] = starts
+        f["seq_start"][:n_real] = starts
+        f["seq_slot"][:n_real] = slots
+        np.add(f["seq_start"][:n_real], 1, out=f["seq_len"][:n_real])
+    else:
+        h.holds = None
+        _write_all(f, n_real, n_seq, spare, slots, starts, tokens, new, scratch_slot)
+        h.holds = layout
+    buf.upload()
+    return StepBatch(
+        mode=mode, n_seq=n_seq, n_tok=n_tok, n_real_seq=n_real, n_real_tok=n_real_tok,
+        max_new=new_bound if new_bound is not None else max(new + [1 if pad_seqs else 0]),
+        max_pos_after=new_bound if new_bound is not None else max([s + n for s, n in zip(starts, new)] + [1]),
+        plan_len=plan_len, **buf.dev_views(n_tok, n_seq + spare),
+        host_slots=list(slots) + [scratch_slot] * pad_seqs, host_starts=list(starts) + [0] * pad_seqs,
+        host_new=new + [1] * pad_seqs,
+    )
+
+
+def _write_all(f, n_real, n_seq, spare, slots, starts, tokens, new, scratch_slot) -> None:
+    ids, pos, seq, sl, st, nw, ln, cu = (f[name] for name in BatchBuffers.FIELDS)
     o = 0
     for i in range(n_real):
         n = new[i]
@@ -142,16 +199,3 @@ def fill_batch(buf: BatchBuffers, mode: str, slots: Sequence[int], starts: Seque
     nw[n_seq:] = 0
     ln[n_seq:] = 1
     cu[n_seq + 1:] = o
-    buf.upload()
-    return StepBatch(
-        mode=mode, n_seq=n_seq, n_tok=n_tok, n_real_seq=n_real, n_real_tok=n_real_tok,
-        max_new=new_bound if new_bound is not None else max(new + [1 if pad_seqs else 0]),
-        max_pos_after=new_bound if new_bound is not None else max([s + n for s, n in zip(starts, new)] + [1]),
-        plan_len=plan_len,
-        token_ids=buf.dev_view("token_ids")[:n_tok], tok_pos=buf.dev_view("tok_pos")[:n_tok],
-        tok_seq=buf.dev_view("tok_seq")[:n_tok], seq_slot=buf.dev_view("seq_slot")[:n_seq + spare],
-        seq_start=buf.dev_view("seq_start")[:n_seq + spare], seq_new=buf.dev_view("seq_new")[:n_seq + spare],
-        seq_len=buf.dev_view("seq_len")[:n_seq + spare], cu_new=buf.dev_view("cu_new")[:n_seq + 1 + spare],
-        host_slots=list(slots) + [scratch_slot] * pad_seqs, host_starts=list(starts) + [0] * pad_seqs,
-        host_new=new + [1] * pad_seqs,
-    )
