@@ -301,8 +301,8 @@ def swiglu(gu: torch.Tensor, pairs: bool = False) -> torch.Tensor:
 def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, act: str = "silu", limit: float = 0.0) -> torch.Tensor:
     """x[M, K] times w_pairs[2*I, K] (rows gate_0, up_0, gate_1, up_1, ...) followed by the
     gated activation act(gate) * up -> [M, I]; act "silu" or "gelu_tanh", or "clamped_swish" with its ``limit``
-    (see ``gated_act``).  The activation runs in the product's epilogue where the tensor-core kernel takes the
-    shape and knows the activation, else as a kernel of its own.  x may be a PendingNorm."""
+    (see ``gated_act``).  The activation runs in the product's epilogue where the tensor-core kernel or the few-row
+    float32 kernel takes the shape, else as a kernel of its own.  x may be a PendingNorm."""
     if act not in GATE_ACTS:
         raise KernelError(f"linear_swiglu: unknown activation {act!r}; known: {sorted(GATE_ACTS)}")
     if isinstance(x, PendingNorm):
@@ -319,7 +319,8 @@ def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, act: str = "silu", lim
     M, K = x.shape
     N = w_pairs.shape[0]
     ldx, ldw = _row_stride(x, "linear x"), _row_stride(w_pairs, "linear w")
-    if gemm.tc_eligible(x, w_pairs, K, ldx, ldw) or gemm.f32_eligible(x, w_pairs, M, K, ldx, ldw):
+    if (gemm.tc_eligible(x, w_pairs, K, ldx, ldw) or gemm.f32_eligible(x, w_pairs, M, K, ldx, ldw)
+            or gemm.rows_eligible(x, w_pairs, M, K, ldx, ldw)):
         out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
         gemm.run(x, w_pairs, out, M, N, K, ldx, ldw, gated=1 + GATE_ACTS[act], gate_limit=limit)      # the kernels' codes: 1 silu, 2 gelu, 3 clamped
         return out

@@ -94,11 +94,17 @@ def f32_eligible(x, w, M, K, ldx, ldw) -> bool:
             and ldw % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def rows_eligible(x, w, M, K, ldx, ldw) -> bool:
+    """Whether the few-row float32 kernel (csrc/gemm_simt.cu) can end in a gated activation."""
+    return (M <= 16 and x.dtype == torch.float32 and w.dtype == torch.float32 and K % 4 == 0 and ldx % 4 == 0 and ldw % 4 == 0
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def run(x, w, out, M, N, K, ldx, ldw, gated: int = 0, late_start: bool = False, gate_limit: float = 0.0) -> None:
     """``gated``: 1 (or True) for up * silu(gate), 2 for up * gelu(gate) in the tanh form, 3 for the clamped pair
     g' sigmoid(1.702 g') (u' + 1) with g' = min(gate, gate_limit), u' = clamp(up, -gate_limit, gate_limit), over paired
     weight rows; 4 and 5: no pairs, every value through the squared ReLU or gelu; only for shapes that a tensor-core kernel takes
-    (tc_eligible, f32_eligible).  ``late_start``: the few-token kernels start only when the kernel before them has finished
+    (tc_eligible, f32_eligible; 1 to 3 also rows_eligible).  ``late_start``: the few-token kernels start only when the kernel before them has finished
     (csrc/gemm_skinny.cu)."""
     lib = library()
     out_f32 = 1 if (out.dtype == torch.float32 and x.dtype != torch.float32) else 0
@@ -145,6 +151,9 @@ def run(x, w, out, M, N, K, ldx, ldw, gated: int = 0, late_start: bool = False, 
         workspace = torch.empty(plan[1], dtype=torch.float32, device=x.device) if plan[1] else None
         _call(lib.ti_linear_f32_tc, _ptr(x), _ptr(w), _ptr(out), M, N, K, ldx, ldw, out.stride(0), plan[0], _ptr(workspace), int(gated),
               float(gate_limit), _stream(), launches=plan[2])
+        return
+    if gated and gated <= 3 and rows_eligible(x, w, M, K, ldx, ldw):
+        _call(lib.ti_linear_rows_gated, _ptr(x), _ptr(w), _ptr(out), M, N, K, ldx, ldw, out.stride(0), int(gated), float(gate_limit), _stream())
         return
     if gated:
         raise RuntimeError("linear: the gated epilogue exists in the tensor-core kernels only")

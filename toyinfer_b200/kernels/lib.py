@@ -25,6 +25,7 @@ def _declare(lib) -> None:
         "ti_gather_add": [P, P, P, P, I, I, I, I, P],
         "ti_swiglu": [P, P, I, I, I, I, P],
         "ti_linear_simt": [P, P, P, I, I, I, L, L, L, I, I, P],
+        "ti_linear_rows_gated": [P, P, P, I, I, I, L, L, L, I, F, P],
         "ti_qk_norm_rope_store": [P, P, P, L, L, L, I, I, I, P, P, I, F, P, P, I, I, P, P, P, P,
                                   P, P, P, I, I, I, I, I, I, P],
         "ti_attn_prefill_simt": [P, P, P, P, L, L, L, L, P, I, I, I, I, I, F, I, I, P],
