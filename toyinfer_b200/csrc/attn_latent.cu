@@ -28,6 +28,7 @@
 //   latent_expand  o[m, h] = Wuv_h ol[m, h], times sigmoid(gate[m, h]) where a design gates its heads.
 #include "common.cuh"
 #include "attn_decode.cuh"
+#include "tma.cuh"
 
 #include <algorithm>
 
@@ -62,7 +63,7 @@ __device__ __forceinline__ void store_row_to_pages(const LatentPages& kv, int sl
 
 // ---------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ void latent_prep_body(float* sm, const T* d, long long d_stride, T* q, long long q_stride,
+__device__ __forceinline__ void latent_prep_body(float* sm, int m, const T* d, long long d_stride, T* q, long long q_stride,
                                                  int n_heads, int plain, int rank, int rot, const float* __restrict__ norm_w, float eps,
                                                  const float* __restrict__ cos_t, const float* __restrict__ sin_t, int max_pos,
                                                  const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
@@ -71,23 +72,39 @@ __device__ __forceinline__ void latent_prep_body(float* sm, const T* d, long lon
     float* vals = sm;                    // W floats, then 33, then W values of T
     float* red = sm + W;
     T* rounded = reinterpret_cast<T*>(red + 33);
-    const int m = blockIdx.x, t = threadIdx.x, nt = blockDim.x;
+    const int t = threadIdx.x, nt = blockDim.x;
     const int pos = min(max(tok_pos[m], 0), max_pos - 1);
     const int half = rot >> 1;
     const float* cs = cos_t + (size_t)pos * half;
     const float* sn = sin_t + (size_t)pos * half;
     const T* drow = d + (size_t)m * d_stride;
-    float ss = 0.f;
-    for (int i = t; i < W; i += nt) {
-        const float x = to_f32(drow[i]);
-        vals[i] = x;
-        if (i < rank) ss = fmaf(x, x, ss);
+    // (loads in batches, so that several are on their way at a time, the weights and tables among them)
+    constexpr int AHEAD = 8;
+    float ss = 0.f, nw[AHEAD], c_r = 0.f, s_r = 0.f;
+    for (int i0 = t; i0 < W; i0 += AHEAD * nt) {
+        float x[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) x[j] = i0 + j * nt < W ? to_f32(drow[i0 + j * nt]) : 0.f;
+        if (i0 == t) {
+#pragma unroll
+            for (int j = 0; j < AHEAD; j++) nw[j] = t + j * nt < rank ? norm_w[t + j * nt] : 0.f;
+            if (t < half) { c_r = cs[t]; s_r = sn[t]; }
+        }
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            const int i = i0 + j * nt;
+            if (i < W) vals[i] = x[j];
+            if (i < rank) ss = fmaf(x[j], x[j], ss);
+        }
     }
     ss = block_sum(ss, red);             // (also makes vals visible)
     const float inv = rsqrtf(ss / (float)rank + eps);
-    for (int i = t; i < rank; i += nt) rounded[i] = from_f32<T>(vals[i] * inv * norm_w[i]);
+#pragma unroll
+    for (int j = 0; j < AHEAD; j++)
+        if (t + j * nt < rank) rounded[t + j * nt] = from_f32<T>(vals[t + j * nt] * inv * nw[j]);
+    for (int i = t + AHEAD * nt; i < rank; i += nt) rounded[i] = from_f32<T>(vals[i] * inv * norm_w[i]);
     for (int i = t; i < half; i += nt) {
-        const float u = vals[rank + i], v = vals[rank + i + half], c = cs[i], s = sn[i];
+        const float u = vals[rank + i], v = vals[rank + i + half], c = i == t ? c_r : cs[i], s = i == t ? s_r : sn[i];
         rounded[rank + i] = from_f32<T>(u * c - v * s);
         rounded[rank + i + half] = from_f32<T>(v * c + u * s);
     }
@@ -118,7 +135,7 @@ __global__ void latent_prep_kernel(const T* __restrict__ d, long long d_stride, 
     extern __shared__ float sm[];
     ti_pdl_sync();
     d = ti_dependent(d); q = ti_dependent(q);
-    latent_prep_body<T>(sm, d, d_stride, q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos, tok_seq,
+    latent_prep_body<T>(sm, blockIdx.x, d, d_stride, q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos, tok_seq,
                         seq_slot, lat, kv);
 }
 
@@ -139,7 +156,7 @@ latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* 
     ti_pdl_sync();
     d = ti_dependent(d); q = ti_dependent(q);
     if ((int)blockIdx.y == n_heads) {
-        latent_prep_body<T>(sm, d, d_stride, (T*)nullptr, 0, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos,
+        latent_prep_body<T>(sm, blockIdx.x, d, d_stride, (T*)nullptr, 0, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos,
                             tok_seq, seq_slot, lat, kv);
         return;
     }
@@ -215,6 +232,122 @@ latent_prep_absorb_kernel(const T* __restrict__ d, long long d_stride, const T* 
     }
 }
 
+// A line towards L2.  Nothing is read into the program, so that this may run before the wait for the kernels before it whatever they
+// write: L2 is where their writes arrive.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
+
+// The same for several tokens at a time, bfloat16: a block takes one head, 64 elements of the latent and up to TOK tokens, so that an
+// element of Wuk is read once for all of them (a block a token and head read a head's whole matrix for one token: 17 MB from L2 for 16
+// tokens of 16 heads of 64 x 512; 9 us there, 6 so, and 31 -> 14 for 64 tokens).  A lane has two neighbouring elements, a warp every fourth row of Wuk; the four
+// warps' sums meet in shared memory.  The blocks behind the heads' do the tokens' rows.
+constexpr int AR_THREADS = 128, AR_COLS = 64;
+
+template <int TOK> constexpr size_t absorb_rows_smem(int plain) { return (size_t)(plain * TOK + 4 * TOK * AR_COLS) * sizeof(float); }
+
+template <int TOK>
+__global__ void __launch_bounds__(AR_THREADS)
+latent_absorb_rows_kernel(const bf16* __restrict__ d, long long d_stride, const bf16* __restrict__ q, long long q_stride,
+                          int n_heads, int plain, int rank, int rot, const float* __restrict__ norm_w, float eps,
+                          const float* __restrict__ cos_t, const float* __restrict__ sin_t, int max_pos,
+                          const int* __restrict__ tok_pos, const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
+                          bf16* __restrict__ lat, LatentPages kv, const bf16* __restrict__ uk, float* __restrict__ qa, int M, int chunks) {
+    ti_pdl_trigger();
+    extern __shared__ __align__(16) float sm[];
+    if ((int)blockIdx.x < n_heads * chunks) {            // (into L2 only: see prefetch_l2)
+        const bf16* from = uk + (size_t)(blockIdx.x / chunks) * plain * rank + blockIdx.x % chunks * AR_COLS;
+        for (int e = threadIdx.x; e < plain; e += AR_THREADS) prefetch_l2(from + (size_t)e * rank);
+    }
+    ti_pdl_sync();
+    d = ti_dependent(d); q = ti_dependent(q);
+    const int m0 = blockIdx.y * TOK, n = min(TOK, M - m0);
+    if ((int)blockIdx.x >= n_heads * chunks) {
+        const int i = blockIdx.x - n_heads * chunks;
+        if (i < n)
+            latent_prep_body<bf16>(sm, m0 + i, d, d_stride, (bf16*)nullptr, 0, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos,
+                                   tok_seq, seq_slot, lat, kv);
+        return;
+    }
+    const int h = blockIdx.x / chunks, chunk = blockIdx.x - h * chunks, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int hd = plain + rot, W = rank + rot, half = rot >> 1, r = chunk * AR_COLS + 2 * lane;
+    float* qs = sm;                      // [plain][TOK]
+    float* part = sm + plain * TOK;      // [4][TOK][AR_COLS]
+    // (loads in batches, so that several are on their way at a time: a warp every fourth token, a lane every 32nd element)
+    for (int e0 = 0; e0 < plain; e0 += 64) {
+        float x[TOK / 4][2];
+#pragma unroll
+        for (int i = 0; i < TOK / 4; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int tok = warp + 4 * i, e = e0 + lane + 32 * j;
+                x[i][j] = tok < n && e < plain ? to_f32(q[(size_t)(m0 + tok) * q_stride + (size_t)h * hd + e]) : 0.f;
+            }
+#pragma unroll
+        for (int i = 0; i < TOK / 4; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+                if (e0 + lane + 32 * j < plain) qs[(e0 + lane + 32 * j) * TOK + warp + 4 * i] = x[i][j];
+    }
+    // the rotated parts of the tokens chunk, chunk + chunks, ...
+    for (int i = t; i < (n - chunk + chunks - 1) / chunks * half; i += AR_THREADS) {
+        const int tok = chunk + i / half * chunks, e = i % half;
+        if (tok >= n) continue;
+        const bf16* qh = q + (size_t)(m0 + tok) * q_stride + (size_t)h * hd + plain;
+        float* dst = qa + ((size_t)(m0 + tok) * n_heads + h) * W + rank;
+        const int pos = min(max(tok_pos[m0 + tok], 0), max_pos - 1);
+        // (rounded to the engine's type as the rotation in place would have left it)
+        const float u = to_f32(qh[e]), v = to_f32(qh[e + half]), c = cos_t[(size_t)pos * half + e], sn = sin_t[(size_t)pos * half + e];
+        dst[e] = to_f32(from_f32<bf16>(u * c - v * sn));
+        dst[e + half] = to_f32(from_f32<bf16>(v * c + u * sn));
+    }
+    __syncthreads();
+    float acc[TOK][2];
+#pragma unroll
+    for (int i = 0; i < TOK; i++) acc[i][0] = acc[i][1] = 0.f;
+    const bf16* from = uk + (size_t)h * plain * rank + r;
+    for (int e0 = warp; e0 < plain; e0 += 4 * 16) {
+        uint32_t w[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) w[j] = e0 + 4 * j < plain && r < rank ? *reinterpret_cast<const uint32_t*>(from + (size_t)(e0 + 4 * j) * rank) : 0u;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            if (e0 + 4 * j >= plain) break;
+            const float w0 = __uint_as_float(w[j] << 16), w1 = __uint_as_float(w[j] & 0xffff0000u);
+#pragma unroll
+            for (int i = 0; i < TOK; i += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(qs + (e0 + 4 * j) * TOK + i);
+                acc[i][0] = fmaf(x.x, w0, acc[i][0]); acc[i][1] = fmaf(x.x, w1, acc[i][1]);
+                acc[i + 1][0] = fmaf(x.y, w0, acc[i + 1][0]); acc[i + 1][1] = fmaf(x.y, w1, acc[i + 1][1]);
+                acc[i + 2][0] = fmaf(x.z, w0, acc[i + 2][0]); acc[i + 2][1] = fmaf(x.z, w1, acc[i + 2][1]);
+                acc[i + 3][0] = fmaf(x.w, w0, acc[i + 3][0]); acc[i + 3][1] = fmaf(x.w, w1, acc[i + 3][1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TOK; i++) *reinterpret_cast<float2*>(part + (warp * TOK + i) * AR_COLS + 2 * lane) = make_float2(acc[i][0], acc[i][1]);
+    __syncthreads();
+    for (int i = t; i < n * AR_COLS; i += AR_THREADS) {
+        const int tok = i / AR_COLS, e = i - tok * AR_COLS;
+        if (chunk * AR_COLS + e < rank)
+            qa[((size_t)(m0 + tok) * n_heads + h) * W + chunk * AR_COLS + e] =
+                (part[i] + part[TOK * AR_COLS + i]) + (part[2 * TOK * AR_COLS + i] + part[3 * TOK * AR_COLS + i]);
+    }
+}
+
+template <int TOK>
+int launch_absorb_rows(const void* d, long long d_stride, const void* q, long long q_stride, int n_heads, int plain, int rank, int rot,
+                       const float* norm_w, float eps, const float* cos_t, const float* sin_t, int max_pos, const int* tok_pos,
+                       const int* tok_seq, const int* seq_slot, void* lat, const LatentPages& kv, const void* uk, float* qa, int M, size_t row,
+                       cudaStream_t stream) {
+    const int chunks = (rank + AR_COLS - 1) / AR_COLS;
+    const size_t smem = std::max(row, absorb_rows_smem<TOK>(plain));
+    if (smem > 48 * 1024) TI_CUDA(cudaFuncSetAttribute(latent_absorb_rows_kernel<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TI_CUDA(ti_launch_class<2>(latent_absorb_rows_kernel<TOK>, dim3(n_heads * chunks + std::min(M, TOK), (M + TOK - 1) / TOK), dim3(AR_THREADS), smem, stream,
+                               (const bf16*)d, d_stride, (const bf16*)q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos,
+                               tok_pos, tok_seq, seq_slot, (bf16*)lat, kv, (const bf16*)uk, qa, M, chunks));
+    TI_CHECK_LAUNCH("latent_prep_absorb");
+    return 0;
+}
+
 // For steps of few tokens: the merge of the key splits and the way out through Wuv in one launch.  Block (token, head):
 // the splits' unnormalised sums are weighed and added into the latent result (shared memory), then
 // o[v] = sum_r uv[h, v, r] * result[r], a warp per output element, four elements at a time.
@@ -226,32 +359,44 @@ latent_merge_expand_kernel(const float* __restrict__ part_o, const float* __rest
     ti_pdl_trigger();
     extern __shared__ float res[];       // [rank], then [64] weights
     float* w_s = res + rank;
+    if (sizeof(T) == 2)          // the head's Wuv towards L2 meanwhile, a part a token (see prefetch_l2)
+        for (int i = ((int)blockIdx.x * blockDim.x + threadIdx.x) * 64; i < vdim * rank; i += gridDim.x * blockDim.x * 64) prefetch_l2(uv + (size_t)blockIdx.y * vdim * rank + i);
     ti_pdl_sync();
     part_o = ti_dependent(part_o); part_ml = ti_dependent(part_ml);
     const int b = blockIdx.x, h = blockIdx.y, t = threadIdx.x;
     const size_t base = ((size_t)b * n_heads + h) * n_splits;
-    float m = -INFINITY;
-    for (int s = 0; s < n_splits; s++) m = fmaxf(m, part_ml[(base + s) * 2]);
-    float l = 0.f;
-    for (int s = 0; s < n_splits; s++) {
-        const float ms = part_ml[(base + s) * 2];
-        const float w = ms > -INFINITY ? expf(ms - m) : 0.f;
-        if (t == 0) w_s[s] = w;
-        l += w > 0.f ? w * part_ml[(base + s) * 2 + 1] : 0.f;
+    // every warp: the splits' maxima and denominators, two a lane (n_splits is at most 64)
+    float ms[2], ls[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const int s = (t & 31) + 32 * j;
+        const float2 ml = s < n_splits ? *reinterpret_cast<const float2*>(part_ml + (base + s) * 2) : make_float2(-INFINITY, 0.f);
+        ms[j] = ml.x; ls[j] = ml.y;
     }
+    const float m = warp_max(fmaxf(ms[0], ms[1]));
+    float l = 0.f;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const float w = ms[j] > -INFINITY ? expf(ms[j] - m) : 0.f;
+        l += w > 0.f ? w * ls[j] : 0.f;
+        if (t < 32) w_s[t + 32 * j] = w;
+    }
+    l = warp_sum(l);
+    const unsigned some = __ballot_sync(0xffffffffu, ms[0] > -INFINITY), more = __ballot_sync(0xffffffffu, ms[1] > -INFINITY);
+    const int last = more ? 64 - __clz(more) : 32 - __clz(some);      // (the splits behind are empty)
     __syncthreads();
     float inv = l > 0.f ? 1.f / l : 0.f;
     if (gate) inv *= head_gate(ti_dependent(gate), gate_stride, b, h);      // (the way out is linear)
     for (int e = t; e < rank; e += blockDim.x) {
         float acc = 0.f;
-        for (int s0 = 0; s0 < n_splits; s0 += 8) {      // eight splits' numbers on their way together
-            float x[8];
+        for (int s0 = 0; s0 < last; s0 += 16) {          // sixteen splits' numbers on their way together
+            float x[16];
 #pragma unroll
-            for (int j = 0; j < 8; j++)          // (an empty split's numbers were never written)
-                x[j] = s0 + j < n_splits && w_s[s0 + j] > 0.f ? part_o[(base + s0 + j) * rank + e] : 0.f;
+            for (int j = 0; j < 16; j++)         // (an empty split's numbers were never written)
+                x[j] = s0 + j < last && w_s[s0 + j] > 0.f ? part_o[(base + s0 + j) * rank + e] : 0.f;
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                if (s0 + j < n_splits) acc = fmaf(w_s[s0 + j], x[j], acc);
+            for (int j = 0; j < 16; j++)
+                if (s0 + j < last) acc = fmaf(w_s[s0 + j], x[j], acc);
         }
         res[e] = acc * inv;
     }
@@ -261,6 +406,7 @@ latent_merge_expand_kernel(const float* __restrict__ part_o, const float* __rest
         // 16-byte pieces of four rows at a time: eight loads on their way per lane
         for (int v0 = warp * 4; v0 < vdim; v0 += rows) {
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
             for (int c = lane; c < (rank >> 3); c += 32) {
                 uint4 w[4];
 #pragma unroll
@@ -570,18 +716,20 @@ latent_attn_kernel(const float* __restrict__ qa, const T* __restrict__ lat, floa
 // ---------------------------------------------------------------------------
 // One query per sequence, bfloat16, on the tensor cores (`mma.sync m16n8k16`, float32 accumulation).  A block takes one
 // sequence, 16 * MT heads and one share of the keys, 32 positions at a time: the rows [c | r] of a tile go to shared memory
-// as they are; S = Qa L^T (a warp per 8 keys), the softmax in 32-bit where the scores are (a row's maximum meets over the
-// warps in shared memory), P rounded to bfloat16 as the second product's operand, O += P L[:, :rank] (the latent's columns
-// shared out over the warps).  Unnormalised sums, maxima and denominators go to the merging kernel when the keys are split.
+// as they are; S = Qa L^T (every warp a quarter of a row's elements for all 32 keys; the quarters meet in shared memory), the softmax
+// in 32-bit (a warp four heads of every 16), P rounded to bfloat16 as the second product's operand, O += P L[:, :rank] (the latent's
+// columns shared out over the warps).  Unnormalised sums, maxima and denominators go to the merging kernel when the keys are split.
 // Rows of a tile outside the query's reach are zeroed: a weight of zero times whatever stood there must stay zero.
 //
-// What bounds it: the read of the rows.  A tile is on its way (cp.async) while the one before it is worked off, and two blocks
-// share an SM when 16 heads or fewer share the rows, so some 70 KB are in flight per SM; a tile of 37 KB takes an SM's share of
-// the memory 1,600 cycles, its arithmetic in two blocks about as long.  16 sequences of 1,000 to 4,000 positions, 16 heads, rows of
-// 512 + 64: 120 us when a tile was fetched, scored and summed one after another (a row's softmax by one thread, the latent's
-// columns as 16-bit reads), 30 now; the way into the latent before it 26 -> 9, the merge and the way out after it 10 -> 12 (of
-// twice the splits).
-constexpr int DK = 32, D_THREADS = 128, P_LD = DK + 8;
+// What bounds it: a tile's chain of steps.  A tile is on its way (a bulk copy a row) while the one before it is worked off, and two
+// blocks share an SM where there is room; 16 sequences of 1,000 to 4,000 positions, 16 heads, rows of 512 + 64, us a tile of a block:
+// the queue of copies and the look-up of the next tile's page 1.4 -> 0.2 (16-byte copies by all threads before, the page's number
+// awaited at once), scores 0.9 -> 0.5 (queries in registers where they fit), softmax and its two barriers 0.5, values 0.65.  All
+// sequences' splits are equally many tiles; with splits of equal number a sequence's own the longest sequence's blocks ended
+// last (7 tiles where the mean is 4).  The layer's step 65.6 -> 53.0, of which the attention 30 -> 21, the way into the latent before it 9 ->
+// 6; the merge and the way out after it 12, bound by 34 MB of Wuv from L2 (a cluster of eight blocks that read it once, shared their
+// results and took 13: not kept).
+constexpr int DK = 32, D_THREADS = 128;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -595,93 +743,156 @@ __device__ __forceinline__ void ld_matrix4_trans(uint32_t (&r)[4], uint32_t addr
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-template <int MT> size_t decode_mma_smem(int W, int tiles) {
-    return (size_t)(16 * MT + tiles * DK) * (W + 8) * 2 + (size_t)16 * MT * P_LD * 2 + (size_t)16 * MT * 8 * 4;
+constexpr int Q_STEPS = 10;          // QREG: steps of 16 elements of a row that a warp has at most (rows of up to 640)
+
+// Scores of a tile as the warps leave them: [shares][ROWS][pitch] floats, 32 keys a row; later a row's weights (bfloat16, in place) and,
+// behind them, the factor of its sums so far.
+constexpr int S_FACTOR = 16;         // where in a row of 32 floats that factor stands
+struct DecodeShape { int tiles, shares, pitch; size_t smem; };
+template <int MT, bool QREG> DecodeShape decode_mma_shape(int W) {
+    auto bytes = [&](int tiles, int shares, int pitch) {
+        return (size_t)((QREG ? 0 : 16 * MT) + tiles * DK) * (W + 8) * 2 + (size_t)shares * 16 * MT * pitch * 4;
+    };
+    DecodeShape s{2, 4, 40, 0};
+    if (bytes(2, 4, 40) > 227 * 1024) s.tiles = 1;                                            // wide rows: one tile of them
+    if (bytes(s.tiles, 4, 40) > 227 * 1024) { s.shares = 1; s.pitch = 32; }                  // the widest: the warps add to one place in turn
+    s.smem = bytes(s.tiles, s.shares, s.pitch);
+    return s;
 }
 
-template <int MT, int NTW>
+// QREG: a warp's quarter of the queries stays in its registers (one tile of 16 heads, rows of up to 640 elements), else they lie in
+// shared memory.
+template <int MT, int NTW, bool QREG>
 __global__ void __launch_bounds__(D_THREADS)
 latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ lat, float* __restrict__ ol,
                          const int* __restrict__ cu_new, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
                          int n_heads, int rank, int rot, float scale, int window, const float* __restrict__ sink,
-                         LatentPages kv, int n_splits, float* __restrict__ part_o, float* __restrict__ part_ml, int tiles) {
+                         LatentPages kv, int n_splits, int room, float* __restrict__ part_o, float* __restrict__ part_ml, int tiles,
+                         int shares, int pitch, int* status) {
     ti_pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ uint64_t full[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    if (tid == 0) { mbar_init(&full[0], 1); mbar_init(&full[1], 1); mbar_fence_init(); }
     ti_pdl_sync();
     qa = ti_dependent(qa); lat = ti_dependent(lat);
     constexpr int ROWS = 16 * MT;
     const int ahead = tiles - 1;                                   // (1, or 0: rows so wide that only one tile of them fits)
-    const int W = rank + rot, LD = W + 8;
-    bf16* Qs = reinterpret_cast<bf16*>(smem_raw);                  // [ROWS][LD]
-    bf16* Ls = Qs + ROWS * LD;                                     // [tiles][DK][LD]
-    bf16* Ps = Ls + tiles * DK * LD;                                 // [ROWS][P_LD]
-    float* mx_s = reinterpret_cast<float*>(Ps + ROWS * P_LD);      // [4][ROWS] the warps' maxima, later their denominators
-    const int split = blockIdx.x, h0 = blockIdx.y * ROWS, b = blockIdx.z;
-    const int tok = cu_new[b];
-    if (cu_new[b + 1] - tok <= 0) return;
-    const int qi = seq_start[b], slot = seq_slot[b];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    const int W = rank + rot, LD = W + 8, steps = W >> 4;
+    float* Sp = reinterpret_cast<float*>(smem_raw);
+    bf16* Ls = reinterpret_cast<bf16*>(smem_raw + (size_t)shares * ROWS * pitch * 4);      // [tiles][DK][LD]
+    bf16* Qs = Ls + tiles * DK * LD;                               // [ROWS][LD]
+    const int split = blockIdx.z, h0 = blockIdx.y * ROWS, b = blockIdx.x;        // (the splits that are empty come last)
+    const int tok = cu_new[b], tok_end = cu_new[b + 1], qi = seq_start[b], slot = seq_slot[b];
+    // Tiles of a split: the same for all sequences, so that the blocks of long and short ones take as long; as many as give every
+    // block that runs at once its share of the step's tiles, and no fewer than the longest sequence needs for n_splits splits.
+    int sum = 0, most = 0;
+    for (int s = lane; s < (int)gridDim.x; s += 32) {
+        const int q = seq_start[s], n = cu_new[s + 1] > cu_new[s] ? q / DK - (window > 0 ? max(0, q - window + 1) : 0) / DK + 1 : 0;
+        sum += n;
+        most = max(most, n);
+    }
+    if (tok_end - tok <= 0) return;
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    most = __reduce_max_sync(0xffffffffu, most);
     const int lo = window > 0 ? max(0, qi - window + 1) : 0;
     const int kt_first = lo / DK, kt_last = qi / DK;
-    const int per = (kt_last - kt_first + n_splits) / n_splits;
+    const int per = max((int)(((long long)sum * gridDim.y + room - 1) / room), (most + n_splits - 1) / n_splits);
     const int kt_a = kt_first + split * per, kt_b = min(kt_last, kt_a + per - 1);
     const int n_tiles8 = rank >> 3;
-    // where this thread's row of a tile lives (four threads a row); null: out of the query's reach
-    auto row_of = [&](int kt) -> const bf16* {
-        const int p = kt * DK + (tid >> 2);
-        if (kt > kt_b || p > qi || p < lo) return nullptr;
-        if (p == qi) return lat + (size_t)tok * W;
+    if (kt_a > kt_last && part_o != nullptr) {                     // nothing is left for this split
+        for (int r = tid; r < ROWS; r += D_THREADS)
+            if (h0 + r < n_heads) {
+                float* ml = part_ml + (((size_t)tok * n_heads + h0 + r) * n_splits + split) * 2;
+                ml[0] = -INFINITY; ml[1] = 0.f;
+            }
+        return;
+    }
+    // The first warp brings the tiles, a lane a row: one bulk copy each, zeros where the row is out of the query's reach.  Where the
+    // tiles lie is looked up for 32 of them at a time, a lane a tile (a tile lies inside one page): looked up tile by tile, the chain of
+    // a load and its use cost the warp 1.4 us of every tile's 3.5.
+    const bool whole = kv.page_size % DK == 0;                     // (else row by row)
+    auto row_at = [&](int p) -> long long {                        // of position p among the cache's rows, or -1
         const int row = kv.ring_rows > 0 ? p % kv.ring_rows : p;
         const int pidx = row / kv.page_size;
         const int page = pidx < kv.table_width ? kv.page_table[(size_t)slot * kv.table_width + pidx] : -1;
-        return page >= 0 && page < kv.n_pages ? (const bf16*)kv.pages + ((size_t)page * kv.page_size + row % kv.page_size) * W : nullptr;
+        return page >= 0 && page < kv.n_pages ? (long long)page * kv.page_size + row % kv.page_size : -1;
     };
-    const uint32_t ls0 = (uint32_t)__cvta_generic_to_shared(Ls), qs0 = (uint32_t)__cvta_generic_to_shared(Qs), ps0 = (uint32_t)__cvta_generic_to_shared(Ps);
-    auto fetch = [&](int kt, const bf16* src) {
-        const uint32_t to = ls0 + (uint32_t)((((kt - kt_a) & ahead) * DK + (tid >> 2)) * LD) * 2;
-        const int bytes = src ? 16 : 0;                            // the rest is filled with zeros
-        const bf16* from = src ? src : lat;
-        for (int e = (tid & 3) * 8; e < W; e += 32)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + e * 2), "l"(src ? from + e : from), "r"(bytes) : "memory");
-    };
-    const bf16* next = nullptr;
-    if (kt_a <= kt_b) {
-        fetch(kt_a, row_of(kt_a));
-        next = row_of(kt_a + 1);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    // (global loads in batches, so that several are on their way at a time)
-    {
-        const int per_row = W >> 2, total = ROWS * per_row;        // pieces of four floats
-        for (int i0 = 0; i0 < total; i0 += 6 * D_THREADS) {
-            float4 x[6];
+    long long tile_row = -1;                                       // of the first position of tile kt_a + 32 n + lane
+    if (whole && warp == 0 && kt_a + lane <= kt_b) tile_row = row_at((kt_a + lane) * DK);
+    uint32_t qf[QREG ? Q_STEPS : 1][4];
+    float2 qx[QREG ? Q_STEPS : 1][4];
+    if constexpr (QREG) {
+        const float* q0 = qa + ((size_t)tok * n_heads + h0 + g) * W + 2 * t4;
+        const bool ok0 = h0 + g < n_heads, ok1 = h0 + g + 8 < n_heads;
 #pragma unroll
-            for (int u = 0; u < 6; u++) {
+        for (int i = 0; i < Q_STEPS; i++) {
+            const int ks = warp + 4 * i;
+#pragma unroll
+            for (int j = 0; j < 4; j++)          // (row g, k), (row g + 8, k), (row g, k + 8), (row g + 8, k + 8)
+                qx[i][j] = ks < steps && (j & 1 ? ok1 : ok0) ? *reinterpret_cast<const float2*>(q0 + (size_t)(j & 1) * 8 * W + ks * 16 + (j >> 1) * 8) : make_float2(0.f, 0.f);
+        }
+    }
+    auto fetch = [&](int kt) {                   // by the whole first warp
+        const int nth = kt - kt_a, at = nth & ahead, p = kt * DK + lane;
+        if (whole && nth > 0 && (nth & 31) == 0) tile_row = kt + lane <= kt_b ? row_at((kt + lane) * DK) : -1;
+        long long row = whole ? __shfl_sync(0xffffffffu, tile_row, nth & 31) : -1;
+        if (whole) row += row >= 0 ? lane : 0;
+        else if (p >= lo && p < qi) row = row_at(p);
+        const bf16* src = p == qi ? lat + (size_t)tok * W : p >= lo && p < qi && row >= 0 ? (const bf16*)kv.pages + (size_t)row * W : nullptr;
+        bf16* to = Ls + (size_t)(at * DK + lane) * LD;
+        const int live = __popc(__ballot_sync(0xffffffffu, src != nullptr));
+        if (src == nullptr)
+            for (int e = 0; e < W; e += 8) *reinterpret_cast<uint4*>(to + e) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();             // (a place that held zeros is written by a copy next)
+        if (lane == 0) { if (live) mbar_expect_tx(&full[at], (uint32_t)live * W * 2); else mbar_arrive(&full[at]); }
+        __syncwarp();
+        if (src != nullptr)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_u32(to)), "l"(src), "r"(W * 2), "r"(smem_u32(&full[at])) : "memory");
+    };
+    const uint32_t ls0 = smem_u32(Ls), qs0 = smem_u32(Qs), sp0 = smem_u32(Sp);
+    if (warp == 0) fetch(kt_a);
+    if constexpr (QREG) {
+#pragma unroll
+        for (int i = 0; i < Q_STEPS; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const __nv_bfloat162 p = __floats2bfloat162_rn(qx[i][j].x, qx[i][j].y);
+                qf[i][j] = *reinterpret_cast<const uint32_t*>(&p);
+            }
+    } else {
+        // (global loads in batches, so that several are on their way at a time)
+        const int per_row = W >> 2, total = ROWS * per_row;        // pieces of four floats
+        for (int i0 = 0; i0 < total; i0 += 12 * D_THREADS) {
+            float4 x[12];
+#pragma unroll
+            for (int u = 0; u < 12; u++) {
                 const int idx = i0 + u * D_THREADS + tid, r = idx / per_row, e = idx - r * per_row;
                 x[u] = (idx < total && h0 + r < n_heads) ? reinterpret_cast<const float4*>(qa + ((size_t)tok * n_heads + h0 + r) * W)[e]
                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
-            for (int u = 0; u < 6; u++) {
+            for (int u = 0; u < 12; u++) {
                 const int idx = i0 + u * D_THREADS + tid, r = idx / per_row, e = idx - r * per_row;
                 if (idx < total) {
-                    bf16* dst = Qs + r * LD + 4 * e;
-                    dst[0] = from_f32<bf16>(x[u].x); dst[1] = from_f32<bf16>(x[u].y); dst[2] = from_f32<bf16>(x[u].z); dst[3] = from_f32<bf16>(x[u].w);
+                    const __nv_bfloat162 a = __floats2bfloat162_rn(x[u].x, x[u].y), c = __floats2bfloat162_rn(x[u].z, x[u].w);
+                    *reinterpret_cast<uint2*>(Qs + r * LD + 4 * e) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c));
                 }
             }
         }
     }
-    // per row g and g + 8 of every 16: the running maximum (the same in all threads of the row) and this thread's share of the denominator
-    float m_run[MT][2], l_run[MT][2];
+    // The softmax: a warp has four rows of every 16, a lane four of a row's 32 keys.  The row's running maximum (the same in its eight
+    // lanes) and this lane's share of the denominator:
+    const int srow = warp * 4 + (lane >> 3), skey = (lane & 7) * 4;
+    float m_run[MT], l_run[MT];
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const int h = h0 + mt * 16 + g + 8 * r;
-            const bool with_sink = sink && split == 0 && h < n_heads;
-            m_run[mt][r] = with_sink ? sink[h] : -INFINITY;
-            l_run[mt][r] = with_sink && warp == 0 && t4 == 0 ? 1.f : 0.f;
-        }
+    for (int mt = 0; mt < MT; mt++) {
+        const int h = h0 + mt * 16 + srow;
+        const bool with_sink = sink && split == 0 && h < n_heads;
+        m_run[mt] = with_sink ? sink[h] : -INFINITY;
+        l_run[mt] = with_sink && skey == 0 ? 1.f : 0.f;
+    }
     float O[MT][NTW][4];
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
@@ -689,98 +900,117 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
         for (int i = 0; i < NTW; i++)
 #pragma unroll
             for (int c = 0; c < 4; c++) O[mt][i][c] = 0.f;
+    bool ok = true;
     for (int kt = kt_a; kt <= kt_b; kt++) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                 // this tile is there (at first Qs too); the other place is no longer read
-        if (ahead && kt < kt_b) {
-            fetch(kt + 1, next);
-            next = row_of(kt + 2);       // looked up a tile ahead
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const uint32_t ls = ls0 + (uint32_t)(((kt - kt_a) & ahead) * DK * LD) * 2;
-        // scores: this warp's 8 keys against all rows, in four chains of sums
-        float c[MT][4][4] = {};
+        const int nth = kt - kt_a;
+        if (!mbar_wait(&full[nth & ahead], (uint32_t)((ahead ? nth >> 1 : nth) & 1))) { ti_report(status, TI_STATUS_TMA_WAIT); ok = false; }
+        if (!__syncthreads_and(ok)) {            // (given up: not before the copies under way have arrived, or their wait has run out too)
+            if (tid == 0) mbar_wait(&full[nth & ahead], (uint32_t)((ahead ? nth >> 1 : nth) & 1));
+            __syncthreads();
+            return;
+        }                                // this tile is there (at first the queries too); the other place and the scores are no longer read
+        if (ahead && kt < kt_b && warp == 0) fetch(kt + 1);
+        const uint32_t ls = ls0 + (uint32_t)((nth & ahead) * DK * LD) * 2;
+        // scores: this warp's steps of the rows' elements (every fourth) of all 32 keys
         {
-            const uint32_t kaddr = ls + (uint32_t)((warp * 8 + (lane & 7)) * LD + (lane >> 3) * 8) * 2;
+            float c[MT][4][4] = {};
+            const uint32_t kaddr = ls + (uint32_t)(((lane & 7) + ((lane >> 4) & 1) * 8) * LD + ((lane >> 3) & 1) * 8) * 2;
             const uint32_t qaddr = qs0 + (uint32_t)((lane & 15) * LD + (lane >> 4) * 8) * 2;
-            int kk = 0;
-#pragma unroll 2
-            for (; kk + 32 <= W; kk += 32) {
-                uint32_t kb[4];          // two steps of 16
-                ld_matrix4(kb, kaddr + kk * 2);
-                const int ch = (kk >> 5) & 1;
+            auto step = [&](int ks, const uint32_t (&a)[MT][4]) {
+                uint32_t k0[4], k1[4];       // keys 0-7 and 8-15, 16-23 and 24-31: two halves of the step each
+                ld_matrix4(k0, kaddr + (uint32_t)(ks * 16) * 2);
+                ld_matrix4(k1, kaddr + (uint32_t)(16 * LD + ks * 16) * 2);
 #pragma unroll
                 for (int mt = 0; mt < MT; mt++) {
-                    uint32_t a0[4], a1[4];
-                    ld_matrix4(a0, qaddr + (uint32_t)(mt * 16 * LD + kk) * 2);
-                    ld_matrix4(a1, qaddr + (uint32_t)(mt * 16 * LD + kk + 16) * 2);
-                    if (ch) { mma_bf16_16816(c[mt][2], a0, kb[0], kb[1]); mma_bf16_16816(c[mt][3], a1, kb[2], kb[3]); }
-                    else { mma_bf16_16816(c[mt][0], a0, kb[0], kb[1]); mma_bf16_16816(c[mt][1], a1, kb[2], kb[3]); }
+                    mma_bf16_16816(c[mt][0], a[mt], k0[0], k0[1]);
+                    mma_bf16_16816(c[mt][1], a[mt], k0[2], k0[3]);
+                    mma_bf16_16816(c[mt][2], a[mt], k1[0], k1[1]);
+                    mma_bf16_16816(c[mt][3], a[mt], k1[2], k1[3]);
+                }
+            };
+            if constexpr (QREG) {
+#pragma unroll
+                for (int i = 0; i < Q_STEPS; i++)
+                    if (warp + 4 * i < steps) {
+                        const uint32_t a[1][4] = {{qf[i][0], qf[i][1], qf[i][2], qf[i][3]}};
+                        step(warp + 4 * i, a);
+                    }
+            } else {
+#pragma unroll 4
+                for (int ks = warp; ks < steps; ks += 4) {
+                    uint32_t a[MT][4];
+#pragma unroll
+                    for (int mt = 0; mt < MT; mt++) ld_matrix4(a[mt], qaddr + (uint32_t)(mt * 16 * LD + ks * 16) * 2);
+                    step(ks, a);
                 }
             }
-            if (kk < W) {                // sixteen left
-                const bf16* krow = Ls + (size_t)((kt - kt_a) & ahead) * DK * LD + (warp * 8 + g) * LD + 2 * t4 + kk;
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(krow), b1 = *reinterpret_cast<const uint32_t*>(krow + 8);
+            for (int w = 0; w < 4; w++) {
+                if (shares == 4 ? w == 0 : w == warp) {
+                    float* mine = Sp + (size_t)(shares == 4 ? warp : 0) * ROWS * pitch + 2 * t4;
+                    const bool add = shares == 1 && warp > 0;
 #pragma unroll
-                for (int mt = 0; mt < MT; mt++) {
-                    uint32_t a[4];
-                    ld_matrix4(a, qaddr + (uint32_t)(mt * 16 * LD + kk) * 2);
-                    mma_bf16_16816(c[mt][0], a, b0, b1);
+                    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                        for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+                            for (int r = 0; r < 2; r++) {
+                                float2* at = reinterpret_cast<float2*>(mine + (mt * 16 + g + 8 * r) * pitch + nt * 8);
+                                const float2 had = add ? *at : make_float2(0.f, 0.f);
+                                *at = make_float2(had.x + c[mt][nt][2 * r], had.y + c[mt][nt][2 * r + 1]);
+                            }
                 }
+                __syncthreads();
+                if (shares == 4) break;
             }
         }
-        const int p0 = kt * DK + warp * 8 + 2 * t4;
-        const bool in0 = p0 >= lo && p0 <= qi, in1 = p0 + 1 >= lo && p0 + 1 <= qi;
-        float s[MT][2][2];
-#pragma unroll
-        for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const bool head_ok = h0 + mt * 16 + g + 8 * r < n_heads;
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const float v = (c[mt][0][2 * r + e] + c[mt][1][2 * r + e]) + (c[mt][2][2 * r + e] + c[mt][3][2 * r + e]);
-                    s[mt][r][e] = head_ok && (e ? in1 : in0) ? v * scale : -INFINITY;
-                }
-                float mx = fmaxf(s[mt][r][0], s[mt][r][1]);
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                if (t4 == 0) mx_s[warp * ROWS + mt * 16 + g + 8 * r] = mx;
-            }
-        __syncthreads();
-        float alpha[MT][2];
-#pragma unroll
-        for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const int row = mt * 16 + g + 8 * r;
-                const float m_new = fmaxf(fmaxf(fmaxf(mx_s[row], mx_s[ROWS + row]), fmaxf(mx_s[2 * ROWS + row], mx_s[3 * ROWS + row])), m_run[mt][r]);
-                const bool any = m_new > -INFINITY;
-                alpha[mt][r] = any ? expf(m_run[mt][r] - m_new) : 1.f;
-                const float e0 = s[mt][r][0] == -INFINITY ? 0.f : expf(s[mt][r][0] - m_new);
-                const float e1 = s[mt][r][1] == -INFINITY ? 0.f : expf(s[mt][r][1] - m_new);
-                m_run[mt][r] = m_new;
-                l_run[mt][r] = l_run[mt][r] * alpha[mt][r] + (e0 + e1);
-                const __nv_bfloat162 pk = __floats2bfloat162_rn(e0, e1);
-                *reinterpret_cast<uint32_t*>(Ps + row * P_LD + warp * 8 + 2 * t4) = *reinterpret_cast<const uint32_t*>(&pk);
-            }
-        __syncthreads();
-        // O += P L: a warp has pairs of tiles of 8 columns of the latent, warp, warp + 4, ...
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
-            if (__any_sync(0xffffffffu, alpha[mt][0] != 1.f || alpha[mt][1] != 1.f)) {
-#pragma unroll
-                for (int i = 0; i < NTW; i++) {
-                    O[mt][i][0] *= alpha[mt][0]; O[mt][i][1] *= alpha[mt][0]; O[mt][i][2] *= alpha[mt][1]; O[mt][i][3] *= alpha[mt][1];
-                }
+            float* row = Sp + (mt * 16 + srow) * pitch;
+            float4 x = *reinterpret_cast<const float4*>(row + skey);
+            if (shares == 4) {
+                const float4 x1 = *reinterpret_cast<const float4*>(row + ROWS * pitch + skey), x2 = *reinterpret_cast<const float4*>(row + 2 * ROWS * pitch + skey);
+                const float4 x3 = *reinterpret_cast<const float4*>(row + 3 * ROWS * pitch + skey);
+                x = make_float4((x.x + x1.x) + (x2.x + x3.x), (x.y + x1.y) + (x2.y + x3.y), (x.z + x1.z) + (x2.z + x3.z), (x.w + x1.w) + (x2.w + x3.w));
             }
+            const int p0 = kt * DK + skey;
+            const bool head_ok = h0 + mt * 16 + srow < n_heads;
+            float s[4] = {x.x, x.y, x.z, x.w}, mx = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s[e] = head_ok && p0 + e >= lo && p0 + e <= qi ? s[e] * scale : -INFINITY;
+                mx = fmaxf(mx, s[e]);
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float m_new = fmaxf(mx, m_run[mt]), alpha = m_new > -INFINITY ? expf(m_run[mt] - m_new) : 1.f;
+            m_run[mt] = m_new;
+            float sum_e = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s[e] = s[e] == -INFINITY ? 0.f : expf(s[e] - m_new);
+                sum_e += s[e];
+            }
+            l_run[mt] = l_run[mt] * alpha + sum_e;
+            const __nv_bfloat162 p01 = __floats2bfloat162_rn(s[0], s[1]), p23 = __floats2bfloat162_rn(s[2], s[3]);
+            __syncwarp();                // the row's scores have been read
+            reinterpret_cast<uint2*>(row)[lane & 7] = make_uint2(*reinterpret_cast<const uint32_t*>(&p01), *reinterpret_cast<const uint32_t*>(&p23));
+            if (skey == 0) row[S_FACTOR] = alpha;
         }
+        __syncthreads();
+        // O += P L: a warp has pairs of tiles of 8 columns of the latent, warp, warp + 4, ...
         uint32_t a[MT][2][4];
 #pragma unroll
-        for (int mt = 0; mt < MT; mt++)
+        for (int mt = 0; mt < MT; mt++) {
+            const float f0 = Sp[(mt * 16 + g) * pitch + S_FACTOR], f1 = Sp[(mt * 16 + g + 8) * pitch + S_FACTOR];
+            if (__any_sync(0xffffffffu, f0 != 1.f || f1 != 1.f)) {
 #pragma unroll
-            for (int ks = 0; ks < 2; ks++)
-                ld_matrix4(a[mt][ks], ps0 + (uint32_t)((mt * 16 + (lane & 15)) * P_LD + ks * 16 + (lane >> 4) * 8) * 2);
+                for (int i = 0; i < NTW; i++) {
+                    O[mt][i][0] *= f0; O[mt][i][1] *= f0; O[mt][i][2] *= f1; O[mt][i][3] *= f1;
+                }
+            }
+#pragma unroll
+            for (int ks = 0; ks < 2; ks++) ld_matrix4(a[mt][ks], sp0 + (uint32_t)((mt * 16 + (lane & 15)) * pitch * 4 + ks * 32 + (lane >> 4) * 16));
+        }
 #pragma unroll
         for (int i = 0; i < NTW; i += 2) {
             const int nt = 2 * warp + 4 * i;                      // this tile and the next
@@ -799,33 +1029,32 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
         }
         if (!ahead && kt < kt_b) {
             __syncthreads();             // the one tile is no longer read
-            fetch(kt + 1, next);
-            next = row_of(kt + 2);
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (warp == 0) fetch(kt + 1);
         }
     }
-    __syncthreads();
+    if (part_o == nullptr) __syncthreads();
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++)
+    for (int mt = 0; mt < MT; mt++) {
+        const int h = h0 + mt * 16 + srow;
+        float l = l_run[mt];
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-            float l = l_run[mt][r];
-            l += __shfl_xor_sync(0xffffffffu, l, 1);
-            l += __shfl_xor_sync(0xffffffffu, l, 2);
-            if (t4 == 0) mx_s[warp * ROWS + mt * 16 + g + 8 * r] = l;
+        for (int o = 1; o < 8; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (skey != 0) continue;
+        if (part_o == nullptr) Sp[(mt * 16 + srow) * pitch + S_FACTOR] = l > 0.f ? 1.f / l : 0.f;
+        else if (h < n_heads) {
+            const size_t at = ((size_t)tok * n_heads + h) * n_splits + split;
+            part_ml[at * 2] = m_run[mt]; part_ml[at * 2 + 1] = l;
         }
-    __syncthreads();
+    }
+    if (part_o == nullptr) __syncthreads();
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
         for (int half = 0; half < 2; half++) {
             const int r = mt * 16 + g + 8 * half, h = h0 + r;
             if (h >= n_heads) continue;
-            const float l = (mx_s[r] + mx_s[ROWS + r]) + (mx_s[2 * ROWS + r] + mx_s[3 * ROWS + r]);
-            const size_t at = ((size_t)tok * n_heads + h) * n_splits + split;
-            if (part_o != nullptr && t4 == 0 && warp == 0) { part_ml[at * 2] = m_run[mt][half]; part_ml[at * 2 + 1] = l; }
-            float* dst = part_o != nullptr ? part_o + at * rank : ol + ((size_t)tok * n_heads + h) * rank;
-            const float f = part_o != nullptr ? 1.f : l > 0.f ? 1.f / l : 0.f;
+            float* dst = part_o != nullptr ? part_o + (((size_t)tok * n_heads + h) * n_splits + split) * rank : ol + ((size_t)tok * n_heads + h) * rank;
+            const float f = part_o != nullptr ? 1.f : Sp[r * pitch + S_FACTOR];
 #pragma unroll
             for (int i = 0; i < NTW; i++) {
                 const int nt = 2 * warp + 4 * (i & ~1) + (i & 1);
@@ -835,25 +1064,57 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
         }
 }
 
+// (SMs of the current device, asked once for each)
+int latent_sms(int* sms) {
+    static int known[64] = {0};
+    int dev = 0;
+    TI_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || known[dev] == 0) {
+        TI_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
+        if (dev >= 0 && dev < 64) known[dev] = *sms;
+        return 0;
+    }
+    *sms = known[dev];
+    return 0;
+}
+
+template <int MT, int NTW, bool QREG>
+int launch_decode_form(const float* qa, const void* lat, float* ol, const int* cu_new, const int* seq_start, const int* seq_slot,
+                       int n_seq, int n_heads, int rank, int rot, float scale, int window, const float* sink,
+                       const LatentPages& kv, int n_splits, float* part_o, float* part_ml, cudaStream_t stream) {
+    constexpr int ROWS = 16 * MT;
+    const int W = rank + rot;
+    const DecodeShape shape = decode_mma_shape<MT, QREG>(W);
+    const size_t smem = shape.smem;
+    int* status = ti_status_ptr();
+    TI_REQUIRE(status != nullptr, "latent_attention: no status word");
+    static size_t configured = 0;
+    if (smem > 48 * 1024 && smem > configured) {
+        TI_CUDA(cudaFuncSetAttribute(latent_decode_mma_kernel<MT, NTW, QREG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured = smem;
+    }
+    int sms = 0;
+    if (int rc = latent_sms(&sms)) return rc;
+    const int room = sms * (smem <= 113 * 1024 ? 2 : 1);
+    dim3 grid(n_seq, (n_heads + ROWS - 1) / ROWS, n_splits);
+    TI_CUDA(ti_launch_class<3>(latent_decode_mma_kernel<MT, NTW, QREG>, grid, dim3(D_THREADS), smem, stream, qa, (const bf16*)lat, ol, cu_new,
+                               seq_start, seq_slot, n_heads, rank, rot, scale, window, sink, kv, n_splits, room, part_o, part_ml, shape.tiles, shape.shares, shape.pitch, status));
+    TI_CHECK_LAUNCH("latent_attention (one token, tensor cores)");
+    return 0;
+}
+
 template <int MT, int NTW>
 int launch_decode_mma(const float* qa, const void* lat, float* ol, const int* cu_new, const int* seq_start, const int* seq_slot,
                       int n_seq, int n_heads, int rank, int rot, float scale, int window, const float* sink,
                       const LatentPages& kv, int n_splits, float* part_o, float* part_ml, int n_tok, cudaStream_t stream,
                       const void* uv = nullptr, void* o = nullptr, long long o_stride = 0, int vdim = 0, const void* gate = nullptr,
                       long long gate_stride = 0) {
-    constexpr int ROWS = 16 * MT;
-    const int W = rank + rot;
-    const int tiles = decode_mma_smem<MT>(W, 2) <= 227 * 1024 ? 2 : 1;
-    const size_t smem = decode_mma_smem<MT>(W, tiles);
-    static size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        TI_CUDA(cudaFuncSetAttribute(latent_decode_mma_kernel<MT, NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = smem;
-    }
-    dim3 grid(n_splits, (n_heads + ROWS - 1) / ROWS, n_seq);
-    TI_CUDA(ti_launch_class<3>(latent_decode_mma_kernel<MT, NTW>, grid, dim3(D_THREADS), smem, stream, qa, (const bf16*)lat, ol, cu_new,
-                               seq_start, seq_slot, n_heads, rank, rot, scale, window, sink, kv, n_splits, part_o, part_ml, tiles));
-    TI_CHECK_LAUNCH("latent_attention (one token, tensor cores)");
+    int rc;
+    if (MT == 1 && rank + rot <= 64 * Q_STEPS)
+        rc = launch_decode_form<1, NTW, true>(qa, lat, ol, cu_new, seq_start, seq_slot, n_seq, n_heads, rank, rot, scale, window, sink, kv, n_splits, part_o, part_ml, stream);
+    else
+        rc = launch_decode_form<MT, NTW, false>(qa, lat, ol, cu_new, seq_start, seq_slot, n_seq, n_heads, rank, rot, scale, window, sink, kv, n_splits, part_o, part_ml, stream);
+    if (rc) return rc;
     if (uv) {
         // (128 / 256 / 512 threads, us a layer of 16 sequences and 16 heads: a latent of 512 83 / 67 / 60, of 256 49 / 49 / 47; four
         // sequences, eight heads, a latent of 256 40 / 35 / 40)
@@ -963,6 +1224,12 @@ extern "C" int ti_latent_prep_absorb(const void* d, long long d_stride, const vo
         using T = decltype(t);
         const size_t row = (size_t)(W + 33) * sizeof(float) + (size_t)W * sizeof(T);
         TI_REQUIRE(row <= 48 * 1024 && (size_t)plain * sizeof(float) <= 48 * 1024, "latent_prep_absorb: rows of %d elements are too long", W);
+        if constexpr (sizeof(T) == 2)
+            if (rank % 2 == 0 && ((uintptr_t)uk & 3) == 0 && plain <= 512 && (long long)n_heads * ((rank + AR_COLS - 1) / AR_COLS) < (1 << 24)) {
+                auto go = M <= 4 ? launch_absorb_rows<4> : launch_absorb_rows<8>;
+                return go(d, d_stride, q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos, tok_pos, tok_seq, seq_slot, lat, kv, uk,
+                          qa, M, row, stream);
+            }
         // (a head's query and its groups' sums: ABSORB_THREADS / (rank / 8) groups of `rank` sums, or a row's own)
         const size_t smem = std::max(row, (size_t)(plain + std::max(8 * ABSORB_THREADS, rank)) * sizeof(float));
         if (smem > 48 * 1024) TI_CUDA(cudaFuncSetAttribute(latent_prep_absorb_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
