@@ -148,6 +148,17 @@ struct SampleArgs {
     int* out;
 };
 
+// The rows' keys and step counts as a kernel's argument: the first kernel of a draw leaves them where a.keys and a.steps point.  (A
+// copy from pinned memory between the logits and the draw waited for the product and cost 20 us of its own on the device.)
+constexpr int ROWS_BY_VALUE = 256;
+struct RowsHost { long long keys[ROWS_BY_VALUE]; int steps[ROWS_BY_VALUE]; };
+struct RowsNone {};
+__device__ __forceinline__ void leave_rows(const SampleArgs& a, const RowsHost& rows, int row) {
+    const_cast<long long*>(a.keys)[row] = rows.keys[row];
+    const_cast<int*>(a.steps)[row] = rows.steps[row];
+}
+__device__ __forceinline__ void leave_rows(const SampleArgs&, const RowsNone&, int) {}
+
 // top_k in [1, MAXK], top_k < V.  Keeps exactly top_k entries (ties at the k-th value
 // go to the lowest indices), then applies top_p on the sorted list.
 __global__ void __launch_bounds__(SB) sample_topk_kernel(SampleArgs a) {
@@ -552,6 +563,7 @@ __global__ void __launch_bounds__(SB) sample_full_kernel(SampleArgs a) {
 //     marks the row done; the tiered kernel runs after it and leaves such rows alone.
 // ---------------------------------------------------------------------------
 constexpr int CHUNK = 4096;       // positions of a row per block of the first kernel
+constexpr int STATS_KEPT = 128;     // chunks of a row whose maxima and sums a merging kernel holds in shared memory
 constexpr int NUCLEUS_K = 64;     // candidates within which a nucleus (top_p without top_k) is looked for first
 constexpr int CB = 512;           // threads of the first kernels
 
@@ -713,9 +725,34 @@ __device__ float block_sum_ordered(float v, float* sm /* 33 entries */) {
     return sm[32];
 }
 
-// The block's chunk: its k largest entries to cand[row][chunk][0 .. k), and, with `stats`, the
+// The smallest of the k largest of n values (n a multiple of four, k at most n) that some threads hold and all have left in key[0 .. n):
+// found by counting those above one's own.  `holds`: whether this thread holds one.  s: a word of shared memory that is -1.
+__device__ __forceinline__ unsigned kth_of(const unsigned* key, int n, int k, bool holds, unsigned own, int* s) {
+    int above = 0;
+    if (holds)
+        for (int i = 0; i < n; i += 4) {
+            const uint4 o = *reinterpret_cast<const uint4*>(key + i);
+            above += (o.x > own) + (o.y > own) + (o.z > own) + (o.w > own);
+        }
+    const unsigned least = __reduce_min_sync(0xffffffffu, holds && above < k ? own : 0xFFFFFFFFu);
+    if ((threadIdx.x & 31) == 0) atomicMin(reinterpret_cast<unsigned*>(s), least);
+    __syncthreads();
+    return *reinterpret_cast<volatile unsigned*>(s);
+}
+
+// The block's chunk: its k largest entries to cand[row][chunk][0 .. k), and, with STATS, the
 // chunk's maximum m and sum of exp(x - m) (as softmax_chunk_kernel leaves them).
-__global__ void __launch_bounds__(K1B) topk_chunk_kernel(SampleArgs a, int k, int chunks, unsigned long long* cand, float* stats) {
+//
+// Few entries (k <= FEW_K): the k-th largest of the threads' own maxima is a bound that at least k entries reach, and few more do.
+// Ranks by counting, among the maxima and then among the entries that reach the bound; no histogram (whose first byte is
+// the same for most logits, so that its counts queue for a few words of shared memory).  Without STATS the bound is looked for among
+// the logits as they are and only what comes near it is divided by the temperature (a quotient is no smaller than that of a smaller
+// logit; two may be the same, hence "near" and the comparison of quotients): with all 16 a thread divided and packed into words first
+// the kernel took 43 us for 64 rows of 151,936 logits, top_k 20, and by histograms 73; so 22.  Chunks with infinities, values that are
+// not a number or quotients outside 1e-30 .. 1e30 are divided and packed whole.
+template <bool STATS, typename Rows>
+__global__ void __launch_bounds__(K1B, STATS ? 4 : 5)
+topk_chunk_kernel(SampleArgs a, int k, int chunks, unsigned long long* cand, float* stats, const __grid_constant__ Rows rows) {
     ti_pdl_trigger();
     __shared__ __align__(16) int hist[256];
     __shared__ int sh[3];
@@ -725,16 +762,72 @@ __global__ void __launch_bounds__(K1B) topk_chunk_kernel(SampleArgs a, int k, in
     const int row = blockIdx.x, c = blockIdx.y, lo = c * CHUNK, t = threadIdx.x;
     const int n = min(CHUNK, a.V - lo);
     const float* x = a.logits + (size_t)row * a.ld + lo;
-    unsigned long long w[CHUNK / K1B];
+    constexpr int EPT = CHUNK / K1B;
+    if (c == 0 && t == 0) leave_rows(a, rows, row);
+    unsigned long long* out = cand + ((size_t)row * chunks + c) * k;
+    unsigned* key = reinterpret_cast<unsigned*>(hist);
+    if (!STATS && k <= FEW_K) {
+        float v[EPT];
+        bool odd = false;
+        unsigned own = 0;
+#pragma unroll
+        for (int e = 0; e < EPT; e++) v[e] = t + e * K1B < n ? x[t + e * K1B] : 0.f;
+#pragma unroll
+        for (int e = 0; e < EPT; e++)
+            if (t + e * K1B < n) {
+                odd |= !(fabsf(v[e]) < 1e30f);
+                own = max(own, order_key(v[e] + 0.0f));      // (-0 counts as +0)
+            }
+        if (t == 0) { sh[0] = 0; sh[1] = -1; }
+        int n_keys = K1B;
+        bool holds = true;
+        if (k <= 24) {                   // the maxima of four threads each: a quarter of the counting, a few entries more
+            own = max(own, __shfl_xor_sync(0xffffffffu, own, 1));
+            own = max(own, __shfl_xor_sync(0xffffffffu, own, 2));
+            n_keys = K1B / 4;
+            holds = (t & 3) == 0;
+            if (holds) key[t >> 2] = own;
+        } else key[t] = own;
+        odd = __syncthreads_or(odd);
+        const unsigned bound = kth_of(key, n_keys, k, holds, own, &sh[1]);
+        const float b = entry_value((unsigned long long)bound << 32), qb = bound ? b / a.temperature : 1.f;
+        if (!odd && fabsf(qb) < 1e30f && fabsf(qb) > 1e-30f) {
+            const float near = bound ? b - fabsf(b) * 4.8e-7f : -INFINITY;      // (a quotient's rounding, several times over)
+            const unsigned qkey = bound ? order_key(qb) : 0u;
+#pragma unroll
+            for (int e = 0; e < EPT; e++)
+                if (t + e * K1B < n && v[e] >= near) {
+                    const unsigned long long w = pack_entry(v[e] / a.temperature, lo + t + e * K1B);
+                    if ((unsigned)(w >> 32) >= qkey) {
+                        const int p = atomicAdd(&sh[0], 1);
+                        if (p < MAXK) kept[p] = w;
+                    }
+                }
+            __syncthreads();
+            const int m = sh[0];
+            if (m <= FEW_K * EPT) {          // (more: ties beyond count, left to the histograms)
+                for (int i = t; i < m; i += K1B) {
+                    const unsigned long long mine = kept[i];
+                    int r = 0;
+                    for (int j = 0; j < m; j++) r += kept[j] > mine;
+                    if (r < k) out[r] = mine;
+                }
+                for (int i = m + t; i < k; i += K1B) out[i] = 0ull;
+                return;
+            }
+        }
+        __syncthreads();
+    }
+    unsigned long long w[EPT];
     float mx = -INFINITY;
 #pragma unroll
-    for (int e = 0; e < CHUNK / K1B; e++) {
+    for (int e = 0; e < EPT; e++) {
         const int i = t + e * K1B;
         const float v = i < n ? x[i] / a.temperature : -INFINITY;
         w[e] = i < n ? pack_entry(v, lo + i) : 0ull;
         mx = fmaxf(mx, v);
     }
-    if (stats) {
+    if (STATS) {
         mx = warp_max(mx);
         if ((t & 31) == 0) red[t >> 5] = mx;
         __syncthreads();
@@ -746,71 +839,88 @@ __global__ void __launch_bounds__(K1B) topk_chunk_kernel(SampleArgs a, int k, in
         mx = red[32];
         float part = 0.f;
 #pragma unroll
-        for (int e = 0; e < CHUNK / K1B; e++) part += (w[e] != 0ull && mx > -INFINITY) ? expf(entry_value(w[e]) - mx) : 0.f;
+        for (int e = 0; e < EPT; e++) part += (w[e] != 0ull && mx > -INFINITY) ? expf(entry_value(w[e]) - mx) : 0.f;
         const float sum = block_sum_ordered(part, red);
         if (t == 0) {
             stats[((size_t)row * chunks + c) * 2] = mx;
             stats[((size_t)row * chunks + c) * 2 + 1] = sum;
         }
-    }
-    unsigned long long* out = cand + ((size_t)row * chunks + c) * k;
-    if (k <= FEW_K) {
-        // Few entries: the k-th largest of the threads' own maxima is a bound that at least k entries reach, and few more do.
-        // Ranks by counting, among the maxima and then among the entries that reach the bound; no histogram (whose first byte is
-        // the same for most logits, so that its counts queue for a few words of shared memory).  64 rows of 151,936 logits, top_k
-        // 20: the kernel 73 us by histograms, 43 so; the merge 26 and 10 with pick_bin.
-        unsigned own = 0;
+        if (k <= FEW_K) {
+            unsigned own = 0;
 #pragma unroll
-        for (int e = 0; e < CHUNK / K1B; e++) own = max(own, (unsigned)(w[e] >> 32));
-        unsigned* key = reinterpret_cast<unsigned*>(hist);
-        int n_keys = K1B;
-        if (k <= 24) {                   // the maxima of four threads each: a quarter of the counting, a few entries more
-            own = max(own, __shfl_xor_sync(0xffffffffu, own, 1));
-            own = max(own, __shfl_xor_sync(0xffffffffu, own, 2));
-            n_keys = K1B / 4;
-            if ((t & 3) == 0) key[t >> 2] = own;
-        } else key[t] = own;
-        if (t == 0) { sh[0] = 0; sh[1] = -1; }
-        __syncthreads();
-        int above = 0;
-        for (int i = 0; i < n_keys; i += 4) {
-            const uint4 o = *reinterpret_cast<const uint4*>(key + i);
-            above += (o.x > own) + (o.y > own) + (o.z > own) + (o.w > own);
-        }
-        const unsigned least = __reduce_min_sync(0xffffffffu, above < k ? own : 0xFFFFFFFFu);
-        if ((t & 31) == 0) atomicMin(reinterpret_cast<unsigned*>(&sh[1]), least);
-        __syncthreads();
-        const unsigned bound = (unsigned)sh[1];
+            for (int e = 0; e < EPT; e++) own = max(own, (unsigned)(w[e] >> 32));
+            key[t] = own;
+            if (t == 0) { sh[0] = 0; sh[1] = -1; }
+            __syncthreads();
+            const unsigned bound = kth_of(key, K1B, k, true, own, &sh[1]);
 #pragma unroll
-        for (int e = 0; e < CHUNK / K1B; e++)
-            if (w[e] != 0ull && (unsigned)(w[e] >> 32) >= bound) {
-                const int p = atomicAdd(&sh[0], 1);
-                if (p < MAXK) kept[p] = w[e];
+            for (int e = 0; e < EPT; e++)
+                if (w[e] != 0ull && (unsigned)(w[e] >> 32) >= bound) {
+                    const int p = atomicAdd(&sh[0], 1);
+                    if (p < MAXK) kept[p] = w[e];
+                }
+            __syncthreads();
+            const int m = sh[0];
+            if (m <= FEW_K * EPT) {
+                for (int i = t; i < m; i += K1B) {
+                    const unsigned long long mine = kept[i];
+                    int r = 0;
+                    for (int j = 0; j < m; j++) r += kept[j] > mine;
+                    if (r < k) out[r] = mine;
+                }
+                for (int i = m + t; i < k; i += K1B) out[i] = 0ull;
+                return;
             }
-        __syncthreads();
-        const int m = sh[0];
-        if (m <= FEW_K * CHUNK / K1B) {          // (more: ties beyond count, left to the histograms)
-            for (int i = t; i < m; i += K1B) {
-                const unsigned long long mine = kept[i];
-                int r = 0;
-                for (int j = 0; j < m; j++) r += kept[j] > mine;
-                if (r < k) out[r] = mine;
-            }
-            for (int i = m + t; i < k; i += K1B) out[i] = 0ull;
-            return;
+            __syncthreads();
         }
-        __syncthreads();
     }
-    select_largest<CHUNK / K1B>(w, k, kept, hist, sh);
+    select_largest<EPT>(w, k, kept, hist, sh);
     for (int i = t; i < k; i += K1B) out[i] = kept[i];
 }
 
 // The row's k largest among the chunks' candidates, sorted, in kept[0 .. k) (the rest of kept up to
-// the next power of two is 0).  All threads call it.
+// the next power of two is 0).  All threads call it.  Few of them, as in the chunks: by the maxima of eight threads each and ranks (64
+// rows of 38 chunks' 20: the kernel 10 us by histograms and a sort, 7 so).
 __device__ int merge_candidates(const unsigned long long* cand, int n_cand, int k, unsigned long long* kept, int* hist, int* sh) {
+    const int t = threadIdx.x;
     int n2 = 1;
     while (n2 < k) n2 <<= 1;
-    for (int i = threadIdx.x; i < n2; i += blockDim.x) kept[i] = 0ull;
+    for (int i = t; i < n2; i += blockDim.x) kept[i] = 0ull;
+    constexpr int EPT = 4;
+    if (k <= FEW_K && n_cand <= EPT * SB && blockDim.x == SB) {
+        __shared__ unsigned long long near[MAXK];
+        unsigned long long w[EPT];
+        unsigned own = 0;
+#pragma unroll
+        for (int e = 0; e < EPT; e++) w[e] = t + e * SB < n_cand ? cand[t + e * SB] : 0ull;
+#pragma unroll
+        for (int e = 0; e < EPT; e++) own = max(own, (unsigned)(w[e] >> 32));
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) own = max(own, __shfl_xor_sync(0xffffffffu, own, o));
+        unsigned* key = reinterpret_cast<unsigned*>(hist);
+        if ((t & 7) == 0) key[t >> 3] = own;
+        if (t == 0) { sh[0] = 0; sh[1] = -1; }
+        __syncthreads();
+        const unsigned bound = kth_of(key, SB / 8, k, (t & 7) == 0, own, &sh[1]);
+#pragma unroll
+        for (int e = 0; e < EPT; e++)
+            if (w[e] != 0ull && (unsigned)(w[e] >> 32) >= bound) {
+                const int p = atomicAdd(&sh[0], 1);
+                if (p < MAXK) near[p] = w[e];
+            }
+        __syncthreads();
+        const int m = sh[0];
+        if (m <= MAXK) {
+            if (t < m) {
+                const unsigned long long mine = near[t];
+                int r = 0;
+                for (int j = 0; j < m; j++) r += near[j] > mine;
+                if (r < k) kept[r] = mine;
+            }
+            __syncthreads();
+            return n2;
+        }
+    }
     __syncthreads();
     select_largest_of(cand, n_cand, k, kept, hist, sh);
     sort_descending(kept, n2);
@@ -819,10 +929,10 @@ __device__ int merge_candidates(const unsigned long long* cand, int n_cand, int 
 
 __global__ void __launch_bounds__(SB) topk_merge_kernel(SampleArgs a, int chunks, const unsigned long long* cand) {
     ti_pdl_trigger();
-    __shared__ int hist[256];
+    __shared__ __align__(16) int hist[256];
     __shared__ int sh[3];
     __shared__ unsigned long long kept[MAXK];
-    __shared__ float cval[MAXK];
+    __shared__ float cval[MAXK], s_sum;
     ti_pdl_sync();
     cand = ti_dependent(cand);
     const int t = threadIdx.x, row = blockIdx.x, k = a.top_k;
@@ -834,11 +944,19 @@ __global__ void __launch_bounds__(SB) topk_merge_kernel(SampleArgs a, int chunks
     __syncthreads();
     if (t == 0) {
         float sum = 0.f;
+#pragma unroll 8
         for (int i = 0; i < n; i++) sum += cval[i];
+        s_sum = sum;
+    }
+    __syncthreads();
+    const float sum = s_sum;
+    for (int i = t; i < n; i += SB) cval[i] = cval[i] / sum;
+    __syncthreads();
+    if (t == 0) {
         float acc = 0.f;
         int keep = n;
         for (int i = 0; i < n; i++) {
-            acc += cval[i] / sum;
+            acc += cval[i];
             if (acc > a.top_p) { keep = i + 1; break; }
         }
         const float u = uniform_from(a.seed, (unsigned long long)a.keys[row], (unsigned long long)a.steps[row]);
@@ -846,7 +964,7 @@ __global__ void __launch_bounds__(SB) topk_merge_kernel(SampleArgs a, int chunks
         float run = 0.f;
         int pick = entry_index(kept[keep - 1]);
         for (int i = 0; i < keep; i++) {
-            run += cval[i] / sum;
+            run += cval[i];
             if (run > coin) { pick = entry_index(kept[i]); break; }
         }
         a.out[row] = pick;
@@ -862,7 +980,7 @@ __global__ void __launch_bounds__(SB) topk_merge_kernel(SampleArgs a, int chunks
 __global__ void __launch_bounds__(SB) nucleus_merge_kernel(SampleArgs a, int chunks, const unsigned long long* cand, const float* stats,
                                                            int* done) {
     ti_pdl_trigger();
-    __shared__ int hist[256];
+    __shared__ __align__(16) int hist[256];
     __shared__ int sh[3];
     __shared__ unsigned long long kept[NUCLEUS_K];
     ti_pdl_sync();
@@ -870,16 +988,30 @@ __global__ void __launch_bounds__(SB) nucleus_merge_kernel(SampleArgs a, int chu
     const int t = threadIdx.x, row = blockIdx.x;
     const int k = min(NUCLEUS_K, a.V);
     merge_candidates(cand + (size_t)row * chunks * NUCLEUS_K, chunks * NUCLEUS_K, k, kept, hist, sh);
+    // the chunks' maxima and sums, read at once where they fit; added up in the chunks' order by one thread
+    __shared__ float st_s[2 * STATS_KEPT], prob[NUCLEUS_K], s_mx, s_sum;
+    const float* st = stats + (size_t)row * chunks * 2;
+    if (chunks <= STATS_KEPT) {
+        for (int i = t; i < 2 * chunks; i += SB) st_s[i] = st[i];
+        st = st_s;
+    }
+    __syncthreads();
     if (t == 0) {
-        const float* st = stats + (size_t)row * chunks * 2;
         float mx = -INFINITY;
         for (int c = 0; c < chunks; c++) mx = fmaxf(mx, st[2 * c]);
         float sum = 0.f;
+#pragma unroll 4
         for (int c = 0; c < chunks; c++) sum += st[2 * c] > -INFINITY ? st[2 * c + 1] * expf(st[2 * c] - mx) : 0.f;
+        s_mx = mx; s_sum = sum;
+    }
+    __syncthreads();
+    if (t < k) prob[t] = kept[t] != 0ull ? expf(entry_value(kept[t]) - s_mx) / s_sum : 0.f;
+    __syncthreads();
+    if (t == 0) {
         float acc = 0.f;
         int keep = 0;
         for (int i = 0; i < k && kept[i] != 0ull; i++) {
-            acc += expf(entry_value(kept[i]) - mx) / sum;
+            acc += prob[i];
             if (acc > a.top_p) { keep = i + 1; break; }
         }
         if (keep == 0 && k == a.V) keep = k;            // a vocabulary this small is in `kept` whole
@@ -889,7 +1021,7 @@ __global__ void __launch_bounds__(SB) nucleus_merge_kernel(SampleArgs a, int chu
             float run = 0.f;
             int pick = entry_index(kept[keep - 1]);
             for (int i = 0; i < keep; i++) {
-                run += expf(entry_value(kept[i]) - mx) / sum;
+                run += prob[i];
                 if (run > coin) { pick = entry_index(kept[i]); break; }
             }
             a.out[row] = pick;
@@ -898,13 +1030,15 @@ __global__ void __launch_bounds__(SB) nucleus_merge_kernel(SampleArgs a, int chu
     }
 }
 
-__global__ void __launch_bounds__(CB) softmax_chunk_kernel(SampleArgs a, int chunks, float* stats) {
+template <typename Rows>
+__global__ void __launch_bounds__(CB) softmax_chunk_kernel(SampleArgs a, int chunks, float* stats, const __grid_constant__ Rows rows) {
     ti_pdl_trigger();
     __shared__ float red[33];
     ti_pdl_sync();
     const int row = blockIdx.x, c = blockIdx.y, lo = c * CHUNK, t = threadIdx.x;
     const int n = min(CHUNK, a.V - lo);
     const float* x = a.logits + (size_t)row * a.ld + lo;
+    if (c == 0 && t == 0) leave_rows(a, rows, row);
     float v[CHUNK / CB];
     float mx = -INFINITY;
 #pragma unroll
@@ -940,7 +1074,13 @@ __global__ void __launch_bounds__(CB) sample_full_merge_kernel(SampleArgs a, int
     ti_pdl_sync();
     stats = ti_dependent(stats);
     const int row = blockIdx.x, t = threadIdx.x;
+    __shared__ float st_s[2 * STATS_KEPT];
     const float* st = stats + (size_t)row * chunks * 2;
+    if (chunks <= STATS_KEPT) {
+        for (int i = t; i < 2 * chunks; i += CB) st_s[i] = st[i];
+        st = st_s;
+    }
+    __syncthreads();
     if (t == 0) {
         float mx = -INFINITY;
         for (int c = 0; c < chunks; c++) mx = fmaxf(mx, st[2 * c]);
@@ -1022,6 +1162,31 @@ extern "C" long long ti_sample_scratch_bytes(int R, int V, int top_k, float top_
     return 0;
 }
 
+namespace {
+// The two forms over many blocks (scratch as ti_sample_scratch_bytes says).
+template <typename Rows>
+int sample_in_chunks(const SampleArgs& a, int R, int chunks, void* scratch, const Rows& rows, cudaStream_t stream) {
+    const bool k_off = a.top_k <= 0 || a.top_k >= a.V;
+    TI_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 7) == 0 && chunks <= 65535, "sample: bad scratch or too many chunks");
+    if (k_off && a.top_p >= 1.0f) {
+        TI_CUDA(ti_launch(softmax_chunk_kernel<Rows>, dim3(R, chunks), dim3(CB), 0, stream, a, chunks, (float*)scratch, rows));
+        TI_CUDA(ti_launch(sample_full_merge_kernel, dim3(R), dim3(CB), 0, stream, a, chunks, (const float*)scratch));
+    } else if (!k_off) {
+        TI_CUDA(ti_launch(topk_chunk_kernel<false, Rows>, dim3(R, chunks), dim3(K1B), 0, stream, a, a.top_k, chunks, (unsigned long long*)scratch, (float*)nullptr, rows));
+        TI_CUDA(ti_launch(topk_merge_kernel, dim3(R), dim3(SB), 0, stream, a, chunks, (const unsigned long long*)scratch));
+    } else {
+        unsigned long long* cand = (unsigned long long*)scratch;
+        float* stats = (float*)(cand + (size_t)R * chunks * NUCLEUS_K);
+        int* done = (int*)(stats + (size_t)R * chunks * 2);
+        TI_CUDA(ti_launch(topk_chunk_kernel<true, Rows>, dim3(R, chunks), dim3(K1B), 0, stream, a, NUCLEUS_K, chunks, cand, stats, rows));
+        TI_CUDA(ti_launch(nucleus_merge_kernel, dim3(R), dim3(SB), 0, stream, a, chunks, (const unsigned long long*)cand, (const float*)stats, done));
+        TI_CUDA(ti_launch(sample_tiered_kernel, dim3(R), dim3(SB), 0, stream, a, (const int*)done));
+    }
+    TI_CHECK_LAUNCH("sample");
+    return 0;
+}
+}  // namespace
+
 // `scratch`: ti_sample_scratch_bytes(...) bytes, 8-byte aligned, or null (one block per row then).
 extern "C" int ti_sample(const float* logits, long long ld, int R, int V, float temperature, int top_k,
                          float top_p, unsigned long long seed, const long long* keys, const int* steps,
@@ -1035,25 +1200,7 @@ extern "C" int ti_sample(const float* logits, long long ld, int R, int V, float 
     a.top_p = top_p; a.seed = seed; a.keys = keys; a.steps = steps; a.out = out;
     const bool k_off = top_k <= 0 || top_k >= V;
     const int chunks = (V + CHUNK - 1) / CHUNK;
-    if (scratch && ti_sample_scratch_bytes(R, V, top_k, top_p) > 0) {
-        TI_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 7) == 0 && chunks <= 65535, "sample: bad scratch or too many chunks");
-        if (k_off && top_p >= 1.0f) {
-            TI_CUDA(ti_launch(softmax_chunk_kernel, dim3(R, chunks), dim3(CB), 0, stream, a, chunks, (float*)scratch));
-            TI_CUDA(ti_launch(sample_full_merge_kernel, dim3(R), dim3(CB), 0, stream, a, chunks, (const float*)scratch));
-        } else if (!k_off) {
-            TI_CUDA(ti_launch(topk_chunk_kernel, dim3(R, chunks), dim3(K1B), 0, stream, a, top_k, chunks, (unsigned long long*)scratch, (float*)nullptr));
-            TI_CUDA(ti_launch(topk_merge_kernel, dim3(R), dim3(SB), 0, stream, a, chunks, (const unsigned long long*)scratch));
-        } else {
-            unsigned long long* cand = (unsigned long long*)scratch;
-            float* stats = (float*)(cand + (size_t)R * chunks * NUCLEUS_K);
-            int* done = (int*)(stats + (size_t)R * chunks * 2);
-            TI_CUDA(ti_launch(topk_chunk_kernel, dim3(R, chunks), dim3(K1B), 0, stream, a, NUCLEUS_K, chunks, cand, stats));
-            TI_CUDA(ti_launch(nucleus_merge_kernel, dim3(R), dim3(SB), 0, stream, a, chunks, (const unsigned long long*)cand, (const float*)stats, done));
-            TI_CUDA(ti_launch(sample_tiered_kernel, dim3(R), dim3(SB), 0, stream, a, (const int*)done));
-        }
-        TI_CHECK_LAUNCH("sample");
-        return 0;
-    }
+    if (scratch && ti_sample_scratch_bytes(R, V, top_k, top_p) > 0) return sample_in_chunks(a, R, chunks, scratch, RowsNone{}, stream);
     if (k_off && top_p >= 1.0f) {
         TI_CUDA(ti_launch(sample_full_kernel, dim3(R), dim3(SB), 0, stream, a));
     } else if (!k_off && top_k <= MAXK) {
@@ -1067,6 +1214,25 @@ extern "C" int ti_sample(const float* logits, long long ld, int R, int V, float 
     }
     TI_CHECK_LAUNCH("sample");
     return 0;
+}
+
+// The same in the forms over many blocks, for up to 256 rows whose keys and step counts lie on the host (read before the call
+// returns).  scratch: ti_sample_scratch_bytes(...) rounded up to 8 bytes, then 12 bytes a row.
+extern "C" int ti_sample_rows(const float* logits, long long ld, int R, int V, float temperature, int top_k, float top_p,
+                              unsigned long long seed, const long long* keys, const int* steps, int* out, void* scratch, cudaStream_t stream) {
+    if (R == 0) return 0;
+    TI_REQUIRE(R > 0 && R <= ROWS_BY_VALUE && V > 0 && ld >= V && keys && steps && scratch, "sample_rows: bad sizes R=%d V=%d ld=%lld", R, V, ld);
+    TI_REQUIRE(temperature > 0.f && top_p > 0.f, "sample_rows: temperature %g and top_p %g must be positive", temperature, top_p);
+    const long long need = (ti_sample_scratch_bytes(R, V, top_k, top_p) + 7) / 8 * 8;
+    TI_REQUIRE(need > 0, "sample_rows: top_k %d has only the form of one block per row", top_k);
+    RowsHost rows;
+    for (int i = 0; i < R; i++) { rows.keys[i] = keys[i]; rows.steps[i] = steps[i]; }
+    SampleArgs a;
+    a.logits = logits; a.ld = ld; a.V = V; a.temperature = temperature; a.top_k = top_k; a.top_p = top_p; a.seed = seed; a.out = out;
+    long long* dev_keys = reinterpret_cast<long long*>(static_cast<char*>(scratch) + need);
+    a.keys = dev_keys;
+    a.steps = reinterpret_cast<const int*>(dev_keys + R);
+    return sample_in_chunks(a, R, (V + CHUNK - 1) / CHUNK, scratch, rows, stream);
 }
 
 extern "C" float ti_uniform_from(unsigned long long seed, unsigned long long key, unsigned long long step) {

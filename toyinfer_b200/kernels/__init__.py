@@ -519,6 +519,33 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, s
     return out
 
 
+SAMPLE_ROWS_MAX = 256        # rows whose keys and step counts travel as a kernel's argument
+
+
+def sample_rows(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, seed: int, keys, steps) -> Optional[torch.Tensor]:
+    """``sample`` with the rows' keys and step counts on the host (numpy int64 and int32, dense): they go with the launch, without
+    a copy.  None where this is not possible: more than ``SAMPLE_ROWS_MAX`` rows, a setting that has only the
+    one-block-per-row form, or a stream that is being captured (the launch's arguments would be the same in every replay)."""
+    _need_cuda(logits, what="sample")
+    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1:
+        raise KernelError("sample: expected float32 [rows, vocab] with dense rows")
+    R, V = logits.shape
+    if keys.shape != (R,) or steps.shape != (R,) or keys.dtype.str[1:] != "i8" or steps.dtype.str[1:] != "i4":
+        raise KernelError("sample: keys must be int64[rows] and steps int32[rows]")
+    if not two_kernel_sampling or R > SAMPLE_ROWS_MAX or R == 0 or torch.cuda.is_current_stream_capturing():
+        return None
+    lib = library()
+    need = int(lib.ti_sample_scratch_bytes(R, V, int(top_k), float(top_p)))
+    if need <= 0:
+        return None
+    out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+    scratch = torch.empty((need + 7) // 8 + (12 * R + 7) // 8, dtype=torch.int64, device=logits.device)
+    _call(lib.ti_sample_rows, _ptr(logits), logits.stride(0), R, V, float(temperature), int(top_k), float(top_p),
+          ctypes.c_uint64(seed & 0xFFFFFFFFFFFFFFFF), keys.ctypes.data, steps.ctypes.data, _ptr(out), _ptr(scratch), _stream(),
+          launches=3 if (top_p < 1.0 and not 0 < top_k < V) else 2)
+    return out
+
+
 def uniform_from(seed: int, key: int, step: int) -> float:
     """The uniform number in [0, 1) that ``sample`` draws for (seed, key, step)."""
     return float(library().ti_uniform_from(ctypes.c_uint64(seed & 0xFFFFFFFFFFFFFFFF),

@@ -49,6 +49,7 @@ def _declare(lib) -> None:
         "ti_read_status": [P],
         "ti_argmax": [P, L, I, I, I, P, P, P, P],
         "ti_sample": [P, L, I, I, F, I, F, c_uint64, P, P, P, P, P],
+        "ti_sample_rows": [P, L, I, I, F, I, F, c_uint64, P, P, P, P, P],
     }
     for name, args in sig.items():
         fn = getattr(lib, name)

@@ -14,6 +14,7 @@ from __future__ import annotations
 
 from typing import Sequence
 
+import numpy as np
 import torch
 
 from .. import kernels as K
@@ -61,7 +62,11 @@ class Sampler:
         p = self.params
         if p.greedy:
             return K.argmax(logits)
-        keys_t, steps_t = self._upload(keys, steps)
         vocab = logits.shape[1]
         top_k = p.top_k if 0 < p.top_k < vocab else 0
+        if self.device.type == "cuda" and len(keys) <= K.SAMPLE_ROWS_MAX:
+            picked = K.sample_rows(logits, p.temperature, top_k, p.top_p, p.seed, np.array(keys, dtype=np.int64), np.array(steps, dtype=np.int32))
+            if picked is not None:
+                return picked
+        keys_t, steps_t = self._upload(keys, steps)
         return K.sample(logits, p.temperature, top_k, p.top_p, p.seed, keys_t, steps_t)
