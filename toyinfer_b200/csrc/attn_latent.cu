@@ -771,16 +771,17 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
                          int shares, int pitch, int* status) {
     ti_pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ uint64_t full[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
-    if (tid == 0) { mbar_init(&full[0], 1); mbar_init(&full[1], 1); mbar_fence_init(); }
-    ti_pdl_sync();
-    qa = ti_dependent(qa); lat = ti_dependent(lat);
     constexpr int ROWS = 16 * MT;
     const int ahead = tiles - 1;                                   // (1, or 0: rows so wide that only one tile of them fits)
     const int W = rank + rot, LD = W + 8, steps = W >> 4;
     float* Sp = reinterpret_cast<float*>(smem_raw);
     bf16* Ls = reinterpret_cast<bf16*>(smem_raw + (size_t)shares * ROWS * pitch * 4);      // [tiles][DK][LD]
+    // (the barriers stand in the 16 bytes between the first two rows, which nothing else uses: the widest rows leave no byte beside them)
+    uint64_t* full = reinterpret_cast<uint64_t*>(Ls + W);
+    if (tid == 0) { mbar_init(&full[0], 1); mbar_init(&full[1], 1); mbar_fence_init(); }
+    ti_pdl_sync();
+    qa = ti_dependent(qa); lat = ti_dependent(lat);
     bf16* Qs = Ls + tiles * DK * LD;                               // [ROWS][LD]
     const int split = blockIdx.z, h0 = blockIdx.y * ROWS, b = blockIdx.x;        // (the splits that are empty come last)
     const int tok = cu_new[b], tok_end = cu_new[b + 1], qi = seq_start[b], slot = seq_slot[b];
