@@ -95,12 +95,11 @@ def expert_pairs(x: torch.Tensor, perm: torch.Tensor, off: torch.Tensor, w_gate_
         rows = pad_src.numel()
         xs = torch.empty((rows, H), dtype=x.dtype, device=dev)
         _call(_fn("ti_moe_gather_rows", [P, L, P, P, I, I, I, P]), _ptr(x), x.stride(0), _ptr(pad_src), _ptr(xs), rows, H, code, _stream())
-        grouped = _fn("ti_linear_grouped_tc", [P, P, P, P, I, I, I, I, L, P])
-        gu = torch.empty((rows, 2 * ff), dtype=x.dtype, device=dev)
-        _call(grouped, _ptr(xs), _ptr(w_gate_up), _ptr(gu), _ptr(tile_group), rows, E, 2 * ff, H, 2 * ff, _stream())
-        y = act_pair(gu, limit, alpha, shift)
+        grouped = _fn("ti_linear_grouped_tc", [P, P, P, P, I, I, I, I, L, I, F, F, F, P])
+        y = torch.empty((rows, ff), dtype=x.dtype, device=dev)
+        _call(grouped, _ptr(xs), _ptr(w_gate_up), _ptr(y), _ptr(tile_group), rows, E, ff, H, ff, 1, float(limit), float(alpha), float(shift), _stream())
         z = torch.empty((rows, H), dtype=x.dtype, device=dev)
-        _call(grouped, _ptr(y), _ptr(w_down), _ptr(z), _ptr(tile_group), rows, E, H, ff, H, _stream())
+        _call(grouped, _ptr(y), _ptr(w_down), _ptr(z), _ptr(tile_group), rows, E, H, ff, H, 0, 0.0, 0.0, 0.0, _stream())
         return z, pad_of_pair, True
     fn = _fn("ti_moe_grouped", [P, L, P, P, P, L, P, P, I, I, I, I, I, I, I, I, F, F, F, F, L, I, P])
     y = torch.empty((Pn, ff), dtype=x.dtype, device=x.device)
@@ -248,12 +247,11 @@ def experts_relu2(x: torch.Tensor, perm: torch.Tensor, off: torch.Tensor, w_up: 
               _ptr(pad_of_pair), _ptr(tile_group), _stream())
         xs = torch.empty((rows, H), dtype=x.dtype, device=dev)
         _call(_fn("ti_moe_gather_rows", [P, L, P, P, I, I, I, P]), _ptr(x), x.stride(0), _ptr(pad_src), _ptr(xs), rows, H, code, _stream())
-        grouped = _fn("ti_linear_grouped_tc", [P, P, P, P, I, I, I, I, L, P])
-        u = torch.empty((rows, ff), dtype=x.dtype, device=dev)
-        _call(grouped, _ptr(xs), _ptr(w_up), _ptr(u), _ptr(tile_group), rows, E, ff, H, ff, _stream())
-        y = relu2(u)
+        grouped = _fn("ti_linear_grouped_tc", [P, P, P, P, I, I, I, I, L, I, F, F, F, P])
+        y = torch.empty((rows, ff), dtype=x.dtype, device=dev)
+        _call(grouped, _ptr(xs), _ptr(w_up), _ptr(y), _ptr(tile_group), rows, E, ff, H, ff, 4, 0.0, 0.0, 0.0, _stream())
         z = torch.empty((rows, H), dtype=x.dtype, device=dev)
-        _call(grouped, _ptr(y), _ptr(w_down), _ptr(z), _ptr(tile_group), rows, E, H, ff, H, _stream())
+        _call(grouped, _ptr(y), _ptr(w_down), _ptr(z), _ptr(tile_group), rows, E, H, ff, H, 0, 0.0, 0.0, 0.0, _stream())
         return z, pad_of_pair
     fn = _fn("ti_moe_grouped", [P, L, P, P, P, L, P, P, I, I, I, I, I, I, I, I, F, F, F, F, L, I, P])
     u = torch.empty((Pn, ff), dtype=x.dtype, device=dev)
