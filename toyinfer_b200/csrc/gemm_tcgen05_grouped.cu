@@ -9,7 +9,7 @@
 // What bounds it: the operands' way into an SM (115 B/ns: 0.28 us a step of 32 KB), and with one block an SM the start and the end of
 // every tile, in which nothing is on its way.  Two blocks of three stages each share an SM instead of one of six where there are tiles
 // for it, and the activation of a gated pair is applied at the end (a tile of 64 gate and 64 up columns; a kernel of its own read and
-// wrote the pairs again, rounded in between).  The whole layer, bfloat16, hidden 2,048, two choices a token, us before / with the activation inside
+// wrote the pairs again).  The whole layer, bfloat16, hidden 2,048, two choices a token, us before / with the activation inside
 // / two blocks an SM too: 16 experts of 1,024, 3,000 tokens 176 / 168 / 149, 777 tokens with a shared expert 111 / 106 / 102.  Where the tiles fit one
 // round, two blocks lose: 8 experts of 1,000 with 600 tokens 39.7 / 36.5 / 39.6, 4 of 600 with 150 tokens 28.9 / 26.8 / 28.9.
 #include "gemm_tcgen05.cuh"
@@ -18,7 +18,9 @@ namespace tigemm {
 namespace {
 constexpr int GBN = 128;
 
-// What a gated pair's tile stores: g' sigmoid(alpha g') (u' + shift), g' = min(g, limit), u' = clamp(u, -limit, limit).
+// What a gated pair's tile stores: g' sigmoid(alpha g') (u' + shift), g' = min(g, limit), u' = clamp(u, -limit, limit).  g and u are
+// rounded to bfloat16 first, as the groups of fewer places have them (moe_rows.cuh, moe_grouped.cu): a token's result must not depend
+// on how many others share its step.
 struct PairAct { float limit, alpha, shift; };
 
 template <int GSTAGES, bool PAIR>
@@ -106,7 +108,8 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_c
                     tmem_ld16(taddr + GBN / 2 + c, u);
 #pragma unroll
                     for (int e = 0; e < 16; e++) {
-                        const float gate = fminf(r[e], act.limit), up = fminf(fmaxf(u[e], -act.limit), act.limit);
+                        const float gate = fminf(to_f32(from_f32<bf16>(r[e])), act.limit);
+                        const float up = fminf(fmaxf(to_f32(from_f32<bf16>(u[e])), -act.limit), act.limit);
                         r[e] = gate * (ti_over(1.0f, 1.0f + expf(-act.alpha * gate))) * (up + act.shift);
                     }
                 }
