@@ -780,6 +780,7 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
     // (the barriers stand in the 16 bytes between the first two rows, which nothing else uses: the widest rows leave no byte beside them)
     uint64_t* full = reinterpret_cast<uint64_t*>(Ls + W);
     if (tid == 0) { mbar_init(&full[0], 1); mbar_init(&full[1], 1); mbar_fence_init(); }
+    __syncthreads();                     // (all warps wait on them below; here the meeting falls into the wait for the kernel before)
     ti_pdl_sync();
     qa = ti_dependent(qa); lat = ti_dependent(lat);
     bf16* Qs = Ls + tiles * DK * LD;                               // [ROWS][LD]
