@@ -53,3 +53,20 @@ def test_single_tokens(monkeypatch, H, rank, rot, page, window, ring):
     check_status()
     # queries in the latent space and softmax weights are rounded to bfloat16 (2^-9 each), the result too
     assert float((got.double() - want).norm() / want.norm()) < 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,rank", [(8, 256), (16, 512), (20, 256)])
+def test_a_sequence_does_not_depend_on_the_others(H, rank):
+    """The same bits whatever the lengths of the sequences beside it: the step is planned for its longest, and a split is a part of
+    the sequence's own keys."""
+    from toyinfer_b200.kernels import latent as KL, check_status
+    longest = [1000, 3000, 2900, 1700, 2000, 2500]
+    d, q, norm_w, tables, uk, uv, batch, mem = sizes.layer(torch.bfloat16, H, 64, 64, rank, 48, longest)
+    got = []
+    for held in (longest, [1000, 3000, 40, 70, 0, 31]):
+        batch.tok_pos, batch.seq_start = (torch.tensor(held, dtype=torch.int32, device="cuda") for _ in range(2))
+        batch.seq_len = batch.seq_start + 1
+        got.append(KL.attention_single(d, q, rank, 64, norm_w, 1e-6, tables, uk, uv, 48, 128 ** -0.5, 0, None, batch, mem))
+    check_status()
+    assert torch.equal(got[0][:2], got[1][:2])

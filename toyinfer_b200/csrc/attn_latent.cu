@@ -724,11 +724,11 @@ latent_attn_kernel(const float* __restrict__ qa, const T* __restrict__ lat, floa
 // What bounds it: a tile's chain of steps.  A tile is on its way (a bulk copy a row) while the one before it is worked off, and two
 // blocks share an SM where there is room; 16 sequences of 1,000 to 4,000 positions, 16 heads, rows of 512 + 64, us a tile of a block:
 // the queue of copies and the look-up of the next tile's page 1.4 -> 0.2 (16-byte copies by all threads before, the page's number
-// awaited at once), scores 0.9 -> 0.5 (queries in registers where they fit), softmax and its two barriers 0.5, values 0.65.  All
-// sequences' splits are equally many tiles; with splits of equal number a sequence's own the longest sequence's blocks ended
-// last (7 tiles where the mean is 4).  The layer's step 65.6 -> 53.0, of which the attention 30 -> 21, the way into the latent before it 9 ->
-// 6; the merge and the way out after it 12, bound by 34 MB of Wuv from L2 (a cluster of eight blocks that read it once, shared their
-// results and took 13: not kept).
+// awaited at once), scores 0.9 -> 0.5 (queries in registers where they fit), softmax and its two barriers 0.5, values 0.65.  The longest
+// sequence's blocks end last (7 tiles where the mean is 4): splits of equally many tiles over all sequences took 53.4 us for the layer's
+// step where these take 59.2 (66.2 before), 196 and 312 for 32 sequences of up to 8,000 with 32 heads, but a sequence's results then
+// changed by 0.0025 with the lengths of the others beside it.  The way into the latent before it 9 -> 6; the merge and the way out after
+// it 12, bound by 34 MB of Wuv from L2 (a cluster of eight blocks that read it once, shared their results and took 13: not kept).
 constexpr int DK = 32, D_THREADS = 128;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(D_THREADS)
 latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ lat, float* __restrict__ ol,
                          const int* __restrict__ cu_new, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
                          int n_heads, int rank, int rot, float scale, int window, const float* __restrict__ sink,
-                         LatentPages kv, int n_splits, int room, float* __restrict__ part_o, float* __restrict__ part_ml, int tiles,
+                         LatentPages kv, int n_splits, float* __restrict__ part_o, float* __restrict__ part_ml, int tiles,
                          int shares, int pitch, int* status) {
     ti_pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -786,20 +786,12 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
     bf16* Qs = Ls + tiles * DK * LD;                               // [ROWS][LD]
     const int split = blockIdx.z, h0 = blockIdx.y * ROWS, b = blockIdx.x;        // (the splits that are empty come last)
     const int tok = cu_new[b], tok_end = cu_new[b + 1], qi = seq_start[b], slot = seq_slot[b];
-    // Tiles of a split: the same for all sequences, so that the blocks of long and short ones take as long; as many as give every
-    // block that runs at once its share of the step's tiles, and no fewer than the longest sequence needs for n_splits splits.
-    int sum = 0, most = 0;
-    for (int s = lane; s < (int)gridDim.x; s += 32) {
-        const int q = seq_start[s], n = cu_new[s + 1] > cu_new[s] ? q / DK - (window > 0 ? max(0, q - window + 1) : 0) / DK + 1 : 0;
-        sum += n;
-        most = max(most, n);
-    }
     if (tok_end - tok <= 0) return;
-    sum = __reduce_add_sync(0xffffffffu, sum);
-    most = __reduce_max_sync(0xffffffffu, most);
     const int lo = window > 0 ? max(0, qi - window + 1) : 0;
     const int kt_first = lo / DK, kt_last = qi / DK;
-    const int per = max((int)(((long long)sum * gridDim.y + room - 1) / room), (most + n_splits - 1) / n_splits);
+    // (equal parts of the sequence's own keys: where a split ends decides what its weights are rounded against, so that this must not
+    // follow from the other sequences of the step)
+    const int per = (kt_last - kt_first + n_splits) / n_splits;
     const int kt_a = kt_first + split * per, kt_b = min(kt_last, kt_a + per - 1);
     const int n_tiles8 = rank >> 3;
     if (kt_a > kt_last && part_o != nullptr) {                     // nothing is left for this split
@@ -1066,20 +1058,6 @@ latent_decode_mma_kernel(const float* __restrict__ qa, const bf16* __restrict__ 
         }
 }
 
-// (SMs of the current device, asked once for each)
-int latent_sms(int* sms) {
-    static int known[64] = {0};
-    int dev = 0;
-    TI_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || known[dev] == 0) {
-        TI_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
-        if (dev >= 0 && dev < 64) known[dev] = *sms;
-        return 0;
-    }
-    *sms = known[dev];
-    return 0;
-}
-
 template <int MT, int NTW, bool QREG>
 int launch_decode_form(const float* qa, const void* lat, float* ol, const int* cu_new, const int* seq_start, const int* seq_slot,
                        int n_seq, int n_heads, int rank, int rot, float scale, int window, const float* sink,
@@ -1095,12 +1073,9 @@ int launch_decode_form(const float* qa, const void* lat, float* ol, const int* c
         TI_CUDA(cudaFuncSetAttribute(latent_decode_mma_kernel<MT, NTW, QREG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured = smem;
     }
-    int sms = 0;
-    if (int rc = latent_sms(&sms)) return rc;
-    const int room = sms * (smem <= 113 * 1024 ? 2 : 1);
     dim3 grid(n_seq, (n_heads + ROWS - 1) / ROWS, n_splits);
     TI_CUDA(ti_launch_class<3>(latent_decode_mma_kernel<MT, NTW, QREG>, grid, dim3(D_THREADS), smem, stream, qa, (const bf16*)lat, ol, cu_new,
-                               seq_start, seq_slot, n_heads, rank, rot, scale, window, sink, kv, n_splits, room, part_o, part_ml, shape.tiles, shape.shares, shape.pitch, status));
+                               seq_start, seq_slot, n_heads, rank, rot, scale, window, sink, kv, n_splits, part_o, part_ml, shape.tiles, shape.shares, shape.pitch, status));
     TI_CHECK_LAUNCH("latent_attention (one token, tensor cores)");
     return 0;
 }

@@ -185,9 +185,7 @@ def attention_single(d: torch.Tensor, q: torch.Tensor, rank: int, rot: int, norm
           _ptr(d), d.stride(0), _ptr(q), q.stride(0), nh, plain, rank, rot, _ptr(norm_w), float(eps), _ptr(cos), _ptr(sin), max_pos,
           _ptr(batch.tok_pos), _ptr(batch.tok_seq), _ptr(batch.seq_slot), _ptr(batch.seq_len), _ptr(lat), *_pages(mem), _ptr(uk),
           _ptr(qa), M, _code(q, "latent_attention"), _stream())
-    # (twice the planned splits: a split takes as many tiles in every sequence, and the short sequences leave theirs empty)
     splits = plan(batch.n_seq, nh, window, batch.plan_len, q.device)
-    splits = min(2 * splits, 64) if splits > 1 else 1
     part_o = torch.empty((M, nh, splits, rank), dtype=torch.float32, device=q.device)
     part_ml = torch.empty((M, nh, splits, 2), dtype=torch.float32, device=q.device)
     o = torch.empty((M, nh * vdim), dtype=q.dtype, device=q.device)
