@@ -1,5 +1,6 @@
-"""The few-row float32 product at the edges of its tiles: 1 to 16 tokens in passes of 1, 2, 4 and 8, weight rows that end inside a group of
-four, contractions that end inside a warp's turn or leave slices without work, both matrix sizes, plain and gated."""
+"""The few-row product at the edges of its tiles: 1 to 16 tokens in passes of 1, 2, 4 and 8, weight rows that end inside a group of four,
+contractions that end inside a warp's turn or leave slices without work, both matrix sizes, plain and gated; float32, and both types
+where rows lie off the 16-byte boundary."""
 from __future__ import annotations
 
 import pytest
@@ -47,3 +48,41 @@ def test_gated(M, N, Kd, act):
         g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
         want = g * torch.sigmoid(1.702 * g) * (u + 1)
     assert (got.double() - want).abs().max() <= 2e-5 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,Kd", [(1, 1), (33, 70), (130, 1023)])
+def test_rows_off_the_boundary(dtype, M, N, Kd):
+    import toyinfer_b200.kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M * N + Kd)
+    x, w = torch.randn(M, Kd + 1, generator=g, device="cuda").to(dtype)[:, 1:], (torch.randn(N, Kd, generator=g, device="cuda") / Kd ** 0.5).to(dtype)
+    out, want = K.linear(x, w, out_dtype=torch.float32).double(), x.double() @ w.double().T
+    assert (out - want).norm() <= BOUND * x.double().norm() * w.double().norm() / Kd ** 0.5
+    assert (out - want).abs().max() <= 1e-5 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_one_token_off_the_boundary_is_not_worked_off_as_eight(dtype):
+    """The time of one token's product against eight tokens' over a matrix that L2 holds: a pass of eight rows whatever their number
+    would take the same, the reads of seven rows and their multiplications more than halve."""
+    import toyinfer_b200.kernels as K
+    w = torch.randn(2048, 2045, device="cuda").to(dtype)
+
+    def time_of(M):
+        x, best = torch.randn(M, 2045, device="cuda").to(dtype), []
+        graph = torch.cuda.CUDAGraph()
+        K.linear(x, w)
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                K.linear(x, w)
+        for _ in range(9):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            best.append(a.elapsed_time(b))
+        return min(best)
+
+    assert time_of(1) < 0.8 * time_of(8)

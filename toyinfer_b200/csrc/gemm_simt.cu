@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(GV_THREADS, R == 4 ? (MR >= 4 ? 2 : 3) : 4)
 gemv_rows_kernel(const T* __restrict__ X, const T* __restrict__ W, OT* __restrict__ out,
                  int M, int N, int K, long long ldx, long long ldw, long long ldo, int kind, float limit) {
     ti_pdl_trigger();
-    constexpr int AHEAD = R == 4 ? (MR == 1 || MR == 4 ? 3 : 2) : R * MR >= 16 ? 2 : 4, SUMS = R * MR;
+    constexpr int AHEAD = V == 1 && MR == 8 && KS == 1 ? 8 : R == 4 ? (MR == 1 || MR == 4 ? 3 : 2) : R * MR >= 16 ? 2 : 4, SUMS = R * MR;
     __shared__ float part[KS > 1 ? GV_WARPS * 32 : 1];
     ti_pdl_sync();
     X = ti_dependent(X);
@@ -210,21 +210,28 @@ bool rows_aligned(const void* x, const void* w, int K, long long ldx, long long 
     return K % V == 0 && ldx % V == 0 && ldw % V == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }
 
+// Four weight rows a warp, the contraction in as many slices as give the SMs warps.
+template <typename T, typename OT, int V, int MR, bool PAIR>
+int launch_rows_sliced(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo, int kind, float limit,
+                       cudaStream_t stream) {
+    const int groups = (N + 3) / 4, steps = (K + 32 * V - 1) / (32 * V);      // groups of four rows, turns of a warp over K
+    int ks = 1;
+    while (ks < 8 && groups * ks < 148 * 16 && steps >= ks * 4) ks *= 2;
+    switch (ks) {
+        case 1: return launch_rows<T, OT, V, 4, MR, 1, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
+        case 2: return launch_rows<T, OT, V, 4, MR, 2, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
+        case 4: return launch_rows<T, OT, V, 4, MR, 4, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
+        default: return launch_rows<T, OT, V, 4, MR, 8, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
+    }
+}
+
 // 32-bit operands on 16-byte boundaries.
 template <int MR, bool PAIR>
 int launch_rows_f32(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo, int kind, float limit,
                     cudaStream_t stream) {
     constexpr int R1 = PAIR ? 2 : 1;
     if ((long long)N * K < ROWS_LARGE) return launch_rows<float, float, 4, R1, MR, 1, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
-    const int groups = (N + 3) / 4, steps = (K + 127) / 128;      // groups of four rows, turns of a warp over K
-    int ks = 1;
-    while (ks < 8 && groups * ks < 148 * 16 && steps >= ks * 4) ks *= 2;
-    switch (ks) {
-        case 1: return launch_rows<float, float, 4, 4, MR, 1, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
-        case 2: return launch_rows<float, float, 4, 4, MR, 2, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
-        case 4: return launch_rows<float, float, 4, 4, MR, 4, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
-        default: return launch_rows<float, float, 4, 4, MR, 8, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
-    }
+    return launch_rows_sliced<float, float, 4, MR, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
 }
 template <bool PAIR>
 int launch_rows_f32(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo, int kind, float limit,
@@ -242,7 +249,10 @@ int launch_simt(const void* x, const void* w, void* out, int M, int N, int K, lo
         if constexpr (sizeof(T) == 4)
             if (rows_aligned(x, w, K, ldx, ldw, 4)) return launch_rows_f32<false>(x, w, out, M, N, K, ldx, ldw, ldo, 0, 0.f, stream);
         // (bfloat16 comes here off the 16-byte boundary only: gemm_skinny.cu takes the rest)
-        return launch_rows<T, OT, 1, 1, 8, 1, false>(x, w, out, M, N, K, ldx, ldw, ldo, 0, 0.f, stream);
+        if (M == 1) return launch_rows_sliced<T, OT, 1, 1, false>(x, w, out, M, N, K, ldx, ldw, ldo, 0, 0.f, stream);
+        if (M == 2) return launch_rows_sliced<T, OT, 1, 2, false>(x, w, out, M, N, K, ldx, ldw, ldo, 0, 0.f, stream);
+        if (M <= 4) return launch_rows_sliced<T, OT, 1, 4, false>(x, w, out, M, N, K, ldx, ldw, ldo, 0, 0.f, stream);
+        return launch_rows_sliced<T, OT, 1, 8, false>(x, w, out, M, N, K, ldx, ldw, ldo, 0, 0.f, stream);
     }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     TI_REQUIRE(grid.y <= 65535, "linear: %d rows exceed the tiled kernel's grid", M);
