@@ -14,6 +14,7 @@
 #define TI_BF16 1
 
 void ti_set_error(const char* fmt, ...);
+int ti_sm_count();      // SMs of the current device, asked once for each (runtime.cu)
 
 #define TI_FAIL(...)                \
     do {                            \

@@ -70,11 +70,26 @@ __global__ void moe_route_table_kernel(const int* __restrict__ ids, const int* _
 // 8 elements (16-byte loads).  With MI = 2 a tile has 64 places (a warp 32 x 32): every weight fragment then feeds two
 // multiplications, which is what the shared memory's bandwidth allows the tensor cores; groups of few places take MI = 1.
 constexpr int TN = 128, TK = 64, T_THREADS = 256, T_LD = TK + 8;
-// Places an expert on average: beyond the first a block of the 32-bit product takes 32 of them (30 places, 1,024 x 600, 86 us a step
-// against 102; at 5 they would leave three of four warps idle); up to the second bfloat16 runs from registers (20 places 97 us against
-// 118; at 31 the tiles below, which read a weight once for 32 places, take 84).
+// Places an expert on average beyond which a block of the 32-bit product takes 32 of them (30 places, 1,024 x 600, 86 us a step
+// against 102; at 5 they would leave three of four warps idle).
 constexpr int ROWS_SMALL_PLACES = 12;
+
+// How many tiles of eight places a warp of the bfloat16 product takes from registers (moe_rows.cuh), 0: shared-memory tiles on mma.sync.
+// The register form reads an expert's weights once for 8 or 16 of its places (32: slower up to 18 places, where a second tile is the
+// exception: 2,048 x 1,024 pairs, 64 experts of 9, 153 us against 117) and grows with its tiles; the tiles below read them once for 32
+// and take the same from 1 place to 32, but no less than their chain of steps over K takes, however few experts there are.  So from
+// registers with up to eight places, and beyond them as long as its tiles' reads (some 5 TB/s, most of them from L2) take less than that
+// chain, 1.65 us a step of 64 (1.3 the shorter chains of a pair).  Weights and steps both grow with K, which cancels.
+// us a product, registers / tiles, at 9, 16 and 24 places: 8 experts, 2,048 x 1,280 pairs 22, 28, 37 / 53; 16 experts 39, 53, 66 / 58;
+// 32 experts 72, 96, 129 / 92; 64 experts 147, 204, 268 / 149; 64 experts of 1,024 x 256 23, 30, 40 / 31.
 constexpr int SKINNY_MAX_PLACES = 24;
+int skinny_tiles(int n_experts, int P, int N, int K, bool pair, int sms) {
+    if (P <= 2 * n_experts) return 1;
+    if (P <= 8 * n_experts) return 2;
+    const long long tiles = P / 16 + n_experts / 2;
+    if (P > SKINNY_MAX_PLACES * n_experts || tiles * N * (pair ? 2 : 1) > (long long)sms * (pair && K <= 1024 ? 340 : 432)) return 0;
+    return P <= 18 * n_experts ? 2 : 4;
+}
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -376,6 +391,9 @@ extern "C" int ti_moe_route_table(const int* ids, const int* table, int vocab, i
     return 0;
 }
 
+// skinny_tiles above for the tests.
+extern "C" int ti_moe_skinny_tiles(int n_experts, int P, int N, int K, int pair, int sms) { return skinny_tiles(n_experts, P, N, K, pair != 0, sms); }
+
 // P places.  pair != 0: out[i, 0:N] = act(a_i W[e]^T, a_i W2[e]^T).  Else out[(scatter ? perm[i] : i)] = a_i W[e]^T * scale.
 extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const void* W2, void* out, long long ldo,
                               const int* perm, const int* off, int n_experts, int P, int N, int K, int top, int gather,
@@ -388,10 +406,11 @@ extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const
     const bool tensor_cores = dtype == TI_BF16 && K % 8 == 0 && lda % 8 == 0 && ((uintptr_t)a & 15) == 0 && ((uintptr_t)W & 15) == 0 &&
                               (!W2 || ((uintptr_t)W2 & 15) == 0);
     timoe::RowsArgs r{a, lda, W, pair ? W2 : nullptr, out, ldo, perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride};
-    if (tensor_cores && P <= SKINNY_MAX_PLACES * n_experts) {
-        if (P <= 2 * n_experts) return timoe::launch_skinny<1>(r, P, stream);
-        if (P <= 8 * n_experts) return timoe::launch_skinny<2>(r, P, stream);
-        return timoe::launch_skinny<4>(r, P, stream);
+    if (tensor_cores) switch (skinny_tiles(n_experts, P, N, K, pair != 0, ti_sm_count())) {
+        case 1: return timoe::launch_skinny<1>(r, P, stream);
+        case 2: return timoe::launch_skinny<2>(r, P, stream);
+        case 4: return timoe::launch_skinny<4>(r, P, stream);
+        default: break;
     }
     if (tensor_cores) {
         const bool big = P >= 48 * n_experts;         // groups of 48 places and more on average: tiles of 64

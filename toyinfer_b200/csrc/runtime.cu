@@ -34,6 +34,18 @@ int ti_pdl_enabled(int cls) { return (g_pdl_mask >> (cls & 31)) & 1u; }
 extern "C" int ti_set_pdl(int on) { g_pdl_mask = on ? ~0u : 0u; return 0; }
 extern "C" int ti_set_pdl_mask(unsigned mask) { g_pdl_mask = mask; return 0; }
 
+int ti_sm_count() {
+    static int known[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (known[dev] == 0) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+        known[dev] = n;
+    }
+    return known[dev];
+}
+
 int* ti_status_ptr() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
