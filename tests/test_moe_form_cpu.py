@@ -1,4 +1,4 @@
-"""Which form the experts' bfloat16 product takes (csrc/moe_grouped.cu, skinny_tiles): the register form up to eight places an expert and
+"""Which form the experts' bfloat16 product takes (csrc/moe_grouped.cu): the register form up to eight places an expert and
 wherever the experts are few, shared-memory tiles where the register form's repeated reads of the weights were measured to take longer.
 Needs nvcc to build the library, no GPU."""
 from __future__ import annotations
@@ -50,3 +50,17 @@ def test_limits():
                     assert got[:2] == [1, 1] and got[2:8] == [2] * 6 and set(got[8:18]) <= {0, 2} and set(got[18:24]) <= {0, 4}
                     assert got[24:] == [0] * 5
                     assert not any(a == 0 and b > 0 for a, b in zip(got, got[1:]))       # once in tiles, always in tiles
+
+
+# rows off the 16-byte boundary: us from registers / in staged tiles
+@pytest.mark.parametrize("E,places,N,pair,staged", [(16, 80, 1023, True, True),       # 942 / 799
+                                                    (16, 320, 391, True, True),       # 676 / 403
+                                                    (4, 320, 1023, True, True),       # 860 / 567
+                                                    (16, 80, 2047, False, True),      # 495 / 428
+                                                    (16, 40, 1023, True, False),      # 503 / 606
+                                                    (16, 80, 391, True, False),       # 176 / 230
+                                                    (4, 160, 2047, False, False),     # 219 / 277
+                                                    (32, 2, 4096, True, False)])
+def test_rows_off_the_boundary(E, places, N, pair, staged):
+    from toyinfer_b200.kernels.lib import library
+    assert bool(library().ti_moe_staged_tiles(E, E * places, N, int(pair), 148)) == staged

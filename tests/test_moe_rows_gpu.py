@@ -57,3 +57,10 @@ def test_bfloat16(counts, H, ff, top):
 
 def test_bfloat16_off_the_boundary():
     run(torch.bfloat16, [5, 0, 12], 70, 13, 1, BF16, shift=1)
+
+
+@pytest.mark.parametrize("counts,H,ff", [([900, 1, 0, 650, 33, 32], 70, 1003), ([1300], 513, 900)])
+def test_many_places_off_the_boundary(counts, H, ff):
+    """Staged tiles for the first product (more than seven blocks an SM), either form for the second."""
+    run(torch.float32, counts, H, ff, 1, F32, shift=1)
+    run(torch.bfloat16, counts, H, ff, 1, BF16, shift=1)

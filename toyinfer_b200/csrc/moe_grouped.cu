@@ -14,7 +14,8 @@
 //                   the tokens' order), scaled by the pair's weight
 // A tile of places lies inside one expert's group (groups are walked tile by tile: the grid has an upper bound of tiles,
 // ceil(P / tile) + experts).  32-bit operands, and bfloat16 groups of few places, run from registers (moe_rows.cuh); bfloat16
-// groups of some tens of places as shared-memory tiles on mma.sync (below), of many on tcgen05 (gemm_tcgen05_grouped.cu).
+// groups of some tens of places as shared-memory tiles on mma.sync (below), of many on tcgen05 (gemm_tcgen05_grouped.cu); rows off the
+// 16-byte boundary with many places as shared-memory tiles on the CUDA cores (below).
 //
 // `moe_combine`: out[m] = sum_j z[m * top + j], summed in the order of j.
 //
@@ -60,6 +61,111 @@ __global__ void moe_route_table_kernel(const int* __restrict__ ids, const int* _
     for (int p = threadIdx.x; p < P; p += blockDim.x) {
         const int e = pair_expert[p];
         perm[offs[e] + atomicAdd(&cur[e], 1)] = p;
+    }
+}
+
+constexpr int GM = 32, GN = 64, GK = 32, G_THREADS = 256;
+
+// The product of rows off the 16-byte boundary with many places an expert, 32-bit arithmetic: tiles of 32 places x 64 weight rows staged in
+// shared memory element by element.  Where such tiles fill the device they read a weight once for 32 places; the register form
+// (moe_rows.cuh), whose loads are single elements there, once for 8, and it is bound by them: see staged_tiles below.
+// out: PAIR -> out[i, n] = act(gate, up);  else out[(scatter ? perm[i] : i), n] = product * scale.
+template <typename T, bool PAIR>
+__global__ void __launch_bounds__(G_THREADS)
+moe_staged_kernel(const T* __restrict__ a, long long lda, const T* __restrict__ W, const T* __restrict__ W2,
+                   T* __restrict__ out, long long ldo, const int* __restrict__ perm, const int* __restrict__ off,
+                   int n_experts, int N, int K, int top, int gather, int scatter, float scale, float limit, float alpha, float shift,
+                   long long w_estride) {
+    ti_pdl_trigger();
+    __shared__ float As[GK][GM + 1];
+    __shared__ float Ws[GK][GN + 1];
+    __shared__ float W2s[PAIR ? GK : 1][GN + 1];
+    __shared__ int rows[GM];
+    __shared__ int where[3];             // expert, first place, places in the tile
+    ti_pdl_sync();
+    a = ti_dependent(a); perm = ti_dependent(perm); off = ti_dependent(off);
+    if (threadIdx.x < 32) {
+        int found = -1, at = 0, n = 0;
+        if (!timoe::find_tile<GM>(off, n_experts, blockIdx.x, found, at, n)) found = -1;
+        if (threadIdx.x == 0) { where[0] = found; where[1] = at; where[2] = n; }
+    }
+    __syncthreads();
+    const int e = where[0], first = where[1], cnt = where[2];
+    if (e < 0) return;
+    const int n0 = blockIdx.y * GN;
+    if (threadIdx.x < GM) {
+        const int i = first + threadIdx.x;
+        int r = -1;
+        if (threadIdx.x < cnt) r = gather ? perm[i] / top : i;
+        rows[threadIdx.x] = r;
+    }
+    __syncthreads();
+    const T* We = W + (size_t)e * w_estride;
+    const T* W2e = PAIR ? W2 + (size_t)e * w_estride : nullptr;
+    // thread (ty, tx): places ty, ty + 8, ty + 16, ty + 24; weight rows tx, tx + 32
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    float acc[4][2], acc2[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) { acc[i][j] = 0.f; acc2[i][j] = 0.f; }
+    // (a step's 32 products are added up by themselves: sums of thousands one after another lose a digit)
+    for (int k0 = 0; k0 < K; k0 += GK) {
+        for (int idx = threadIdx.x; idx < GM * GK; idx += G_THREADS) {
+            const int r = idx / GK, kk = idx - r * GK;
+            const int src = rows[r];
+            As[kk][r] = (src >= 0 && k0 + kk < K) ? to_f32(a[(size_t)src * lda + k0 + kk]) : 0.f;
+        }
+        for (int idx = threadIdx.x; idx < GN * GK; idx += G_THREADS) {
+            const int r = idx / GK, kk = idx - r * GK;
+            const bool ok = n0 + r < N && k0 + kk < K;
+            Ws[kk][r] = ok ? to_f32(We[(size_t)(n0 + r) * K + k0 + kk]) : 0.f;
+            if constexpr (PAIR) W2s[kk][r] = ok ? to_f32(W2e[(size_t)(n0 + r) * K + k0 + kk]) : 0.f;
+        }
+        __syncthreads();
+        float part[4][2] = {}, part2[4][2] = {};
+#pragma unroll 8
+        for (int kk = 0; kk < GK; kk++) {
+            float av[4], wv[2], w2v[2];
+#pragma unroll
+            for (int i = 0; i < 4; i++) av[i] = As[kk][ty + 8 * i];
+#pragma unroll
+            for (int j = 0; j < 2; j++) { wv[j] = Ws[kk][tx + 32 * j]; w2v[j] = PAIR ? W2s[kk][tx + 32 * j] : 0.f; }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    part[i][j] = fmaf(av[i], wv[j], part[i][j]);
+                    if constexpr (PAIR) part2[i][j] = fmaf(av[i], w2v[j], part2[i][j]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) { acc[i][j] += part[i][j]; acc2[i][j] += part2[i][j]; }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int r = ty + 8 * i;
+        if (r >= cnt) continue;
+        const int place = first + r;
+        const size_t orow = scatter ? (size_t)perm[place] : (size_t)place;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int n = n0 + tx + 32 * j;
+            if (n >= N) continue;
+            float y;
+            if constexpr (PAIR) {
+                // the two products are rounded to the engine's type first (as in moe_rows.cuh)
+                const float g = fminf(to_f32(from_f32<T>(acc[i][j])), limit);
+                const float u = fminf(fmaxf(to_f32(from_f32<T>(acc2[i][j])), -limit), limit);
+                y = g * ti_over(1.0f, 1.0f + expf(-alpha * g)) * (u + shift);
+            } else {
+                y = acc[i][j] * scale;
+            }
+            out[orow * ldo + n] = from_f32<T>(y);
+        }
     }
 }
 
@@ -391,7 +497,16 @@ extern "C" int ti_moe_route_table(const int* ids, const int* table, int vocab, i
     return 0;
 }
 
-// skinny_tiles above for the tests.
+// Whether a product of rows off the 16-byte boundary runs in staged tiles: with more than 48 places an expert, where the tiles are more
+// than seven blocks an SM (a pair's counted twice, it reads two matrices).  us a product, registers / tiles, float32, 16 experts: pairs of 2,047 x 1,023, 40 places an
+// expert 503 / 606, 80 942 / 799, 160 1,794 / 1,082, 320 3,462 / 1,829; 1,023 x 391, 80 places 176 / 230, 160 336 / 268; single matrices
+// of 2,047 x 1,023, 40 places 265 / 330, 80 495 / 428; four experts of pairs of 2,047 x 1,023, 160 places 441 / 477, 320 860 / 567.
+bool staged_tiles(int n_experts, int P, int N, bool pair, int sms) {
+    return P > 48LL * n_experts && ((long long)P / GM + n_experts / 2) * ((N + GN - 1) / GN) * (pair ? 2 : 1) > 7LL * sms;
+}
+
+// skinny_tiles and staged_tiles above for the tests.
+extern "C" int ti_moe_staged_tiles(int n_experts, int P, int N, int pair, int sms) { return staged_tiles(n_experts, P, N, pair != 0, sms); }
 extern "C" int ti_moe_skinny_tiles(int n_experts, int P, int N, int K, int pair, int sms) { return skinny_tiles(n_experts, P, N, K, pair != 0, sms); }
 
 // P places.  pair != 0: out[i, 0:N] = act(a_i W[e]^T, a_i W2[e]^T).  Else out[(scatter ? perm[i] : i)] = a_i W[e]^T * scale.
@@ -432,7 +547,15 @@ extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const
         const bool vec = K % V == 0 && lda % V == 0 && w_estride % V == 0 && (((uintptr_t)a | (uintptr_t)W | (uintptr_t)r.W2) & 15) == 0;
         if constexpr (sizeof(T) == 4)
             if (vec) return P > ROWS_SMALL_PLACES * n_experts ? timoe::launch_rows<T, V, 4>(r, P, stream) : timoe::launch_rows<T, V, 1>(r, P, stream);
-        return timoe::launch_rows<T, 1, 1>(r, P, stream);
+        if (!staged_tiles(n_experts, P, N, pair != 0, ti_sm_count())) return timoe::launch_rows<T, 1, 1>(r, P, stream);
+        const dim3 grid((P + GM - 1) / GM + n_experts, (N + GN - 1) / GN);
+        TI_REQUIRE(grid.y <= 65535, "moe_grouped: %d weight rows are too many for one launch", N);
+#define TI_MOE_LAUNCH(PAIR) TI_CUDA(ti_launch(moe_staged_kernel<T, PAIR>, grid, dim3(G_THREADS), 0, stream, (const T*)a, lda, (const T*)W, (const T*)W2, (T*)out, ldo, \
+                                              perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride))
+        if (pair) TI_MOE_LAUNCH(true); else TI_MOE_LAUNCH(false);
+#undef TI_MOE_LAUNCH
+        TI_CHECK_LAUNCH("moe_grouped");
+        return 0;
     });
 }
 
