@@ -129,6 +129,22 @@ def test_router_with_its_product_not_a_number():
     w[:, 0] = torch.tensor([nan, 3.0, 2.0, 1.0])          # x = unit vectors: a row's logits are w's columns; 0 * nan reaches the others
     perm, off, _, _ = KM.route_rows(x[:1].contiguous(), w, None, 2, 1.0, None, 64)
     assert sorted(perm.tolist()) == [0, 1] and off.tolist() == [0, 1, 2, 2, 2]
-    w[:, 0] = torch.tensor([0.0, nan, -0.0, -1.0])
+    w[:, 0] = torch.tensor([0.0, nan, -0.0, -1.0])          # 0 wins over -0 as the lower index; then the lowest open one is no number
     perm, off, _, _ = KM.route_rows(x[:1].contiguous(), w, None, 2, 1.0, None, 64)
-    assert off.tolist() == [0, 1, 2, 2, 2] or off.tolist() == [0, 1, 1, 2, 2]
+    assert off.tolist() == [0, 1, 2, 2, 2]
+    w[:, 0] = torch.tensor([0.0, -1.0, nan, -0.0])          # where the lowest open one is a number, a score that is none never wins
+    perm, off, _, _ = KM.route_rows(x[:1].contiguous(), w, None, 2, 1.0, None, 64)
+    assert off.tolist() == [0, 1, 1, 1, 2]
+    for column in w.T[:1].contiguous(), torch.tensor([[0.0, nan, -0.0, -1.0]], device="cuda"), torch.tensor([[nan, nan, 1.0, 2.0]], device="cuda"):
+        w[:, 0] = column[0]
+        got, want = KM.route_rows(x[:1].contiguous(), w, None, 2, 1.0, None, 64), KM.route_softmax(column, None, 4, 2)
+        assert torch.equal(got[1], want[1]) and torch.equal(got[0], want[0])          # as the router of finished logits chooses
+
+
+@pytest.mark.parametrize("M,E,H,takes", [(2048, 8, 4096, True), (1, 8, 4096, False), (1, 8, 2048, True), (1, 16, 4096, True), (2049, 16, 4096, False), (8192, 8, 2048, True), (8193, 8, 2048, False),
+                                         (8193, 16, 2048, True), (8193, 32, 4096, True)])
+def test_where_the_product_of_its_own_is_faster(M, E, H, takes):
+    from toyinfer_b200.kernels import moe as KM
+    x, w = torch.empty(M, H, dtype=torch.bfloat16, device="cuda"), torch.empty(E, H, dtype=torch.bfloat16, device="cuda")
+    assert KM.route_rows_eligible(x, w, 0, 2) == takes
+    assert KM.route_rows_eligible(x.float(), w.float(), 0, 2)

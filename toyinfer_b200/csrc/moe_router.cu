@@ -194,6 +194,8 @@ int route_few(const float* z, long long ldz, const float* logit_bias, const floa
 // expert, choose as moe_route_few_kernel does.  The choices go to moe_place_kernel, which counts and places the pairs.
 // (The product alone, a tcgen05 tile of which 16 of 128 rows were used, took 12 us at 40 to 777 tokens, and the one-block router after
 // it 7 us at one token and 9 at 777: what bounds both is a chain of dependent steps, not work.)
+// Pieces on their way and blocks an SM so that nothing spills: 32 experts in bfloat16 with four pieces and three blocks took, rows of
+// 2,048, 10.3, 19.4 and 22.9 us at 1, 296 and 777 tokens; with two and two 6.9, 8.6 and 13.4.
 constexpr int RK_THREADS = 256;
 
 // Smaller than every number's key: not a number.  Equal numbers (zeros of both signs too) have equal keys.
@@ -204,12 +206,12 @@ __device__ __forceinline__ unsigned order_key(float c) {
 }
 
 template <typename T, int EPW, int TOK>
-__global__ void __launch_bounds__(RK_THREADS, TOK == 1 ? 2 : 3)
+__global__ void __launch_bounds__(RK_THREADS, TOK == 1 || EPW * 16 / sizeof(T) > 16 ? 2 : 3)
 moe_router_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ w, int K, const float* __restrict__ logit_bias,
                   const float* __restrict__ correction, int n_experts, int top, float scale, int M, int* __restrict__ pair_expert,
                   float* __restrict__ pair_w) {
     ti_pdl_trigger();
-    constexpr int V = 16 / sizeof(T), AHEAD = TOK == 1 ? 4 : 1;
+    constexpr int V = 16 / sizeof(T), AHEAD = TOK > 1 ? 1 : EPW * V > 16 ? 2 : 4;
     struct alignas(16) Pack { T v[V]; };
     __shared__ float logits[TOK][32];
     ti_pdl_sync();
@@ -540,7 +542,7 @@ extern "C" int ti_moe_route_rows(const void* x, long long ldx, const void* w, in
             return 0;
         };
         // a token a block while all blocks fit the device at once
-        const int rc = M <= 296 ? go(std::integral_constant<int, 1>()) : go(std::integral_constant<int, 4>());
+        const int rc = M <= 2 * ti_sm_count() ? go(std::integral_constant<int, 1>()) : go(std::integral_constant<int, 4>());
         if (rc) return rc;
         TI_CHECK_LAUNCH("moe_route_rows");
         return 0;

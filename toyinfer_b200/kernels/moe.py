@@ -170,12 +170,19 @@ def route_softmax(z: torch.Tensor, correction, n_experts: int, top: int, n_group
 
 
 def route_rows_eligible(x: torch.Tensor, w: torch.Tensor, n_groups: int, top: int) -> bool:
-    """Whether ``route_rows`` takes this router: up to 32 experts, no runs, rows on 16-byte boundaries."""
+    """Whether ``route_rows`` takes this router: up to 32 experts, no runs, rows on 16-byte boundaries; in bfloat16 up to 16 experts
+    only so many tokens, as it reads the router's matrix again for every four and the tcgen05 product does not.  us, both kernels /
+    product and router: rows of 4,096, 8 experts, 1,500 tokens 16.8 / 16.6, 4,096 29.5 / 24.2; 16 experts 20.3 / 26.4 and 43.5 / 40.8;
+    rows of 2,048, 8 experts, 8,192 tokens 36.8 / 36.8, 16,384 70.9 / 62.5; 16 experts, 16,384 104 / 114.  (32 experts, 8,192 tokens
+    of 4,096: 143 / 235; float32, 16,384 tokens: 172 / 220 at 8 experts of 4,096, its largest part.)  One token, 8 experts of 4,096:
+    7.2 / 5.7; of 2,048 5.3 / 5.7."""
     E, H = w.shape
-    v = 16 // x.element_size()
+    M, v = x.shape[0], 16 // x.element_size()
+    if x.dtype == torch.bfloat16 and E <= 16 and (M > 2048 or M == 1 and E <= 8 if H > 2048 else M > 8192 and E <= 8):
+        return False
     return (E <= 32 and n_groups <= 1 and top <= 16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] == H and x.dtype == w.dtype
             and w.is_contiguous() and H % v == 0 and x.stride(0) % v == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and x.shape[0] * top * 32 < 2 ** 31)
+            and M * top * 32 < 2 ** 31)
 
 
 def route_rows(x: torch.Tensor, w: torch.Tensor, correction, top: int, scale: float, logit_bias, ff: int):
