@@ -81,3 +81,24 @@ def test_products_are_rounded_before_the_activation(act):
     assert float((got != want.to(torch.bfloat16)).float().mean()) < 0.03
     few = run(40)
     assert float((got[:40] != few).float().mean()) < 0.03
+
+
+def test_the_squared_relu_takes_products_in_32_bits():
+    """As above for the experts whose activation is the squared ReLU: every form squares the products before they are rounded."""
+    from toyinfer_b200.kernels import moe as KM, check_status
+    M, E, H = 300, 2, 256
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randn(M, H, generator=g, device="cuda").to(torch.bfloat16)
+    expert, perm, off = places(M, E, 1)
+    up = (torch.randn(E, H, H, generator=g, device="cuda") * H ** -0.5).to(torch.bfloat16)
+    down = torch.eye(H, device="cuda").to(torch.bfloat16).expand(E, H, H).contiguous()
+    want = torch.stack([(x[m].double() @ up[expert[m]].double().T).clamp(min=0) ** 2 for m in range(M)]).to(torch.bfloat16)
+    # padded; tiles of some tens of places; from registers, several and one an expert
+    for rows in (300, 90, 40, 6, 1):
+        order = perm[perm < rows].contiguous()
+        at = torch.tensor([0] + torch.bincount(expert[:rows], minlength=E).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+        z, place = KM.experts_relu2(x[:rows], order, at, up, down, 1)
+        check_status()
+        got = z if place is None else z[place.long()]
+        # (sums within 2^-20 fall on another side of a rounding to 8 bits in fewer than one case of a hundred)
+        assert float((got != want[:rows]).float().mean()) < 0.03

@@ -74,7 +74,7 @@ template <typename T, bool PAIR>
 __global__ void __launch_bounds__(G_THREADS)
 moe_staged_kernel(const T* __restrict__ a, long long lda, const T* __restrict__ W, const T* __restrict__ W2,
                    T* __restrict__ out, long long ldo, const int* __restrict__ perm, const int* __restrict__ off,
-                   int n_experts, int N, int K, int top, int gather, int scatter, float scale, float limit, float alpha, float shift,
+                   int n_experts, int N, int K, int top, int gather, int scatter, int relu2, float scale, float limit, float alpha, float shift,
                    long long w_estride) {
     ti_pdl_trigger();
     __shared__ float As[GK][GM + 1];
@@ -162,7 +162,7 @@ moe_staged_kernel(const T* __restrict__ a, long long lda, const T* __restrict__ 
                 const float u = fminf(fmaxf(to_f32(from_f32<T>(acc2[i][j])), -limit), limit);
                 y = g * ti_over(1.0f, 1.0f + expf(-alpha * g)) * (u + shift);
             } else {
-                y = acc[i][j] * scale;
+                y = timoe::single<T>(relu2, scale, acc[i][j]);
             }
             out[orow * ldo + n] = from_f32<T>(y);
         }
@@ -207,7 +207,7 @@ template <bool PAIR, int MI>
 __global__ void __launch_bounds__(T_THREADS)
 moe_grouped_mma_kernel(const bf16* __restrict__ a, long long lda, const bf16* __restrict__ W, const bf16* __restrict__ W2,
                        bf16* __restrict__ out, long long ldo, const int* __restrict__ perm, const int* __restrict__ off,
-                       int n_experts, int N, int K, int top, int gather, int scatter, float scale, float limit, float alpha, float shift,
+                       int n_experts, int N, int K, int top, int gather, int scatter, int relu2, float scale, float limit, float alpha, float shift,
                        long long w_estride) {
     ti_pdl_trigger();
     constexpr int TM = 32 * MI;
@@ -323,7 +323,7 @@ moe_grouped_mma_kernel(const bf16* __restrict__ a, long long lda, const bf16* __
                     const float u = fminf(fmaxf(to_f32(from_f32<bf16>(acc2[m][j][2 * half + c])), -limit), limit);
                     y = gt * (ti_over(1.0f, 1.0f + expf(-alpha * gt))) * (u + shift);
                 } else {
-                    y = acc[m][j][2 * half + c] * scale;
+                    y = timoe::single<bf16>(relu2, scale, acc[m][j][2 * half + c]);
                 }
                 out[orow * ldo + n] = from_f32<bf16>(y);
             }
@@ -509,7 +509,8 @@ bool staged_tiles(int n_experts, int P, int N, bool pair, int sms) {
 extern "C" int ti_moe_staged_tiles(int n_experts, int P, int N, int pair, int sms) { return staged_tiles(n_experts, P, N, pair != 0, sms); }
 extern "C" int ti_moe_skinny_tiles(int n_experts, int P, int N, int K, int pair, int sms) { return skinny_tiles(n_experts, P, N, K, pair != 0, sms); }
 
-// P places.  pair != 0: out[i, 0:N] = act(a_i W[e]^T, a_i W2[e]^T).  Else out[(scatter ? perm[i] : i)] = a_i W[e]^T * scale.
+// P places.  pair != 0: out[i, 0:N] = act(a_i W[e]^T, a_i W2[e]^T).  Else out[(scatter ? perm[i] : i)] = a_i W[e]^T * scale, or, pair 2
+// without W2, the squared ReLU of a_i W[e]^T.
 extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const void* W2, void* out, long long ldo,
                               const int* perm, const int* off, int n_experts, int P, int N, int K, int top, int gather,
                               int scatter, int pair, float scale, float limit, float alpha, float shift, long long w_estride, int dtype,
@@ -517,10 +518,12 @@ extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const
     if (P == 0) return 0;
     if (w_estride <= 0) w_estride = (long long)N * K;          // elements from one expert's matrix to the next
     TI_REQUIRE(P > 0 && N > 0 && K > 0 && n_experts > 0 && top > 0, "moe_grouped: bad sizes");
+    const int relu2 = pair == 2 && !W2;
+    if (relu2) pair = 0;
     TI_REQUIRE(!pair || W2, "moe_grouped: the paired form needs a second matrix");
     const bool tensor_cores = dtype == TI_BF16 && K % 8 == 0 && lda % 8 == 0 && ((uintptr_t)a & 15) == 0 && ((uintptr_t)W & 15) == 0 &&
                               (!W2 || ((uintptr_t)W2 & 15) == 0);
-    timoe::RowsArgs r{a, lda, W, pair ? W2 : nullptr, out, ldo, perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride};
+    timoe::RowsArgs r{a, lda, W, pair ? W2 : nullptr, out, ldo, perm, off, n_experts, N, K, top, gather, scatter, relu2, scale, limit, alpha, shift, w_estride};
     if (tensor_cores) switch (skinny_tiles(n_experts, P, N, K, pair != 0, ti_sm_count())) {
         case 1: return timoe::launch_skinny<1>(r, P, stream);
         case 2: return timoe::launch_skinny<2>(r, P, stream);
@@ -534,7 +537,7 @@ extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const
         const int nblk = (N + TN - 1) / TN;
         TI_REQUIRE(nblk <= 65535, "moe_grouped: %d weight rows are too many for one launch", N);
 #define TI_MOE_LAUNCH(PAIR, MI) TI_CUDA(ti_launch(moe_grouped_mma_kernel<PAIR, MI>, dim3(tiles, nblk), dim3(T_THREADS), 0, stream, (const bf16*)a, lda, \
-                              (const bf16*)W, (const bf16*)W2, (bf16*)out, ldo, perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride))
+                              (const bf16*)W, (const bf16*)W2, (bf16*)out, ldo, perm, off, n_experts, N, K, top, gather, scatter, relu2, scale, limit, alpha, shift, w_estride))
         if (pair) { if (big) TI_MOE_LAUNCH(true, 2); else TI_MOE_LAUNCH(true, 1); }
         else { if (big) TI_MOE_LAUNCH(false, 2); else TI_MOE_LAUNCH(false, 1); }
 #undef TI_MOE_LAUNCH
@@ -551,7 +554,7 @@ extern "C" int ti_moe_grouped(const void* a, long long lda, const void* W, const
         const dim3 grid((P + GM - 1) / GM + n_experts, (N + GN - 1) / GN);
         TI_REQUIRE(grid.y <= 65535, "moe_grouped: %d weight rows are too many for one launch", N);
 #define TI_MOE_LAUNCH(PAIR) TI_CUDA(ti_launch(moe_staged_kernel<T, PAIR>, grid, dim3(G_THREADS), 0, stream, (const T*)a, lda, (const T*)W, (const T*)W2, (T*)out, ldo, \
-                                              perm, off, n_experts, N, K, top, gather, scatter, scale, limit, alpha, shift, w_estride))
+                                              perm, off, n_experts, N, K, top, gather, scatter, relu2, scale, limit, alpha, shift, w_estride))
         if (pair) TI_MOE_LAUNCH(true); else TI_MOE_LAUNCH(false);
 #undef TI_MOE_LAUNCH
         TI_CHECK_LAUNCH("moe_grouped");

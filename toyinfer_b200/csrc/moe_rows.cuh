@@ -27,6 +27,7 @@ struct RowsArgs {
     void* out; long long ldo;                // pair: out[i] = act(gate, up); else out[scatter ? perm[i] : i] = product * scale
     const int* perm; const int* off;
     int n_experts, N, K, top, gather, scatter;
+    int relu2;                               // without a pair: every product through the squared ReLU instead of times `scale`
     float scale, limit, alpha, shift;
     long long w_estride;                     // elements from one expert's matrix to the next
 };
@@ -65,6 +66,13 @@ __device__ __forceinline__ float pair_act(const RowsArgs& a, float gate, float u
     const float g = fminf(to_f32(from_f32<T>(gate)), a.limit);
     const float u = fminf(fmaxf(to_f32(from_f32<T>(up)), -a.limit), a.limit);
     return g * (ti_over(1.0f, 1.0f + expf(-a.alpha * g))) * (u + a.shift);
+}
+
+// a product without a pair, before it is stored
+template <typename T>
+__device__ __forceinline__ float single(int relu2, float scale, float x) {
+    if (!relu2) return x * scale;
+    return sizeof(T) == 2 ? ti_pointwise_bf16(x, 4) : ti_pointwise(x, 4);
 }
 
 // 32-bit arithmetic on the CUDA cores.  A warp takes four weight rows (two of each matrix of a pair) and eight places; its lanes
@@ -146,7 +154,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 2) moe_rows_kernel(RowsArgs p) {
     const int r = lane & 7, n = n0 + (PAIR ? (lane >> 3 & 1) : lane >> 3);
     if (r >= cnt || n >= p.N || (PAIR && lane >= 16)) return;
     const size_t row = p.scatter ? (size_t)p.perm[first + r] : (size_t)(first + r);
-    ((T*)p.out)[row * p.ldo + n] = from_f32<T>(PAIR ? pair_act<T>(p, sum, second) : sum * p.scale);
+    ((T*)p.out)[row * p.ldo + n] = from_f32<T>(PAIR ? pair_act<T>(p, sum, second) : single<T>(p.relu2, p.scale, sum));
 }
 
 // bfloat16 on mma.sync, as the dense product of a few tokens does it (gemm_skinny.cu): a warp owns 16 weight rows (8 of each
@@ -246,8 +254,8 @@ __global__ void __launch_bounds__(SK_WARPS * 32, NT == 4 ? 2 : 3) moe_skinny_ker
             if (PAIR) {
                 if (lo_ok) out[n_lo] = from_f32<bf16>(pair_act<bf16>(p, c[n][i], c[n][i + 2]));
             } else {
-                if (lo_ok) out[n_lo] = from_f32<bf16>(c[n][i] * p.scale);
-                if (hi_ok) out[n_hi] = from_f32<bf16>(c[n][i + 2] * p.scale);
+                if (lo_ok) out[n_lo] = from_f32<bf16>(single<bf16>(p.relu2, p.scale, c[n][i]));
+                if (hi_ok) out[n_hi] = from_f32<bf16>(single<bf16>(p.relu2, p.scale, c[n][i + 2]));
             }
         }
 }

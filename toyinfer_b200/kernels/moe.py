@@ -261,10 +261,9 @@ def experts_relu2(x: torch.Tensor, perm: torch.Tensor, off: torch.Tensor, w_up: 
         _call(grouped, _ptr(y), _ptr(w_down), _ptr(z), _ptr(tile_group), rows, E, H, ff, H, 0, 0.0, 0.0, 0.0, _stream())
         return z, pad_of_pair
     fn = _fn("ti_moe_grouped", [P, L, P, P, P, L, P, P, I, I, I, I, I, I, I, I, F, F, F, F, L, I, P])
-    u = torch.empty((Pn, ff), dtype=x.dtype, device=dev)
-    _call(fn, _ptr(x), x.stride(0), _ptr(w_up), None, _ptr(u), ff, _ptr(perm), _ptr(off), E, Pn, ff, H, top, 1, 0, 0,
+    y = torch.empty((Pn, ff), dtype=x.dtype, device=dev)
+    _call(fn, _ptr(x), x.stride(0), _ptr(w_up), None, _ptr(y), ff, _ptr(perm), _ptr(off), E, Pn, ff, H, top, 1, 0, 2,
           1.0, 0.0, 0.0, 0.0, 0, code, _stream())
-    y = relu2(u)
     z = torch.empty((Pn, H), dtype=x.dtype, device=dev)
     _call(fn, _ptr(y), ff, _ptr(w_down), None, _ptr(z), H, _ptr(perm), _ptr(off), E, Pn, H, ff, top, 0, 1, 0,
           1.0, 0.0, 0.0, 0.0, 0, code, _stream())
