@@ -164,8 +164,8 @@ static inline cudaError_t ti_launch_after(void (*kernel)(KArgs...), dim3 grid, d
 __device__ __forceinline__ float ti_over(float z, float d) {
     float r;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-    const float q = z * r, rest = fmaf(-q, d, z);
-    return fabsf(rest) < INFINITY ? fmaf(rest, r, q) : q;
+    const float q = z * r, over = fmaf(q, d, -z);        // (over = -rest: of a zero z it is +0, and the sum below keeps the sign of q)
+    return fabsf(over) < INFINITY ? fmaf(-over, r, q) : q;
 }
 
 // The activation of a gated product's gate.  kind 1: silu, z / (1 + exp(-z)); kind 2: the tanh form of gelu,
