@@ -56,3 +56,24 @@ def test_where_rows_do_not_go_with_the_launch():
     with torch.cuda.graph(g):
         assert K.sample_rows(x[:5], 1.0, 20, 0.9, 1, keys[:5], steps[:5]) is None    # a capture
         x[:5] * 2
+
+
+@pytest.mark.parametrize("V", [1025, 4096, 4097, 8191, 20001])
+@pytest.mark.parametrize("kind", ["plain", "ties", "masked"])
+def test_ranks_beyond_the_first_candidates(kind, V):
+    """A wide nucleus, walked tier by tier, at lengths around a turn of the block over the row: the token that the rule gives in 64 bits."""
+    import toyinfer_b200.kernels as K
+    x = rows(kind, 4, V) * 0.1 if kind != "masked" else rows(kind, 4, V)
+    keys, steps = np.arange(4, dtype=np.int64), np.arange(4, dtype=np.int32)
+    got = K.sample_rows(x, 1.0, 0, 0.97, 5, keys, steps).tolist()
+    p = torch.softmax(x.double(), dim=1).cpu()
+    for r in range(4):
+        row = x[r].tolist()
+        order = sorted(range(V), key=lambda i: (-row[i], i))
+        run = torch.cumsum(p[r][order], 0)
+        cut = int((run > 0.97).nonzero()[0])
+        coin = K.uniform_from(5, int(keys[r]), int(steps[r])) * float(run[cut])
+        at = int((run > coin).nonzero()[0])
+        # (sums of up to 20,000 probabilities in 32 bits, one after another: an entry whose running sum lies within 1e-4 may be passed)
+        near = {order[i] for i in range(max(0, at - 400), min(V, at + 400)) if abs(float(run[i]) - coin) < 1e-4 + float(p[r][order[i]])}
+        assert got[r] in near | {order[at]}

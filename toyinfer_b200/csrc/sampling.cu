@@ -296,10 +296,11 @@ __global__ void __launch_bounds__(SB) sample_topk_kernel(SampleArgs a) {
 // walks many (a nucleus of 34,000 entries: 34 tiers).  The kept set's sum is formed first, in a
 // fixed order (a contiguous run of entries per thread, then a scan over the threads).
 //
-// What bounds it: the passes over the row by one SM, four a rank and one a tier (their counts go to shared memory once a warp and byte
-// value, the byte is found by a warp, the walk reads eight entries at a time and divides none: one thread did all three alone), and
-// the walk's chain of sums, which has to keep its order.  14 rows of 8,845 logits, a nucleus of 0.9: 134 -> 67 us; 8 of 60,000, flat
-// ones, 1,380 -> 1,146.
+// What bounds it: the passes over the row by one SM, four a rank and one a tier, and the walk's chain of sums, which has to keep its
+// order.  The byte is found by a warp, the walk reads eight entries at a time and divides none (one thread did both alone); the first
+// byte's counts, of a few values, go to shared memory once a warp and value, those of the other three one by one (all four once a warp
+// and value, which compares the lanes of every warp of the row: 2,931 us for a row of 151,936 logits, a nucleus of 0.95; so 2,118; all
+// one by one, the walk by one thread, 2,504).  8 rows of 32,000, flat ones: 4,449 -> 2,218; 14 of 8,845, a nucleus of 0.9: 134 -> 67.
 // ---------------------------------------------------------------------------
 constexpr int MAX_TIERS = 1024;
 
@@ -341,6 +342,8 @@ __device__ __forceinline__ void pick_bin(const int* hist, int rem, int* s) {
     s[2] = above + in < rem ? 1 : in == rem - above ? 2 : 0;
 }
 
+constexpr int RANK_AHEAD = 4;     // logits a thread has on their way
+
 // The bound of sorted rank `k` (1 <= k <= V): the k entries at or before it are exactly the k
 // first of the sorted order.  All threads call it and get the same answer.
 __device__ Bound select_rank(const float* x, int V, float temp, int k, int* hist, int* scan_i, int* s_bin, int* s_idx) {
@@ -350,13 +353,26 @@ __device__ Bound select_rank(const float* x, int V, float temp, int k, int* hist
     for (int pass = 3; pass >= 0; pass--) {
         if (t < 256) hist[t] = 0;
         __syncthreads();
-        // one count a warp and byte value (most logits share their first byte: their counts would queue for one word)
-        for (int i0 = t - (t & 31); i0 < V; i0 += SB) {
-            const int i = i0 + (t & 31);
-            const unsigned key = i < V ? order_key(x[i] / temp) : 0u;
-            const int bin = i < V && (key & mask) == prefix ? (int)((key >> (8 * pass)) & 255) : -1;
-            const unsigned same = __match_any_sync(0xffffffffu, bin);
-            if (bin >= 0 && (t & 31) == __ffs(same) - 1) atomicAdd(&hist[bin], __popc(same));
+        if (pass == 3) {
+            // one count a warp and byte value (most logits share their first byte: their counts would queue for one word)
+            for (int i0 = t - (t & 31); i0 < V; i0 += RANK_AHEAD * SB) {
+                float v[RANK_AHEAD];
+#pragma unroll
+                for (int j = 0; j < RANK_AHEAD; j++) v[j] = i0 + j * SB + (t & 31) < V ? x[i0 + j * SB + (t & 31)] : 0.f;
+#pragma unroll
+                for (int j = 0; j < RANK_AHEAD; j++) {
+                    if (i0 + j * SB >= V) break;                  // (the same for the warp)
+                    const int bin = i0 + j * SB + (t & 31) < V ? (int)(order_key(v[j] / temp) >> 24) : -1;
+                    const unsigned same = __match_any_sync(0xffffffffu, bin);
+                    if (bin >= 0 && (t & 31) == __ffs(same) - 1) atomicAdd(&hist[bin], __popc(same));
+                }
+            }
+        } else {
+            // few of a warp's lanes still count, and their bytes differ
+            for (int i = t; i < V; i += SB) {
+                const unsigned key = order_key(x[i] / temp);
+                if ((key & mask) == prefix) atomicAdd(&hist[(key >> (8 * pass)) & 255], 1);
+            }
         }
         __syncthreads();
         pick_bin(hist, rem, s_bin);
