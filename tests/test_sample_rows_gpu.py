@@ -58,6 +58,18 @@ def test_where_rows_do_not_go_with_the_launch():
         x[:5] * 2
 
 
+@pytest.mark.parametrize("kind", ["plain", "ties", "neighbours"])
+@pytest.mark.parametrize("top_k", [32, 33, 63])
+def test_merges_of_many_candidates(monkeypatch, kind, top_k):
+    """Chunks enough for thousands of candidates, at the number of entries where the merge takes closer bounds."""
+    import toyinfer_b200.kernels as K
+    x = rows(kind, 5, 151936)
+    keys, steps = np.arange(5, dtype=np.int64), np.arange(5, dtype=np.int32)
+    got = K.sample_rows(x, 0.8, top_k, 0.97, 3, keys, steps)
+    monkeypatch.setattr(K, "two_kernel_sampling", False)
+    assert torch.equal(K.sample(x, 0.8, top_k, 0.97, 3, torch.from_numpy(keys).cuda(), torch.from_numpy(steps).cuda()), got)
+
+
 @pytest.mark.parametrize("V", [1025, 4096, 4097, 8191, 20001])
 @pytest.mark.parametrize("kind", ["plain", "ties", "masked"])
 def test_ranks_beyond_the_first_candidates(kind, V):

@@ -924,13 +924,18 @@ __device__ int merge_candidates(const unsigned long long* cand, int n_cand, int 
         for (int e = 0; e < EPT; e++) w[e] = t + e * SB < n_cand ? cand[t + e * SB] : 0ull;
 #pragma unroll
         for (int e = 0; e < EPT; e++) own = max(own, (unsigned)(w[e] >> 32));
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) own = max(own, __shfl_xor_sync(0xffffffffu, own, o));
+        // the maxima of eight threads each, of four where more entries are asked for (64 of 128 maxima are a loose bound: 64 rows of
+        // 38 chunks' 64 entries left several hundred above it)
+        const int share = k <= 32 ? 8 : 4;
+        own = max(own, __shfl_xor_sync(0xffffffffu, own, 1));
+        own = max(own, __shfl_xor_sync(0xffffffffu, own, 2));
+        if (share == 8) own = max(own, __shfl_xor_sync(0xffffffffu, own, 4));
         unsigned* key = reinterpret_cast<unsigned*>(hist);
-        if ((t & 7) == 0) key[t >> 3] = own;
+        const bool holds = t % share == 0;
+        if (holds) key[t / share] = own;
         if (t == 0) { sh[0] = 0; sh[1] = -1; }
         __syncthreads();
-        const unsigned bound = kth_of(key, SB / 8, k, (t & 7) == 0, own, &sh[1]);
+        const unsigned bound = kth_of(key, SB / share, k, holds, own, &sh[1]);
 #pragma unroll
         for (int e = 0; e < EPT; e++)
             if (w[e] != 0ull && (unsigned)(w[e] >> 32) >= bound) {
