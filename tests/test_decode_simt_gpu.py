@@ -46,15 +46,15 @@ def exact(q, rows, scale, window):
     return torch.stack(out)
 
 
-def run(monkeypatch, dtype, nh, nkv, hd, window, splits, offset=0):
+def run(monkeypatch, dtype, nh, nkv, hd, window, splits, offset=0, lens=LENS):
     from toyinfer_b200.kernels import attention
-    mem, rows = paged(LENS, nkv, hd, dtype, window, nh * hd, offset)
+    mem, rows = paged(lens, nkv, hd, dtype, window, nh * hd, offset)
     g = torch.Generator("cuda").manual_seed(5)
-    q = torch.randn((len(LENS), nh * hd + 3), generator=g, device="cuda").to(dtype)[:, 3:].view(len(LENS), nh, hd)
-    batch = SimpleNamespace(plan_len=max(LENS), n_real_seq=len(LENS), seq_slot=torch.arange(len(LENS), dtype=torch.int32, device="cuda"),
-                            seq_len=torch.tensor(LENS, dtype=torch.int32, device="cuda"))
+    q = torch.randn((len(lens), nh * hd + 3), generator=g, device="cuda").to(dtype)[:, 3:].view(len(lens), nh, hd)
+    batch = SimpleNamespace(plan_len=max(lens), n_real_seq=len(lens), seq_slot=torch.arange(len(lens), dtype=torch.int32, device="cuda"),
+                            seq_len=torch.tensor(lens, dtype=torch.int32, device="cuda"))
     monkeypatch.setattr(attention, "decode_plan", lambda *a: (splits, 0))
-    out = torch.full((len(LENS), nh, hd), float("nan"), dtype=dtype, device="cuda")
+    out = torch.full((len(lens), nh, hd), float("nan"), dtype=dtype, device="cuda")
     scale = 1 / math.sqrt(hd)
     attention.decode(q, mem, out, scale, window, batch)
     want = exact(q, rows, scale, window)
@@ -81,3 +81,11 @@ def test_bfloat16(monkeypatch, nh, nkv, hd, window, splits):
 @pytest.mark.parametrize("hd", [32, 68, 160])
 def test_pages_off_the_boundary(monkeypatch, dtype, hd):
     run(monkeypatch, dtype, 4, 2, hd, 0, 3, offset=1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("splits", [8, 9, 16])
+@pytest.mark.parametrize("nh,nkv,hd", [(6, 1, 32), (5, 1, 96), (2, 2, 256)])
+def test_clusters(monkeypatch, dtype, nh, nkv, hd, splits):
+    """Two sequences, whose clusters find room (more of them meet through scratch memory): splits with and without keys."""
+    run(monkeypatch, dtype, nh, nkv, hd, 0, splits, lens=[1300, 70])

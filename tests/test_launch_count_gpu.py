@@ -1,5 +1,5 @@
-"""The count of launches against the kernels of a captured graph, where it depends on the shape: the float32 product's pieces and
-the short convolution's two forms."""
+"""The count of launches against the kernels of a captured graph, where it depends on the shape: the float32 product's pieces, the
+short convolution's two forms, the CUDA-core decode attention's ways of merging its splits."""
 from __future__ import annotations
 
 from types import SimpleNamespace
@@ -46,3 +46,18 @@ def test_short_conv(taps, n, pad):
                             n_seq=1, max_new=n)
     kernels = 2 if taps > 1 and n > (16 if taps <= 4 and pad == 4 else 64) else 1
     assert counted_and_captured(lambda: KR.short_conv(x, w, state, 0, batch)) == (kernels, kernels)
+
+
+@pytest.mark.parametrize("n_seq,length,kernels", [(1, 300, 1), (1, 2000, 1), (4, 2000, 2), (64, 300, 1), (3, 7000, 2)])
+def test_decode_attention_clusters_only_where_all_find_room(n_seq, length, kernels):
+    """24 heads of 128 over 4 in float32: one sequence's four clusters find room, four sequences' sixteen of eight blocks do not (as
+    clusters they took 27.9 us, through scratch memory 17.2); one split, and more than sixteen."""
+    from toyinfer_b200.kernels import attention
+    pages = -(-length // 64)
+    k = torch.randn(n_seq * pages, 4, 64, 128, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    mem = SimpleNamespace(k_pages=k, v_pages=k, page_table=torch.arange(n_seq * pages, **i32).view(n_seq, pages), page_size=64, ring_rows=0, n_kv_heads=4)
+    batch = SimpleNamespace(plan_len=length, n_real_seq=n_seq, seq_slot=torch.arange(n_seq, **i32), seq_len=torch.full((n_seq,), length, **i32))
+    q = torch.randn(n_seq, 24, 128, device="cuda")
+    out = torch.empty_like(q)
+    assert counted_and_captured(lambda: attention.decode(q, mem, out, 0.1, 0, batch)) == (kernels, kernels)

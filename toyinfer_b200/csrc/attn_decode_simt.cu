@@ -21,8 +21,8 @@
 // Measured, a layer's step in us against the form that staged tiles in shared memory (one thread a score): 4 sequences of up to
 // 589 positions, 32 heads of 128 over 8, 114 -> 52 (the attention 70 -> 12); 16 of up to 2,000, 40 over 8, 437 -> 185 (307 -> 57,
 // 4.6 TB/s); one of 2,000, 24 over 4, 123 -> 42; heads of 32 at some twenty positions 12 -> 4 and no merging kernel.
-// Up to CLUSTER_SPLITS splits are launched as one cluster and merge through distributed shared memory; more go through
-// global scratch and `attn_decode_combine_kernel`.  With one split the result is written directly.
+// Up to CLUSTER_SPLITS splits are launched as one cluster and merge through distributed shared memory where all clusters find room
+// (launch_form); else they go through global scratch and `attn_decode_combine_kernel`.  With one split the result is written directly.
 #include "attn_decode.cuh"
 
 #include <cooperative_groups.h>
@@ -239,14 +239,52 @@ attn_decode_kernel(DecodeArgs a, int chunks, int in_cluster) {
     cluster.sync();        // nobody leaves while its shared memory may still be read
 }
 
+// How many clusters of n_splits blocks the device holds at once, asked once for each.
 template <typename T, int LPK, int NV, int G, bool VEC>
-int launch_form(const DecodeArgs& a, int n_seq, cudaStream_t stream) {
+int cluster_room(int n_splits, size_t smem, int* room) {
+    static int known[64][CLUSTER_SPLITS + 1] = {};       // room + 1
+    int dev = 0;
+    TI_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && known[dev][n_splits] > 0) { *room = known[dev][n_splits] - 1; return 0; }
+    auto* kernel = attn_decode_kernel<T, LPK, NV, G, VEC>;
+    if (n_splits > 8) TI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, n_splits);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = (unsigned)n_splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    TI_CUDA(cudaOccupancyMaxActiveClusters(room, kernel, &cfg));
+    if (dev >= 0 && dev < 64) known[dev][n_splits] = *room + 1;
+    return 0;
+}
+
+// kernels != null: nothing is launched, only the number of kernels that would be is left there.
+//
+// Clusters are placed whole, inside one part of the chip; those that find no room with the others wait for a whole one to end.  So
+// they are taken only where all of them fit at once with some to spare (as the tensor-core kernel's plan asks, kernels/attention.py), else
+// the splits meet through scratch memory.  us, as clusters / through scratch: 24 query heads of 128 over 4, four sequences of 2,000
+// positions (16 clusters of 8) 27.9 / 17.2; 32 over 8, three of 7,000 (24 of 12) 57 / 38; 64 of 32 over 8, one of 2,000 (16 of 8) 13.7 /
+// 8.1; where they fit: 32 of 128 over 8, one of 300 10.7 / 11.5, 16 of 32 over one, one of 300 5.7 / 7.1.
+template <typename T, int LPK, int NV, int G, bool VEC>
+int launch_form(const DecodeArgs& a, int n_seq, cudaStream_t stream, int* kernels) {
     const int g = a.n_heads / a.n_kv_heads, hd = a.hd, chunks = (g + G - 1) / G;
     const size_t smem = (size_t)WARPS * G * hd * sizeof(float);
     TI_REQUIRE((long long)a.n_kv_heads * chunks <= 65535, "attention_decode: %d kv heads with %d query heads each", a.n_kv_heads, g);
     if (smem > 48 * 1024)
         TI_CUDA(cudaFuncSetAttribute(attn_decode_kernel<T, LPK, NV, G, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int in_cluster = a.n_splits > 1 && a.n_splits <= CLUSTER_SPLITS;
+    int in_cluster = 0;
+    if (a.n_splits > 1 && a.n_splits <= CLUSTER_SPLITS) {
+        int room = 0;
+        if (int rc = cluster_room<T, LPK, NV, G, VEC>(a.n_splits, smem, &room)) return rc;
+        in_cluster = (long long)n_seq * a.n_kv_heads * chunks * 27 <= room * 25LL;
+    }
+    if (kernels) { *kernels = a.n_splits > 1 && !in_cluster ? 2 : 1; return 0; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_seq, a.n_kv_heads * chunks, a.n_splits);
     cfg.blockDim = dim3(THREADS);
@@ -281,29 +319,29 @@ int launch_form(const DecodeArgs& a, int n_seq, cudaStream_t stream) {
 // Query heads a block takes: all that share a kv head up to six (more registers leave one block on an SM), chunks of four
 // beyond; wide heads, whose elements already fill the registers, one or two.
 template <typename T, int LPK, bool VEC>
-int launch_narrow(const DecodeArgs& a, int n_seq, cudaStream_t stream) {
+int launch_narrow(const DecodeArgs& a, int n_seq, cudaStream_t stream, int* kernels) {
     const int g = a.n_heads / a.n_kv_heads;
-    if (!VEC || g == 1) return launch_form<T, LPK, 1, 1, VEC>(a, n_seq, stream);
-    if (g == 2) return launch_form<T, LPK, 1, 2, true>(a, n_seq, stream);
-    if (g == 5 || g == 6) return launch_form<T, LPK, 1, 6, true>(a, n_seq, stream);
-    return launch_form<T, LPK, 1, 4, true>(a, n_seq, stream);
+    if (!VEC || g == 1) return launch_form<T, LPK, 1, 1, VEC>(a, n_seq, stream, kernels);
+    if (g == 2) return launch_form<T, LPK, 1, 2, true>(a, n_seq, stream, kernels);
+    if (g == 5 || g == 6) return launch_form<T, LPK, 1, 6, true>(a, n_seq, stream, kernels);
+    return launch_form<T, LPK, 1, 4, true>(a, n_seq, stream, kernels);
 }
 
 template <typename T, bool VEC>
-int launch_width(const DecodeArgs& a, int n_seq, cudaStream_t stream) {
+int launch_width(const DecodeArgs& a, int n_seq, cudaStream_t stream, int* kernels) {
     const int hd = a.hd;
-    if (hd <= 32) return launch_narrow<T, 8, VEC>(a, n_seq, stream);
-    if (hd <= 64) return launch_narrow<T, 16, VEC>(a, n_seq, stream);
-    if (hd <= 128) return launch_narrow<T, 32, VEC>(a, n_seq, stream);
-    if (hd <= 256) return VEC && a.n_heads / a.n_kv_heads > 1 ? launch_form<T, 32, 2, 2, true>(a, n_seq, stream) : launch_form<T, 32, 2, 1, VEC>(a, n_seq, stream);
-    return launch_form<T, 32, 4, 1, VEC>(a, n_seq, stream);
+    if (hd <= 32) return launch_narrow<T, 8, VEC>(a, n_seq, stream, kernels);
+    if (hd <= 64) return launch_narrow<T, 16, VEC>(a, n_seq, stream, kernels);
+    if (hd <= 128) return launch_narrow<T, 32, VEC>(a, n_seq, stream, kernels);
+    if (hd <= 256) return VEC && a.n_heads / a.n_kv_heads > 1 ? launch_form<T, 32, 2, 2, true>(a, n_seq, stream, kernels) : launch_form<T, 32, 2, 1, VEC>(a, n_seq, stream, kernels);
+    return launch_form<T, 32, 4, 1, VEC>(a, n_seq, stream, kernels);
 }
 
 template <typename T>
-int launch(const DecodeArgs& a, int n_seq, cudaStream_t stream) {
+int launch(const DecodeArgs& a, int n_seq, cudaStream_t stream, int* kernels) {
     const uintptr_t mask = 4 * sizeof(T) - 1;
     const bool vec = a.hd % 4 == 0 && ((uintptr_t)a.k_pages & mask) == 0 && ((uintptr_t)a.v_pages & mask) == 0;
-    return vec ? launch_width<T, true>(a, n_seq, stream) : launch_width<T, false>(a, n_seq, stream);
+    return vec ? launch_width<T, true>(a, n_seq, stream, kernels) : launch_width<T, false>(a, n_seq, stream, kernels);
 }
 }  // namespace
 
@@ -336,7 +374,17 @@ extern "C" int ti_attn_decode_simt(const void* q, long long q_stride, const void
     a.seq_slot = seq_slot; a.seq_len = seq_len; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.hd = head_dim;
     a.window = window; a.n_splits = n_splits; a.scale = scale; a.out = out; a.o_stride = o_stride;
     a.part_o = part_o; a.part_ml = part_ml;
-    return ti_dispatch_dtype(dtype, [&](auto t) -> int { return launch<decltype(t)>(a, n_seq, stream); });
+    return ti_dispatch_dtype(dtype, [&](auto t) -> int { return launch<decltype(t)>(a, n_seq, stream, nullptr); });
+}
+
+// The kernels that ti_attn_decode_simt launches for these sizes (its pages at these addresses).
+extern "C" int ti_attn_decode_simt_kernels(const void* k_pages, const void* v_pages, int n_seq, int n_heads, int n_kv_heads, int head_dim,
+                                           int n_splits, int dtype, int* kernels) {
+    TI_REQUIRE(n_seq > 0 && n_heads > 0 && n_kv_heads > 0 && n_heads % n_kv_heads == 0 && head_dim > 0 && head_dim <= 512 && n_splits >= 1 && kernels,
+               "attention_decode: bad sizes");
+    DecodeArgs a = {};
+    a.k_pages = k_pages; a.v_pages = v_pages; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.hd = head_dim; a.n_splits = n_splits;
+    return ti_dispatch_dtype(dtype, [&](auto t) -> int { return launch<decltype(t)>(a, n_seq, nullptr, kernels); });
 }
 
 // ---------------------------------------------------------------------------

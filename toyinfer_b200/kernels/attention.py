@@ -52,7 +52,7 @@ def prefill(q, k, v, out, scale, window, batch) -> None:
           _code(q, "attention_prefill"), _stream())
 
 
-MAX_CLUSTER = 16     # splits that the decode kernels merge themselves, as one thread-block cluster
+MAX_CLUSTER = 16     # splits that the decode kernels merge themselves, as one thread-block cluster, where there is room for all
 
 
 def chunk(q, k, v, mem, out, scale, window, batch) -> None:
@@ -158,6 +158,21 @@ def decode_plan(n_seq: int, n_heads: int, n_kv_heads: int, hd: int, max_len: int
     return splits, scratch_mode
 
 
+_simt_known: dict = {}
+
+
+def _simt_kernels(q, mem, splits: int) -> int:
+    """Kernels of the CUDA-core decode attention: one where the splits meet in clusters, which the library asks the device."""
+    (B, nh, hd), k, v = q.shape, mem.k_pages.data_ptr(), mem.v_pages.data_ptr()
+    key = (q.device, B, nh, mem.n_kv_heads, hd, splits, q.dtype, k % 16, v % 16)
+    if key not in _simt_known:
+        n = ctypes.c_int(0)
+        _call(library().ti_attn_decode_simt_kernels, _ptr(mem.k_pages), _ptr(mem.v_pages), B, nh, mem.n_kv_heads, hd, splits,
+              _code(q, "attention_decode"), ctypes.byref(n), launches=0)
+        _simt_known[key] = n.value
+    return _simt_known[key]
+
+
 def decode(q, mem, out, scale, window, batch) -> None:
     B, nh, hd = q.shape
     nkv = mem.n_kv_heads
@@ -173,11 +188,15 @@ def decode(q, mem, out, scale, window, batch) -> None:
     batch.drained_after_attention = tensor_cores and splits > 1 and mode == 1
     fn = lib.ti_attn_decode_mma if tensor_cores else lib.ti_attn_decode_simt
     extra = (mode,) if tensor_cores else ()
+    if tensor_cores:
+        launches = 2 if splits > 1 and mode != 2 else 1
+    else:
+        launches = _simt_kernels(q, mem, splits) if 1 < splits <= MAX_CLUSTER else 1 + (splits > 1)
     _call(fn, _ptr(q), _row_stride(q, "q"), _ptr(mem.k_pages), _ptr(mem.v_pages),
           _ptr(pt), pt.shape[1], mem.page_size, mem.ring_rows, mem.k_pages.shape[0],
           _ptr(batch.seq_slot), _ptr(batch.seq_len), B, nh, nkv, hd, scale, window, splits,
           _ptr(out), out.stride(0), _ptr(part_o), _ptr(part_ml), _code(q, "attention_decode"), *extra, _stream(),
-          launches=2 if splits > (1 if tensor_cores else MAX_CLUSTER) and mode != 2 else 1)
+          launches=launches)
 
 
 def decode_fused_eligible(q, k, v, q_w, k_w, tables, mem) -> bool:
