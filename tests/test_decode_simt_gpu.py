@@ -83,6 +83,13 @@ def test_pages_off_the_boundary(monkeypatch, dtype, hd):
     run(monkeypatch, dtype, 4, 2, hd, 0, 3, offset=1)
 
 
+@pytest.mark.parametrize("dtype,offset", [(torch.float32, 0), (torch.float32, 1), (torch.bfloat16, 0), (torch.bfloat16, 1)])
+@pytest.mark.parametrize("nh,nkv,hd,splits", [(4, 2, 260, 1), (3, 1, 384, 7), (2, 2, 448, 17), (2, 1, 401, 2)])
+def test_heads_of_four_runs(monkeypatch, dtype, offset, nh, nkv, hd, splits):
+    """Wider than any layer's (kernels/attention.py stops at 256): the C entry's own range."""
+    run(monkeypatch, dtype, nh, nkv, hd, 0, splits, offset=offset)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("splits", [8, 9, 16])
 @pytest.mark.parametrize("nh,nkv,hd", [(6, 1, 32), (5, 1, 96), (2, 2, 256)])

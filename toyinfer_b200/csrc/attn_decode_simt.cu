@@ -108,6 +108,15 @@ attn_decode_kernel(DecodeArgs a, int chunks, int in_cluster) {
         if (page < 0 || page >= a.n_pages) page = 0;
         const size_t first = (((size_t)page * a.n_kv_heads + kvh) * TILE + row0 % TILE) * hd;
         float kx[KEYS][NV][4], vx[KEYS][NV][4];
+        auto values = [&]() {
+#pragma unroll
+            for (int k = 0; k < KEYS; k++) {
+                const int r = k * GROUPS + grp, p = p0 + r;
+                const int n = p >= lo && p < L ? hd : 0;
+#pragma unroll
+                for (int i = 0; i < NV; i++) load4<VEC>(vx[k][i], (const T*)a.v_pages + first + (size_t)r * hd, i * LPK + sub, n);
+            }
+        };
 #pragma unroll
         for (int k = 0; k < KEYS; k++) {
             const int r = k * GROUPS + grp, p = p0 + r;
@@ -115,13 +124,7 @@ attn_decode_kernel(DecodeArgs a, int chunks, int in_cluster) {
 #pragma unroll
             for (int i = 0; i < NV; i++) load4<VEC>(kx[k][i], (const T*)a.k_pages + first + (size_t)r * hd, i * LPK + sub, n);
         }
-#pragma unroll
-        for (int k = 0; k < KEYS; k++) {
-            const int r = k * GROUPS + grp, p = p0 + r;
-            const int n = p >= lo && p < L ? hd : 0;
-#pragma unroll
-            for (int i = 0; i < NV; i++) load4<VEC>(vx[k][i], (const T*)a.v_pages + first + (size_t)r * hd, i * LPK + sub, n);
-        }
+        if constexpr (NV < 4) values();                                  // (four runs: no registers for both; one head, scored first)
         // the key whose scores this lane ends up with, of its group's eight
         const int mine = sub / (LPK / 8), p_mine = p0 + mine * GROUPS + grp;
         const bool live = p_mine >= lo && p_mine < L;
@@ -146,6 +149,7 @@ attn_decode_kernel(DecodeArgs a, int chunks, int in_cluster) {
                     s[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                 }
             }
+            if constexpr (NV >= 4) values();
             float x = s[0];
 #pragma unroll
             for (int o = LPK / 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -276,8 +280,7 @@ int launch_form(const DecodeArgs& a, int n_seq, cudaStream_t stream, int* kernel
     const int g = a.n_heads / a.n_kv_heads, hd = a.hd, chunks = (g + G - 1) / G;
     const size_t smem = (size_t)WARPS * G * hd * sizeof(float);
     TI_REQUIRE((long long)a.n_kv_heads * chunks <= 65535, "attention_decode: %d kv heads with %d query heads each", a.n_kv_heads, g);
-    if (smem > 48 * 1024)
-        TI_CUDA(cudaFuncSetAttribute(attn_decode_kernel<T, LPK, NV, G, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static_assert(WARPS * G * LPK * NV * 4 * sizeof(float) <= 48 * 1024, "the warps' sums fit without a setting of the kernel's");
     int in_cluster = 0;
     if (a.n_splits > 1 && a.n_splits <= CLUSTER_SPLITS) {
         int room = 0;
@@ -362,8 +365,8 @@ extern "C" int ti_attn_decode_simt(const void* q, long long q_stride, const void
     TI_REQUIRE((n_heads / n_kv_heads) * head_dim <= MAX_OUTPUTS,
                "attention_decode: %d query heads per kv head of size %d exceed this kernel's %d outputs per kv head",
                n_heads / n_kv_heads, head_dim, MAX_OUTPUTS);
-    // (the host refuses the same sizes before a model is built, kernels/attention.py: a page of keys and values beside the
-    // group's queries and weights in 227 KB)
+    // (kernels/attention.py refuses the same sizes before a model is built.  They are what a form of this kernel with a page of keys
+    // and values in shared memory could hold; this one could take more, and no caller has more: heads of up to 449 elements pass)
     TI_REQUIRE(((long long)(n_heads / n_kv_heads) * (head_dim + TILE + 3) + TILE * (2LL * head_dim + 1)) * 4 <= 227 * 1024,
                "attention_decode: %d query heads per kv head of size %d are too many", n_heads / n_kv_heads, head_dim);
     TI_REQUIRE(n_splits >= 1 && n_splits <= 65535 && n_kv_heads <= 65535, "attention_decode: bad split count %d", n_splits);
