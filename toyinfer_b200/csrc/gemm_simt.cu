@@ -116,7 +116,7 @@ constexpr long long ROWS_LARGE = 1 << 19;      // weights from which several tok
 // 4.7, 5.4, 6.7; 2,560 x 9,728 40, 80, 117 / 17, 27, 41; 19,456 x 2,560 41, 56, 83 / 32, 43, 68 (the read of the weights alone takes 30);
 // 384 x 96 2.1, 2.4, 2.8 / 1.4, 1.5, 1.8.
 template <typename T, typename OT, int V, int R, int MR, int KS, bool PAIR>
-__global__ void __launch_bounds__(GV_THREADS, R == 4 ? (MR >= 4 ? 2 : 3) : 4)
+__global__ void __launch_bounds__(GV_THREADS, R == 4 ? (MR >= 4 ? 2 : 3) : MR == 8 ? 2 : MR == 4 ? 3 : 4)
 gemv_rows_kernel(const T* __restrict__ X, const T* __restrict__ W, OT* __restrict__ out,
                  int M, int N, int K, long long ldx, long long ldw, long long ldo, int kind, float limit) {
     ti_pdl_trigger();
@@ -198,7 +198,7 @@ int launch_rows(const void* x, const void* w, void* out, int M, int N, int K, lo
                 cudaStream_t stream) {
     const int groups = GV_WARPS / KS * R;           // weight rows of a block
     long long blocks = ((long long)N + groups - 1) / groups;
-    if (KS == 1 && blocks > 148 * 8) blocks = 148 * 8;
+    if (KS == 1) blocks = blocks < 8LL * ti_sm_count() ? blocks : 8LL * ti_sm_count();
     const dim3 grid((unsigned)blocks, (M + MR - 1) / MR);
     TI_CUDA(ti_launch(gemv_rows_kernel<T, OT, V, R, MR, KS, PAIR>, grid, dim3(GV_THREADS), 0, stream, (const T*)x, (const T*)w, (OT*)out, M, N, K, ldx, ldw, ldo,
                       kind, limit));
@@ -216,7 +216,7 @@ int launch_rows_sliced(const void* x, const void* w, void* out, int M, int N, in
                        cudaStream_t stream) {
     const int groups = (N + 3) / 4, steps = (K + 32 * V - 1) / (32 * V);      // groups of four rows, turns of a warp over K
     int ks = 1;
-    while (ks < 8 && groups * ks < 148 * 16 && steps >= ks * 4) ks *= 2;
+    while (ks < 8 && groups * ks < 16 * ti_sm_count() && steps >= ks * 4) ks *= 2;
     switch (ks) {
         case 1: return launch_rows<T, OT, V, 4, MR, 1, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
         case 2: return launch_rows<T, OT, V, 4, MR, 2, PAIR>(x, w, out, M, N, K, ldx, ldw, ldo, kind, limit, stream);
