@@ -9,9 +9,13 @@
 // What bounds it: the operands' way into an SM (115 B/ns: 0.28 us a step of 32 KB), and with one block an SM the start and the end of
 // every tile, in which nothing is on its way.  Two blocks of three stages each share an SM instead of one of six where there are tiles
 // for it, and the activation of a gated pair is applied at the end (a tile of 64 gate and 64 up columns; a kernel of its own read and
-// wrote the pairs again).  The whole layer, bfloat16, hidden 2,048, two choices a token, us before / with the activation inside
-// / two blocks an SM too: 16 experts of 1,024, 3,000 tokens 176 / 168 / 149, 777 tokens with a shared expert 111 / 106 / 102.  Where the tiles fit one
-// round, two blocks lose: 8 experts of 1,000 with 600 tokens 39.7 / 36.5 / 39.6, 4 of 600 with 150 tokens 28.9 / 26.8 / 28.9.
+// wrote the pairs again).  The whole layer, hidden 2,048, two choices a token, us before / with the activation inside
+// / two blocks an SM too: 16 experts of 1,024, 3,000 tokens 176 / 168 / 149, 777 tokens with a shared expert 111 / 106 / 102.
+// The gather and both products, one block an SM / two, at the tiles of the first and the second product that the rule counts: 8 experts
+// of 1,000, 600 tokens with two choices (224, 224) 54.1 / 48.3; 16 of 640, 1,100 with one (170, 272) 52.0 / 45.5; 8 of 768, 512 with two
+// (144, 192) 43.0 / 37.6; contractions of a few steps gain nothing, 16 of 512, hidden 1,024 (168, 168) 27.7 / 29.0, 8 of 1,280, hidden
+// 1,024, one choice (240, 96) 30.0 / 30.5.  Where the tiles fit one round, two blocks lose: 8 of 1,000, 600 with one choice (144, 144)
+// 35.1 / 44.3, 4 of 600, 150 with two (50, 80) 24.4 / 31.5.
 #include "gemm_tcgen05.cuh"
 
 namespace tigemm {
@@ -108,8 +112,10 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_c
                     tmem_ld16(taddr + GBN / 2 + c, u);
 #pragma unroll
                     for (int e = 0; e < 16; e++) {
-                        const float gate = fminf(to_f32(from_f32<bf16>(r[e])), act.limit);
-                        const float up = fminf(fmaxf(to_f32(from_f32<bf16>(u[e])), -act.limit), act.limit);
+                        const __nv_bfloat162 gu = __floats2bfloat162_rn(r[e], u[e]);        // (both in one conversion)
+                        const uint32_t both = *reinterpret_cast<const uint32_t*>(&gu);
+                        const float gate = fminf(__uint_as_float(both << 16), act.limit);
+                        const float up = fminf(fmaxf(__uint_as_float(both & 0xffff0000u), -act.limit), act.limit);
                         r[e] = gate * (ti_over(1.0f, 1.0f + expf(-act.alpha * gate))) * (up + act.shift);
                     }
                 }
@@ -167,7 +173,7 @@ extern "C" int ti_linear_grouped_tc(const void* a, const void* W, void* out, con
     const PairAct pa{limit, alpha, shift};
     // Two blocks an SM where the tiles are more than one round of SMs (the groups' padding leaves half a tile each empty on average; how
     // many tiles hold rows is known on the device only); else one, with all its memory for the stages.
-    const bool two = ((long long)grid.x - groups / 2) * grid.y > 148;
+    const bool two = ((long long)grid.x - groups / 2) * grid.y > ti_sm_count();
     if (pair) return two ? launch_grouped<3, true>(grid, am, bm, g, tile_group, per_group, pa, status, stream)
                          : launch_grouped<6, true>(grid, am, bm, g, tile_group, per_group, pa, status, stream);
     return two ? launch_grouped<3, false>(grid, am, bm, g, tile_group, per_group, pa, status, stream)
