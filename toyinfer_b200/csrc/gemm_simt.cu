@@ -114,7 +114,8 @@ constexpr long long ROWS_LARGE = 1 << 19;      // weights from which several tok
 // PAIR: rows come in (gate, up) pairs, out is ti_gate_pair of them, [M, N / 2].
 // us, one row a warp without slices / so, at 1, 4 and 8 tokens: 512 x 4,096 11.3, 18.3, 26 / 3.6, 4.3, 5.3; 2,048 x 2,048 8.1, 11.6, 15.6 /
 // 4.7, 5.4, 6.7; 2,560 x 9,728 40, 80, 117 / 17, 27, 41; 19,456 x 2,560 41, 56, 83 / 32, 43, 68 (the read of the weights alone takes 30);
-// 384 x 96 2.1, 2.4, 2.8 / 1.4, 1.5, 1.8.
+// 384 x 96 2.4, 2.7, 3.0 / 1.6, 1.8, 1.8; 1,024 x 400 at 8 tokens 5.1 / 3.0, gated 6.3 / 3.2.  Rows off the 16-byte boundary, elements one by
+// one, at 1, 5 and 16 tokens: float32 2,048 x 2,045 17.4, 18.8, 22.7 / 3.2, 7.8, 13.9; bfloat16 9,728 x 2,559 50, 53, 108 / 21, 49, 74.
 template <typename T, typename OT, int V, int R, int MR, int KS, bool PAIR>
 __global__ void __launch_bounds__(GV_THREADS, R == 4 ? (MR >= 4 ? 2 : 3) : MR == 8 ? 2 : MR == 4 ? 3 : 4)
 gemv_rows_kernel(const T* __restrict__ X, const T* __restrict__ W, OT* __restrict__ out,
