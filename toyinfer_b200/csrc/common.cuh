@@ -169,24 +169,28 @@ __device__ __forceinline__ float ti_over(float z, float d) {
 }
 
 // The activation of a gated product's gate.  kind 1: silu, z / (1 + exp(-z)); kind 2: the tanh form of gelu,
-// 0.5 z (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))).
+// 0.5 z (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))).  FLAT: without a branch (ti_over), else by the compiler's division, whose slow
+// path stands apart: for kernels whose ungated form pays for the longer code.
+template <bool FLAT = true>
 __device__ __forceinline__ float ti_gate_act(float z, int kind) {
     if (kind == 2) {
         const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
         return 0.5f * z * (1.0f + tanhf(u));
     }
-    return ti_over(z, 1.0f + expf(-z));
+    return FLAT ? ti_over(z, 1.0f + expf(-z)) : z / (1.0f + expf(-z));
 }
 
 // What a gated product stores for its (gate, up) pair.  kind 1 and 2: up * act(gate) as above; kind 3: a clamped gate
 // under a sharpened sigmoid, times the clamped up value plus one: g' = min(gate, limit), u' = clamp(up, -limit, limit),
 // g' sigmoid(1.702 g') (u' + 1).
+template <bool FLAT = true>
 __device__ __forceinline__ float ti_gate_pair(float gate, float up, int kind, float limit) {
     if (kind == 3) {
         const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-        return ti_over(g, 1.0f + expf(-1.702f * g)) * (u + 1.0f);
+        const float d = 1.0f + expf(-1.702f * g);
+        return (FLAT ? ti_over(g, d) : g / d) * (u + 1.0f);
     }
-    return up * ti_gate_act(gate, kind);
+    return up * ti_gate_act<FLAT>(gate, kind);
 }
 
 // Activations without a gate, applied value by value.  kind 4: the squared ReLU; kind 5: gelu by the error function,
