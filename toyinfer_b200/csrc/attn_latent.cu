@@ -340,7 +340,7 @@ int launch_absorb_rows(const void* d, long long d_stride, const void* q, long lo
                        cudaStream_t stream) {
     const int chunks = (rank + AR_COLS - 1) / AR_COLS;
     const size_t smem = std::max(row, absorb_rows_smem<TOK>(plain));
-    if (smem > 48 * 1024) TI_CUDA(cudaFuncSetAttribute(latent_absorb_rows_kernel<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (below 48 KB: the entry takes heads of up to 512 elements here and refuses longer rows)
     TI_CUDA(ti_launch_class<2>(latent_absorb_rows_kernel<TOK>, dim3(n_heads * chunks + std::min(M, TOK), (M + TOK - 1) / TOK), dim3(AR_THREADS), smem, stream,
                                (const bf16*)d, d_stride, (const bf16*)q, q_stride, n_heads, plain, rank, rot, norm_w, eps, cos_t, sin_t, max_pos,
                                tok_pos, tok_seq, seq_slot, (bf16*)lat, kv, (const bf16*)uk, qa, M, chunks));
