@@ -47,7 +47,7 @@ def test_limits():
             for K in (8, 640, 1032, 8192):
                 for pair in (False, True):
                     got = [tiles(E, p, N, K, pair) for p in range(1, 30)]
-                    assert got[:2] == [1, 1] and got[2:8] == [2] * 6 and set(got[8:18]) <= {0, 2} and set(got[18:24]) <= {0, 4}
+                    assert got[:4] == [1] * 4 and got[4:8] == [2] * 4 and set(got[8:18]) <= {0, 2} and set(got[18:24]) <= {0, 4}
                     assert got[24:] == [0] * 5
                     assert not any(a == 0 and b > 0 for a, b in zip(got, got[1:]))       # once in tiles, always in tiles
 

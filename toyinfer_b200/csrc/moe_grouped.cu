@@ -188,9 +188,11 @@ constexpr int ROWS_SMALL_PLACES = 12;
 // chain, 1.65 us a step of 64 (1.3 the shorter chains of a pair).  Weights and steps both grow with K, which cancels.
 // us a product, registers / tiles, at 9, 16 and 24 places: 8 experts, 2,048 x 1,280 pairs 22, 28, 37 / 53; 16 experts 39, 53, 66 / 58;
 // 32 experts 72, 96, 129 / 92; 64 experts 147, 204, 268 / 149; 64 experts of 1,024 x 256 23, 30, 40 / 31.
+// Eight places a warp up to four an expert, us at 1, 2, 4, 6 and 8 places with eight a warp / sixteen: 16 experts, 2,048 x 1,024 pairs 18.7,
+// 22.6, 24.6, 29.8, 31.5 / 20.7, 24.9, 27.6, 30.3, 30.9; 64 experts 59, 78, 93, 109, 127 / 64, 85, 100, 108, 114.
 constexpr int SKINNY_MAX_PLACES = 24;
 int skinny_tiles(int n_experts, int P, int N, int K, bool pair, int sms) {
-    if (P <= 2 * n_experts) return 1;
+    if (P <= 4 * n_experts) return 1;
     if (P <= 8 * n_experts) return 2;
     const long long tiles = P / 16 + n_experts / 2;
     if (P > SKINNY_MAX_PLACES * n_experts || tiles * N * (pair ? 2 : 1) > (long long)sms * (pair && K <= 1024 ? 340 : 432)) return 0;
